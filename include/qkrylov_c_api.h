@@ -298,7 +298,14 @@ int qkrylov_set_projection_kernel(int method);
  * qkrylov_debug_device_wait_probe: one kernel waits on an mbarrier that nothing
  * completes, for limit_ns of GPU global time (clamped to 1 us .. 1 s), and
  * counts the give-up as qkrylov_device_wait_timeouts does; no copy is in
- * flight, the GPU stays usable. */
+ * flight, the GPU stays usable.
+ * qkrylov_debug_packed_apply_host: y = the off-diagonal part of H x (reference
+ * order, interleaved complex) from the packed SpMV's tables, walked on the host
+ * with every index checked; *form receives the amplitude form (0 uniform, 1
+ * signed, 2 coded; + 4 where all magnitudes are equal, + 8 where amplitudes are
+ * complex) or -1, with y untouched, where the packed kernel does not apply. */
+int qkrylov_debug_packed_apply_host(qkrylov_basis_h basis, qkrylov_site_h site, qkrylov_opsum_h ops, const double* x,
+                                    double* y, int* form);
 int qkrylov_debug_inject_alloc_failure(int64_t after_n);
 int64_t qkrylov_debug_live_allocations(void);
 int qkrylov_debug_device_wait_probe(int64_t limit_ns);

@@ -123,6 +123,7 @@ _SIGS = {
     "qkrylov_set_projection_kernel": (_i, [_i]),
     "qkrylov_lanczos_ritz_values": (_i, [_vp, _i, _c.c_uint64, _i, _i, _dp, _ip, _ip]),
     "qkrylov_debug_live_allocations": (_c.c_int64, []),
+    "qkrylov_debug_packed_apply_host": (_i, [_vp, _vp, _vp, _dp, _dp, _ip]),
     "qkrylov_debug_device_wait_probe": (_i, [_c.c_int64]),
     "qkrylov_vector_dot_device_f64": (_i, [_vp, _vp, _u64, _dp, _vp]),
     "qkrylov_vector_dot_device_f32": (_i, [_vp, _vp, _u64, _dp, _vp]),
@@ -472,9 +473,10 @@ class MatrixFreeHamiltonian(_Handle):
     def tuning(self, fp32=True):
         """(variant, {variant: autotuned ms}) of the fast kernel used in mode 0;
         variant names: "row", "staged", "rows4", "rows4_staged", "rows4_wide",
-        "tile1", "tile2", "tile4", "class" ("generic" when it does not apply)."""
+        "tile1", "tile2", "tile4", "class", and "packed", which is taken untimed
+        wherever it applies ("generic" when none does)."""
         v = _c.c_int()
-        names = ["row", "staged", "rows4", "rows4_staged", "rows4_wide", "tile1", "tile2", "tile4", "class"]
+        names = ["row", "staged", "rows4", "rows4_staged", "rows4_wide", "tile1", "tile2", "tile4", "class", "packed"]
         ms = (_c.c_double * len(names))()
         _check(lib().qkrylov_hamiltonian_tuning_ex(self._h, int(bool(fp32)), _c.byref(v), ms, len(names)))
         return ("generic" if v.value < 0 else names[v.value]), {names[i]: ms[i] for i in range(len(names))}

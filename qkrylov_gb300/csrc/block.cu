@@ -456,7 +456,8 @@ public:
         oj_ = false;
         for (size_t h = 0; h < hs.size(); ++h) {
             Hamiltonian& H = *hs[h];
-            QKG_REQUIRE(H.fast(), "batched Lanczos needs every Hamiltonian on the fast SpMV kernel");
+            H.ensure_fast();
+            QKG_REQUIRE(H.has_fast_tables() && H.fast(), "batched Lanczos needs every Hamiltonian on the fast SpMV kernel");
             QKG_REQUIRE(H.device() == hs[0]->device(), "batched Lanczos needs every Hamiltonian on one device");
             QKG_CUDA(cudaStreamSynchronize(H.stream()));
             H.fast_params(P[h]);
@@ -551,9 +552,9 @@ public:
         if (tmp.bytes < n * sizeof(double2)) tmp.alloc(n * sizeof(double2));
         QKG_CUDA(cudaMemcpyAsync(tmp.p, host_ref, n * sizeof(double2), cudaMemcpyHostToDevice, s_));
         const double2* src = tmp.as<double2>();
-        if (H.permuted()) {
+        if (H.basis().permuted) {
             if (tmp2.bytes < n * sizeof(double2)) tmp2.alloc(n * sizeof(double2));
-            H.to_internal_f64(tmp.as<double2>(), tmp2.as<double2>(), s_);
+            H.to_basis_f64(tmp.as<double2>(), tmp2.as<double2>(), s_);
             src = tmp2.as<double2>();
         }
         const int g = (int)std::min<uint64_t>((n + 255) / 256, 152ull * 16);

@@ -349,11 +349,16 @@ int qkrylov_hamiltonian_apply_device_f64(qkrylov_hamiltonian_h h, const void* dx
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const auto* x = static_cast<const double2*>(dx);
         auto* y = static_cast<double2*>(dy);
+        const uint64_t n = H.dim();
         if (!H.permuted()) {
+            if (x + n > y && y + n > x) {  // overlapping vectors: from a copy of x
+                ensure(h->x64, n * sizeof(double2));
+                QKG_CUDA(cudaMemcpyAsync(h->x64.p, x, n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+                x = h->x64.as<double2>();
+            }
             H.apply_f64(x, y, s);
             return;
         }
-        const uint64_t n = H.dim();
         ensure(h->x64, n * sizeof(double2));
         ensure(h->y64, n * sizeof(double2));
         H.to_internal_f64(x, h->x64.as<double2>(), s);
@@ -369,11 +374,16 @@ int qkrylov_hamiltonian_apply_device_f32(qkrylov_hamiltonian_h h, const void* dx
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const auto* x = static_cast<const float2*>(dx);
         auto* y = static_cast<float2*>(dy);
+        const uint64_t n = H.dim();
         if (!H.permuted()) {
+            if (x + n > y && y + n > x) {  // overlapping vectors: from a copy of x
+                ensure(h->x32, n * sizeof(float2));
+                QKG_CUDA(cudaMemcpyAsync(h->x32.p, x, n * sizeof(float2), cudaMemcpyDeviceToDevice, s));
+                x = h->x32.as<float2>();
+            }
             H.apply_f32(x, y, s);
             return;
         }
-        const uint64_t n = H.dim();
         ensure(h->x32, n * sizeof(float2));
         ensure(h->y32, n * sizeof(float2));
         H.to_internal_f32(x, h->x32.as<float2>(), s);
@@ -417,9 +427,11 @@ int qkrylov_hamiltonian_info(qkrylov_hamiltonian_h h, int* no, int* ni, int* nm,
 
 int qkrylov_hamiltonian_select_kernel(qkrylov_hamiltonian_h h, int generic, int* fast_in_use) {
     if (!h || !h->ptr || generic < 0 || generic > qkg::Hamiltonian::kMaxMode) return QKRYLOV_ERROR_INVALID_ARG;
-    h->ptr->set_kernel_mode(generic);
-    if (fast_in_use) *fast_in_use = h->ptr->fast() ? 1 : 0;
-    return QKRYLOV_SUCCESS;
+    return guarded([&] {
+        set_device(h);
+        h->ptr->set_kernel_mode(generic);
+        if (fast_in_use) *fast_in_use = h->ptr->fast() ? 1 : 0;
+    });
 }
 
 int qkrylov_hamiltonian_tuning(qkrylov_hamiltonian_h h, int fp32, int* variant, double* ms) {
@@ -701,6 +713,11 @@ int qkrylov_debug_inject_alloc_failure(int64_t after_n) {
     return QKRYLOV_SUCCESS;
 }
 int64_t qkrylov_debug_live_allocations(void) { return qkg::live_device_allocs(); }
+int qkrylov_debug_packed_apply_host(qkrylov_basis_h b, qkrylov_site_h site, qkrylov_opsum_h ops, const double* x,
+                                    double* y, int* form) {
+    if (!b || !b->ptr || !site || !ops || !x || !y || !form) return QKRYLOV_ERROR_INVALID_ARG;
+    return guarded([&] { *form = qkg::packed_apply_host(*b->ptr, site->kind, ops->terms, x, y); });
+}
 int qkrylov_debug_device_wait_probe(int64_t limit_ns) {
     if (limit_ns <= 0) return QKRYLOV_ERROR_INVALID_ARG;
     return guarded([&] { qkg::tilek::wait_probe((long long)limit_ns); });

@@ -78,7 +78,7 @@ uint64_t permute_mask(const Basis& b, uint64_t m) {
 }
 }  // namespace
 
-std::vector<HostTerm> compile_terms(const Basis& b, SiteKind site, const std::vector<Term>& terms) {
+std::vector<HostTerm> compile_terms(const Basis& b, SiteKind site, const std::vector<Term>& terms, bool reference) {
     std::vector<HostTerm> out;
     const uint64_t phantom = (b.nbits >= 64) ? 0 : ~below(b.nbits);  // bits every basis state has at 0
     for (size_t ti = 0; ti < terms.size(); ++ti) {
@@ -145,6 +145,13 @@ std::vector<HostTerm> compile_terms(const Basis& b, SiteKind site, const std::ve
             if (b.no_double) h.check = true;
         }
         if (dead || b.dim == 0) continue;
+        if (reference) {
+            h.C = C; h.V = V; h.X = X; h.J = J;
+            for (size_t i = 0; i < keep.size(); ++i) {
+                h.vars[i].sm = keep[i].sm;
+                h.vars[i].pf = keep[i].pf;
+            }
+        }
         out.push_back(std::move(h));
     }
     return out;

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <complex>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -37,7 +38,8 @@ enum DiagMode : int { DIAG_U8 = 0, DIAG_U16 = 1, DIAG_FULL = 2 };
 // kernel (spmv_tile.cu).
 enum FastVariant : int {
     FV_ROW = 0, FV_STAGED = 1, FV_ROWS4 = 2, FV_ROWS4_STAGED = 3, FV_ROWS4_WIDE = 4,
-    FV_TILE1 = 5, FV_TILE2 = 6, FV_TILE4 = 7, FV_CLASS = 8
+    FV_TILE1 = 5, FV_TILE2 = 6, FV_TILE4 = 7, FV_CLASS = 8,
+    FV_PACKED = 9  // the packed kernel (pack.hpp), where it applies: not tuned, always taken
 };
 constexpr int kFastVariants = 9;
 constexpr int kFastVariantsV1 = 5;  // variants reported by qkrylov_hamiltonian_tuning
@@ -74,12 +76,17 @@ struct LanczosHooks {
 namespace fastk {
 template <class A> struct FastParams;
 }
+namespace packk {
+template <class A> struct Params;
+}
 
 // Per-precision copy of the compiled term lists.
 struct TermSet {
     DBuf outer, inner, mixed, diag, all, vars;
     int n_outer = 0, n_inner = 0, n_mixed = 0, n_diag = 0, n_all = 0;
 };
+
+class PackPlan;
 
 class Hamiltonian {
 public:
@@ -91,21 +98,32 @@ public:
     cudaStream_t stream() const { return stream_; }
     int device() const { return dev_; }
     const DevBasis& dbasis() const { return *db_; }
-    bool permuted() const { return basis_->permuted; }
+    // The order of the vectors that apply_* and the solvers work on.  packed():
+    // the reference's (the packed kernel, mode 0); else the basis' internal order,
+    // which permuted() says differs from the reference's.
+    bool packed() const { return pack_ && mode_ == 0; }
+    bool permuted() const { return !packed() && basis_->permuted; }
     bool all_real() const { return all_real_; }
 
-    // y = H x on device vectors in internal order (interleaved complex).
+    // y = H x on device vectors in the order above (interleaved complex; x and
+    // y must not overlap).
     void apply_f64(const double2* x, double2* y, cudaStream_t s) const;
     void apply_f32(const float2* x, float2* y, cudaStream_t s) const;
     // One FP32 SpMV of the device-resident Lanczos step (fast kernel only);
     // writes n_items() partials to lz.apart.
     void apply_lanczos_f32(const LanczosHooks& lz, cudaStream_t s) const;
 
-    // Diagonal H_ii (complex, internal order) into a device buffer.
+    // Seeded Gaussian start vectors: element i of the basis' internal order takes
+    // the generator's block i whatever order the vector is in.
+    void philox_f64(uint64_t seed, uint64_t stream, double2* out, cudaStream_t s) const;
+    void philox_f32(uint64_t seed, uint64_t stream, float2* out, cudaStream_t s) const;
+
+    // Diagonal H_ii (complex, in the vectors' order) into a device buffer.
     void diagonal_f64(double2* d, cudaStream_t s) const;
 
-    // Reference order <-> internal order for device vectors.
+    // Reference order <-> the vectors' order for device vectors.
     void to_internal_f64(const double2* ref, double2* in, cudaStream_t s) const;
+    void to_basis_f64(const double2* ref, double2* in, cudaStream_t s) const;  // the basis' internal order
     void to_reference_f64(const double2* in, double2* ref, cudaStream_t s) const;
     void to_internal_f32(const float2* ref, float2* in, cudaStream_t s) const;
     void to_reference_f32(const float2* in, float2* ref, cudaStream_t s) const;
@@ -125,14 +143,16 @@ public:
     int n_diag() const { return t64_.n_diag; }
     int diag_mode() const { return diag_mode_; }
     size_t n_items() const { return n_items_; }
-    bool fast() const { return fast_ && !force_generic_; }
+    bool fast() const { return (packed() || fast_) && !force_generic_; }
+    void ensure_fast();
+    bool has_fast_tables() const { return fast_; }
     // kernel mode: 0 automatic (autotuned), 1 generic kernel, 2 fast kernel
     // one row per thread, 3 fast kernel with shared-memory staging, 4 fast
     // kernel four rows per thread, 5 four rows per thread with staging, 6 four
     // rows per thread with the larger register budget, 7 / 8 / 9 the tiled
     // kernel over 1 / 2 / 4 outer blocks per CTA, 10 the class-persistent kernel
     static constexpr int kMaxMode = 10;
-    void set_kernel_mode(int m) { mode_ = m; force_generic_ = (m == 1); }
+    void set_kernel_mode(int m);
     void force_generic(bool on) { set_kernel_mode(on ? 1 : 0); }
     // fast-kernel variant for vectors of elem_bytes per element
     // dynamic shared memory of a staged variant: the largest outer block's slice
@@ -167,6 +187,7 @@ public:
         if (mode_ == 4) return FV_ROWS4;
         if (mode_ == 5) return can_stage ? FV_ROWS4_STAGED : FV_ROWS4;
         if (mode_ == 6) return FV_ROWS4_WIDE;
+        if (packed()) return FV_PACKED;
         const FastVariant v = pref_[elem_bytes == 16 ? 1 : 0];
         if (tile_g(v) && !can_tile(tile_g(v), elem_bytes)) return FV_ROWS4;
         if (v == FV_CLASS && !can_class(elem_bytes)) return FV_ROWS4;
@@ -183,6 +204,15 @@ public:
     // Fast-kernel parameters (one work item per <= 1024 rows of an outer
     // block) for arithmetic type A (float or double).
     template <class A> void fast_params(fastk::FastParams<A>& p) const;
+    template <class A> void pack_params(packk::Params<A>& p, const PackPlan& plan) const;
+    // The packed plan for block vectors: classes of about class_rows rows, of
+    // amplitude form `form` or a more general one; null where none applies.  Built
+    // on first use and kept.
+    const PackPlan* block_plan(uint32_t class_rows, int form);
+    // reference index of each row of the basis' internal order (null: the same)
+    const uint32_t* permutation() const {
+        return basis_->permuted ? static_cast<const uint32_t*>(db_->ref_of_int) : nullptr;
+    }
     bool uniform_inner() const { return unif_; }
     const WorkItem* items_device() const { return items_.as<WorkItem>(); }
     // host copy of the fast kernel's work items
@@ -205,6 +235,7 @@ public:
 private:
     void build_diagonal();
     void build_fast();
+    void build_pack(const std::vector<Term>& terms);
     template <class S> void upload_terms(const std::vector<HostTerm>& ht);
 
     // fast-path data (see spmv_fast_kernel)
@@ -216,7 +247,7 @@ private:
     void autotune();
     // the work-item list and count a fast variant runs on
     const WorkItem* items_of(FastVariant v, size_t* n) const;
-    bool fast_ = false, force_generic_ = false, unif_ = false;
+    bool fast_ = false, fast_tried_ = false, force_generic_ = false, unif_ = false;
     int mode_ = 0;
     FastVariant pref_[2] = {FV_ROWS4, FV_ROWS4};
     double tune_ms_[2][kFastVariants] = {};
@@ -233,6 +264,12 @@ private:
     FastSet f64s_, f32s_;
     DBuf iptr_, ient_;
     DBuf optr_, mptr_, ment_;  // per-block outer-entry / straddling-term list offsets and straddling entries
+
+    std::unique_ptr<PackPlan> pack_;
+    std::vector<Term> terms_;  // for the block plans
+    std::map<std::pair<uint32_t, int>, std::unique_ptr<PackPlan>> block_plans_;
+    std::mutex block_plans_mu_;
+    DBuf dcode_ref_;  // diagonal codes in reference order (where the internal order differs)
 
     std::shared_ptr<Basis> basis_;
     const DevBasis* db_ = nullptr;

@@ -24,6 +24,8 @@
 //            same block, rank = block offset + inner_rank[b'];
 //   mixed  - everything else: full rank of the target.
 #include "fast_common.cuh"
+#include "pack.hpp"
+#include "solvers.hpp"
 #include "tile.hpp"
 
 #include <algorithm>
@@ -947,7 +949,22 @@ Hamiltonian::Hamiltonian(std::shared_ptr<Basis> basis, SiteKind site, const std:
     upload_vec(items_, items);
     QKG_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     build_diagonal();
-    build_fast();
+    build_pack(terms);
+    if (!pack_) {
+        build_fast();
+        autotune();
+    }
+}
+
+// The tables of the other fast kernels, for a Hamiltonian on the packed one:
+// built when a kernel mode or the batched engine first asks for them.
+void Hamiltonian::ensure_fast() {
+    if (pack_ && !fast_tried_) build_fast();
+}
+void Hamiltonian::set_kernel_mode(int m) {
+    if (m >= 2) ensure_fast();
+    mode_ = m;
+    force_generic_ = m == 1;
 }
 
 namespace {
@@ -966,6 +983,7 @@ static void allow_stage_smem(size_t bytes);
 void Hamiltonian::build_fast() {
     const Basis& B = *basis_;
     fast_ = false;
+    fast_tried_ = true;
     if (B.rank_kind != RANK_TABLE || wide_ || dim() == 0 || dim() >= (1ull << 31) || diag_mode_ == DIAG_FULL) return;
     const uint64_t inm = db_->in_mask;
     std::vector<const HostTerm*> outer, inner, mixed;
@@ -1223,14 +1241,42 @@ void Hamiltonian::build_fast() {
         if (t32) tilek::tile_allow_smem<float, float>(t32);
         if (t64) tilek::tile_allow_smem<double, double>(t64);
     }
-    autotune();
+}
+
+template <class C>
+__global__ void scatter_code_kernel(const C* __restrict__ src, C* __restrict__ dst, const uint32_t* __restrict__ perm,
+                                    uint64_t n) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        dst[perm[i]] = src[i];
+}
+
+// The packed plan of the sectors that the fast kernels take (32-bit states and
+// row indices, coded diagonal).
+void Hamiltonian::build_pack(const std::vector<Term>& terms) {
+    if (wide_ || dim() == 0 || diag_mode_ == DIAG_FULL) return;
+    PackTables tables;
+    if (!tables.build(*basis_, site_, terms)) return;
+    auto plan = std::make_unique<PackPlan>(tables);
+    if (basis_->permuted) {
+        const uint64_t n = dim();
+        const uint32_t* perm = static_cast<const uint32_t*>(db_->ref_of_int);
+        dcode_ref_.alloc(dcode_.bytes);
+        if (diag_mode_ == DIAG_U8)
+            scatter_code_kernel<uint8_t><<<grid_for(n), kBlock, 0, stream_>>>(dcode_.as<uint8_t>(), dcode_ref_.as<uint8_t>(), perm, n);
+        else
+            scatter_code_kernel<uint16_t><<<grid_for(n), kBlock, 0, stream_>>>(dcode_.as<uint16_t>(), dcode_ref_.as<uint16_t>(), perm, n);
+        QKG_LAUNCHED();
+        QKG_CUDA(cudaStreamSynchronize(stream_));
+    }
+    pack_ = std::move(plan);
+    terms_ = terms;
 }
 
 // Autotuner: for sectors large enough to matter, time each fast-kernel
 // variant per precision and keep the fastest for mode 0.
 void Hamiltonian::autotune() {
     const uint64_t n = dim();
-    if (n < (1ull << 20)) return;  // small sectors: four rows per thread
+    if (!fast_ || n < (1ull << 20)) return;  // small sectors: four rows per thread
     const int saved = mode_;
     for (int prec = 0; prec < 2; ++prec) {
         const size_t e = prec ? sizeof(double2) : sizeof(float2);
@@ -1679,7 +1725,38 @@ static void launch_spmv(const DevBasis& b, const TermSet& ts, const DBuf& items,
     QKG_LAUNCHED();
 }
 
+template <class A>
+void Hamiltonian::pack_params(packk::Params<A>& p, const PackPlan& plan) const {
+    plan.params(p);
+    p.diag_mode = diag_mode_;
+    p.cdiag = all_real_ ? 0 : 1;
+    p.dcode = basis_->permuted ? dcode_ref_.p : dcode_.p;
+    p.dtab = (sizeof(A) == 8 ? dtab64_ : dtab32_).template as<A>();
+}
+
+template void Hamiltonian::pack_params<float>(packk::Params<float>&, const PackPlan&) const;
+template void Hamiltonian::pack_params<double>(packk::Params<double>&, const PackPlan&) const;
+
+const PackPlan* Hamiltonian::block_plan(uint32_t class_rows, int form) {
+    if (!pack_) return nullptr;
+    std::lock_guard<std::mutex> lk(block_plans_mu_);
+    auto it = block_plans_.find({class_rows, form});
+    if (it == block_plans_.end()) {
+        PackTables t;
+        std::unique_ptr<PackPlan> plan;
+        if (t.build(*basis_, site_, terms_, class_rows, (packk::AmpMode)form)) plan = std::make_unique<PackPlan>(t);
+        it = block_plans_.emplace(std::make_pair(class_rows, form), std::move(plan)).first;
+    }
+    return it->second.get();
+}
+
 void Hamiltonian::apply_f64(const double2* x, double2* y, cudaStream_t s) const {
+    if (packed()) {
+        packk::Params<double> p;
+        pack_params(p, *pack_);
+        pack_apply_f64(*pack_, p, x, y, s);
+        return;
+    }
     if (fast()) {
         const FastVariant v = variant(16);
         if (tile_g(v) || v == FV_CLASS) {
@@ -1706,6 +1783,14 @@ void Hamiltonian::apply_f64(const double2* x, double2* y, cudaStream_t s) const 
 
 void Hamiltonian::apply_lanczos_f32(const LanczosHooks& lz, cudaStream_t s) const {
     QKG_REQUIRE(fast(), "the device-resident Lanczos step needs the fast SpMV kernel");
+    if (packed()) {
+        packk::Params<float> p;
+        pack_params(p, *pack_);
+        p.lz = lz.op;
+        p.apart = lz.apart;
+        pack_apply_f32(*pack_, p, nullptr, nullptr, s);
+        return;
+    }
     const FastVariant v = variant(8);
     const bool st = v == FV_STAGED || v == FV_ROWS4_STAGED;
     FastParams<float> p;
@@ -1726,6 +1811,7 @@ void Hamiltonian::apply_lanczos_f32(const LanczosHooks& lz, cudaStream_t s) cons
 }
 
 size_t Hamiltonian::lanczos_parts() const {
+    if (packed()) return pack_ctas(*pack_);
     if (!fast()) return n_items_;
     if (variant(8) == FV_CLASS) return class_grid_;
     if (tile_g(variant(8))) return n_tile_items(tile_g(variant(8)));
@@ -1744,6 +1830,12 @@ const WorkItem* Hamiltonian::items_of(FastVariant v, size_t* n) const {
 }
 
 void Hamiltonian::apply_f32(const float2* x, float2* y, cudaStream_t s) const {
+    if (packed()) {
+        packk::Params<float> p;
+        pack_params(p, *pack_);
+        pack_apply_f32(*pack_, p, x, y, s);
+        return;
+    }
     if (fast()) {
         const FastVariant v = variant(8);
         if (tile_g(v) || v == FV_CLASS) {
@@ -1774,7 +1866,8 @@ void Hamiltonian::diagonal_f64(double2* d, cudaStream_t s) const {
         QKG_CUDA(cudaMemcpyAsync(d, dfull64_.p, n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
         return;
     }
-    diag_expand_kernel<double><<<grid_for(n), kBlock, 0, s>>>(dcode_.p, diag_mode_ == DIAG_U8 ? 1 : 2, dtab64_.as<double>(), n, d);
+    const void* codes = packed() && basis_->permuted ? dcode_ref_.p : dcode_.p;
+    diag_expand_kernel<double><<<grid_for(n), kBlock, 0, s>>>(codes, diag_mode_ == DIAG_U8 ? 1 : 2, dtab64_.as<double>(), n, d);
     QKG_LAUNCHED();
 }
 
@@ -1810,9 +1903,27 @@ static void permute(const DevBasis& b, bool permuted, const V* src, V* dst, uint
 }
 
 void Hamiltonian::to_internal_f64(const double2* r, double2* i, cudaStream_t s) const { permute(*db_, permuted(), r, i, dim(), true, s); }
+void Hamiltonian::to_basis_f64(const double2* r, double2* i, cudaStream_t s) const { permute(*db_, basis_->permuted, r, i, dim(), true, s); }
 void Hamiltonian::to_reference_f64(const double2* i, double2* r, cudaStream_t s) const { permute(*db_, permuted(), i, r, dim(), false, s); }
 void Hamiltonian::to_internal_f32(const float2* r, float2* i, cudaStream_t s) const { permute(*db_, permuted(), r, i, dim(), true, s); }
 void Hamiltonian::to_reference_f32(const float2* i, float2* r, cudaStream_t s) const { permute(*db_, permuted(), i, r, dim(), false, s); }
+
+template <class V, bool F64>
+__global__ void philox_order_kernel(uint64_t seed, uint64_t stream, const uint32_t* __restrict__ perm, V* __restrict__ out,
+                                    uint64_t n) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        out[perm[i]] = philox_cnormal<V, F64>(seed, stream, i);
+}
+void Hamiltonian::philox_f64(uint64_t seed, uint64_t stream, double2* out, cudaStream_t s) const {
+    if (!packed() || !basis_->permuted) return philox_normal_f64(seed, stream, out, dim(), s);
+    philox_order_kernel<double2, true><<<grid_for(dim()), kBlock, 0, s>>>(seed, stream, static_cast<const uint32_t*>(db_->ref_of_int), out, dim());
+    QKG_LAUNCHED();
+}
+void Hamiltonian::philox_f32(uint64_t seed, uint64_t stream, float2* out, cudaStream_t s) const {
+    if (!packed() || !basis_->permuted) return philox_normal_f32(seed, stream, out, dim(), s);
+    philox_order_kernel<float2, false><<<grid_for(dim()), kBlock, 0, s>>>(seed, stream, static_cast<const uint32_t*>(db_->ref_of_int), out, dim());
+    QKG_LAUNCHED();
+}
 
 void Hamiltonian::emit_entries(std::vector<uint64_t>& row_offsets, std::vector<uint64_t>& cols,
                                std::vector<std::complex<double>>& vals) const {

@@ -341,7 +341,7 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
 
     float2* v0 = static_cast<float2*>(vptr[0]);
     if (o.device_start) {
-        philox_normal_f32(o.seed, 0, v0, n, st);
+        H.philox_f32(o.seed, 0, v0, st);
     } else {
         // the caller's vector is copied straight from its buffer (pinned memory takes the DMA path)
         std::vector<cd> h;

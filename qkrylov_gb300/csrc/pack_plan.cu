@@ -1,0 +1,578 @@
+// Host side of the packed SpMV plan (pack.hpp): the blocks and classes of the
+// reference order, the terms' classification, and the tables.
+#include "pack.hpp"
+#include "solvers.hpp"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <map>
+#include <tuple>
+
+namespace qkg {
+using namespace packk;
+namespace {
+
+inline int popc(uint64_t x) { return __builtin_popcountll(x); }
+
+// A compiled term without variable factors: conditions, flips, parity, amplitude.
+struct PTerm {
+    uint64_t C, V, X, J;
+    cd amp;
+};
+
+// A term's variable factors are of two kinds: (a0 = -a1) on one bit is a sign,
+// so the bit joins the parity mask; a0 = 0 is a condition on its bits.  A
+// parity bit that a condition pins is a constant sign.  False: another kind.
+bool simplify(const HostTerm& h, PTerm& t, bool& dead) {
+    t = {h.C, h.V, h.X, h.J, h.amp};
+    dead = false;
+    for (const DVar& v : h.vars) {
+        const cd a0(v.a0r, v.a0i), a1(v.a1r, v.a1i);
+        if (a0 == cd(0.0)) {  // all of sm's bits of s ^ pf set
+            const uint64_t need = ~v.pf & v.sm, both = t.C & v.sm;
+            if ((t.V & both) != (need & both)) { dead = true; return true; }
+            t.C |= v.sm;
+            t.V = (t.V & ~v.sm) | need;
+            t.amp *= a1;
+        } else if (a0 == -a1 && popc(v.sm) == 1) {
+            // a1 where the bit of s ^ pf is 1: (-1)^bit(s) times a0 (pf = 0) or a1 (pf = 1)
+            t.J ^= v.sm;
+            t.amp *= (v.pf & v.sm) ? a1 : a0;
+        } else {
+            return false;
+        }
+    }
+    const uint64_t pinned = t.J & t.C;
+    if (popc(pinned & t.V) & 1) t.amp = -t.amp;
+    t.J &= ~pinned;
+    return true;
+}
+
+int top_bit(uint64_t x) { return x ? 63 - __builtin_clzll(x) : -1; }
+
+// Appends v to the image of a plan's tables; returns its offset (16-byte aligned).
+template <class T>
+size_t append(std::vector<char>& image, const std::vector<T>& v) {
+    const size_t at = (image.size() + 15) / 16 * 16;
+    image.resize(at + v.size() * sizeof(T));
+    if (!v.empty()) std::memcpy(image.data() + at, v.data(), v.size() * sizeof(T));
+    return at;
+}
+
+constexpr size_t kMaxTable = 32ull << 20;  // uint2 entries of all tables (256 MB)
+
+}  // namespace
+
+bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& terms, uint32_t class_target,
+                       AmpMode at_least) {
+    *this = PackTables();
+    dim = B.dim;
+    const int nb = B.nbits;
+    if (B.rank_kind != RANK_TABLE || nb > 32 || B.dim == 0 || B.dim >= (1ull << 31)) return false;
+    // popcount groups in the reference encoding
+    uint64_t gm[2] = {0, 0};
+    for (int g = 0; g < B.ngroups; ++g) gm[g] = B.to_reference(B.gmask[g]);
+    const int ng = B.ngroups;
+    // --- terms
+    std::vector<PTerm> list;
+    for (const HostTerm& h : compile_terms(B, site, terms, true)) {
+        if (h.X == 0) continue;
+        PTerm t;
+        bool dead;
+        if (!simplify(h, t, dead)) return false;
+        if (!dead) list.push_back(t);
+    }
+    // --- the split: the most inner bits whose largest class keeps to class_target
+    // rows (a block of x then fits in L1 beside its neighbours') and whose tables
+    // stay below a quarter of the sector's rows (they are built for every
+    // Hamiltonian), whole sites for interleaved bases
+    const int unit = B.split ? 2 : 1;
+    // rows of the largest class that a sector leaves, and of all of them
+    auto class_rows = [&](int n_in, bool all) {
+        uint64_t most = 1;
+        uint64_t free_bits = (1ull << n_in) - 1;
+        for (int g = 0; g < ng; ++g) {
+            const int in = popc(gm[g] & ((1ull << n_in) - 1)), out = popc(gm[g]) - in;
+            uint64_t m = 0;
+            for (int k = 0; k <= in; ++k)
+                if (B.gpop[g] - k >= 0 && B.gpop[g] - k <= out) m = all ? m + binom(in, k) : std::max(m, binom(in, k));
+            most *= m;
+            free_bits &= ~gm[g];
+        }
+        return most << popc(free_bits);
+    };
+    int n_in = std::min(nb, unit);
+    while (n_in + unit <= nb && n_in + unit <= 16 && class_rows(n_in + unit, false) <= class_target &&
+           class_rows(n_in + unit, true) <= std::max<uint64_t>(4096, B.dim / 4))
+        n_in += unit;
+    const int n_out = nb - n_in;
+    if (n_out > 22 || class_rows(n_in, false) > 0xFFFE) return false;
+    const uint64_t inm = (1ull << n_in) - 1;
+    // --- classes of inner configurations (by the groups' popcounts)
+    const int w1 = ng > 1 ? popc(gm[1] & inm) + 1 : 1, w0 = ng > 0 ? popc(gm[0] & inm) + 1 : 1;
+    const int ncls = w0 * w1;
+    auto class_of_inner = [&](uint64_t b) {
+        const int k0 = ng > 0 ? popc(b & gm[0]) : 0, k1 = ng > 1 ? popc(b & gm[1]) : 0;
+        return k0 * w1 + k1;
+    };
+    auto class_of_outer = [&](uint64_t a) {  // the class that block a holds, -1: none
+        const uint64_t s = a << n_in;
+        int k0 = 0, k1 = 0;
+        if (ng > 0) { k0 = B.gpop[0] - popc(s & gm[0]); if (k0 < 0 || k0 >= w0) return -1; }
+        if (ng > 1) { k1 = B.gpop[1] - popc(s & gm[1]); if (k1 < 0 || k1 >= w1) return -1; }
+        return k0 * w1 + k1;
+    };
+    std::vector<std::vector<uint32_t>> members(ncls);
+    std::vector<uint16_t> rank(1ull << n_in), cls(1ull << n_in);
+    for (uint64_t b = 0; b <= inm; ++b) {
+        const int c = class_of_inner(b);
+        cls[b] = (uint16_t)c;
+        rank[b] = (uint16_t)std::min<size_t>(members[c].size(), 0xFFFF);
+        members[c].push_back((uint32_t)b);
+    }
+    const uint64_t n_a = 1ull << n_out;
+    std::vector<uint32_t> off(n_a + 1, 0);
+    std::vector<int> bcls(n_a, -1);
+    std::vector<char> present(ncls, 0);
+    uint64_t total = 0;
+    for (uint64_t a = 0; a < n_a; ++a) {
+        off[a] = (uint32_t)total;
+        bcls[a] = class_of_outer(a);
+        if (bcls[a] < 0) continue;
+        present[bcls[a]] = 1;
+        total += members[bcls[a]].size();
+    }
+    off[n_a] = (uint32_t)total;
+    QKG_REQUIRE(total == B.dim, "packed plan: blocks do not add up to the sector");
+    // --- terms by class, merged by their flips
+    struct Group {
+        uint64_t X;
+        std::vector<PTerm> t;
+    };
+    std::vector<Group> inner, outer, mixed;
+    auto add = [](std::vector<Group>& v, const PTerm& t) {
+        for (auto& g : v)
+            if (g.X == t.X) { g.t.push_back(t); return; }
+        v.push_back({t.X, {t}});
+    };
+    for (const PTerm& t : list) {
+        const uint64_t m = t.X | t.C | t.J;
+        if (!(m & ~inm)) add(inner, t);
+        else if (!(m & inm)) add(outer, t);
+        else add(mixed, t);
+    }
+    // far flips first: the lanes of a warp (consecutive rows) share their high
+    // bits, so their first entries mostly flip the same bond and read one run
+    std::stable_sort(inner.begin(), inner.end(), [](const Group& x, const Group& y) { return top_bit(x.X) > top_bit(y.X); });
+    for (const auto& g : mixed)
+        if (g.t.size() > 24) return false;
+    real = true;
+    for (const auto* v : {&inner, &outer, &mixed})
+        for (const auto& g : *v)
+            for (const auto& t : g.t) real = real && t.amp.imag() == 0.0;
+    auto sum_at = [](const std::vector<PTerm>& ts, uint64_t s, cd& amp) {  // amplitude of the merged terms on s
+        bool any = false;
+        for (const auto& t : ts)
+            if ((s & t.C) == t.V) {
+                const cd v = t.J && (popc(s & t.J) & 1) ? -t.amp : t.amp;
+                amp = any ? amp + v : v;
+                any = true;
+            }
+        return any;
+    };
+    // --- raw tables: (rank, amplitude) per slot and row, then packed by mode
+    struct Raw {
+        std::vector<uint16_t> r;  // [slot][row of the class, padded to tiles]
+        std::vector<uint16_t> c;  // amplitude index
+    };
+    std::map<std::pair<uint64_t, uint64_t>, uint32_t> amp_id;
+    bool too_many = false;
+    // codes met since `used` was last cleared, and the last ones looked up
+    std::vector<char> used;
+    cd seen[4];
+    uint16_t seen_id[4];
+    int n_seen = 0, next_seen = 0;
+    auto code_of = [&](cd a) -> uint16_t {
+        for (int i = 0; i < n_seen; ++i)
+            if (seen[i] == a) {
+                used[seen_id[i]] = 1;
+                return seen_id[i];
+            }
+        uint64_t k[2];
+        const double re = a.real() + 0.0, im = a.imag() + 0.0;  // no negative zeros
+        std::memcpy(k, &re, 8);
+        std::memcpy(k + 1, &im, 8);
+        auto it = amp_id.find({k[0], k[1]});
+        if (it == amp_id.end()) {
+            if (amps.size() >= 4096) { too_many = true; return 0; }
+            it = amp_id.emplace(std::make_pair(k[0], k[1]), (uint32_t)amps.size()).first;
+            amps.push_back(cd(re, im));
+            used.push_back(0);
+        }
+        seen[next_seen] = cd(re, im);
+        seen_id[next_seen] = (uint16_t)it->second;
+        n_seen = std::min(n_seen + 1, 4);
+        next_seen = (next_seen + 1) & 3;
+        used[it->second] = 1;
+        return (uint16_t)it->second;
+    };
+    // the magnitude of the used codes (-1: none used), and which signs occur; one =
+    // false: several magnitudes
+    struct Mag {
+        double mag = -1.0;
+        bool plus = false, minus = false, one = true;
+    };
+    auto magnitude = [&]() {
+        Mag m;
+        for (size_t i = 0; i < amps.size(); ++i) {
+            if (!used[i]) continue;
+            const double v = amps[i].real();
+            if (m.mag < 0.0) m.mag = std::abs(v);
+            m.one = m.one && std::abs(v) == m.mag;
+            (std::signbit(v) ? m.minus : m.plus) = true;
+        }
+        std::fill(used.begin(), used.end(), 0);
+        return m;
+    };
+    std::vector<uint32_t> ctile(ncls, 0);  // first inner tile of a class
+        std::vector<uint16_t> er, ec;  // entries: [(slot * 32 + lane) * 4 + q]
+    size_t longest = 0;            // inner entries of a row
+    auto tiles_of = [&](int c) { return (uint32_t)((members[c].size() + kTile - 1) / kTile); };
+    // emit(row, target rank, amplitude index) for the rows of class c on which the
+    // merged terms ts give an entry in class c2.  A few terms have a few sums: the
+    // amplitude index is looked up by which terms hold, and with which signs.
+    std::vector<int> sums;
+    auto each = [&](int c, int c2, const std::vector<PTerm>& ts, uint32_t flip, auto&& emit) {
+        const size_t T = ts.size();
+        const bool few = T <= 5;
+        if (few) sums.assign((size_t)1 << (2 * T), -1);
+        uint32_t C[5], V[5], J[5];
+        for (size_t k = 0; few && k < T; ++k) C[k] = (uint32_t)ts[k].C, V[k] = (uint32_t)ts[k].V, J[k] = (uint32_t)ts[k].J;
+        const auto& mem = members[c];
+        for (uint32_t r = 0; r < mem.size(); ++r) {
+            const uint32_t bb = mem[r], b2 = bb ^ flip;
+            if (few) {
+                uint32_t key = 0;
+                for (size_t k = 0; k < T; ++k)
+                    if ((bb & C[k]) == V[k]) key |= (J[k] && __builtin_parity(bb & J[k]) ? ((1u << T) | 1u) : 1u) << k;
+                if (!key || cls[b2] != c2) continue;
+                int& id = sums[key];
+                if (id < 0) {  // code_of also marks the code as used
+                    cd amp;
+                    sum_at(ts, bb, amp);
+                    id = code_of(amp);
+                }
+                emit(r, rank[b2], (uint16_t)id);
+            } else {
+                cd amp;
+                if (!sum_at(ts, bb, amp) || cls[b2] != c2) continue;
+                emit(r, rank[b2], code_of(amp));
+            }
+        }
+    };
+    std::vector<uint16_t> rr, rc;  // a class' rows: entries in group order
+    std::vector<uint8_t> rn;       // how many
+    for (int c = 0; c < ncls; ++c) {
+        ctile[c] = (uint32_t)tile.size();
+        if (!present[c]) continue;
+        const size_t W = members[c].size(), most_slots = inner.size();
+        if (most_slots > 255) return false;
+        rn.assign(W, 0);
+        rr.resize(W * most_slots);
+        rc.resize(W * most_slots);
+        for (const auto& g : inner)
+            each(c, c, g.t, (uint32_t)g.X, [&](uint32_t r, uint16_t to, uint16_t code) {
+                const size_t at = r * most_slots + rn[r]++;
+                rr[at] = to;
+                rc[at] = code;
+            });
+        for (uint32_t t = 0; t < tiles_of(c); ++t) {
+            uint2 rec = make_uint2((uint32_t)(er.size() / kTile), 0u);
+            for (uint32_t q = 0; q < 4; ++q) {
+                const size_t r0 = (size_t)t * kTile + q * 32, r1 = std::min(W, r0 + 32);
+                size_t most = 0;
+                for (size_t r = r0; r < r1; ++r) most = std::max<size_t>(most, rn[r]);
+                rec.y |= (uint32_t)most << (8 * q);
+                longest = std::max(longest, most);
+                const size_t e0 = er.size(), nq = (most + 3) / 4;
+                er.resize(e0 + nq * kTile, (uint16_t)kNone16);
+                ec.resize(er.size(), 0);
+                for (size_t r = r0; r < r1; ++r)
+                    for (size_t j = 0; j < rn[r]; ++j) {
+                        const size_t at = e0 + ((j / 4) * 32 + (r - r0)) * 4 + (j & 3);
+                        er[at] = rr[r * most_slots + j];
+                        ec[at] = rc[r * most_slots + j];
+                    }
+            }
+            tile.push_back(rec);
+            if (er.size() / 4 > kMaxTable || too_many) return false;
+        }
+    }
+    // the kernels read one quad ahead
+    er.resize(er.size() + kTile, (uint16_t)kNone16);
+    ec.resize(er.size(), 0);
+    const Mag inner_mag = magnitude();
+    // --- per block: outer entries and straddling tables
+    blk.assign(n_a, Blk{});
+    struct O { int32_t d; cd a; };
+    struct M { uint32_t tab, off; };
+    std::vector<O> olist;
+    std::vector<M> slist;
+    std::map<std::tuple<int, uint32_t, uint32_t, uint32_t, int>, uint32_t> tables;  // -> first entry / 4 (uint2 index)
+    std::vector<std::pair<uint32_t, Mag>> table_mag;  // of each straddling table
+    size_t outer_most = 0, mixed_most = 0;
+    for (uint64_t a = 0; a < n_a; ++a) {
+        blk[a].o0 = (uint32_t)olist.size();
+        blk[a].m0 = (uint32_t)slist.size();
+        if (bcls[a] >= 0) {
+            const uint64_t sa = a << n_in;
+            for (const auto& g : outer) {
+                const uint64_t a2 = a ^ (g.X >> n_in);
+                cd amp;
+                if (bcls[a2] != bcls[a] || !sum_at(g.t, sa, amp)) continue;
+                olist.push_back({(int32_t)((int64_t)off[a2] - (int64_t)off[a]), amp});
+            }
+            for (size_t gi = 0; gi < mixed.size(); ++gi) {
+                const auto& g = mixed[gi];
+                const uint64_t a2 = a ^ (g.X >> n_in);
+                if (bcls[a2] < 0) continue;
+                uint32_t valid = 0, neg = 0;
+                for (size_t k = 0; k < g.t.size(); ++k)
+                    if ((sa & g.t[k].C & ~inm) == (g.t[k].V & ~inm)) {
+                        valid |= 1u << k;
+                        if (popc(sa & g.t[k].J & ~inm) & 1) neg |= 1u << k;
+                    }
+                if (!valid) continue;
+                const auto key = std::make_tuple(bcls[a], (uint32_t)gi, valid, neg, bcls[a2]);
+                auto it = tables.find(key);
+                if (it == tables.end()) {
+                    std::vector<PTerm> ts;
+                    for (size_t k = 0; k < g.t.size(); ++k)
+                        if (valid >> k & 1) {
+                            PTerm t = g.t[k];
+                            t.C &= inm;
+                            t.V &= inm;
+                            t.J &= inm;
+                            if (neg >> k & 1) t.amp = -t.amp;
+                            ts.push_back(t);
+                        }
+                    const int c = bcls[a], c2 = bcls[a2];
+                    const size_t e0 = er.size();
+                    er.resize(e0 + (size_t)tiles_of(c) * kTile, (uint16_t)kNone16);
+                    ec.resize(er.size(), 0);
+                    bool any = false;
+                    each(c, c2, ts, (uint32_t)(g.X & inm), [&](uint32_t r, uint16_t to, uint16_t code) {
+                        const size_t t = r / kTile, i = r % kTile;
+                        const size_t at = e0 + (t * 32 + (i & 31)) * 4 + (i >> 5);
+                        er[at] = to;
+                        ec[at] = code;
+                        any = true;
+                    });
+                    if (er.size() / 4 > kMaxTable || too_many) return false;
+                    uint32_t id = 0xFFFFFFFFu;  // no row of the class has an entry
+                    if (any) {
+                        id = (uint32_t)(e0 / 4);
+                        table_mag.push_back({id, magnitude()});
+                    } else {
+                        er.resize(e0);
+                        ec.resize(e0);
+                    }
+                    it = tables.emplace(key, id).first;
+                }
+                if (it->second != 0xFFFFFFFFu) slist.push_back({it->second, off[a2]});
+            }
+        }
+        blk[a].o1 = (uint32_t)olist.size();
+        blk[a].m1 = (uint32_t)slist.size();
+        outer_most = std::max<size_t>(outer_most, blk[a].o1 - blk[a].o0);
+        mixed_most = std::max<size_t>(mixed_most, blk[a].m1 - blk[a].m0);
+        if (olist.size() > 0x7FFFFFFFull || slist.size() > 0x7FFFFFFFull) return false;
+    }
+    // --- amplitude mode: one magnitude per inner table and per straddling table?
+    size_t widest = 0;
+    for (int c = 0; c < ncls; ++c)
+        if (present[c]) widest = std::max(widest, members[c].size());
+    bool one = real && inner_mag.one, sgn = inner_mag.plus && inner_mag.minus;
+    const double umag = inner_mag.mag;
+    std::map<uint32_t, double> smag;  // straddling table -> its amplitude (its magnitude where signs differ)
+    equal = real;
+    u = umag < 0.0 ? 0.0 : (inner_mag.plus ? umag : -umag);
+    for (const auto& t : table_mag) {
+        one = one && t.second.one;
+        sgn = sgn || (t.second.plus && t.second.minus);
+    }
+    sgn = sgn || at_least == AMP_SIGNED;
+    if (sgn && widest > 0x7FFF) one = false;
+    mode = one && at_least != AMP_CODED ? (sgn ? AMP_SIGNED : AMP_UNIFORM) : AMP_CODED;
+    if (mode == AMP_CODED && amps.size() > (size_t)kMaxAmps) return false;
+    if (mode != AMP_CODED) {
+        if (mode == AMP_SIGNED) {
+            // rank | sign << 15; amplitudes are magnitudes
+            std::vector<uint16_t> bit(amps.size());
+            for (size_t i = 0; i < amps.size(); ++i) bit[i] = std::signbit(amps[i].real()) ? 0x8000u : 0u;
+            for (size_t e = 0; e < er.size(); ++e)
+                er[e] = er[e] == kNone16 ? (uint16_t)kNone15 : (uint16_t)(er[e] | bit[ec[e]]);
+            u = std::max(umag, 0.0);
+        }
+        for (const auto& t : table_mag)
+            smag[t.first] = mode == AMP_SIGNED || t.second.plus ? t.second.mag : -t.second.mag;
+        double mag = umag;
+        auto same = [&](double v) {
+            v = std::abs(v);
+            if (mag < 0.0) mag = v;
+            if (v != mag) equal = false;
+        };
+        for (const auto& o : olist) same(o.a.real());
+        for (const auto& s : smag) same(s.second);
+        if (umag < 0.0) u = std::max(mag, 0.0);  // no inner entry: the common magnitude
+    } else {
+        equal = false;
+    }
+    if (longest + outer_most + mixed_most > (size_t)kMaxRowEntries) equal = false;
+    // --- items: the tiles of every block; blocks that a straddling flip of the
+    // highest outer bit joins run side by side, so that the rows they gather from
+    // one another are still in L2
+    int pair_bit = -1;
+    for (const auto& g : mixed) pair_bit = std::max(pair_bit, top_bit(g.X >> n_in));
+    std::vector<uint32_t> order;
+    for (uint64_t a = 0; a < n_a; ++a)
+        if (bcls[a] >= 0) order.push_back((uint32_t)a);
+    if (pair_bit >= 0) {
+        const uint32_t m = 1u << pair_bit;
+        auto key = [&](uint32_t a) { return ((uint64_t)(a & ~m) << 1) | ((a & m) ? 1u : 0u); };
+        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return key(x) < key(y); });
+    }
+    for (uint32_t a : order) {
+        const size_t W = members[bcls[a]].size();
+        for (size_t t = 0; t * kTile < W; ++t)
+            items.push_back({(uint32_t)(off[a] + t * kTile), a, ctile[bcls[a]] + (uint32_t)t,
+                             (uint32_t)(t << 8 | std::min<size_t>(kTile, W - t * kTile))});
+    }
+    // --- the packed tables
+    tab.resize(er.size() / 4);
+    if (!er.empty()) std::memcpy(tab.data(), er.data(), er.size() * 2);
+    if (mode == AMP_CODED) {
+        codes.resize(er.size() / 4);
+        for (size_t e = 0; e < codes.size(); ++e)
+            codes[e] = (uint32_t)ec[4 * e] | (uint32_t)ec[4 * e + 1] << 8 | (uint32_t)ec[4 * e + 2] << 16 | (uint32_t)ec[4 * e + 3] << 24;
+    }
+    for (const auto& o : olist) out.push_back({o.d, 0u, o.a.real(), o.a.imag()});
+    for (const auto& m : slist) {
+        const double v = mode == AMP_CODED ? 0.0 : smag[m.tab];
+        str.push_back({m.tab, m.off, v, 0.0});
+    }
+    return true;
+}
+
+void PackTables::apply_host(const cd* x, cd* y) const {
+    auto in = [](bool ok) { QKG_REQUIRE(ok, "packed tables: index out of range"); };
+    for (const Item& it : items) {
+        const uint32_t cnt = it.tc & 0xFFu, tin = it.tc >> 8;
+        in(it.a < blk.size() && it.tile < tile.size() && cnt <= (uint32_t)kTile);
+        const Blk b = blk[it.a];
+        in(b.o1 <= out.size() && b.m1 <= str.size() && tin * (uint64_t)kTile <= it.row0);
+        for (uint32_t i = 0; i < (uint32_t)kTile; ++i) {
+            const uint32_t lane = i & 31u, q = i >> 5;
+            const uint64_t row = (uint64_t)it.row0 + i;
+            cd s = 0.0;
+            if (i < cnt)
+                for (uint32_t k = b.o0; k < b.o1; ++k) {
+                    const int64_t t = (int64_t)row + out[k].delta;
+                    in(row < dim && t >= 0 && t < (int64_t)dim);
+                    s += cd(out[k].ar, out[k].ai) * x[t];
+                }
+            auto entry = [&](uint64_t at, uint32_t k, uint64_t base, double amp) {
+                in(at < tab.size() && k < 4);
+                const uint32_t w = (k & 2u) ? tab[at].y : tab[at].x;
+                uint32_t r = (k & 1u) ? w >> 16 : w & 0xFFFFu;
+                cd a = amp;
+                if (mode == AMP_SIGNED) {
+                    if (r & 0x8000u) a = -a;
+                    r &= 0x7FFFu;
+                    if (r == kNone15) return;
+                } else if (r == kNone16) {
+                    return;
+                }
+                if (mode == AMP_CODED) {
+                    in(at < codes.size());
+                    const uint32_t c = (codes[at] >> (8 * k)) & 0xFFu;
+                    in(c < amps.size());
+                    a = amps[c];
+                }
+                in(i < cnt && base + r < dim);  // rows past the block's end have no entries
+                s += a * x[base + r];
+            };
+            uint64_t quad = tile[it.tile].x;
+            for (uint32_t g = 0; g < q; ++g) quad += (((tile[it.tile].y >> (8 * g)) & 0xFFu) + 3u) / 4u;
+            const uint32_t slots = (tile[it.tile].y >> (8 * q)) & 0xFFu;
+            for (uint32_t j = 0; j < slots; ++j)
+                entry((quad + j / 4) * 32 + lane, j & 3u, it.row0 - tin * (uint64_t)kTile, u);
+            in((quad + (slots + 3) / 4) * 32 + lane < tab.size());  // the quad read ahead
+            for (uint32_t k = b.m0; k < b.m1; ++k) entry(str[k].tab + tin * 32ull + lane, q, str[k].off, str[k].ar);
+            if (i < cnt) y[row] = s;
+        }
+    }
+}
+
+PackPlan::PackPlan(const PackTables& t)
+    : real_(t.real), equal_(t.equal), mode_(t.mode), n_items_((uint32_t)t.items.size()), n_amps_((int)t.codes.size() ? (int)t.amps.size() : 0), u_(t.u) {
+    for (const Item& it : t.items) {
+        if ((it.tc >> 8) == 0) blocks_.push_back({it.row0, it.a, it.tile, 0});
+        blocks_.back().rows += it.tc & 0xFFu;
+    }
+    std::vector<char> image;
+    items_ = append(image, t.items);
+    blk_ = append(image, t.blk);
+    tile_ = append(image, t.tile);
+    tab_ = append(image, t.tab);
+    out64_ = append(image, t.out);
+    str64_ = append(image, t.str);
+    std::vector<Out<float>> o32;
+    for (const auto& o : t.out) o32.push_back({o.delta, 0u, (float)o.ar, (float)o.ai});
+    std::vector<Str<float>> s32;
+    for (const auto& s : t.str) s32.push_back({s.tab, s.off, (float)s.ar, (float)s.ai});
+    out32_ = append(image, o32);
+    str32_ = append(image, s32);
+    if (mode_ == AMP_CODED) {
+        codes_ = append(image, t.codes);
+        std::vector<float2> a32;
+        std::vector<double2> a64;
+        for (const cd& a : t.amps) {
+            a32.push_back(make_float2((float)a.real(), (float)a.imag()));
+            a64.push_back(make_double2(a.real(), a.imag()));
+        }
+        amps32_ = append(image, a32);
+        amps64_ = append(image, a64);
+    }
+    all_.alloc(std::max<size_t>(16, image.size()));
+    if (!image.empty()) QKG_CUDA(cudaMemcpy(all_.p, image.data(), image.size(), cudaMemcpyHostToDevice));
+}
+
+int packed_apply_host(const Basis& B, SiteKind site, const std::vector<Term>& terms, const double* x, double* y) {
+    PackTables t;
+    if (!t.build(B, site, terms)) return -1;
+    t.apply_host(reinterpret_cast<const cd*>(x), reinterpret_cast<cd*>(y));
+    return (int)t.mode + (t.equal ? 4 : 0) + (t.real ? 0 : 8);
+}
+
+template <class A>
+void PackPlan::params(Params<A>& p) const {
+    std::memset(&p, 0, sizeof(p));
+    const bool d = sizeof(A) == 8;
+    p.items = at<Item>(items_);
+    p.n_items = n_items_;
+    p.blk = at<Blk>(blk_);
+    p.out = at<Out<A>>(d ? out64_ : out32_);
+    p.str = at<Str<A>>(d ? str64_ : str32_);
+    p.tile = at<uint2>(tile_);
+    p.tab = at<uint2>(tab_);
+    p.codes = mode_ == AMP_CODED ? at<uint32_t>(codes_) : nullptr;
+    p.amps = mode_ == AMP_CODED ? at<A>(d ? amps64_ : amps32_) : nullptr;
+    p.n_amps = n_amps_;
+    p.u = (A)u_;
+}
+template void PackPlan::params<float>(Params<float>&) const;
+template void PackPlan::params<double>(Params<double>&) const;
+
+}  // namespace qkg

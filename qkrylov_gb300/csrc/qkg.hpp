@@ -203,7 +203,8 @@ enum SiteKind : int { SITE_SPIN = 0, SITE_FERMION = 1, SITE_HUBBARD = 2, SITE_TJ
 
 // Compile an OpSum for a basis and a site kind.  Dead terms (never valid on
 // the basis) are dropped; unknown operators and sites outside [0, 64) for the
-// site's bit layout throw Error(INVALID_ARG).
-std::vector<HostTerm> compile_terms(const Basis& b, SiteKind site, const std::vector<Term>& terms);
+// site's bit layout throw Error(INVALID_ARG).  reference: masks on the
+// reference's encoding instead of the basis' internal one.
+std::vector<HostTerm> compile_terms(const Basis& b, SiteKind site, const std::vector<Term>& terms, bool reference = false);
 
 }  // namespace qkg

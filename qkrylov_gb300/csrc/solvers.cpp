@@ -486,7 +486,7 @@ LanczosOut lanczos_f64(Hamiltonian& H, const LanczosOpts& o) {
     DBuf w(n * sizeof(double2)), tmp;
     double2* v = V.push();
     if (o.device_start) {
-        philox_normal_f64(o.seed, 0, v, n, st);
+        H.philox_f64(o.seed, 0, v, st);
     } else {
         std::vector<cd> h;
         const cd* src = o.v0_ref;
@@ -615,7 +615,7 @@ LanczosOut lanczos_mixed(Hamiltonian& H, const LanczosOpts& o) {
     DBuf w(n * sizeof(float2)), tmp;
     float2* v = V.push();
     if (o.device_start) {
-        philox_normal_f32(o.seed, 0, v, n, st);
+        H.philox_f32(o.seed, 0, v, st);
     } else {
         std::vector<cd> h;
         const cd* src = o.v0_ref;

@@ -67,6 +67,11 @@ struct NormalStream {
     }
 };
 // Device Philox4x32-10 (Salmon et al., SC'11) Gaussian complex vectors.
+// Test hook: the off-diagonal part of H x (reference order) from the packed
+// SpMV plan's tables, walked on the host with every index checked; returns the
+// amplitude form (0 uniform, 1 signed, 2 coded; + 4 equal magnitudes, + 8
+// complex), or -1 where the plan does not apply.
+int packed_apply_host(const Basis& B, SiteKind site, const std::vector<Term>& terms, const double* x, double* y);
 void philox_normal_f64(uint64_t seed, uint64_t stream, double2* out, uint64_t n, cudaStream_t s);
 void philox_normal_f32(uint64_t seed, uint64_t stream, float2* out, uint64_t n, cudaStream_t s);
 

@@ -1,0 +1,485 @@
+// SpMV kernels of the packed plan (pack.hpp): a tile of 128 consecutive rows is
+// one warp's work (NQ = 4: lane l holds rows l, l + 32, l + 64 and l + 96) or
+// four warps' (NQ = 1: 32 rows each).
+//
+// What bounds them.  FP32: the latency of the gathers (long-scoreboard stalls, half
+// the issue slots used), so the entries are cheap to decode (a 64-bit load holds four
+// ranks; a gather, its address and one packed FMA an entry), four gathers are in
+// flight a warp, and the registers are held to 48 warps a SM.  Reading and writing
+// vectors in the reference's order makes the lanes of a warp consecutive states:
+// far flips, listed first, read one run.  L = 28 ring (40.1 M rows): 0.42 ms = 1.52
+// TB/s of x and y; the kernel on the domain-wall order 0.66 ms, and 0.19 ms for each of
+// the two permutation passes of an apply that this order does without.
+// FP64: the integer pipe (60% busy) for equal magnitudes, 1.65 ms; the FP64 pipe (88%
+// busy) otherwise and before, 2.80 ms.
+#include "pack.hpp"
+
+#include <type_traits>
+
+namespace qkg {
+using namespace fastk;
+using namespace packk;
+namespace {
+
+using u64 = unsigned long long;
+
+// CTAs of four warps.  Resident CTAs the register allocation is held to: the
+// kernels wait for gathers, so FP32 takes 48 warps a SM at 40 registers (L = 28
+// ring: 32 warps 0.47 ms, 40 0.46, 48 0.42, 56 0.44), FP64 24 warps at 80 (16
+// warps 2.05 ms, 24 1.65, 32 1.65).
+constexpr int kThreads = 128;
+constexpr int kCtas32 = 12, kCtas64 = 6;
+
+// Two FP32 FMAs in one instruction: d = a * b + c on (re, im) pairs.
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 pair(float x, float y) {
+    u64 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ float2 unpair(u64 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+// ---- sums of one row -------------------------------------------------------
+// FP32, real amplitudes.
+struct SumF32 {
+    using V = u64;  // one complex element
+    u64 s;
+    __device__ __forceinline__ void init() { s = 0ull; }
+    __device__ __forceinline__ void add(float a, V x) { s = fma2(pair(a, a), x, s); }
+    __device__ __forceinline__ void add(float ar, float ai, V x) {
+        const float2 v = unpair(x);
+        s = fma2(pair(ar, ar), x, s);
+        s = fma2(pair(-ai, ai), pair(v.y, v.x), s);
+    }
+};
+// FP64 on the FP64 pipe.
+struct SumF64 {
+    using V = double2;
+    double r, i;
+    __device__ __forceinline__ void init() { r = i = 0.0; }
+    __device__ __forceinline__ void add(double a, V x) {
+        r = fma(a, x.x, r);
+        i = fma(a, x.y, i);
+    }
+    __device__ __forceinline__ void add(double ar, double ai, V x) {
+        r = fma(-ai, x.y, fma(ar, x.x, r));
+        i = fma(ai, x.x, fma(ar, x.y, i));
+    }
+};
+
+// FP64 sums by integers aligned to the largest exponent met so far.  All
+// amplitudes of the row have the same magnitude, so the row is that magnitude
+// times a sum of +-x, and each x is its 53-bit significand shifted right by its
+// exponent's distance from the largest: GB300 adds doubles at 2 a clock and SM,
+// integers at 64.  The significand keeps 4 bits below its last place and 6
+// above its first (up to 64 addends), so an addend loses less than 2^-56 of the
+// largest one where a chain of FP64 additions rounds each partial sum to 2^-53.
+// Infinities, NaN and rows below 2^-959 are left to the FP64 pipe (bad()).
+struct IntSum {
+    long long s;
+    int e;
+    // PTX shifts clamp: a distance of 64 or more leaves nothing
+    static __device__ __forceinline__ u64 shift(u64 v, int d) {
+        u64 r;
+        asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(d));
+        return r;
+    }
+    static __device__ __forceinline__ long long shift(long long v, int d) {
+        long long r;
+        asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(d));
+        return r;
+    }
+    __device__ __forceinline__ void init() {
+        s = 0;
+        e = 0;
+    }
+    // x with its sign bit flipped by the top bit of `flip`
+    __device__ __forceinline__ void add(uint32_t flip, double x) {
+        const uint32_t hi = (uint32_t)__double2hiint(x);
+        const uint32_t lo = (uint32_t)__double2loint(x);
+        const int ex = (int)((hi >> 20) & 0x7FFu);
+        const int em = max(e, ex);
+        s = shift(s, em - e);
+        e = em;
+        u64 m = ((u64)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+        m = shift(m << 4, em - ex);
+        const long long sg = (long long)((int)(hi ^ flip) >> 31);  // 0 or -1
+        s += ((long long)m ^ sg) - sg;
+    }
+    __device__ __forceinline__ bool bad() const { return e == 0x7FF || e < 64; }
+    // u times the sum (s counts units of 2^(e - 1079)); v = u * 2^-56
+    __device__ __forceinline__ double value(double v) const { return v * __hiloint2double(e << 20, 0) * (double)s; }
+};
+struct SumI64 {
+    using V = double2;
+    IntSum r, i;
+    __device__ __forceinline__ void init() {
+        r.init();
+        i.init();
+    }
+    __device__ __forceinline__ void add(double a, V x) {  // a = +-u
+        const uint32_t flip = (uint32_t)__double2hiint(a);
+        r.add(flip, x.x);
+        i.add(flip, x.y);
+    }
+    __device__ __forceinline__ void add(double, double, V) {}  // never called: coded amplitudes go to SumF64
+    __device__ __forceinline__ bool bad() const { return r.bad() || i.bad(); }
+};
+
+// a with the sign of the top bit of w applied
+__device__ __forceinline__ float with_sign(float a, uint32_t w) {
+    return __uint_as_float(__float_as_uint(a) ^ (w & 0x80000000u));
+}
+__device__ __forceinline__ double with_sign(double a, uint32_t w) {
+    return __hiloint2double(__double2hiint(a) ^ (int)(w & 0x80000000u), __double2loint(a));
+}
+
+// Element i of v; on = false: zero, without a load.
+template <class T> struct Elem;
+template <> struct Elem<float> {
+    using V = u64;
+    static __device__ __forceinline__ V load(const float2* p) { return __ldg(reinterpret_cast<const u64*>(p)); }
+    static __device__ __forceinline__ V load_if(const float2* p, bool on) {
+        V v;
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.b64 %0, 0;\n\t@p ld.global.nc.b64 %0, [%1];\n\t}"
+            : "=l"(v) : "l"(p), "r"((uint32_t)on));
+        return v;
+    }
+};
+template <> struct Elem<double> {
+    using V = double2;
+    static __device__ __forceinline__ V load(const double2* p) { return __ldg(p); }
+    static __device__ __forceinline__ V load_if(const double2* p, bool on) {
+        V v;
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\tmov.f64 %1, 0d0000000000000000;\n\t"
+            "@p ld.global.nc.v2.f64 {%0, %1}, [%2];\n\t}"
+            : "=d"(v.x), "=d"(v.y) : "l"(p), "r"((uint32_t)on));
+        return v;
+    }
+};
+
+// The off-diagonal sums of a warp's tile.  MODE: AmpMode; CPLX: complex
+// amplitudes (coded).
+template <class T, class Sum, int MODE, bool CPLX, int NQ>
+__device__ __forceinline__ void walk(const Params<T>& p, const Item& it, uint32_t q0, const typename V2<T>::t* __restrict__ x,
+                                     const T* s_amp, Sum (&acc)[NQ]) {
+    using E = Elem<T>;
+    using V = typename E::V;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t cnt = it.tc & 0xFFu, tin = it.tc >> 8;
+    const uint4 b4 = __ldg(reinterpret_cast<const uint4*>(p.blk) + it.a);
+    const uint2 t2 = __ldg(p.tile + it.tile);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) acc[q].init();
+    // outer entries: one offset and amplitude for the whole block
+    const auto* xr = x + it.row0 + lane + 32u * q0;
+    if (cnt >= 32u * (q0 + NQ)) {
+#pragma unroll(NQ == 4 ? 2 : 4)
+        for (uint32_t k = b4.x; k < b4.y; ++k) {
+            const Out<T> o = p.out[k];
+            const auto* xo = xr + o.delta;
+            V v[NQ];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) v[q] = E::load(xo + 32 * q);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                if (CPLX) acc[q].add(o.ar, o.ai, v[q]);
+                else acc[q].add(o.ar, v[q]);
+            }
+        }
+    } else {
+        for (uint32_t k = b4.x; k < b4.y; ++k) {
+            const Out<T> o = p.out[k];
+            const auto* xo = xr + o.delta;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                if (lane + 32u * (q0 + q) < cnt) {
+                    const V v = E::load(xo + 32 * q);
+                    if (CPLX) acc[q].add(o.ar, o.ai, v);
+                    else acc[q].add(o.ar, v);
+                }
+        }
+    }
+    // entry k of a quad: rank, whether there is one, amplitude
+    auto rank_of = [&](const uint2& e, int k, bool& on) -> uint32_t {
+        const uint32_t w = (k & 2) ? e.y : e.x;
+        const uint32_t r = (k & 1) ? w >> 16 : w & 0xFFFFu;
+        if (MODE == AMP_SIGNED) {
+            on = (r & 0x7FFFu) != kNone15;
+            return r & 0x7FFFu;
+        }
+        on = r != kNone16;
+        return r;
+    };
+    auto add_entry = [&](const uint2& e, int k, uint32_t code, Sum& s, const V& v, T u) {
+        if (MODE == AMP_CODED) {
+            const uint32_t c = (code >> (8 * k)) & 0xFFu;
+            if (CPLX) s.add(s_amp[2 * c], s_amp[2 * c + 1], v);
+            else s.add(s_amp[2 * c], v);
+        } else if (MODE == AMP_SIGNED) {
+            const uint32_t w = (k & 2) ? e.y : e.x;
+            s.add(with_sign(u, (k & 1) ? w : w << 16), v);
+        } else {
+            s.add(u, v);
+        }
+    };
+    // inner entries, row group by row group; the next quad is loaded before this
+    // one's gathers
+    {
+        const auto* xb = x + (it.row0 - tin * (uint32_t)kTile);
+        uint32_t first = t2.x;
+        if (NQ == 1) {  // the quads of the row groups before this one
+            if (q0 > 0) first += ((t2.y & 0xFFu) + 3u) >> 2;
+            if (q0 > 1) first += (((t2.y >> 8) & 0xFFu) + 3u) >> 2;
+            if (q0 > 2) first += (((t2.y >> 16) & 0xFFu) + 3u) >> 2;
+        }
+        uint32_t at = first * 32u + lane;
+        uint2 nxt = __ldg(p.tab + at);
+        uint32_t cn = MODE == AMP_CODED ? __ldg(p.codes + at) : 0u;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            for (int n = (int)((t2.y >> (8 * (q0 + q))) & 0xFFu); n > 0; n -= 4) {
+                const uint2 e = nxt;
+                const uint32_t c = cn;
+                at += 32u;
+                nxt = __ldg(p.tab + at);
+                if (MODE == AMP_CODED) cn = __ldg(p.codes + at);
+                V v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    bool on;
+                    const uint32_t r = rank_of(e, k, on);
+                    v[k] = E::load_if(xb + r, on);
+                }
+                add_entry(e, 0, c, acc[q], v[0], p.u);
+                add_entry(e, 1, c, acc[q], v[1], p.u);
+                if (sizeof(T) == 4 || n > 2) {  // a slot costs the FP64 sums tens of instructions
+                    add_entry(e, 2, c, acc[q], v[2], p.u);
+                    add_entry(e, 3, c, acc[q], v[3], p.u);
+                }
+            }
+        }
+    }
+    // straddling tables: one entry a row
+    for (uint32_t k = b4.z; k < b4.w; ++k) {
+        const Str<T> s = p.str[k];
+        const uint32_t at = s.tab + tin * 32u + lane;
+        const uint2 e = __ldg(p.tab + at);
+        const uint32_t c = MODE == AMP_CODED ? __ldg(p.codes + at) : 0u;
+        V v[NQ];
+        if (NQ == 4) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                bool on;
+                const uint32_t r = rank_of(e, q, on);
+                v[q] = E::load_if(x + s.off + r, on);
+            }
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) add_entry(e, q, c, acc[q], v[q], s.ar);
+        } else {
+            // entry q0, brought to the first place
+            const uint32_t w = (q0 & 2u) ? e.y : e.x;
+            const uint2 f = make_uint2((q0 & 1u) ? w >> 16 : w, 0u);
+            bool on;
+            const uint32_t r = rank_of(f, 0, on);
+            v[0] = E::load_if(x + s.off + r, on);
+            add_entry(f, 0, c >> (8u * q0), acc[0], v[0], s.ar);
+        }
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void load_amps(const Params<T>& p, T* s_amp) {
+    for (int i = threadIdx.x; i < 2 * p.n_amps; i += blockDim.x) s_amp[i] = p.amps[i];
+    __syncthreads();
+}
+
+template <class T>
+__device__ __forceinline__ void diag_at(const Params<T>& p, uint32_t row, T& dr, T& di) {
+    const uint32_t c = p.diag_mode == DIAG_U8 ? (uint32_t)__ldg(static_cast<const uint8_t*>(p.dcode) + row)
+                                              : (uint32_t)__ldg(static_cast<const uint16_t*>(p.dcode) + row);
+    dr = __ldg(p.dtab + 2 * c);
+    di = __ldg(p.dtab + 2 * c + 1);
+}
+
+// FP32.  LZ: the Lanczos step's form (operands from *p.lz, y = scale H x -
+// bprev vprev, per-CTA partials of Re<x, y>).
+template <int MODE, bool CPLX, bool LZ, int NQ>
+__global__ void __launch_bounds__(kThreads, kCtas32)
+    pack32_kernel(const Params<float> p, const float2* __restrict__ x_in, float2* __restrict__ y_in) {
+    __shared__ float s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
+    if (MODE == AMP_CODED) load_amps(p, s_amp);
+    const float2* __restrict__ x = x_in;
+    float2* __restrict__ y = y_in;
+    float scale = 1.f, bprev = 0.f;
+    const float2* __restrict__ vprev = nullptr;
+    if (LZ) {
+        const LzOperands o = *p.lz;
+        x = static_cast<const float2*>(o.x);
+        y = static_cast<float2*>(o.y);
+        vprev = static_cast<const float2*>(o.vprev);
+        scale = o.scale32;
+        bprev = o.bprev32;
+    }
+    const uint32_t wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    const uint32_t id = NQ == 4 ? wid : wid >> 2, q0 = NQ == 4 ? 0u : wid & 3u;
+    float dot_hi = 0.f, dot_lo = 0.f;
+    if (id < p.n_items) {
+        const uint4 i4 = __ldg(reinterpret_cast<const uint4*>(p.items) + id);
+        const Item it{i4.x, i4.y, i4.z, i4.w};
+        SumF32 acc[NQ];
+        walk<float, SumF32, MODE, CPLX, NQ>(p, it, q0, x, s_amp, acc);
+        const uint32_t cnt = it.tc & 0xFFu;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            if (lane + 32u * (q0 + q) >= cnt) continue;
+            const uint32_t row = it.row0 + lane + 32u * (q0 + q);
+            float dr, di;
+            diag_at(p, row, dr, di);
+            const u64 xv = Elem<float>::load(x + row);
+            if (p.cdiag) acc[q].add(dr, di, xv);
+            else acc[q].add(dr, xv);
+            float2 o = unpair(acc[q].s);
+            if (LZ) {
+                o.x *= scale;
+                o.y *= scale;
+                if (vprev) {  // read once a step: evict-first, so x keeps more of L2
+                    const float2 pv = __ldcs(vprev + row);
+                    o.x = fmaf(-bprev, pv.x, o.x);
+                    o.y = fmaf(-bprev, pv.y, o.y);
+                }
+                const float2 xf = unpair(xv);
+                ffma_acc(dot_hi, dot_lo, xf.x, o.x);
+                ffma_acc(dot_hi, dot_lo, xf.y, o.y);
+            }
+            __stcs(y + row, o);
+        }
+    }
+    if (LZ) {
+        const float2 t = block_sum_ff(dot_hi, dot_lo);
+        if (threadIdx.x == 0) p.apart[blockIdx.x] = make_double2((double)t.x + (double)t.y, 0.0);
+    }
+}
+
+// FP64.  EQUAL: every amplitude has the same magnitude p.u (sums of aligned integers).
+template <int MODE, bool CPLX, bool EQUAL, int NQ>
+__global__ void __launch_bounds__(kThreads, kCtas64)
+    pack64_kernel(const Params<double> p, const double2* __restrict__ x, double2* __restrict__ y) {
+    __shared__ double s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
+    if (MODE == AMP_CODED) load_amps(p, s_amp);
+    const uint32_t wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    const uint32_t id = NQ == 4 ? wid : wid >> 2, q0 = NQ == 4 ? 0u : wid & 3u;
+    if (id >= p.n_items) return;
+    const uint4 i4 = __ldg(reinterpret_cast<const uint4*>(p.items) + id);
+    const Item it{i4.x, i4.y, i4.z, i4.w};
+    const uint32_t cnt = it.tc & 0xFFu;
+    double orr[NQ], oi[NQ];
+    bool redo = !EQUAL;
+    if constexpr (EQUAL) {
+        SumI64 acc[NQ];
+        walk<double, SumI64, MODE, false, NQ>(p, it, q0, x, s_amp, acc);
+        const double v = fabs(p.u) * 0x1p-56;
+        bool bad = false;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            bad = bad || (lane + 32u * (q0 + q) < cnt && acc[q].bad());
+            orr[q] = acc[q].r.value(v);
+            oi[q] = acc[q].i.value(v);
+        }
+        redo = __any_sync(0xffffffffu, bad);
+    }
+    if (redo) {
+        SumF64 acc[NQ];
+        walk<double, SumF64, MODE, CPLX, NQ>(p, it, q0, x, s_amp, acc);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            orr[q] = acc[q].r;
+            oi[q] = acc[q].i;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if (lane + 32u * (q0 + q) >= cnt) continue;
+        const uint32_t row = it.row0 + lane + 32u * (q0 + q);
+        double dr, di;
+        diag_at(p, row, dr, di);
+        const double2 xv = __ldg(x + row);
+        double2 o;
+        o.x = fma(dr, xv.x, orr[q]);
+        o.y = fma(dr, xv.y, oi[q]);
+        if (p.cdiag) {
+            o.x = fma(-di, xv.y, o.x);
+            o.y = fma(di, xv.x, o.y);
+        }
+        __stcs(y + row, o);
+    }
+}
+
+// Four warps a tile (NQ = 1) below 24 tiles a SM: one warp a tile leaves the
+// SMs short of loads in flight there, and pays for itself above, where the four
+// rows share the block's entries.  FP32 / FP64, one against four warps: L = 14
+// 6.3 / 12.3 against 4.3 / 6.2 us, L = 20 (1,700 tiles) 8.5 / 18.5 against 6.3 /
+// 12.6 us, L = 24 (21,500 tiles) 28.9 / 112.9 against 43.2 / 126.0 us.
+bool split_tiles(uint32_t n_items) { return n_items < 152u * 24u; }
+
+}  // namespace
+
+uint32_t pack_ctas(const PackPlan& P) {
+    const uint32_t n = P.n_items(), w = kThreads / 32;
+    return split_tiles(n) ? n : (n + w - 1) / w;
+}
+
+namespace {
+// go(mode, complex amplitudes, rows a lane) for the plan's form
+template <class F>
+void pick(const PackPlan& P, F&& go) {
+    using std::integral_constant;
+    auto rows = [&](auto mode, auto cplx) {
+        if (split_tiles(P.n_items())) go(mode, cplx, integral_constant<int, 1>{});
+        else go(mode, cplx, integral_constant<int, 4>{});
+    };
+    if (P.mode() == AMP_UNIFORM) rows(integral_constant<int, AMP_UNIFORM>{}, std::false_type{});
+    else if (P.mode() == AMP_SIGNED) rows(integral_constant<int, AMP_SIGNED>{}, std::false_type{});
+    else if (P.real()) rows(integral_constant<int, AMP_CODED>{}, std::false_type{});
+    else rows(integral_constant<int, AMP_CODED>{}, std::true_type{});
+}
+}  // namespace
+
+void pack_apply_f32(const PackPlan& P, Params<float>& p, const float2* x, float2* y, cudaStream_t s) {
+    if (!p.n_items) return;
+    const unsigned g = pack_ctas(P), t = kThreads;
+    pick(P, [&](auto m, auto c, auto nq) {
+        constexpr int M = decltype(m)::value, N = decltype(nq)::value;
+        constexpr bool C = decltype(c)::value;
+        if (p.lz) pack32_kernel<M, C, true, N><<<g, t, 0, s>>>(p, x, y);
+        else pack32_kernel<M, C, false, N><<<g, t, 0, s>>>(p, x, y);
+    });
+    QKG_LAUNCHED();
+}
+
+void pack_apply_f64(const PackPlan& P, Params<double>& p, const double2* x, double2* y, cudaStream_t s) {
+    if (!p.n_items) return;
+    const unsigned g = pack_ctas(P), t = kThreads;
+    pick(P, [&](auto m, auto c, auto nq) {
+        constexpr int M = decltype(m)::value, N = decltype(nq)::value;
+        constexpr bool C = decltype(c)::value;
+        if constexpr (M != AMP_CODED) {
+            if (P.equal_magnitude()) {
+                pack64_kernel<M, C, true, N><<<g, t, 0, s>>>(p, x, y);
+                return;
+            }
+        }
+        pack64_kernel<M, C, false, N><<<g, t, 0, s>>>(p, x, y);
+    });
+    QKG_LAUNCHED();
+}
+
+}  // namespace qkg
