@@ -26,6 +26,7 @@
 // first three are one CUDA graph of three steps (a full rotation) replayed,
 // with the step index in device memory.
 #include "block.hpp"
+#include "block_pack.cuh"
 #include "fast_common.cuh"
 #include "solvers.hpp"
 
@@ -446,6 +447,7 @@ template <class T, class A>
 class BlockEngine {
 public:
     using T2 = typename V2<T>::t;
+    static constexpr bool kCountsSteps = false;
     BlockEngine(const std::vector<Hamiltonian*>& hs, int Rp, int Ruser)
         : hs_(hs), Rp_(Rp), Ruser_(Ruser), ws_lock_(hs[0]->workspace_lock()) {
         s_ = hs[0]->stream();
@@ -494,7 +496,7 @@ public:
     size_t n_items() const { return n_items_; }
     T2* buf(int i) { return static_cast<T2*>(buf_[i]); }
 
-    void spmv(int vpl, const T2* x, T2* y, const double* scale, double* apart) {
+    void spmv(int vpl, const T2* x, T2* y, const double* scale, double* apart, int*) {
         const auto* P = params_.as<FastParams<A>>();
         const auto* it = items_.as<BItem>();
         const unsigned g = (unsigned)n_items_;
@@ -506,7 +508,7 @@ public:
 
     // Autotuner: time the block SpMV for each vectors-per-lane choice that
     // divides Rp (at most 32 lanes per row) and keep the fastest.
-    int autotune(std::vector<double>& rec) {
+    int choose_vpl(std::vector<double>& rec) {
         rec.assign(3, 0.0);
         int best = 0;
         double best_ms = 0.0;
@@ -516,9 +518,9 @@ public:
             const int vpl = 1 << vi;
             if (Rp_ % vpl || Rp_ / vpl > 32) continue;
             LaunchTimer tm(s_);
-            spmv(vpl, buf(0), buf(1), nullptr, nullptr);
+            spmv(vpl, buf(0), buf(1), nullptr, nullptr, nullptr);
             tm.start();
-            for (int r = 0; r < 2; ++r) spmv(vpl, buf(0), buf(1), nullptr, nullptr);
+            for (int r = 0; r < 2; ++r) spmv(vpl, buf(0), buf(1), nullptr, nullptr, nullptr);
             tm.stop();
             QKG_CUDA(cudaStreamSynchronize(s_));
             rec[vi] = tm.collect() * 1e3 / 2.0;
@@ -581,15 +583,213 @@ public:
     double* bpart() { return bpart_.as<double>(); }
 };
 
-template <class T, class A>
-BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, int Rp) {
+// The block engine on the packed plans (reference order throughout).
+template <class T>
+class PackedBlockEngine {
+public:
     using T2 = typename V2<T>::t;
+    static constexpr bool kCountsSteps = true;  // the SpMV advances the step counter
+    // whether every Hamiltonian has a plan for block vectors of this width, all of
+    // one amplitude form (a sector's plan may need a more general one than another's)
+    static bool usable(const std::vector<Hamiltonian*>& hs, int Rp) {
+        std::vector<const PackPlan*> p;
+        return plans(hs, Rp, p);
+    }
+    static bool plans(const std::vector<Hamiltonian*>& hs, int Rp, std::vector<const PackPlan*>& out) {
+        int form = packk::AMP_UNIFORM;
+        for (;;) {
+            int most = form;
+            out.clear();
+            for (auto* h : hs) {
+                if (h->dim() && !h->packed()) return false;
+                out.push_back(h->dim() ? h->block_plan(class_rows(Rp), (packk::AmpMode)form) : nullptr);
+                if (!h->dim()) continue;
+                if (!out.back()) return false;
+                most = std::max(most, (int)out.back()->mode());
+            }
+            bool same = true;
+            for (auto* p : out) same = same && (!p || p->mode() == most);
+            if (same) return true;
+            form = most;
+        }
+    }
+    // rows of the largest block aimed at
+    static uint32_t class_rows(int Rp) { return std::max<uint32_t>(8, kSlice / (uint32_t)(Rp * sizeof(T2))); }
+
+    PackedBlockEngine(const std::vector<Hamiltonian*>& hs, int Rp, int Ruser)
+        : hs_(hs), Rp_(Rp), Ruser_(Ruser), ws_lock_(hs[0]->workspace_lock()) {
+        s_ = hs[0]->stream();
+        std::vector<packk::Params<T>> P(hs.size());
+        std::vector<blockk::Tile> items;
+        std::vector<blockk::Cta> ctas;
+        std::vector<blockk::UpdItem> upd;
+        std::vector<uint32_t> range(1, 0), urange(1, 0);
+        std::vector<const uint32_t*> perms;
+        // a CTA's run of tiles: kPasses rows a row group, fewer where that would
+        // leave SMs without CTAs
+        uint64_t total = 0;
+        for (auto* h : hs) total += h->dim();
+        const uint32_t groups = blockk::kBT / std::max(1, Rp / (Rp % 4 == 0 ? 4 : Rp % 2 == 0 ? 2 : 1));
+        const uint32_t run = (uint32_t)std::max<uint64_t>(
+            blockk::kTile, std::min<uint64_t>((uint64_t)kPasses * groups, total / (152 * 4)) / blockk::kTile * blockk::kTile);
+        bool real = true;
+        std::vector<const PackPlan*> plan_of;
+        QKG_REQUIRE(plans(hs, Rp, plan_of), "batched Lanczos: no packed plan");
+        for (size_t h = 0; h < hs.size(); ++h) {
+            Hamiltonian& H = *hs[h];
+            QKG_REQUIRE(H.device() == hs[0]->device(), "batched Lanczos needs every Hamiltonian on one device");
+            QKG_CUDA(cudaStreamSynchronize(H.stream()));
+            perms.push_back(H.permutation());
+            if (H.dim()) {
+                const PackPlan& plan = *plan_of[h];
+                H.pack_params(P[h], plan);
+                real = real && plan.real();
+                mode_ = plan.mode();
+                uint32_t rows = 0;
+                for (const auto& t : plan.tiles()) {
+                    if (!rows || rows + blockk::kTile > run || ctas.back().count == (uint32_t)blockk::kMaxRun) {
+                        ctas.push_back({(uint32_t)items.size(), 0});
+                        rows = 0;
+                    }
+                    ++ctas.back().count;
+                    rows += blockk::kTile;  // a run walks whole tiles
+                    items.push_back({t.row0, t.a, t.tile, t.tc, (uint32_t)h, 0u, rows_});
+                }
+            }
+            range.push_back((uint32_t)ctas.size());
+            for (uint64_t r = 0; r < H.dim(); r += kUpdRows)
+                upd.push_back({rows_ + r, (uint32_t)std::min<uint64_t>(kUpdRows, H.dim() - r), (uint32_t)h});
+            urange.push_back((uint32_t)upd.size());
+            dims_.push_back(H.dim());
+            bases_.push_back(rows_);
+            rows_ += H.dim();
+        }
+        real_ = real;
+        n_ctas_ = ctas.size();
+        n_upd_ = upd.size();
+        auto up = [](DBuf& b, const auto& v) {
+            using E = typename std::decay_t<decltype(v)>::value_type;
+            b.alloc(std::max<size_t>(1, v.size()) * sizeof(E));
+            if (!v.empty()) QKG_CUDA(cudaMemcpy(b.p, v.data(), v.size() * sizeof(E), cudaMemcpyHostToDevice));
+        };
+        up(params_, P);
+        up(items_, items);
+        up(ctas_, ctas);
+        up(upd_, upd);
+        range.insert(range.end(), urange.begin(), urange.end());
+        up(range_, range);
+        up(perms_, perms);
+        up(dbases_, bases_);
+        // the three rotating block vectors live in the first Hamiltonian's
+        // Krylov workspace, kept between calls (freeing 13 GB costs milliseconds
+        // and fresh pages slow the first steps)
+        const size_t vbytes = (std::max<uint64_t>(1, rows_) * Rp * sizeof(T2) + 255) / 256 * 256;
+        char* ws = static_cast<char*>(hs[0]->krylov_workspace(3 * vbytes).p);
+        for (int i = 0; i < 3; ++i) {
+            buf_[i] = ws + (size_t)i * vbytes;
+            QKG_CUDA(cudaMemsetAsync(buf_[i], 0, vbytes, s_));
+        }
+        apart_.alloc(std::max<size_t>(1, n_ctas_) * Rp * sizeof(double));
+        bpart_.alloc(std::max<size_t>(1, n_upd_) * Rp * sizeof(double));
+    }
+
+    uint64_t rows() const { return rows_; }
+    T2* buf(int i) { return static_cast<T2*>(buf_[i]); }
+    cudaStream_t stream() const { return s_; }
+    double* apart() { return apart_.as<double>(); }
+    double* bpart() { return bpart_.as<double>(); }
+    // vectors per lane: 16-byte units, two of them where the width allows
+    int choose_vpl(std::vector<double>& rec) {
+        rec.assign(3, 0.0);
+        return Rp_ % 4 == 0 ? 4 : Rp_ % 2 == 0 ? 2 : 1;
+    }
+
+    void spmv(int vpl, const T2* x, T2* y, const double* scale, double* apart, int* kstep) {
+        if (!n_ctas_) return;
+        if (vpl == 4) spmv_v<4>(x, y, scale, apart, kstep);
+        else if (vpl == 2) spmv_v<2>(x, y, scale, apart, kstep);
+        else spmv_v<1>(x, y, scale, apart, kstep);
+    }
+    void update(const T2* u, const T2* up, T2* y, const double* ca, const double* cb, double* part) {
+        if (!n_upd_) return;
+        constexpr int W = sizeof(T) == 4 ? 2 : 1;
+        const auto* it = upd_.as<blockk::UpdItem>();
+        if (Rp_ % W == 0)
+            blockk::block_pack_update<T, W><<<(unsigned)n_upd_, blockk::kBT, 0, s_>>>(it, Rp_, y, u, up, ca, cb, part);
+        else
+            blockk::block_pack_update<T, 1><<<(unsigned)n_upd_, blockk::kBT, 0, s_>>>(it, Rp_, y, u, up, ca, cb, part);
+        QKG_LAUNCHED();
+    }
+    void finish(const double* part, int mode, const BState& st) {
+        const uint32_t* r = range_.as<uint32_t>() + (mode == FIN_ALPHA ? 0 : hs_.size() + 1);
+        block_finish_kernel<<<(unsigned)(hs_.size() * Rp_), kBlock, 0, s_>>>(part, r, mode, st);
+        QKG_LAUNCHED();
+    }
+    void philox(uint64_t seed, T2* u) {
+        if (!n_upd_) return;
+        int streams = 1;  // streams a Hamiltonian: the vectors padded to a power of two
+        while (streams < Ruser_) streams *= 2;
+        blockk::block_pack_philox<T2, sizeof(T) == 8><<<(unsigned)n_upd_, blockk::kBT, 0, s_>>>(
+            upd_.as<blockk::UpdItem>(), dbases_.as<uint64_t>(), static_cast<const uint32_t* const*>(perms_.p), Rp_, Ruser_,
+            streams, seed, u);
+        QKG_LAUNCHED();
+    }
+    // column v of Hamiltonian h from a reference-order host vector
+    void set_column(size_t h, int v, const cd* host_ref, DBuf& tmp, DBuf&, T2* u) {
+        const uint64_t n = dims_[h];
+        if (!n) return;
+        if (tmp.bytes < n * sizeof(double2)) tmp.alloc(n * sizeof(double2));
+        QKG_CUDA(cudaMemcpyAsync(tmp.p, host_ref, n * sizeof(double2), cudaMemcpyHostToDevice, s_));
+        const int g = (int)std::min<uint64_t>((n + 255) / 256, 152ull * 16);
+        block_column_kernel<T2><<<g, 256, 0, s_>>>(tmp.as<double2>(), n, Rp_, u + bases_[h] * Rp_ + v);
+        QKG_LAUNCHED();
+        QKG_CUDA(cudaStreamSynchronize(s_));  // host_ref may be reused by the caller
+    }
+
+private:
+    static constexpr uint32_t kSlice = 1200 * 1024;  // bytes of a block of x aimed at
+    static constexpr uint32_t kPasses = 8;
+    static constexpr uint32_t kUpdRows = 512;        // rows of an update CTA
+
+    template <int VPL>
+    void spmv_v(const T2* x, T2* y, const double* scale, double* apart, int* kstep) {
+        auto go = [&](auto mode, auto cplx) {
+            constexpr int M = decltype(mode)::value;
+            constexpr bool C = decltype(cplx)::value;
+            blockk::block_pack_kernel<T, M, C, VPL><<<(unsigned)n_ctas_, blockk::kBT, 0, s_>>>(
+                params_.as<packk::Params<T>>(), items_.as<blockk::Tile>(), ctas_.as<blockk::Cta>(), Rp_, x, y, scale, apart,
+                kstep);
+        };
+        using std::integral_constant;
+        if (mode_ == packk::AMP_UNIFORM) go(integral_constant<int, packk::AMP_UNIFORM>{}, std::false_type{});
+        else if (mode_ == packk::AMP_SIGNED) go(integral_constant<int, packk::AMP_SIGNED>{}, std::false_type{});
+        else if (real_) go(integral_constant<int, packk::AMP_CODED>{}, std::false_type{});
+        else go(integral_constant<int, packk::AMP_CODED>{}, std::true_type{});
+        QKG_LAUNCHED();
+    }
+
+    std::vector<Hamiltonian*> hs_;
+    int Rp_, Ruser_;
+    std::unique_lock<std::mutex> ws_lock_;  // the first Hamiltonian's workspace, held for the engine's life
+    cudaStream_t s_ = nullptr;
+    packk::AmpMode mode_ = packk::AMP_UNIFORM;
+    bool real_ = true;
+    uint64_t rows_ = 0;
+    size_t n_ctas_ = 0, n_upd_ = 0;
+    std::vector<uint64_t> dims_, bases_;
+    DBuf params_, items_, ctas_, upd_, range_, perms_, dbases_, apart_, bpart_;
+    void* buf_[3] = {nullptr, nullptr, nullptr};
+};
+
+template <class Engine>
+BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, int Rp) {
+    using T2 = typename Engine::T2;
     BlockTridiag out;
     out.n_ham = (int)hs.size();
     out.R = o.R;
     out.steps = o.steps;
     out.rp = Rp;
-    BlockEngine<T, A> E(hs, Rp, o.R);
+    Engine E(hs, Rp, o.R);
     cudaStream_t s = E.stream();
     out.rows = E.rows();
     const int V = out.n_ham * Rp;
@@ -600,6 +800,8 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
     QKG_CUDA(cudaMemsetAsync(scal.p, 0, scal.bytes, s));
     QKG_CUDA(cudaMemsetAsync(ab.p, 0, ab.bytes, s));
     QKG_CUDA(cudaMemsetAsync(ints.p, 0, ints.bytes, s));
+    if (Engine::kCountsSteps)  // the first SpMV makes it 0
+        QKG_CUDA(cudaMemsetAsync(ints.as<int>() + 3 * (size_t)V, 0xFF, sizeof(int), s));
     BState st;
     double* d = scal.as<double>();
     st.c_cur = d;
@@ -644,6 +846,7 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
     }
     // tile shape: autotuned once per batch of Hamiltonians, vector width and precision
     int vpl = o.vpl;
+    if (vpl <= 0 && Engine::kCountsSteps) vpl = E.choose_vpl(out.tune_ms);
     if (vpl <= 0) {
         static std::mutex mu;
         static std::map<std::vector<uintptr_t>, std::pair<int, std::vector<double>>> cache;
@@ -653,11 +856,11 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
             key.push_back((uintptr_t)h->dim());
         }
         key.push_back((uintptr_t)Rp);
-        key.push_back((uintptr_t)sizeof(T));
+        key.push_back((uintptr_t)sizeof(T2));
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
         if (it == cache.end()) {
-            vpl = E.autotune(out.tune_ms);
+            vpl = E.choose_vpl(out.tune_ms);
             cache[key] = {vpl, out.tune_ms};
         } else {
             vpl = it->second.first;
@@ -680,15 +883,17 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
         T2* up = E.buf((k + 2) % 3);
         T2* y = E.buf((k + 1) % 3);
         if (t) t->start();
-        E.spmv(vpl, u, y, st.c_cur, E.apart());
+        E.spmv(vpl, u, y, st.c_cur, E.apart(), st.kstep);
         if (t) t->stop();
         E.finish(E.apart(), FIN_ALPHA, st);
         E.update(u, up, y, st.ca, st.cb, E.bpart());
         E.finish(E.bpart(), FIN_BETA, st);
-        block_advance_kernel<<<1, 1, 0, s>>>(st.kstep);
-        QKG_LAUNCHED();
+        if (!Engine::kCountsSteps) {
+            block_advance_kernel<<<1, 1, 0, s>>>(st.kstep);
+            QKG_LAUNCHED();
+        }
     };
-    constexpr int kStepKernels = 5;  // SpMV, alpha finish, update, beta finish, step counter
+    constexpr int kStepKernels = Engine::kCountsSteps ? 4 : 5;  // SpMV, alpha finish, update, beta finish (, step counter)
     const int eager = std::min(M, 3);
     double sp_sum = 0.0;
     for (int k = 0; k < eager; ++k) {
@@ -762,12 +967,19 @@ BlockTridiag block_lanczos(const std::vector<Hamiltonian*>& hs, const BlockOpts&
     QKG_REQUIRE(o.steps >= 0, "negative step count");
     QKG_REQUIRE(o.start != BlockStart::Given || o.given.size() == hs.size() * (size_t)o.R, "start vector count");
     QKG_REQUIRE(o.vpl == 0 || o.vpl == 1 || o.vpl == 2 || o.vpl == 4, "vectors per lane must be 1, 2 or 4");
-    int Rp = 1;
+    // padded width: the packed engine takes any multiple of four above two
+    // vectors, the other one powers of two
+    int Rp = 1, Rq = o.R <= 2 ? o.R : (o.R + 3) / 4 * 4;
     while (Rp < o.R) Rp *= 2;
     int dev = 0;
     QKG_CUDA(cudaGetDevice(&dev));
     QKG_REQUIRE(dev == hs[0]->device(), "current device differs from the Hamiltonians' device");
-    return o.mixed ? run_block<float, float>(hs, o, Rp) : run_block<double, double>(hs, o, Rp);
+    if (o.mixed) {
+        if (PackedBlockEngine<float>::usable(hs, Rq)) return run_block<PackedBlockEngine<float>>(hs, o, Rq);
+        return run_block<BlockEngine<float, float>>(hs, o, Rp);
+    }
+    if (PackedBlockEngine<double>::usable(hs, Rq)) return run_block<PackedBlockEngine<double>>(hs, o, Rq);
+    return run_block<BlockEngine<double, double>>(hs, o, Rp);
 }
 
 void ftlm_observables_block(const BlockTridiag& t, const double* betas, int nb, double* Zo, double* Eo, double* Co,

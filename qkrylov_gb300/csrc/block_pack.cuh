@@ -1,0 +1,523 @@
+// Block SpMV on the packed plan (pack.hpp): y = diag(scale) H x for Rp
+// interleaved vectors of several Hamiltonians in one launch.
+//
+// A CTA takes a run of the plan's 128-row tiles.  G lanes share a row; lane l
+// holds the row's 16-byte units l, l + G, ... (a unit: two FP32 or one FP64
+// vector), so that the G lanes of a row read consecutive units: whole sectors and
+// whole 128-byte lines a load instruction.  A row's index work (its quads, its
+// ranks) is shared by its Rp values.
+#pragma once
+
+#include "pack.hpp"
+
+namespace qkg {
+namespace blockk {
+using namespace fastk;
+using namespace packk;
+using u64 = unsigned long long;
+
+constexpr int kBT = 256;       // threads of a CTA
+constexpr int kBatch = 4;      // outer entries loaded together
+constexpr int kMaxRun = 8;     // tiles of a CTA
+constexpr int kMaxList = 96;   // outer (and straddling) entries of its blocks staged in shared memory
+
+struct Tile {  // one tile of one Hamiltonian (Item with its Hamiltonian)
+    uint32_t row0, a, tile, tc, ham, pad;
+    uint64_t base;  // first row of its Hamiltonian in the block vector
+};
+struct Cta {  // consecutive tiles of one Hamiltonian
+    uint32_t first, count;
+};
+
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 pk(float x, float y) {
+    u64 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ float2 unpk(u64 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+constexpr u64 kMinusOne2 = 0xBF800000BF800000ull;  // (-1, -1)
+__device__ __forceinline__ u64 sub2(u64 a, u64 b) { return fma2(b, kMinusOne2, a); }  // a - b, rounded once
+// (hi, lo) += a * b elementwise, compensated (TwoProduct, TwoSum), both halves at once
+__device__ __forceinline__ void acc2(u64& hi, u64& lo, u64 a, u64 b) {
+    const u64 p = mul2(a, b);
+    const u64 e = fma2(a, b, mul2(p, kMinusOne2));
+    const u64 t = add2(hi, p);
+    const u64 z = sub2(t, hi);
+    const u64 err = add2(sub2(hi, sub2(t, z)), sub2(p, z));
+    lo = add2(lo, add2(err, e));
+    hi = t;
+}
+
+// p + a * b bytes (one 32 x 32 + 64 bit multiply-add)
+template <class E>
+__device__ __forceinline__ const E* offset(const E* p, int a, int b) {
+    return reinterpret_cast<const E*>(reinterpret_cast<const char*>(p) + (long long)a * (long long)b);
+}
+template <class E>
+__device__ __forceinline__ E* offset(E* p, int a, int b) {
+    return reinterpret_cast<E*>(reinterpret_cast<char*>(p) + (long long)a * (long long)b);
+}
+
+// A lane's values of one row: VPL complex values in units.
+// FP32: pairs (re, im) packed in 64 bits.
+template <class T, int VPL> struct Row;
+template <int VPL> struct Row<float, VPL> {
+    static constexpr int U = VPL >= 2 ? VPL / 2 : 1;  // units (VPL = 1: half a unit)
+    u64 v[VPL];
+    __device__ __forceinline__ void load(const float2* p, int G) {  // p: the lane's first unit
+        if constexpr (VPL == 1) {
+            v[0] = *reinterpret_cast<const u64*>(p);
+        } else {
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(p + 2 * j * G);
+                v[2 * j] = q.x;
+                v[2 * j + 1] = q.y;
+            }
+        }
+    }
+    __device__ __forceinline__ void store(float2* p, int G) const {
+        if constexpr (VPL == 1) {
+            __stcs(reinterpret_cast<u64*>(p), v[0]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+                __stcs(reinterpret_cast<ulonglong2*>(p + 2 * j * G), make_ulonglong2(v[2 * j], v[2 * j + 1]));
+        }
+    }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) v[j] = 0ull;
+    }
+    __device__ __forceinline__ void write(float2* p, int G) const {
+        if constexpr (VPL == 1) *reinterpret_cast<u64*>(p) = v[0];
+        else
+#pragma unroll
+            for (int j = 0; j < U; ++j) *reinterpret_cast<ulonglong2*>(p + 2 * j * G) = make_ulonglong2(v[2 * j], v[2 * j + 1]);
+    }
+    __device__ __forceinline__ void axpy(const float (&a)[VPL], const Row& x) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) v[j] = fma2(pk(a[j], a[j]), x.v[j], v[j]);
+    }
+    __device__ __forceinline__ void add(float a, const Row& x) {
+        const u64 aa = pk(a, a);
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) v[j] = fma2(aa, x.v[j], v[j]);
+    }
+    __device__ __forceinline__ void add(float ar, float ai, const Row& x) {
+        const u64 rr = pk(ar, ar), ii = pk(-ai, ai);
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            const float2 q = unpk(x.v[j]);
+            v[j] = fma2(ii, pk(q.y, q.x), fma2(rr, x.v[j], v[j]));
+        }
+    }
+};
+template <int VPL> struct Row<double, VPL> {
+    static constexpr int U = VPL;
+    double2 v[VPL];
+    __device__ __forceinline__ void load(const double2* p, int G) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) v[j] = p[j * G];
+    }
+    __device__ __forceinline__ void store(double2* p, int G) const {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) __stcs(p + j * G, v[j]);
+    }
+    __device__ __forceinline__ void write(double2* p, int G) const {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) p[j * G] = v[j];
+    }
+    __device__ __forceinline__ void axpy(const double (&a)[VPL], const Row& x) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            v[j].x = fma(a[j], x.v[j].x, v[j].x);
+            v[j].y = fma(a[j], x.v[j].y, v[j].y);
+        }
+    }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) v[j] = make_double2(0.0, 0.0);
+    }
+    __device__ __forceinline__ void add(double a, const Row& x) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            v[j].x = fma(a, x.v[j].x, v[j].x);
+            v[j].y = fma(a, x.v[j].y, v[j].y);
+        }
+    }
+    __device__ __forceinline__ void add(double ar, double ai, const Row& x) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            v[j].x = fma(-ai, x.v[j].y, fma(ar, x.v[j].x, v[j].x));
+            v[j].y = fma(ai, x.v[j].x, fma(ar, x.v[j].y, v[j].y));
+        }
+    }
+};
+// Vector of a lane's j-th value.
+template <class T, int VPL>
+__device__ __forceinline__ int vec_of(int l, int j, int G) {
+    if (sizeof(T) == 4 && VPL >= 2) return 2 * (l + (j / 2) * G) + (j & 1);
+    return l + j * G;
+}
+
+// Per-vector sums Re sum conj(x) y.
+template <class T, int VPL> struct Dots;
+template <int VPL> struct Dots<float, VPL> {
+    u64 hi[VPL], lo[VPL], sc[VPL];
+    __device__ __forceinline__ void init(int j, double scale) {
+        hi[j] = lo[j] = 0ull;
+        sc[j] = pk((float)scale, (float)scale);
+    }
+    __device__ __forceinline__ void finish(Row<float, VPL>& y, const Row<float, VPL>& x, bool dot) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            y.v[j] = mul2(y.v[j], sc[j]);
+            if (dot) acc2(hi[j], lo[j], x.v[j], y.v[j]);
+        }
+    }
+    __device__ __forceinline__ void square(const Row<float, VPL>& x) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) acc2(hi[j], lo[j], x.v[j], x.v[j]);
+    }
+    // (hi, lo) of vector j: real and imaginary products together
+    __device__ __forceinline__ double2 get(int j) const {
+        const float2 h = unpk(hi[j]), l = unpk(lo[j]);
+        float a = h.x, b = l.x;
+        ff_add(a, b, h.y, l.y);
+        double2 r;  // kept as a float pair in the two halves of one double's place
+        r.x = __hiloint2double(__float_as_int(a), __float_as_int(b));
+        r.y = 0.0;
+        return r;
+    }
+};
+template <int VPL> struct Dots<double, VPL> {
+    double s[VPL], sc[VPL];
+    __device__ __forceinline__ void init(int j, double scale) {
+        s[j] = 0.0;
+        sc[j] = scale;
+    }
+    __device__ __forceinline__ void finish(Row<double, VPL>& y, const Row<double, VPL>& x, bool dot) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            y.v[j].x *= sc[j];
+            y.v[j].y *= sc[j];
+            if (dot) s[j] = fma(x.v[j].y, y.v[j].y, fma(x.v[j].x, y.v[j].x, s[j]));
+        }
+    }
+    __device__ __forceinline__ void square(const Row<double, VPL>& x) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) s[j] = fma(x.v[j].y, x.v[j].y, fma(x.v[j].x, x.v[j].x, s[j]));
+    }
+    __device__ __forceinline__ double2 get(int j) const { return make_double2(s[j], 0.0); }
+};
+// Partial sums as the CTA adds them: FP32 as float pairs (a double-precision
+// reduction in every CTA would cost more than its rows on the narrow FP64 pipe).
+template <class T> struct Part;
+template <> struct Part<double> {
+    double s = 0.0;
+    __device__ __forceinline__ void add(double v) { s += v; }
+    __device__ __forceinline__ double pack() const { return s; }
+    __device__ __forceinline__ double value() const { return s; }
+};
+template <> struct Part<float> {
+    float hi = 0.f, lo = 0.f;
+    __device__ __forceinline__ void add(double v) {
+        ff_add(hi, lo, __int_as_float(__double2hiint(v)), __int_as_float(__double2loint(v)));
+    }
+    __device__ __forceinline__ double pack() const { return __hiloint2double(__float_as_int(hi), __float_as_int(lo)); }
+    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
+// part[v] = sum over the CTA's n_groups row groups of red[group * Rp + v], all
+// threads taking part (the caller has synchronised after writing red).
+template <class T>
+__device__ __forceinline__ void reduce_vectors(double* red, int n_groups, int Rp, double* part) {
+    const int v = threadIdx.x % Rp, s = threadIdx.x / Rp, ns = kBT / Rp;
+    Part<T> a;
+    if (s < ns)
+        for (int g = s; g < n_groups; g += ns) a.add(red[g * Rp + v]);
+    __syncthreads();
+    if (s < ns) red[s * Rp + v] = a.pack();
+    __syncthreads();
+    int n = ns < n_groups ? ns : n_groups;
+    while (n > 1) {  // halves onto each other
+        const int h = (n + 1) / 2;
+        if (s < n - h) {
+            a.add(red[(s + h) * Rp + v]);
+            red[s * Rp + v] = a.pack();
+        }
+        n = h;
+        __syncthreads();
+    }
+    if ((int)threadIdx.x < Rp) part[threadIdx.x] = a.value();  // s = 0
+}
+
+template <class T, int MODE, bool CPLX, int VPL>
+__global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
+    block_pack_kernel(const Params<T>* __restrict__ P, const Tile* __restrict__ tiles, const Cta* __restrict__ ctas, int Rp,
+                      const typename V2<T>::t* __restrict__ X, typename V2<T>::t* __restrict__ Y,
+                      const double* __restrict__ scale, double* __restrict__ apart, int* kstep) {
+    using T2 = typename V2<T>::t;
+    using R = Row<T, VPL>;
+    __shared__ double red[kBT * VPL];
+    __shared__ T s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
+    if (kstep && blockIdx.x == 0 && threadIdx.x == 0) ++*kstep;  // the step whose kernels follow
+    const Cta cta = ctas[blockIdx.x];
+    const uint32_t ham = tiles[cta.first].ham;
+    const Params<T>& p = P[ham];
+    if (MODE == AMP_CODED) {
+        for (int i = threadIdx.x; i < 2 * p.n_amps; i += kBT) s_amp[i] = p.amps[i];
+        __syncthreads();
+    }
+    const int G = Rp / VPL, NG = kBT / G;
+    const int l = threadIdx.x % G, grp = threadIdx.x / G;
+    constexpr int W0 = (sizeof(T) == 4 && VPL >= 2) ? 2 : 1;  // complex values of a unit
+    Dots<T, VPL> dots;
+#pragma unroll
+    for (int j = 0; j < VPL; ++j)
+        dots.init(j, scale ? scale[(size_t)ham * Rp + vec_of<T, VPL>(l, j, G)] : 1.0);
+    const T u = p.u;
+    const Out<T>* const g_out = p.out;
+    const Str<T>* const g_str = p.str;
+    const uint2* __restrict__ tab = p.tab;
+    const uint32_t* __restrict__ codes = p.codes;
+
+    // the run's tiles and their blocks' lists
+    __shared__ Tile s_tile[kMaxRun];
+    __shared__ uint4 s_blk[kMaxRun];
+    __shared__ uint2 s_rec[kMaxRun];
+    __shared__ Out<T> s_out[kMaxList];
+    __shared__ Str<T> s_str[kMaxList];
+    if (threadIdx.x < cta.count) {
+        const Tile t = tiles[cta.first + threadIdx.x];
+        s_tile[threadIdx.x] = t;
+        s_blk[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(p.blk) + t.a);
+        s_rec[threadIdx.x] = __ldg(p.tile + t.tile);
+    }
+    __syncthreads();
+    uint32_t lo = 0, ls = 0;  // list entries of the whole run
+    for (uint32_t i = 0; i < cta.count; ++i) {
+        lo += s_blk[i].y - s_blk[i].x;
+        ls += s_blk[i].w - s_blk[i].z;
+    }
+    const bool staged = lo <= (uint32_t)kMaxList && ls <= (uint32_t)kMaxList;
+    if (staged) {
+        uint32_t o = 0, q = 0;
+        for (uint32_t i = 0; i < cta.count; ++i) {
+            const uint4 b4 = s_blk[i];
+            if (threadIdx.x < b4.y - b4.x) s_out[o + threadIdx.x] = g_out[b4.x + threadIdx.x];
+            if (threadIdx.x < b4.w - b4.z) s_str[q + threadIdx.x] = g_str[b4.z + threadIdx.x];
+            o += b4.y - b4.x;
+            q += b4.w - b4.z;
+        }
+        __syncthreads();
+    }
+    const int rb = Rp * (int)sizeof(T2);  // bytes of a row
+    const T2* __restrict__ Xh = X + s_tile[0].base * (uint64_t)Rp + l * W0;  // the Hamiltonian's rows
+    T2* __restrict__ Yh = Y + s_tile[0].base * (uint64_t)Rp + l * W0;
+    {
+        uint32_t ti = 0, oo = 0, so = 0;  // the row's tile and where its lists start
+        if (grp < NG)
+            for (int rr = grp; rr < (int)cta.count * kTile; rr += NG) {
+                while (ti < (uint32_t)rr >> 7) {
+                    oo += s_blk[ti].y - s_blk[ti].x;
+                    so += s_blk[ti].w - s_blk[ti].z;
+                    ++ti;
+                }
+                const Tile& it = s_tile[ti];
+                const int r = rr & (kTile - 1);
+                if (r >= (int)(it.tc & 0xFFu)) continue;
+                const uint32_t lane = r & 31u, q = (uint32_t)r >> 5, tin = it.tc >> 8;
+                const uint4 b4 = s_blk[ti];
+                const uint2 rec = s_rec[ti];
+                const uint32_t no = b4.y - b4.x, ns = b4.w - b4.z;
+                const Out<T>* outl = staged ? s_out + oo : g_out + b4.x;
+                const Str<T>* strl = staged ? s_str + so : g_str + b4.z;
+                const uint32_t row = it.row0 + r;
+                const uint32_t dc = p.diag_mode == DIAG_U8 ? (uint32_t)__ldg(static_cast<const uint8_t*>(p.dcode) + row)
+                                                           : (uint32_t)__ldg(static_cast<const uint16_t*>(p.dcode) + row);
+                const T2* xo = offset(Xh, (int)row, rb);
+                const T2* xl = offset(Xh, (int)(it.row0 - tin * (uint32_t)kTile), rb);  // the block's rows
+                R acc;
+                acc.zero();
+                // outer entries, kBatch rows in flight
+                uint32_t k = 0;
+                for (; k + kBatch <= no; k += kBatch) {
+                    R v[kBatch];
+#pragma unroll
+                    for (int i = 0; i < kBatch; ++i) v[i].load(offset(xo, outl[k + i].delta, rb), G);
+#pragma unroll
+                    for (int i = 0; i < kBatch; ++i) {
+                        if (CPLX) acc.add(outl[k + i].ar, outl[k + i].ai, v[i]);
+                        else acc.add(outl[k + i].ar, v[i]);
+                    }
+                }
+                for (; k < no; ++k) {
+                    R v;
+                    v.load(offset(xo, outl[k].delta, rb), G);
+                    if (CPLX) acc.add(outl[k].ar, outl[k].ai, v);
+                    else acc.add(outl[k].ar, v);
+                }
+                uint32_t first = rec.x;
+                if (q > 0) first += ((rec.y & 0xFFu) + 3u) >> 2;
+                if (q > 1) first += (((rec.y >> 8) & 0xFFu) + 3u) >> 2;
+                if (q > 2) first += (((rec.y >> 16) & 0xFFu) + 3u) >> 2;
+                const int slots = (int)((rec.y >> (8 * q)) & 0xFFu);
+                uint32_t at = first * 32u + lane;
+                uint2 nxt = __ldg(tab + at);
+                uint32_t cn = MODE == AMP_CODED ? __ldg(codes + at) : 0u;
+                auto amp_add = [&](uint32_t w16, uint32_t code, T a, const R& v) {
+                    if (MODE == AMP_CODED) {
+                        const uint32_t c = code & 0xFFu;
+                        if (CPLX) acc.add(s_amp[2 * c], s_amp[2 * c + 1], v);
+                        else acc.add(s_amp[2 * c], v);
+                    } else {
+                        acc.add(MODE == AMP_SIGNED && (w16 & 0x8000u) ? -a : a, v);
+                    }
+                };
+                auto rank_of = [](uint32_t w16) { return (int)(MODE == AMP_SIGNED ? w16 & 0x7FFFu : w16); };
+                constexpr int kNone = MODE == AMP_SIGNED ? (int)kNone15 : (int)kNone16;
+                for (int n = slots; n > 0; n -= 4) {
+                    const uint2 e = nxt;
+                    const uint32_t c = cn;
+                    if (n > 4) {
+                        at += 32u;
+                        nxt = __ldg(tab + at);
+                        if (MODE == AMP_CODED) cn = __ldg(codes + at);
+                    }
+                    // a row's entries fill its first slots
+                    const uint32_t w[4] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16};
+#pragma unroll
+                    for (int h = 0; h < 4; h += 2) {
+                        const int r0 = rank_of(w[h]), r1 = rank_of(w[h + 1]);
+                        if (r0 == kNone) break;
+                        R v0, v1;
+                        v0.load(offset(xl, r0, rb), G);
+                        if (r1 != kNone) v1.load(offset(xl, r1, rb), G);
+                        amp_add(w[h], c >> (8 * h), u, v0);
+                        if (r1 != kNone) amp_add(w[h + 1], c >> (8 * h + 8), u, v1);
+                    }
+                }
+                for (uint32_t j = 0; j < ns; ++j) {
+                    const Str<T> s = strl[j];
+                    const uint32_t as = s.tab + tin * 32u + lane;
+                    const uint2 e = __ldg(tab + as);
+                    const uint32_t w = (q & 2u) ? e.y : e.x, w16 = (q & 1u) ? w >> 16 : w & 0xFFFFu;
+                    const uint32_t c = MODE == AMP_CODED ? __ldg(codes + as) >> (8 * q) : 0u;
+                    const int to = rank_of(w16);
+                    if (to == kNone) continue;
+                    R v;
+                    v.load(offset(Xh, (int)s.off + to, rb), G);
+                    amp_add(w16, c, s.ar, v);
+                }
+                R x;
+                x.load(xo, G);
+                const T dr = __ldg(p.dtab + 2 * dc);
+                if (p.cdiag) acc.add(dr, __ldg(p.dtab + 2 * dc + 1), x);
+                else acc.add(dr, x);
+                dots.finish(acc, x, apart != nullptr);
+                acc.store(offset(Yh, (int)row, rb), G);
+            }
+    }
+    if (apart) {
+        if (grp < NG)
+#pragma unroll
+            for (int j = 0; j < VPL; ++j) red[grp * Rp + vec_of<T, VPL>(l, j, G)] = dots.get(j).x;
+        __syncthreads();
+        reduce_vectors<T>(red, NG, Rp, apart + (size_t)blockIdx.x * Rp);
+    }
+}
+
+// w = y - ca u - cb up in place on y, and per CTA the partial ||w_v||^2 (u ==
+// nullptr: only the norms of y).  A CTA takes `count` rows of one Hamiltonian;
+// NU lanes a row, one 16-byte unit (VPL values) each.
+struct UpdItem {
+    uint64_t row0;  // in the block vector
+    uint32_t count, ham;
+};
+template <class T, int VPL>
+__global__ void __launch_bounds__(kBT)
+    block_pack_update(const UpdItem* __restrict__ items, int Rp, typename V2<T>::t* __restrict__ Y,
+                      const typename V2<T>::t* __restrict__ U, const typename V2<T>::t* __restrict__ Up,
+                      const double* __restrict__ ca, const double* __restrict__ cb, double* __restrict__ part) {
+    using R = Row<T, VPL>;
+    __shared__ double red[kBT * VPL];
+    const UpdItem it = items[blockIdx.x];
+    const int G = Rp / VPL, NG = kBT / G;
+    const int l = threadIdx.x % G, grp = threadIdx.x / G;
+    Dots<T, VPL> dots;
+    T a[VPL], b[VPL];
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+        const size_t vid = (size_t)it.ham * Rp + vec_of<T, VPL>(l, j, G);
+        dots.init(j, 1.0);
+        a[j] = U ? -(T)ca[vid] : (T)0;
+        b[j] = U ? -(T)cb[vid] : (T)0;
+    }
+    const uint64_t o = it.row0 * (uint64_t)Rp + l * VPL;
+    if (grp < NG) {
+#pragma unroll 4
+        for (uint32_t r = grp; r < it.count; r += NG) {
+            const uint64_t at = o + (uint64_t)r * Rp;
+            R w;
+            w.load(Y + at, G);
+            if (U) {
+                R u, v;
+                u.load(U + at, G);
+                v.load(Up + at, G);
+                w.axpy(a, u);
+                w.axpy(b, v);
+                w.write(Y + at, G);
+            }
+            dots.square(w);
+        }
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) red[grp * Rp + vec_of<T, VPL>(l, j, G)] = dots.get(j).x;
+    }
+    __syncthreads();
+    reduce_vectors<T>(red, NG, Rp, part + (size_t)blockIdx.x * Rp);
+}
+
+// Seeded Philox Gaussian start vectors in reference order: vector v of
+// Hamiltonian h, element i of its basis' internal order (at row perm[i]), gets
+// the Philox block (counter i, stream h * streams + v); padding vectors are zero.
+template <class T2, bool F64>
+__global__ void __launch_bounds__(kBT)
+    block_pack_philox(const UpdItem* __restrict__ items, const uint64_t* __restrict__ bases,
+                      const uint32_t* const* __restrict__ perms, int Rp, int Ruser, int streams, uint64_t seed,
+                      T2* __restrict__ U) {
+    const UpdItem it = items[blockIdx.x];
+    const uint64_t base = bases[it.ham];
+    const uint32_t* __restrict__ perm = perms[it.ham];
+    const uint32_t i0 = (uint32_t)(it.row0 - base);
+    for (uint32_t e = threadIdx.x; e < it.count * (uint32_t)Rp; e += kBT) {
+        const uint32_t i = i0 + e / Rp, v = e % Rp;
+        T2 o;
+        o.x = 0;
+        o.y = 0;
+        if ((int)v < Ruser) o = philox_cnormal<T2, F64>(seed, (uint64_t)it.ham * streams + v, i);
+        U[(base + (perm ? perm[i] : i)) * (uint64_t)Rp + v] = o;
+    }
+}
+
+}  // namespace blockk
+}  // namespace qkg

@@ -112,11 +112,8 @@ struct PackTables {
 // Their device copies.
 class PackPlan {
 public:
-    struct Block {  // one block: its rows and first inner tile
-        uint32_t row0, a, tile, rows;
-    };
     explicit PackPlan(const PackTables& t);
-    const std::vector<Block>& blocks() const { return blocks_; }  // in launch order
+    const std::vector<packk::Item>& tiles() const { return tiles_; }
     packk::AmpMode mode() const { return mode_; }
     bool real() const { return real_; }
     bool equal_magnitude() const { return equal_; }
@@ -127,7 +124,7 @@ private:
     bool real_ = true, equal_ = false;
     packk::AmpMode mode_ = packk::AMP_UNIFORM;
     uint32_t n_items_ = 0;
-    std::vector<Block> blocks_;
+    std::vector<packk::Item> tiles_;
     int n_amps_ = 0;
     double u_ = 0.0;
     DBuf all_;  // the tables, one after the other

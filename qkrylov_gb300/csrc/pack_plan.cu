@@ -517,10 +517,7 @@ void PackTables::apply_host(const cd* x, cd* y) const {
 
 PackPlan::PackPlan(const PackTables& t)
     : real_(t.real), equal_(t.equal), mode_(t.mode), n_items_((uint32_t)t.items.size()), n_amps_((int)t.codes.size() ? (int)t.amps.size() : 0), u_(t.u) {
-    for (const Item& it : t.items) {
-        if ((it.tc >> 8) == 0) blocks_.push_back({it.row0, it.a, it.tile, 0});
-        blocks_.back().rows += it.tc & 0xFFu;
-    }
+    tiles_ = t.items;
     std::vector<char> image;
     items_ = append(image, t.items);
     blk_ = append(image, t.blk);
