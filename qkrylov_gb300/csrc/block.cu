@@ -447,7 +447,6 @@ template <class T, class A>
 class BlockEngine {
 public:
     using T2 = typename V2<T>::t;
-    static constexpr bool kCountsSteps = false;
     BlockEngine(const std::vector<Hamiltonian*>& hs, int Rp, int Ruser)
         : hs_(hs), Rp_(Rp), Ruser_(Ruser), ws_lock_(hs[0]->workspace_lock()) {
         s_ = hs[0]->stream();
@@ -496,7 +495,7 @@ public:
     size_t n_items() const { return n_items_; }
     T2* buf(int i) { return static_cast<T2*>(buf_[i]); }
 
-    void spmv(int vpl, const T2* x, T2* y, const double* scale, double* apart, int*) {
+    void spmv(int vpl, const T2* x, T2* y, const double* scale, double* apart) {
         const auto* P = params_.as<FastParams<A>>();
         const auto* it = items_.as<BItem>();
         const unsigned g = (unsigned)n_items_;
@@ -508,7 +507,7 @@ public:
 
     // Autotuner: time the block SpMV for each vectors-per-lane choice that
     // divides Rp (at most 32 lanes per row) and keep the fastest.
-    int choose_vpl(std::vector<double>& rec) {
+    int autotune(std::vector<double>& rec) {
         rec.assign(3, 0.0);
         int best = 0;
         double best_ms = 0.0;
@@ -518,9 +517,9 @@ public:
             const int vpl = 1 << vi;
             if (Rp_ % vpl || Rp_ / vpl > 32) continue;
             LaunchTimer tm(s_);
-            spmv(vpl, buf(0), buf(1), nullptr, nullptr, nullptr);
+            spmv(vpl, buf(0), buf(1), nullptr, nullptr);
             tm.start();
-            for (int r = 0; r < 2; ++r) spmv(vpl, buf(0), buf(1), nullptr, nullptr, nullptr);
+            for (int r = 0; r < 2; ++r) spmv(vpl, buf(0), buf(1), nullptr, nullptr);
             tm.stop();
             QKG_CUDA(cudaStreamSynchronize(s_));
             rec[vi] = tm.collect() * 1e3 / 2.0;
@@ -583,121 +582,85 @@ public:
     double* bpart() { return bpart_.as<double>(); }
 };
 
-// The block engine on the packed plans (reference order throughout).
+// The block engine on the packed plans (reference order throughout).  Its
+// vectors, scalars and partial sums live in the first Hamiltonian's Krylov
+// workspace, kept between calls (freeing 13 GB costs milliseconds and fresh pages
+// slow the first steps).
 template <class T>
 class PackedBlockEngine {
 public:
     using T2 = typename V2<T>::t;
-    static constexpr bool kCountsSteps = true;  // the SpMV advances the step counter
-    // whether every Hamiltonian has a plan for block vectors of this width, all of
-    // one amplitude form (a sector's plan may need a more general one than another's)
-    static bool usable(const std::vector<Hamiltonian*>& hs, int Rp) {
+    // whether every Hamiltonian has a plan, all of one amplitude form (a sector's plan
+    // may need a more general one than another's)
+    static bool usable(const std::vector<Hamiltonian*>& hs) {
         std::vector<const PackPlan*> p;
-        return plans(hs, Rp, p);
+        return plans(hs, p);
     }
-    static bool plans(const std::vector<Hamiltonian*>& hs, int Rp, std::vector<const PackPlan*>& out) {
-        int form = packk::AMP_UNIFORM;
-        for (;;) {
-            int most = form;
-            out.clear();
-            for (auto* h : hs) {
-                if (h->dim() && !h->packed()) return false;
-                out.push_back(h->dim() ? h->block_plan(class_rows(Rp), (packk::AmpMode)form) : nullptr);
-                if (!h->dim()) continue;
-                if (!out.back()) return false;
-                most = std::max(most, (int)out.back()->mode());
-            }
-            bool same = true;
-            for (auto* p : out) same = same && (!p || p->mode() == most);
-            if (same) return true;
-            form = most;
-        }
-    }
-    // rows of the largest block aimed at
-    static uint32_t class_rows(int Rp) { return std::max<uint32_t>(8, kSlice / (uint32_t)(Rp * sizeof(T2))); }
 
-    PackedBlockEngine(const std::vector<Hamiltonian*>& hs, int Rp, int Ruser)
+    PackedBlockEngine(const std::vector<Hamiltonian*>& hs, int Rp, int Ruser, size_t extra)
         : hs_(hs), Rp_(Rp), Ruser_(Ruser), ws_lock_(hs[0]->workspace_lock()) {
         s_ = hs[0]->stream();
-        std::vector<packk::Params<T>> P(hs.size());
-        std::vector<blockk::Tile> items;
-        std::vector<blockk::Cta> ctas;
-        std::vector<blockk::UpdItem> upd;
-        std::vector<uint32_t> range(1, 0), urange(1, 0);
-        std::vector<const uint32_t*> perms;
-        // a CTA's run of tiles: kPasses rows a row group, fewer where that would
-        // leave SMs without CTAs
+        std::vector<const PackPlan*> plan_of;
+        QKG_REQUIRE(plans(hs, plan_of), "batched Lanczos: no packed plan");
         uint64_t total = 0;
         for (auto* h : hs) total += h->dim();
+        // a CTA's run of tiles: kPasses rows a row group, fewer where that would
+        // leave SMs without CTAs
         const uint32_t groups = blockk::kBT / std::max(1, Rp / (Rp % 4 == 0 ? 4 : Rp % 2 == 0 ? 2 : 1));
-        const uint32_t run = (uint32_t)std::max<uint64_t>(
-            blockk::kTile, std::min<uint64_t>((uint64_t)kPasses * groups, total / (152 * 4)) / blockk::kTile * blockk::kTile);
-        bool real = true;
-        std::vector<const PackPlan*> plan_of;
-        QKG_REQUIRE(plans(hs, Rp, plan_of), "batched Lanczos: no packed plan");
+        run_ = (int)std::max<uint64_t>(1, std::min<uint64_t>({(uint64_t)kPasses * groups / blockk::kTile,
+                                                              total / (152 * 4) / blockk::kTile, blockk::kMaxRun}));
+        std::vector<packk::Params<T>> P(hs.size());
+        std::vector<blockk::Ham> hams(hs.size());
+        std::vector<uint32_t> range(1, 0), rrange(1, 0);
         for (size_t h = 0; h < hs.size(); ++h) {
             Hamiltonian& H = *hs[h];
             QKG_REQUIRE(H.device() == hs[0]->device(), "batched Lanczos needs every Hamiltonian on one device");
-            QKG_CUDA(cudaStreamSynchronize(H.stream()));
-            perms.push_back(H.permutation());
+            if (h) QKG_CUDA(cudaStreamSynchronize(H.stream()));
+            hams[h] = {rows_, H.dim(), range.back(), rrange.back(), H.permutation()};
+            uint32_t n = 0;
             if (H.dim()) {
-                const PackPlan& plan = *plan_of[h];
-                H.pack_params(P[h], plan);
-                real = real && plan.real();
-                mode_ = plan.mode();
-                uint32_t rows = 0;
-                for (const auto& t : plan.tiles()) {
-                    if (!rows || rows + blockk::kTile > run || ctas.back().count == (uint32_t)blockk::kMaxRun) {
-                        ctas.push_back({(uint32_t)items.size(), 0});
-                        rows = 0;
-                    }
-                    ++ctas.back().count;
-                    rows += blockk::kTile;  // a run walks whole tiles
-                    items.push_back({t.row0, t.a, t.tile, t.tc, (uint32_t)h, 0u, rows_});
-                }
+                H.pack_params(P[h], *plan_of[h]);
+                real_ = real_ && plan_of[h]->real();
+                mode_ = plan_of[h]->mode();
+                n = (plan_of[h]->n_items() + run_ - 1) / run_;
+            } else {
+                std::memset(&P[h], 0, sizeof(P[h]));
             }
-            range.push_back((uint32_t)ctas.size());
-            for (uint64_t r = 0; r < H.dim(); r += kUpdRows)
-                upd.push_back({rows_ + r, (uint32_t)std::min<uint64_t>(kUpdRows, H.dim() - r), (uint32_t)h});
-            urange.push_back((uint32_t)upd.size());
-            dims_.push_back(H.dim());
-            bases_.push_back(rows_);
+            range.push_back(range.back() + n);
+            rrange.push_back(rrange.back() + (uint32_t)((H.dim() + blockk::kRowChunk - 1) / blockk::kRowChunk));
             rows_ += H.dim();
         }
-        real_ = real;
-        n_ctas_ = ctas.size();
-        n_upd_ = upd.size();
-        auto up = [](DBuf& b, const auto& v) {
-            using E = typename std::decay_t<decltype(v)>::value_type;
-            b.alloc(std::max<size_t>(1, v.size()) * sizeof(E));
-            if (!v.empty()) QKG_CUDA(cudaMemcpy(b.p, v.data(), v.size() * sizeof(E), cudaMemcpyHostToDevice));
-        };
-        up(params_, P);
-        up(items_, items);
-        up(ctas_, ctas);
-        up(upd_, upd);
-        range.insert(range.end(), urange.begin(), urange.end());
-        up(range_, range);
-        up(perms_, perms);
-        up(dbases_, bases_);
-        // the three rotating block vectors live in the first Hamiltonian's
-        // Krylov workspace, kept between calls (freeing 13 GB costs milliseconds
-        // and fresh pages slow the first steps)
-        const size_t vbytes = (std::max<uint64_t>(1, rows_) * Rp * sizeof(T2) + 255) / 256 * 256;
-        char* ws = static_cast<char*>(hs[0]->krylov_workspace(3 * vbytes).p);
-        for (int i = 0; i < 3; ++i) {
-            buf_[i] = ws + (size_t)i * vbytes;
-            QKG_CUDA(cudaMemsetAsync(buf_[i], 0, vbytes, s_));
-        }
-        apart_.alloc(std::max<size_t>(1, n_ctas_) * Rp * sizeof(double));
-        bpart_.alloc(std::max<size_t>(1, n_upd_) * Rp * sizeof(double));
+        n_ctas_ = range.back();
+        n_row_ctas_ = rrange.back();
+        range.insert(range.end(), rrange.begin(), rrange.end());
+        // the workspace: three vectors, then everything else, 256-byte aligned
+        auto al = [](size_t b) { return (b + 255) / 256 * 256; };
+        const size_t vbytes = al(std::max<uint64_t>(1, rows_) * Rp * sizeof(T2));
+        const size_t pb = al(P.size() * sizeof(P[0])), hb = al(hams.size() * sizeof(hams[0])), rb = al(range.size() * 4);
+        const size_t ab = al(std::max<size_t>(1, n_ctas_) * Rp * 8), bb = al(std::max<size_t>(1, n_row_ctas_) * Rp * 8);
+        char* ws = static_cast<char*>(hs[0]->krylov_workspace(3 * vbytes + pb + hb + rb + ab + bb + al(extra)).p);
+        for (int i = 0; i < 3; ++i) buf_[i] = ws + (size_t)i * vbytes;
+        char* q = ws + 3 * vbytes;
+        std::vector<char> image(pb + hb + rb);
+        std::memcpy(image.data(), P.data(), P.size() * sizeof(P[0]));
+        std::memcpy(image.data() + pb, hams.data(), hams.size() * sizeof(hams[0]));
+        std::memcpy(image.data() + pb + hb, range.data(), range.size() * 4);
+        QKG_CUDA(cudaMemcpyAsync(q, image.data(), image.size(), cudaMemcpyHostToDevice, s_));  // pageable: copied on return
+        params_ = reinterpret_cast<packk::Params<T>*>(q);
+        hams_ = reinterpret_cast<blockk::Ham*>(q + pb);
+        range_ = reinterpret_cast<uint32_t*>(q + pb + hb);
+        apart_ = reinterpret_cast<double*>(q + pb + hb + rb);
+        bpart_ = reinterpret_cast<double*>(q + pb + hb + rb + ab);
+        extra_ = q + pb + hb + rb + ab + bb;
+        for (size_t h = 0; h < hs.size(); ++h) bases_.push_back(hams[h].base);
     }
 
     uint64_t rows() const { return rows_; }
     T2* buf(int i) { return static_cast<T2*>(buf_[i]); }
     cudaStream_t stream() const { return s_; }
-    double* apart() { return apart_.as<double>(); }
-    double* bpart() { return bpart_.as<double>(); }
+    double* apart() { return apart_; }
+    double* bpart() { return bpart_; }
+    void* extra() { return extra_; }
     // vectors per lane: 16-byte units, two of them where the width allows
     int choose_vpl(std::vector<double>& rec) {
         rec.assign(3, 0.0);
@@ -711,54 +674,73 @@ public:
         else spmv_v<1>(x, y, scale, apart, kstep);
     }
     void update(const T2* u, const T2* up, T2* y, const double* ca, const double* cb, double* part) {
-        if (!n_upd_) return;
+        if (!n_row_ctas_) return;
         constexpr int W = sizeof(T) == 4 ? 2 : 1;
-        const auto* it = upd_.as<blockk::UpdItem>();
         if (Rp_ % W == 0)
-            blockk::block_pack_update<T, W><<<(unsigned)n_upd_, blockk::kBT, 0, s_>>>(it, Rp_, y, u, up, ca, cb, part);
+            blockk::block_pack_update<T, W><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), Rp_, y, u, up, ca, cb, part);
         else
-            blockk::block_pack_update<T, 1><<<(unsigned)n_upd_, blockk::kBT, 0, s_>>>(it, Rp_, y, u, up, ca, cb, part);
+            blockk::block_pack_update<T, 1><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), Rp_, y, u, up, ca, cb, part);
         QKG_LAUNCHED();
     }
     void finish(const double* part, int mode, const BState& st) {
-        const uint32_t* r = range_.as<uint32_t>() + (mode == FIN_ALPHA ? 0 : hs_.size() + 1);
+        const uint32_t* r = range_ + (mode == FIN_ALPHA ? 0 : hs_.size() + 1);
         block_finish_kernel<<<(unsigned)(hs_.size() * Rp_), kBlock, 0, s_>>>(part, r, mode, st);
         QKG_LAUNCHED();
     }
     void philox(uint64_t seed, T2* u) {
-        if (!n_upd_) return;
+        if (!n_row_ctas_) return;
         int streams = 1;  // streams a Hamiltonian: the vectors padded to a power of two
         while (streams < Ruser_) streams *= 2;
-        blockk::block_pack_philox<T2, sizeof(T) == 8><<<(unsigned)n_upd_, blockk::kBT, 0, s_>>>(
-            upd_.as<blockk::UpdItem>(), dbases_.as<uint64_t>(), static_cast<const uint32_t* const*>(perms_.p), Rp_, Ruser_,
-            streams, seed, u);
+        blockk::block_pack_philox<T2, sizeof(T) == 8><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), Rp_, Ruser_,
+                                                                                          streams, seed, u);
         QKG_LAUNCHED();
     }
-    // column v of Hamiltonian h from a reference-order host vector
-    void set_column(size_t h, int v, const cd* host_ref, DBuf& tmp, DBuf&, T2* u) {
-        const uint64_t n = dims_[h];
-        if (!n) return;
-        if (tmp.bytes < n * sizeof(double2)) tmp.alloc(n * sizeof(double2));
-        QKG_CUDA(cudaMemcpyAsync(tmp.p, host_ref, n * sizeof(double2), cudaMemcpyHostToDevice, s_));
-        const int g = (int)std::min<uint64_t>((n + 255) / 256, 152ull * 16);
-        block_column_kernel<T2><<<g, 256, 0, s_>>>(tmp.as<double2>(), n, Rp_, u + bases_[h] * Rp_ + v);
+    // start vector v of Hamiltonian h (reference order, on the host; null: zero) into
+    // the staging memory, which is that of the two other vectors: R pairs of doubles a
+    // row fit there in either precision
+    void stage_column(size_t h, int v, const cd* host_ref) {
+        const uint64_t n = hs_[h]->dim();
+        double2* st = static_cast<double2*>(buf_[1]) + (size_t)v * n;
+        if (host_ref) QKG_CUDA(cudaMemcpyAsync(st, host_ref, n * sizeof(double2), cudaMemcpyHostToDevice, s_));
+        else QKG_CUDA(cudaMemsetAsync(st, 0, n * sizeof(double2), s_));
+    }
+    // the staged vectors of Hamiltonian h into its rows of u
+    void gather_columns(size_t h, T2* u) {
+        const uint64_t n = hs_[h]->dim();
+        blockk::block_pack_gather<T2><<<(unsigned)((n + 31) / 32), blockk::kBT, 0, s_>>>(
+            static_cast<const double2*>(buf_[1]), n, Ruser_, Rp_, u + bases_[h] * Rp_);
         QKG_LAUNCHED();
-        QKG_CUDA(cudaStreamSynchronize(s_));  // host_ref may be reused by the caller
     }
 
 private:
-    static constexpr uint32_t kSlice = 1200 * 1024;  // bytes of a block of x aimed at
     static constexpr uint32_t kPasses = 8;
-    static constexpr uint32_t kUpdRows = 512;        // rows of an update CTA
+
+    static bool plans(const std::vector<Hamiltonian*>& hs, std::vector<const PackPlan*>& out) {
+        int form = packk::AMP_UNIFORM;
+        for (;;) {
+            int most = form;
+            out.clear();
+            for (auto* h : hs) {
+                if (h->dim() && !h->packed()) return false;
+                out.push_back(h->dim() ? h->plan_of_form(form) : nullptr);
+                if (!h->dim()) continue;
+                if (!out.back()) return false;
+                most = std::max(most, (int)out.back()->mode());
+            }
+            bool same = true;
+            for (auto* p : out) same = same && (!p || p->mode() == most);
+            if (same) return true;
+            form = most;
+        }
+    }
 
     template <int VPL>
     void spmv_v(const T2* x, T2* y, const double* scale, double* apart, int* kstep) {
         auto go = [&](auto mode, auto cplx) {
             constexpr int M = decltype(mode)::value;
             constexpr bool C = decltype(cplx)::value;
-            blockk::block_pack_kernel<T, M, C, VPL><<<(unsigned)n_ctas_, blockk::kBT, 0, s_>>>(
-                params_.as<packk::Params<T>>(), items_.as<blockk::Tile>(), ctas_.as<blockk::Cta>(), Rp_, x, y, scale, apart,
-                kstep);
+            blockk::block_pack_kernel<T, M, C, VPL><<<n_ctas_, blockk::kBT, 0, s_>>>(params_, hams_, (int)hs_.size(), run_, Rp_,
+                                                                                    x, y, scale, apart, kstep);
         };
         using std::integral_constant;
         if (mode_ == packk::AMP_UNIFORM) go(integral_constant<int, packk::AMP_UNIFORM>{}, std::false_type{});
@@ -769,27 +751,31 @@ private:
     }
 
     std::vector<Hamiltonian*> hs_;
-    int Rp_, Ruser_;
+    int Rp_, Ruser_, run_ = 1;
     std::unique_lock<std::mutex> ws_lock_;  // the first Hamiltonian's workspace, held for the engine's life
     cudaStream_t s_ = nullptr;
     packk::AmpMode mode_ = packk::AMP_UNIFORM;
     bool real_ = true;
     uint64_t rows_ = 0;
-    size_t n_ctas_ = 0, n_upd_ = 0;
-    std::vector<uint64_t> dims_, bases_;
-    DBuf params_, items_, ctas_, upd_, range_, perms_, dbases_, apart_, bpart_;
+    unsigned n_ctas_ = 0, n_row_ctas_ = 0;
+    std::vector<uint64_t> bases_;
+    packk::Params<T>* params_ = nullptr;
+    blockk::Ham* hams_ = nullptr;
+    uint32_t* range_ = nullptr;
+    double *apart_ = nullptr, *bpart_ = nullptr;
+    void* extra_ = nullptr;
     void* buf_[3] = {nullptr, nullptr, nullptr};
 };
 
-template <class Engine>
+template <class T, class A>
 BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, int Rp) {
-    using T2 = typename Engine::T2;
+    using T2 = typename V2<T>::t;
     BlockTridiag out;
     out.n_ham = (int)hs.size();
     out.R = o.R;
     out.steps = o.steps;
     out.rp = Rp;
-    Engine E(hs, Rp, o.R);
+    BlockEngine<T, A> E(hs, Rp, o.R);
     cudaStream_t s = E.stream();
     out.rows = E.rows();
     const int V = out.n_ham * Rp;
@@ -800,8 +786,6 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
     QKG_CUDA(cudaMemsetAsync(scal.p, 0, scal.bytes, s));
     QKG_CUDA(cudaMemsetAsync(ab.p, 0, ab.bytes, s));
     QKG_CUDA(cudaMemsetAsync(ints.p, 0, ints.bytes, s));
-    if (Engine::kCountsSteps)  // the first SpMV makes it 0
-        QKG_CUDA(cudaMemsetAsync(ints.as<int>() + 3 * (size_t)V, 0xFF, sizeof(int), s));
     BState st;
     double* d = scal.as<double>();
     st.c_cur = d;
@@ -846,7 +830,6 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
     }
     // tile shape: autotuned once per batch of Hamiltonians, vector width and precision
     int vpl = o.vpl;
-    if (vpl <= 0 && Engine::kCountsSteps) vpl = E.choose_vpl(out.tune_ms);
     if (vpl <= 0) {
         static std::mutex mu;
         static std::map<std::vector<uintptr_t>, std::pair<int, std::vector<double>>> cache;
@@ -856,11 +839,11 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
             key.push_back((uintptr_t)h->dim());
         }
         key.push_back((uintptr_t)Rp);
-        key.push_back((uintptr_t)sizeof(T2));
+        key.push_back((uintptr_t)sizeof(T));
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
         if (it == cache.end()) {
-            vpl = E.choose_vpl(out.tune_ms);
+            vpl = E.autotune(out.tune_ms);
             cache[key] = {vpl, out.tune_ms};
         } else {
             vpl = it->second.first;
@@ -883,17 +866,15 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
         T2* up = E.buf((k + 2) % 3);
         T2* y = E.buf((k + 1) % 3);
         if (t) t->start();
-        E.spmv(vpl, u, y, st.c_cur, E.apart(), st.kstep);
+        E.spmv(vpl, u, y, st.c_cur, E.apart());
         if (t) t->stop();
         E.finish(E.apart(), FIN_ALPHA, st);
         E.update(u, up, y, st.ca, st.cb, E.bpart());
         E.finish(E.bpart(), FIN_BETA, st);
-        if (!Engine::kCountsSteps) {
-            block_advance_kernel<<<1, 1, 0, s>>>(st.kstep);
-            QKG_LAUNCHED();
-        }
+        block_advance_kernel<<<1, 1, 0, s>>>(st.kstep);
+        QKG_LAUNCHED();
     };
-    constexpr int kStepKernels = Engine::kCountsSteps ? 4 : 5;  // SpMV, alpha finish, update, beta finish (, step counter)
+    constexpr int kStepKernels = 5;  // SpMV, alpha finish, update, beta finish, step counter
     const int eager = std::min(M, 3);
     double sp_sum = 0.0;
     for (int k = 0; k < eager; ++k) {
@@ -959,6 +940,115 @@ BlockTridiag run_block(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, 
     return out;
 }
 
+// The run on the packed engine: every step four launches, none of them waited for.
+template <class T>
+BlockTridiag run_packed(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, int Rp) {
+    using Engine = PackedBlockEngine<T>;
+    using T2 = typename Engine::T2;
+    BlockTridiag out;
+    out.n_ham = (int)hs.size();
+    out.R = o.R;
+    out.steps = o.steps;
+    out.rp = Rp;
+    const int V = out.n_ham * Rp;
+    const int M = std::max(0, o.steps);
+    // device state: six scalars a vector, alpha and beta of every step, then integers
+    const size_t nd = 6 * (size_t)V + 2 * (size_t)M * V, ni = 3 * (size_t)V + 1;
+    Engine E(hs, Rp, o.R, nd * sizeof(double) + ni * sizeof(int));
+    cudaStream_t s = E.stream();
+    out.rows = E.rows();
+    double* d = static_cast<double*>(E.extra());
+    int* ip = reinterpret_cast<int*>(d + nd);
+    QKG_CUDA(cudaMemsetAsync(d, 0, nd * sizeof(double) + ni * sizeof(int), s));
+    QKG_CUDA(cudaMemsetAsync(ip + 3 * (size_t)V, 0xFF, sizeof(int), s));  // the first SpMV makes it step 0
+    BState st;
+    st.c_cur = d;
+    st.c_prev = d + V;
+    st.beta_prev = d + 2 * V;
+    st.ca = d + 3 * V;
+    st.cb = d + 4 * V;
+    st.norm2 = d + 5 * V;
+    st.alpha = d + 6 * V;
+    st.beta = st.alpha + (size_t)M * V;
+    st.active = ip;
+    st.n_alpha = ip + V;
+    st.n_beta = ip + 2 * V;
+    st.kstep = ip + 3 * V;
+    st.V = V;
+    st.Rp = Rp;
+    st.Ruser = o.R;
+
+    T2* U0 = E.buf(0);
+    if (o.start == BlockStart::Philox) {
+        E.philox(o.seed, U0);
+    } else {
+        std::vector<cd> h;
+        for (size_t hh = 0; hh < hs.size(); ++hh) {
+            const uint64_t n = hs[hh]->dim();
+            if (!n) continue;
+            NormalStream ns(o.f32_stream);  // restarted per Hamiltonian, as one ftlm() call per sector
+            for (int v = 0; v < o.R; ++v) {
+                if (o.start == BlockStart::Given) {
+                    E.stage_column(hh, v, o.given.at(hh * o.R + v));
+                } else {
+                    h.resize(n);
+                    ns.fill(n, h.data());
+                    E.stage_column(hh, v, h.data());
+                }
+            }
+            E.gather_columns(hh, U0);
+        }
+    }
+    int vpl = o.vpl;
+    if (vpl <= 0) vpl = E.choose_vpl(out.tune_ms);
+    QKG_REQUIRE(Rp % vpl == 0 && Rp / vpl <= 32, "vectors per lane must divide the padded block width");
+    out.vpl = vpl;
+
+    LaunchTimer total(s);
+    constexpr int kTimed = 3;  // SpMV launches that are timed
+    std::vector<std::unique_ptr<LaunchTimer>> tsp;
+    for (int k = 0; k < std::min(M, kTimed); ++k) tsp.push_back(std::make_unique<LaunchTimer>(s));
+    total.start();
+    E.update(nullptr, nullptr, U0, nullptr, nullptr, E.bpart());  // ||u_0||^2 partials
+    E.finish(E.bpart(), FIN_INIT, st);
+    // step k: u_k = buf[k % 3], u_{k-1} = buf[(k + 2) % 3], y = buf[(k + 1) % 3]
+    for (int k = 0; k < M; ++k) {
+        T2* u = E.buf(k % 3);
+        T2* up = k ? E.buf((k + 2) % 3) : nullptr;
+        T2* y = E.buf((k + 1) % 3);
+        if (k < kTimed) tsp[k]->start();
+        E.spmv(vpl, u, y, st.c_cur, E.apart(), st.kstep);
+        if (k < kTimed) tsp[k]->stop();
+        E.finish(E.apart(), FIN_ALPHA, st);
+        E.update(u, up, y, st.ca, st.cb, E.bpart());
+        E.finish(E.bpart(), FIN_BETA, st);
+    }
+    total.stop();
+    std::vector<double> hd(nd);
+    std::vector<int> hi(ni);
+    QKG_CUDA(cudaMemcpyAsync(hd.data(), d, nd * sizeof(double), cudaMemcpyDeviceToHost, s));
+    QKG_CUDA(cudaMemcpyAsync(hi.data(), ip, ni * sizeof(int), cudaMemcpyDeviceToHost, s));
+    QKG_CUDA(cudaStreamSynchronize(s));
+    out.seconds = total.collect();
+    double sp = 0.0;
+    for (auto& t : tsp) sp += t->collect();
+    out.spmv_ms = tsp.empty() ? 0.0 : sp * 1e3 / tsp.size();
+    const double *hn = hd.data() + 5 * (size_t)V, *ha = hd.data() + 6 * (size_t)V, *hb = ha + (size_t)M * V;
+    const int *na = hi.data() + V, *nb = hi.data() + 2 * (size_t)V;
+    const int nv = out.n_ham * o.R;
+    out.alpha.resize(nv);
+    out.beta.resize(nv);
+    out.norm2.resize(nv);
+    for (int h = 0; h < out.n_ham; ++h)
+        for (int v = 0; v < o.R; ++v) {
+            const int vid = h * Rp + v, oi = h * o.R + v;
+            out.norm2[oi] = hn[vid];
+            for (int k = 0; k < na[vid]; ++k) out.alpha[oi].push_back(ha[(size_t)k * V + vid]);
+            for (int k = 0; k < nb[vid]; ++k) out.beta[oi].push_back(hb[(size_t)k * V + vid]);
+        }
+    return out;
+}
+
 }  // namespace
 
 BlockTridiag block_lanczos(const std::vector<Hamiltonian*>& hs, const BlockOpts& o) {
@@ -974,12 +1064,8 @@ BlockTridiag block_lanczos(const std::vector<Hamiltonian*>& hs, const BlockOpts&
     int dev = 0;
     QKG_CUDA(cudaGetDevice(&dev));
     QKG_REQUIRE(dev == hs[0]->device(), "current device differs from the Hamiltonians' device");
-    if (o.mixed) {
-        if (PackedBlockEngine<float>::usable(hs, Rq)) return run_block<PackedBlockEngine<float>>(hs, o, Rq);
-        return run_block<BlockEngine<float, float>>(hs, o, Rp);
-    }
-    if (PackedBlockEngine<double>::usable(hs, Rq)) return run_block<PackedBlockEngine<double>>(hs, o, Rq);
-    return run_block<BlockEngine<double, double>>(hs, o, Rp);
+    if (o.mixed) return PackedBlockEngine<float>::usable(hs) ? run_packed<float>(hs, o, Rq) : run_block<float, float>(hs, o, Rp);
+    return PackedBlockEngine<double>::usable(hs) ? run_packed<double>(hs, o, Rq) : run_block<double, double>(hs, o, Rp);
 }
 
 void ftlm_observables_block(const BlockTridiag& t, const double* betas, int nb, double* Zo, double* Eo, double* Co,

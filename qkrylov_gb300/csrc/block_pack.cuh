@@ -21,13 +21,26 @@ constexpr int kBatch = 4;      // outer entries loaded together
 constexpr int kMaxRun = 8;     // tiles of a CTA
 constexpr int kMaxList = 96;   // outer (and straddling) entries of its blocks staged in shared memory
 
-struct Tile {  // one tile of one Hamiltonian (Item with its Hamiltonian)
-    uint32_t row0, a, tile, tc, ham, pad;
-    uint64_t base;  // first row of its Hamiltonian in the block vector
+// One Hamiltonian of the batch: its rows [base, base + dim) of the block vector,
+// its CTAs' range in the SpMV grid (runs of `run` tiles) and in the row grid
+// (chunks of kRowChunk rows).
+struct Ham {
+    uint64_t base, dim;
+    uint32_t cta0, row_cta0;
+    const uint32_t* perm;  // reference index of each internal row (null: the same)
 };
-struct Cta {  // consecutive tiles of one Hamiltonian
-    uint32_t first, count;
-};
+constexpr uint32_t kRowChunk = 512;
+// the Hamiltonian whose range holds CTA c
+template <class F>
+__device__ __forceinline__ int find_ham(const Ham* __restrict__ hams, int n, uint32_t c, F first) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (first(hams[mid]) <= c) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
 
 __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
     u64 d;
@@ -273,7 +286,7 @@ __device__ __forceinline__ void reduce_vectors(double* red, int n_groups, int Rp
 
 template <class T, int MODE, bool CPLX, int VPL>
 __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
-    block_pack_kernel(const Params<T>* __restrict__ P, const Tile* __restrict__ tiles, const Cta* __restrict__ ctas, int Rp,
+    block_pack_kernel(const Params<T>* __restrict__ P, const Ham* __restrict__ hams, int n_hams, int run, int Rp,
                       const typename V2<T>::t* __restrict__ X, typename V2<T>::t* __restrict__ Y,
                       const double* __restrict__ scale, double* __restrict__ apart, int* kstep) {
     using T2 = typename V2<T>::t;
@@ -281,9 +294,11 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
     __shared__ double red[kBT * VPL];
     __shared__ T s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
     if (kstep && blockIdx.x == 0 && threadIdx.x == 0) ++*kstep;  // the step whose kernels follow
-    const Cta cta = ctas[blockIdx.x];
-    const uint32_t ham = tiles[cta.first].ham;
+    const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.cta0; });
     const Params<T>& p = P[ham];
+    const uint32_t tile0 = (blockIdx.x - hams[ham].cta0) * (uint32_t)run;
+    const uint32_t count = min((uint32_t)run, p.n_items - tile0);
+    const uint64_t base = hams[ham].base;
     if (MODE == AMP_CODED) {
         for (int i = threadIdx.x; i < 2 * p.n_amps; i += kBT) s_amp[i] = p.amps[i];
         __syncthreads();
@@ -302,27 +317,28 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
     const uint32_t* __restrict__ codes = p.codes;
 
     // the run's tiles and their blocks' lists
-    __shared__ Tile s_tile[kMaxRun];
+    __shared__ Item s_tile[kMaxRun];
     __shared__ uint4 s_blk[kMaxRun];
     __shared__ uint2 s_rec[kMaxRun];
     __shared__ Out<T> s_out[kMaxList];
     __shared__ Str<T> s_str[kMaxList];
-    if (threadIdx.x < cta.count) {
-        const Tile t = tiles[cta.first + threadIdx.x];
+    if (threadIdx.x < count) {
+        const uint4 i4 = __ldg(reinterpret_cast<const uint4*>(p.items) + tile0 + threadIdx.x);
+        const Item t{i4.x, i4.y, i4.z, i4.w};
         s_tile[threadIdx.x] = t;
         s_blk[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(p.blk) + t.a);
         s_rec[threadIdx.x] = __ldg(p.tile + t.tile);
     }
     __syncthreads();
     uint32_t lo = 0, ls = 0;  // list entries of the whole run
-    for (uint32_t i = 0; i < cta.count; ++i) {
+    for (uint32_t i = 0; i < count; ++i) {
         lo += s_blk[i].y - s_blk[i].x;
         ls += s_blk[i].w - s_blk[i].z;
     }
     const bool staged = lo <= (uint32_t)kMaxList && ls <= (uint32_t)kMaxList;
     if (staged) {
         uint32_t o = 0, q = 0;
-        for (uint32_t i = 0; i < cta.count; ++i) {
+        for (uint32_t i = 0; i < count; ++i) {
             const uint4 b4 = s_blk[i];
             if (threadIdx.x < b4.y - b4.x) s_out[o + threadIdx.x] = g_out[b4.x + threadIdx.x];
             if (threadIdx.x < b4.w - b4.z) s_str[q + threadIdx.x] = g_str[b4.z + threadIdx.x];
@@ -332,18 +348,18 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
         __syncthreads();
     }
     const int rb = Rp * (int)sizeof(T2);  // bytes of a row
-    const T2* __restrict__ Xh = X + s_tile[0].base * (uint64_t)Rp + l * W0;  // the Hamiltonian's rows
-    T2* __restrict__ Yh = Y + s_tile[0].base * (uint64_t)Rp + l * W0;
+    const T2* __restrict__ Xh = X + base * (uint64_t)Rp + l * W0;  // the Hamiltonian's rows
+    T2* __restrict__ Yh = Y + base * (uint64_t)Rp + l * W0;
     {
         uint32_t ti = 0, oo = 0, so = 0;  // the row's tile and where its lists start
         if (grp < NG)
-            for (int rr = grp; rr < (int)cta.count * kTile; rr += NG) {
+            for (int rr = grp; rr < (int)count * kTile; rr += NG) {
                 while (ti < (uint32_t)rr >> 7) {
                     oo += s_blk[ti].y - s_blk[ti].x;
                     so += s_blk[ti].w - s_blk[ti].z;
                     ++ti;
                 }
-                const Tile& it = s_tile[ti];
+                const Item it = s_tile[ti];
                 const int r = rr & (kTile - 1);
                 if (r >= (int)(it.tc & 0xFFu)) continue;
                 const uint32_t lane = r & 31u, q = (uint32_t)r >> 5, tin = it.tc >> 8;
@@ -448,44 +464,42 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
 }
 
 // w = y - ca u - cb up in place on y, and per CTA the partial ||w_v||^2 (u ==
-// nullptr: only the norms of y).  A CTA takes `count` rows of one Hamiltonian;
-// NU lanes a row, one 16-byte unit (VPL values) each.
-struct UpdItem {
-    uint64_t row0;  // in the block vector
-    uint32_t count, ham;
-};
+// nullptr: only the norms of y; Up == nullptr: no previous vector).  A CTA takes
+// kRowChunk rows of one Hamiltonian, a lane one 16-byte unit (VPL values) of a row.
 template <class T, int VPL>
 __global__ void __launch_bounds__(kBT)
-    block_pack_update(const UpdItem* __restrict__ items, int Rp, typename V2<T>::t* __restrict__ Y,
+    block_pack_update(const Ham* __restrict__ hams, int n_hams, int Rp, typename V2<T>::t* __restrict__ Y,
                       const typename V2<T>::t* __restrict__ U, const typename V2<T>::t* __restrict__ Up,
                       const double* __restrict__ ca, const double* __restrict__ cb, double* __restrict__ part) {
     using R = Row<T, VPL>;
     __shared__ double red[kBT * VPL];
-    const UpdItem it = items[blockIdx.x];
+    const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.row_cta0; });
+    const uint32_t row0 = (blockIdx.x - hams[ham].row_cta0) * kRowChunk;
+    const uint32_t count = (uint32_t)min((unsigned long long)kRowChunk, (unsigned long long)(hams[ham].dim - row0));
     const int G = Rp / VPL, NG = kBT / G;
     const int l = threadIdx.x % G, grp = threadIdx.x / G;
     Dots<T, VPL> dots;
     T a[VPL], b[VPL];
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
-        const size_t vid = (size_t)it.ham * Rp + vec_of<T, VPL>(l, j, G);
+        const size_t vid = (size_t)ham * Rp + vec_of<T, VPL>(l, j, G);
         dots.init(j, 1.0);
         a[j] = U ? -(T)ca[vid] : (T)0;
-        b[j] = U ? -(T)cb[vid] : (T)0;
+        b[j] = Up ? -(T)cb[vid] : (T)0;
     }
-    const uint64_t o = it.row0 * (uint64_t)Rp + l * VPL;
+    const uint64_t o = (hams[ham].base + row0) * (uint64_t)Rp + l * VPL;
     if (grp < NG) {
 #pragma unroll 4
-        for (uint32_t r = grp; r < it.count; r += NG) {
+        for (uint32_t r = grp; r < count; r += NG) {
             const uint64_t at = o + (uint64_t)r * Rp;
             R w;
             w.load(Y + at, G);
             if (U) {
                 R u, v;
                 u.load(U + at, G);
-                v.load(Up + at, G);
+                if (Up) v.load(Up + at, G);
                 w.axpy(a, u);
-                w.axpy(b, v);
+                if (Up) w.axpy(b, v);
                 w.write(Y + at, G);
             }
             dots.square(w);
@@ -502,20 +516,41 @@ __global__ void __launch_bounds__(kBT)
 // the Philox block (counter i, stream h * streams + v); padding vectors are zero.
 template <class T2, bool F64>
 __global__ void __launch_bounds__(kBT)
-    block_pack_philox(const UpdItem* __restrict__ items, const uint64_t* __restrict__ bases,
-                      const uint32_t* const* __restrict__ perms, int Rp, int Ruser, int streams, uint64_t seed,
+    block_pack_philox(const Ham* __restrict__ hams, int n_hams, int Rp, int Ruser, int streams, uint64_t seed,
                       T2* __restrict__ U) {
-    const UpdItem it = items[blockIdx.x];
-    const uint64_t base = bases[it.ham];
-    const uint32_t* __restrict__ perm = perms[it.ham];
-    const uint32_t i0 = (uint32_t)(it.row0 - base);
-    for (uint32_t e = threadIdx.x; e < it.count * (uint32_t)Rp; e += kBT) {
+    const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.row_cta0; });
+    const uint64_t base = hams[ham].base;
+    const uint32_t* __restrict__ perm = hams[ham].perm;
+    const uint32_t i0 = (blockIdx.x - hams[ham].row_cta0) * kRowChunk;
+    const uint32_t count = (uint32_t)min((unsigned long long)kRowChunk, (unsigned long long)(hams[ham].dim - i0));
+    for (uint32_t e = threadIdx.x; e < count * (uint32_t)Rp; e += kBT) {
         const uint32_t i = i0 + e / Rp, v = e % Rp;
         T2 o;
         o.x = 0;
         o.y = 0;
-        if ((int)v < Ruser) o = philox_cnormal<T2, F64>(seed, (uint64_t)it.ham * streams + v, i);
+        if ((int)v < Ruser) o = philox_cnormal<T2, F64>(seed, (uint64_t)ham * streams + v, i);
         U[(base + (perm ? perm[i] : i)) * (uint64_t)Rp + v] = o;
+    }
+}
+
+// The vectors of one Hamiltonian (R contiguous FP64 vectors of n elements, one
+// after the other) into its rows of the block vector; padding vectors are zero.
+template <class T2>
+__global__ void __launch_bounds__(kBT)
+    block_pack_gather(const double2* __restrict__ src, uint64_t n, int R, int Rp, T2* __restrict__ dst) {
+    __shared__ double2 t[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint64_t r0 = blockIdx.x * 32ull;
+    for (int v = w; v < Rp; v += kBT / 32)
+        t[lane][v] = v < R && r0 + lane < n ? src[(uint64_t)v * n + r0 + lane] : make_double2(0.0, 0.0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < 32 * Rp; e += kBT) {
+        const int r = e / Rp, v = e % Rp;
+        if (r0 + r >= n) break;
+        T2 o;
+        o.x = t[r][v].x;
+        o.y = t[r][v].y;
+        dst[(r0 + r) * Rp + v] = o;
     }
 }
 

@@ -205,10 +205,10 @@ public:
     // block) for arithmetic type A (float or double).
     template <class A> void fast_params(fastk::FastParams<A>& p) const;
     template <class A> void pack_params(packk::Params<A>& p, const PackPlan& plan) const;
-    // The packed plan for block vectors: classes of about class_rows rows, of
-    // amplitude form `form` or a more general one; null where none applies.  Built
-    // on first use and kept.
-    const PackPlan* block_plan(uint32_t class_rows, int form);
+    // The packed plan in amplitude form `form` or a more general one (the batched
+    // engine runs Hamiltonians of one form together); null where none applies.
+    // Another form than the plan's own is built on first use and kept.
+    const PackPlan* plan_of_form(int form);
     // reference index of each row of the basis' internal order (null: the same)
     const uint32_t* permutation() const {
         return basis_->permuted ? static_cast<const uint32_t*>(db_->ref_of_int) : nullptr;
@@ -266,9 +266,9 @@ private:
     DBuf optr_, mptr_, ment_;  // per-block outer-entry / straddling-term list offsets and straddling entries
 
     std::unique_ptr<PackPlan> pack_;
-    std::vector<Term> terms_;  // for the block plans
-    std::map<std::pair<uint32_t, int>, std::unique_ptr<PackPlan>> block_plans_;
-    std::mutex block_plans_mu_;
+    std::vector<Term> terms_;  // for plans of another form
+    std::map<int, std::unique_ptr<PackPlan>> form_plans_;
+    std::mutex form_plans_mu_;
     DBuf dcode_ref_;  // diagonal codes in reference order (where the internal order differs)
 
     std::shared_ptr<Basis> basis_;

@@ -1737,15 +1737,15 @@ void Hamiltonian::pack_params(packk::Params<A>& p, const PackPlan& plan) const {
 template void Hamiltonian::pack_params<float>(packk::Params<float>&, const PackPlan&) const;
 template void Hamiltonian::pack_params<double>(packk::Params<double>&, const PackPlan&) const;
 
-const PackPlan* Hamiltonian::block_plan(uint32_t class_rows, int form) {
-    if (!pack_) return nullptr;
-    std::lock_guard<std::mutex> lk(block_plans_mu_);
-    auto it = block_plans_.find({class_rows, form});
-    if (it == block_plans_.end()) {
+const PackPlan* Hamiltonian::plan_of_form(int form) {
+    if (!pack_ || (int)pack_->mode() >= form) return pack_.get();
+    std::lock_guard<std::mutex> lk(form_plans_mu_);
+    auto it = form_plans_.find(form);
+    if (it == form_plans_.end()) {
         PackTables t;
         std::unique_ptr<PackPlan> plan;
-        if (t.build(*basis_, site_, terms_, class_rows, (packk::AmpMode)form)) plan = std::make_unique<PackPlan>(t);
-        it = block_plans_.emplace(std::make_pair(class_rows, form), std::move(plan)).first;
+        if (t.build(*basis_, site_, terms_, (packk::AmpMode)form)) plan = std::make_unique<PackPlan>(t);
+        it = form_plans_.emplace(form, std::move(plan)).first;
     }
     return it->second.get();
 }

@@ -20,7 +20,7 @@
 namespace qkg {
 namespace packk {
 
-constexpr uint32_t kClassTarget = 5000;
+constexpr uint32_t kClassTarget = 5000;  // rows of the largest inner class aimed at
 constexpr int kTile = 128;        // rows of a table tile: one warp, four rows a lane
 constexpr uint32_t kNone16 = 0xFFFFu, kNone15 = 0x7FFFu;
 constexpr int kMaxAmps = 256;     // distinct amplitudes of the coded form
@@ -100,9 +100,8 @@ struct PackTables {
     // False where the plan does not apply: ranks by search, states over 32 bits,
     // classes of more than 65,534 rows, more than 256 distinct amplitudes (coded
     // form), tables over 256 MB, more than 24 straddling terms with one flip.
-    // class_target: rows of the largest inner class aimed at; at_least: the least
-    // general amplitude form to give.
-    bool build(const Basis& B, SiteKind site, const std::vector<Term>& terms, uint32_t class_target = packk::kClassTarget,
+    // at_least: the least general amplitude form to give.
+    bool build(const Basis& B, SiteKind site, const std::vector<Term>& terms,
                packk::AmpMode at_least = packk::AMP_UNIFORM);
     // The off-diagonal part of H x as the kernels walk the tables, every index
     // checked against its table (throws Error).
@@ -113,7 +112,6 @@ struct PackTables {
 class PackPlan {
 public:
     explicit PackPlan(const PackTables& t);
-    const std::vector<packk::Item>& tiles() const { return tiles_; }
     packk::AmpMode mode() const { return mode_; }
     bool real() const { return real_; }
     bool equal_magnitude() const { return equal_; }
@@ -124,7 +122,6 @@ private:
     bool real_ = true, equal_ = false;
     packk::AmpMode mode_ = packk::AMP_UNIFORM;
     uint32_t n_items_ = 0;
-    std::vector<packk::Item> tiles_;
     int n_amps_ = 0;
     double u_ = 0.0;
     DBuf all_;  // the tables, one after the other

@@ -64,8 +64,7 @@ constexpr size_t kMaxTable = 32ull << 20;  // uint2 entries of all tables (256 M
 
 }  // namespace
 
-bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& terms, uint32_t class_target,
-                       AmpMode at_least) {
+bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& terms, AmpMode at_least) {
     *this = PackTables();
     dim = B.dim;
     const int nb = B.nbits;
@@ -83,7 +82,7 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         if (!simplify(h, t, dead)) return false;
         if (!dead) list.push_back(t);
     }
-    // --- the split: the most inner bits whose largest class keeps to class_target
+    // --- the split: the most inner bits whose largest class keeps to kClassTarget
     // rows (a block of x then fits in L1 beside its neighbours') and whose tables
     // stay below a quarter of the sector's rows (they are built for every
     // Hamiltonian), whole sites for interleaved bases
@@ -103,7 +102,7 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         return most << popc(free_bits);
     };
     int n_in = std::min(nb, unit);
-    while (n_in + unit <= nb && n_in + unit <= 16 && class_rows(n_in + unit, false) <= class_target &&
+    while (n_in + unit <= nb && n_in + unit <= 16 && class_rows(n_in + unit, false) <= kClassTarget &&
            class_rows(n_in + unit, true) <= std::max<uint64_t>(4096, B.dim / 4))
         n_in += unit;
     const int n_out = nb - n_in;
@@ -517,7 +516,6 @@ void PackTables::apply_host(const cd* x, cd* y) const {
 
 PackPlan::PackPlan(const PackTables& t)
     : real_(t.real), equal_(t.equal), mode_(t.mode), n_items_((uint32_t)t.items.size()), n_amps_((int)t.codes.size() ? (int)t.amps.size() : 0), u_(t.u) {
-    tiles_ = t.items;
     std::vector<char> image;
     items_ = append(image, t.items);
     blk_ = append(image, t.blk);
