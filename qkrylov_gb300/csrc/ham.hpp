@@ -87,6 +87,7 @@ struct TermSet {
 };
 
 class PackPlan;
+struct Workspace;
 
 class Hamiltonian {
 public:
@@ -112,6 +113,9 @@ public:
     // One FP32 SpMV of the device-resident Lanczos step (fast kernel only);
     // writes n_items() partials to lz.apart.
     void apply_lanczos_f32(const LanczosHooks& lz, cudaStream_t s) const;
+    // The FP64 one (packed kernel; false, with nothing launched, elsewhere):
+    // lanczos_parts() partials.
+    bool apply_lanczos_f64(const LanczosHooks& lz, cudaStream_t s) const;
 
     // Seeded Gaussian start vectors: element i of the basis' internal order takes
     // the generator's block i whatever order the vector is in.
@@ -228,8 +232,19 @@ public:
     // call, so two calls on one Hamiltonian from different host threads take
     // turns instead of freeing each other's Krylov space.
     DBuf& krylov_workspace(size_t bytes) const;
-    void release_workspace() const { kws_.reset(); }
-    size_t workspace_bytes() const { return kws_.bytes; }
+    void release_workspace() const;
+    size_t workspace_bytes() const;
+    // Also kept between calls and covered by the lock and the two above: vectors of
+    // `bytes` each for the FP64 Lanczos (slabs of up to 256 MB, allocated as the run
+    // grows), the reductions' scratch, and mapped host memory for scalars.
+    void* krylov_vector(size_t i, size_t bytes) const;
+    bool has_krylov_vector(size_t i) const;  // of the size last asked for
+    void trim_vectors(size_t keep_bytes) const;  // frees slabs from the last while they hold more
+    Workspace& reduction_scratch(size_t partials) const;
+    struct MappedScalars {
+        double *host = nullptr, *dev = nullptr;
+    };
+    MappedScalars mapped_scalars(size_t n) const;
     std::unique_lock<std::mutex> workspace_lock() const { return std::unique_lock<std::mutex>(kws_mu_); }
 
 private:
@@ -286,6 +301,12 @@ private:
     DBuf dcode_, dtab64_, dtab32_, dfull64_, dfull32_;
     int n_dtab_ = 0;
     mutable DBuf kws_;
+    mutable std::vector<DBuf> slabs_;
+    mutable size_t slab_vec_bytes_ = 0;
+    static constexpr size_t kSlabBytes = 256ull << 20;
+    mutable std::unique_ptr<Workspace> red_;
+    mutable MappedScalars mapped_;
+    mutable size_t mapped_n_ = 0;
     mutable std::mutex kws_mu_;
 };
 
@@ -322,6 +343,12 @@ void mdot_f64(const double2* const* V_dev, int k, const double2* w, uint64_t n, 
               Workspace& ws, cudaStream_t s);
 void mdot_f32(const float2* const* V_dev, int k, const float2* w, uint64_t n, std::complex<double>* out,
               Workspace& ws, cudaStream_t s);
+// <V_j, w> as g partial sums a vector, part[j * g + i], left on the device; the g to
+// give for k vectors, and the most partials any k <= k_max takes
+int mdot_f64_chunks(int k, uint64_t n);
+size_t mdot_f64_most_partials(int k_max, uint64_t n);
+void mdot_f64_partials(const double2* const* V_dev, int k, const double2* w, uint64_t n, double2* part, int g,
+                       cudaStream_t s);
 // out[o * k + j] = <V_j, W_o> for j < k, o < nw <= 4: one pass over the V_j for
 // all W_o (compensated FP32; W a host array of device pointers).
 void mdot_multi_f32(const float2* const* V_dev, int k, float2* const* W, int nw, uint64_t n,

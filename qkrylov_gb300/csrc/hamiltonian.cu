@@ -1611,7 +1611,67 @@ static void allow_stage_smem(size_t bytes) {
     done |= bit;
 }
 
+void Hamiltonian::release_workspace() const {
+    kws_.reset();
+    slabs_.clear();
+    red_.reset();
+}
+size_t Hamiltonian::workspace_bytes() const {
+    size_t b = kws_.bytes;
+    for (const auto& s : slabs_) b += s.bytes;
+    return b;
+}
+void* Hamiltonian::krylov_vector(size_t i, size_t bytes) const {
+    bytes = (bytes + 255) / 256 * 256;
+    if (slab_vec_bytes_ != bytes) {
+        slabs_.clear();
+        slab_vec_bytes_ = bytes;
+    }
+    const size_t per = std::max<size_t>(1, std::min<size_t>(64, kSlabBytes / bytes));
+    while (slabs_.size() <= i / per) {
+        size_t fr = 0, tot = 0;
+        QKG_CUDA(cudaMemGetInfo(&fr, &tot));
+        if (fr < per * bytes + (64ull << 20))
+            throw Error(CUDA_ERR, "out of device memory for the Krylov basis (" + std::to_string(slabs_.size() * per) + " vectors held)");
+        slabs_.emplace_back(per * bytes);
+    }
+    return slabs_[i / per].as<char>() + (i % per) * bytes;
+}
+bool Hamiltonian::has_krylov_vector(size_t i) const {
+    return slab_vec_bytes_ && i < slabs_.size() * std::max<size_t>(1, std::min<size_t>(64, kSlabBytes / slab_vec_bytes_));
+}
+void Hamiltonian::trim_vectors(size_t keep_bytes) const {
+    size_t b = 0;
+    for (const auto& s : slabs_) b += s.bytes;
+    while (!slabs_.empty() && b > keep_bytes) {
+        b -= slabs_.back().bytes;
+        slabs_.pop_back();
+    }
+}
+Workspace& Hamiltonian::reduction_scratch(size_t partials) const {
+    if (!red_ || red_->cap_partials < partials) {
+        red_.reset();
+        red_ = std::make_unique<Workspace>(partials);
+    }
+    return *red_;
+}
+Hamiltonian::MappedScalars Hamiltonian::mapped_scalars(size_t n) const {
+    if (mapped_n_ < n) {
+        if (mapped_.host) cudaFreeHost(mapped_.host);
+        mapped_ = {};
+        mapped_n_ = 0;
+        QKG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&mapped_.host), n * sizeof(double), cudaHostAllocMapped));
+        QKG_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped_.dev), mapped_.host, 0));
+        mapped_n_ = n;
+    }
+    return mapped_;
+}
+
 Hamiltonian::~Hamiltonian() {
+    if (mapped_.host) {
+        if (stream_) cudaStreamSynchronize(stream_);
+        cudaFreeHost(mapped_.host);
+    }
     if (stream_) {
         cudaStreamSynchronize(stream_);
         cudaStreamDestroy(stream_);
@@ -1808,6 +1868,16 @@ void Hamiltonian::apply_lanczos_f32(const LanczosHooks& lz, cudaStream_t s) cons
     size_t ni = 0;
     p.items = items_of(v, &ni);
     launch_fast<float, float>(p, ni, all_real_, unif_, nullptr, nullptr, s, v, st ? stage_bytes(8) : 0);
+}
+
+bool Hamiltonian::apply_lanczos_f64(const LanczosHooks& lz, cudaStream_t s) const {
+    if (!packed()) return false;
+    packk::Params<double> p;
+    pack_params(p, *pack_);
+    p.lz = lz.op;
+    p.apart = lz.apart;
+    pack_apply_f64(*pack_, p, nullptr, nullptr, s);
+    return true;
 }
 
 size_t Hamiltonian::lanczos_parts() const {

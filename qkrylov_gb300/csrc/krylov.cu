@@ -744,6 +744,26 @@ void mdot_f64(const double2* const* V, int k, const double2* w, uint64_t n, std:
               cudaStream_t s) {
     mdot_impl<double2, false>(V, k, w, n, out, ws, s);
 }
+// Row chunks of the FP64 projections: every CTA ends with two double sums a vector
+// over its threads, which cost more than an element's products on the FP64 pipe, so
+// the chunks are few (six CTAs a SM over all columns) and a thread has at least four
+// elements where there are that many.
+int mdot_f64_chunks(int k, uint64_t n) {
+    const int cols = std::max(1, (k + KB - 1) / KB);
+    const uint64_t most = std::max<uint64_t>(1, n / (4 * kThreads));
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(most, std::max(8, 152 * 6 / cols)));
+}
+size_t mdot_f64_most_partials(int k_max, uint64_t n) {
+    size_t m = 0;
+    for (int k = 1; k <= k_max; ++k) m = std::max(m, (size_t)k * mdot_f64_chunks(k, n));
+    return m;
+}
+void mdot_f64_partials(const double2* const* V, int k, const double2* w, uint64_t n, double2* part, int g,
+                       cudaStream_t s) {
+    if (k <= 0) return;
+    mdot_kernel<double2, false><<<dim3((k + KB - 1) / KB, g), kThreads, 0, s>>>(V, k, w, n, part, g);
+    QKG_LAUNCHED();
+}
 void mdot_f32(const float2* const* V, int k, const float2* w, uint64_t n, std::complex<double>* out, Workspace& ws,
               cudaStream_t s) {
     mdot_impl<float2, true>(V, k, w, n, out, ws, s);

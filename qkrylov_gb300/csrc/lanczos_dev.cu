@@ -24,6 +24,8 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstring>
+#include <memory>
 #include <type_traits>
 
 namespace qkg {
@@ -268,6 +270,104 @@ __global__ void lz_beta_kernel(const double2* __restrict__ bpart, int nparts, Lz
         o.bprev32 = (float)o.bprev;
         *op = o;
     }
+}
+
+// ---- FP64 ---------------------------------------------------------------------
+// w -= a v in place, ||w||^2 partials.
+__global__ void lz64_update(void* const* __restrict__ vtab, const LzState* __restrict__ st, uint64_t n,
+                            double2* __restrict__ bpart) {
+    const int k = st->k;
+    double2* __restrict__ w = static_cast<double2*>(vtab[k + 1]);
+    const double2* __restrict__ v = static_cast<const double2*>(vtab[k]);
+    const double a = -st->a;
+    double acc = 0.0;
+#pragma unroll 4
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        double2 x = w[i];
+        const double2 c = v[i];
+        x.x = fma(a, c.x, x.x);
+        x.y = fma(a, c.y, x.y);
+        w[i] = x;
+        acc = fma(x.y, x.y, fma(x.x, x.x, acc));
+    }
+    const double2 t = bsum2(acc, 0.0);
+    if (threadIdx.x == 0) bpart[blockIdx.x] = t;
+}
+// y = scale y - bprev vprev and Re<x, y> partials, for an SpMV that does not do it.
+__global__ void lz64_post(const LzOperands* __restrict__ op, uint64_t n, double2* __restrict__ apart) {
+    const LzOperands o = *op;
+    const double2* __restrict__ x = static_cast<const double2*>(o.x);
+    const double2* __restrict__ p = static_cast<const double2*>(o.vprev);
+    double2* __restrict__ y = static_cast<double2*>(o.y);
+    double acc = 0.0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        double2 w = y[i];
+        const double2 c = x[i];
+        w.x *= o.scale;
+        w.y *= o.scale;
+        if (p) {
+            const double2 d = p[i];
+            w.x = fma(-o.bprev, d.x, w.x);
+            w.y = fma(-o.bprev, d.y, w.y);
+        }
+        y[i] = w;
+        acc = fma(c.y, w.y, fma(c.x, w.x, acc));
+    }
+    const double2 t = bsum2(acc, 0.0);
+    if (threadIdx.x == 0) apart[blockIdx.x] = t;
+}
+// coef_j = -sig_j^2 <V_j, w> from the projections' partials (column j at part[j * nparts]).
+__global__ void lz64_coef(const double2* __restrict__ part, int nparts, const double* __restrict__ sig,
+                          double2* __restrict__ coef) {
+    const int j = blockIdx.x;
+    double re = 0.0, im = 0.0;
+    for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
+        const double2 v = part[(size_t)j * nparts + i];
+        re += v.x;
+        im += v.y;
+    }
+    const double2 s = bsum2(re, im);
+    if (threadIdx.x == 0) {
+        const double f = -sig[j] * sig[j];
+        coef[j] = make_double2(f * s.x, f * s.y);
+    }
+}
+// w += sum_j coef_j V_j (j < k), ||w||^2 partials; w = V_k.
+__global__ void __launch_bounds__(kT) lz64_subtract(void* const* __restrict__ vtab, int k, const double2* __restrict__ coef,
+                                                    uint64_t n, double2* __restrict__ bpart) {
+    extern __shared__ double2 s_c[];
+    const double2** s_v = reinterpret_cast<const double2**>(s_c + k);
+    for (int j = threadIdx.x; j < k; j += blockDim.x) {
+        s_c[j] = coef[j];
+        s_v[j] = static_cast<const double2*>(vtab[j]);
+    }
+    __syncthreads();
+    double2* __restrict__ w = static_cast<double2*>(vtab[k]);
+    double acc = 0.0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        double2 x = w[i];
+        int j = 0;
+        for (; j + 4 <= k; j += 4) {  // four vectors' loads in flight
+            double2 a[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[q] = s_v[j + q][i];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double2 c = s_c[j + q];
+                x.x = fma(c.x, a[q].x, fma(-c.y, a[q].y, x.x));
+                x.y = fma(c.x, a[q].y, fma(c.y, a[q].x, x.y));
+            }
+        }
+        for (; j < k; ++j) {
+            const double2 a = s_v[j][i], c = s_c[j];
+            x.x = fma(c.x, a.x, fma(-c.y, a.y, x.x));
+            x.y = fma(c.x, a.y, fma(c.y, a.x, x.y));
+        }
+        w[i] = x;
+        acc = fma(x.y, x.y, fma(x.x, x.x, acc));
+    }
+    const double2 t = bsum2(acc, 0.0);
+    if (threadIdx.x == 0) bpart[blockIdx.x] = t;
 }
 
 using clk = std::chrono::steady_clock;
@@ -579,6 +679,282 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
         QKG_CUDA(cudaStreamSynchronize(st));
     }
     return out;
+}
+
+// The FP64 recurrence with its scalars on the device: the host enqueues steps up
+// to kInFlight ahead and reads alpha and beta (mapped memory) behind them, so
+// nothing waits for the GPU within a step.  v_k = sig_k V_k as in the mixed form.
+//   SpMV (y = sig_k H V_k - beta_{k-1} v_{k-1}, Re<V_k, y> partials), alpha,
+//   update (w -= alpha v_k, and its norm), with `full` the projections of w on
+//   every V_j, their coefficients and the subtraction (one classical
+//   Gram-Schmidt pass, and the norm), beta.
+// vec(i) gives the memory of V_i; keep(j) is called with each completed step j
+// in order and says whether to go on.
+namespace {
+struct Recurrence64 {
+    Hamiltonian& H;
+    uint64_t n;
+    cudaStream_t st;
+    int nmax;
+    bool full;
+    double *ah = nullptr, *bh = nullptr;  // alpha_j, beta_j on the host
+    double t_spmv = 0.0;
+    int n_spmv = 0;
+    Recurrence64(Hamiltonian& h, int steps, bool reorth) : H(h), n(h.dim()), st(h.stream()), nmax(steps), full(reorth) {}
+
+    // V_0 is the start vector (its norm need not be 1: sig0 = 1 / ||V_0||)
+    // slot(i): the vector slot V_i lives in
+    template <class Slot, class Vec, class Keep>
+    void run(double sig0, Slot&& slot, Vec&& vec, Keep&& keep) {
+        const int N = nmax + 2;
+        const int nparts = H.packed() ? (int)H.lanczos_parts() : kUpdGrid;
+        const int g = (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kT - 1) / kT, kUpdGrid));
+        // device scalars: state, operands, pointers, alpha, beta, sig, coefficients, partials
+        auto al = [](size_t b) { return (b + 255) / 256 * 256; };
+        size_t off = 0;
+        auto take = [&](size_t b) { const size_t o = off; off += al(b); return o; };
+        const size_t o_st = take(sizeof(LzState)), o_op = take(sizeof(LzOperands)), o_tab = take(N * sizeof(void*)),
+                     o_al = take(N * 8), o_be = take(N * 8), o_sg = take(N * 8), o_co = take((size_t)N * 16),
+                     o_ap = take((size_t)nparts * 16), o_bp = take((size_t)kUpdGrid * 16), o_p2 = take(kAlphaBlocks * 8),
+                     o_ar = take(sizeof(unsigned int));
+        Workspace& ws = H.reduction_scratch(std::max<size_t>(1 << 16, off / sizeof(double2) + 1 + (full ? mdot_f64_most_partials(N, n) : 0)));
+        char* base = ws.partial.as<char>();
+        auto* state = reinterpret_cast<LzState*>(base + o_st);
+        auto* op = reinterpret_cast<LzOperands*>(base + o_op);
+        auto** tab = reinterpret_cast<void**>(base + o_tab);
+        auto *alpha = reinterpret_cast<double*>(base + o_al), *beta = reinterpret_cast<double*>(base + o_be),
+             *sig = reinterpret_cast<double*>(base + o_sg);
+        auto* coef = reinterpret_cast<double2*>(base + o_co);
+        auto *apart = reinterpret_cast<double2*>(base + o_ap), *bpart = reinterpret_cast<double2*>(base + o_bp);
+        auto* part2 = reinterpret_cast<double*>(base + o_p2);
+        auto* arrived = reinterpret_cast<unsigned int*>(base + o_ar);
+        double2* ppart = reinterpret_cast<double2*>(base + off);
+        const auto m = H.mapped_scalars(2 * (size_t)N);
+        ah = m.host;
+        bh = m.host + N;
+        // initial image: state, operands, the pointers of the vectors there are, sig_0
+        std::vector<void*> ptr(N, nullptr);
+        std::vector<char> image(off, 0);
+        int known = 0;  // pointers the device has
+        auto name_vectors = [&](int need) {  // V_0 .. V_need and those allocated with them
+            int i = known;
+            for (; i <= nmax && (i <= need || H.has_krylov_vector(slot(i))); ++i) ptr[i] = vec(i);
+            return i;
+        };
+        known = name_vectors(std::min(1, nmax));
+        LzOperands op0;
+        op0.x = ptr[0];
+        op0.y = ptr[1];
+        op0.scale = sig0;
+        std::memcpy(image.data() + o_op, &op0, sizeof(op0));
+        std::memcpy(image.data() + o_tab, ptr.data(), (size_t)known * sizeof(void*));
+        std::memcpy(image.data() + o_sg, &sig0, sizeof(double));
+        QKG_CUDA(cudaMemcpyAsync(base, image.data(), image.size(), cudaMemcpyHostToDevice, st));
+        LanczosHooks hooks;
+        hooks.op = op;
+        hooks.apart = apart;
+        struct Events {
+            std::vector<cudaEvent_t> e;
+            ~Events() { for (auto x : e) if (x) cudaEventDestroy(x); }
+        } done{std::vector<cudaEvent_t>(kInFlight + 2, nullptr)};
+        for (auto& e : done.e) QKG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        std::vector<std::unique_ptr<LaunchTimer>> timers;
+        int launched = 0, checked = 0;
+        bool go = true;
+        auto enqueue = [&](int k) {
+            // V_{k+2}, the next step's output, joins the table before a kernel names it
+            if (k + 2 <= nmax && k + 2 >= known) {
+                const int from = known;
+                known = name_vectors(k + 2);
+                QKG_CUDA(cudaMemcpyAsync(tab + from, &ptr[from], (size_t)(known - from) * sizeof(void*), cudaMemcpyHostToDevice, st));
+            }
+            if (k < kTimedSteps) {
+                timers.push_back(std::make_unique<LaunchTimer>(st));
+                timers.back()->start();
+            }
+            const bool fused = H.apply_lanczos_f64(hooks, st);
+            if (!fused) H.apply_f64(static_cast<const double2*>(ptr[k]), static_cast<double2*>(ptr[k + 1]), st);
+            if (k < kTimedSteps) timers.back()->stop();
+            if (!fused) {
+                lz64_post<<<kUpdGrid, kT, 0, st>>>(op, n, apart);
+                QKG_LAUNCHED();
+            }
+            lz_alpha_kernel<<<kAlphaBlocks, kT, 0, st>>>(apart, nparts, state, alpha, beta, sig, m.dev, part2, arrived);
+            QKG_LAUNCHED();
+            lz64_update<<<g, kT, 0, st>>>(tab, state, n, bpart);
+            QKG_LAUNCHED();
+            if (full) {
+                const int gm = mdot_f64_chunks(k + 1, n);
+                mdot_f64_partials(reinterpret_cast<const double2* const*>(tab), k + 1, static_cast<const double2*>(ptr[k + 1]),
+                                  n, ppart, gm, st);
+                lz64_coef<<<k + 1, kT, 0, st>>>(ppart, gm, sig, coef);
+                QKG_LAUNCHED();
+                lz64_subtract<<<g, kT, (size_t)(k + 1) * (sizeof(double2) + sizeof(void*)), st>>>(tab, k + 1, coef, n, bpart);
+                QKG_LAUNCHED();
+            }
+            lz_beta_kernel<<<1, kT, 0, st>>>(bpart, g, state, beta, sig, m.dev + N, tab, nmax, op);
+            QKG_LAUNCHED();
+        };
+        try {
+            while (launched < nmax && go) {
+                enqueue(launched);
+                QKG_CUDA(cudaEventRecord(done.e[launched % done.e.size()], st));
+                ++launched;
+                while (checked < launched && go) {
+                    cudaEvent_t e = done.e[checked % done.e.size()];
+                    if (launched < nmax && launched - checked < kInFlight) {
+                        const cudaError_t q = cudaEventQuery(e);
+                        if (q == cudaErrorNotReady) break;
+                        QKG_CUDA(q);
+                    } else {
+                        QKG_CUDA(cudaEventSynchronize(e));
+                    }
+                    go = keep(checked++);
+                }
+            }
+            QKG_CUDA(cudaStreamSynchronize(st));
+        } catch (...) {
+            cudaStreamSynchronize(st);  // nothing of this run is in flight when its memory is reused
+            throw;
+        }
+        for (auto& t : timers) t_spmv += t->collect();
+        n_spmv = (int)timers.size();
+    }
+};
+}  // namespace
+
+// src/solvers/lanczos.cpp:101-202 in FP64: full reorthogonalisation, the
+// reference's start vector and stopping rules.
+LanczosOut lanczos_f64_device(Hamiltonian& H, const LanczosOpts& o) {
+    LanczosOut out;
+    const uint64_t n = H.dim();
+    if (n == 0) return out;
+    const auto lock = H.workspace_lock();
+    cudaStream_t st = H.stream();
+    const int nmax = (int)std::min<uint64_t>((uint64_t)std::max(o.maxiter, 0), n);
+    const size_t vb = n * sizeof(double2);
+    auto vec = [&](int i) { return H.krylov_vector((size_t)i, vb); };
+    struct Trim {  // a long run's vectors are not kept
+        Hamiltonian& H;
+        ~Trim() { H.trim_vectors(2ull << 30); }
+    } trim{H};
+    double2* v0 = static_cast<double2*>(vec(0));
+    double2* v1 = static_cast<double2*>(vec(1));
+    if (o.device_start) {
+        H.philox_f64(o.seed, 0, v0, st);
+    } else {
+        std::vector<cd> h;
+        const cd* src = o.v0_ref;
+        if (!src) {
+            h.resize(n);
+            ref_uniform_complex(1234, n, h.data(), o.f32_stream);  // src/solvers/lanczos.cpp:115-120
+            src = h.data();
+        }
+        QKG_CUDA(cudaMemcpyAsync(H.permuted() ? v1 : v0, src, vb, cudaMemcpyHostToDevice, st));
+        if (H.permuted()) H.to_internal_f64(v1, v0, st);
+        QKG_CUDA(cudaStreamSynchronize(st));
+    }
+    double nr0;
+    {
+        Workspace& ws = H.reduction_scratch(1 << 16);
+        nr0 = std::sqrt(nrm2sq_f64(v0, n, ws, st));
+        if (nr0 != 0.0) scal_f64(1.0 / nr0, v0, n, st);
+    }
+    auto& alphas = out.alphas;
+    auto& betas = out.betas;
+    double e_old = 1e100;
+    Recurrence64 R(H, nmax, true);
+    const auto t0 = clk::now();
+    R.run(1.0, [](int i) { return (size_t)i; }, vec, [&](int j) {
+        alphas.push_back(R.ah[j]);
+        const double b = R.bh[j];
+        out.iters = j + 1;
+        if (b < 1e-15) {
+            out.converged = true;
+            return false;
+        }
+        if (j + 1 == nmax) return false;
+        betas.push_back(b);
+        if (j > 0 && !o.fixed_steps) {
+            const double e = tridiag_lowest(alphas.data(), betas.data(), j + 1);
+            if (std::abs(e - e_old) < o.tol) {
+                out.converged = true;
+                return false;
+            }
+            e_old = e;
+        }
+        return true;
+    });
+    out.t_loop = secs(t0, clk::now());
+    out.t_spmv = R.t_spmv;
+    out.n_spmv = R.n_spmv;
+    std::vector<double> s;
+    out.energy = tridiag_ground(alphas.data(), betas.data(), (int)alphas.size(), s);
+    out.energy_tridiag = out.energy;
+    out.residual = -1.0;
+    if (o.want_vec) {
+        // Ritz vector into the place of the first vector past the basis used
+        const int m = (int)s.size();
+        std::vector<cd> c(m);
+        double sg = 1.0;
+        for (int i = 0; i < m; ++i) {
+            c[i] = s[i] * sg;
+            sg = 1.0 / R.bh[i];
+        }
+        Workspace& ws = H.reduction_scratch(1 << 16);
+        std::vector<const double2*> p(m);
+        for (int i = 0; i < m; ++i) p[i] = static_cast<const double2*>(vec(i));
+        DBuf tab(std::max(1, m) * sizeof(void*));
+        QKG_CUDA(cudaMemcpy(tab.p, p.data(), m * sizeof(void*), cudaMemcpyHostToDevice));
+        double2* ritz = static_cast<double2*>(vec(m));
+        QKG_CUDA(cudaMemsetAsync(ritz, 0, vb, st));
+        mcombine_f64(static_cast<const double2* const*>(tab.p), m, c.data(), ritz, n, ws, st);
+        const double nr = std::sqrt(nrm2sq_f64(ritz, n, ws, st));
+        if (nr != 0.0) scal_f64(1.0 / nr, ritz, n, st);
+        cd* dst = o.evec_out;
+        if (!dst) {
+            out.evec.resize(n);
+            dst = out.evec.data();
+        }
+        const double2* src = ritz;
+        if (H.permuted()) {
+            double2* t2 = static_cast<double2*>(vec(0));
+            H.to_reference_f64(ritz, t2, st);
+            src = t2;
+        }
+        QKG_CUDA(cudaMemcpyAsync(dst, src, vb, cudaMemcpyDeviceToHost, st));
+        QKG_CUDA(cudaStreamSynchronize(st));
+    }
+    return out;
+}
+
+// The three-term recurrence without reorthogonalisation from a reference-order
+// host vector (dynamics.cpp:38-56, ftlm.cpp:36-52): alphas, betas until beta <
+// 1e-15 or n_steps; returns the start vector's squared norm (below min_norm^2:
+// nothing recorded).
+double three_term_f64(Hamiltonian& H, const cd* v_ref, int n_steps, double min_norm, std::vector<double>& alphas,
+                      std::vector<double>& betas) {
+    const uint64_t n = H.dim();
+    const auto lock = H.workspace_lock();
+    cudaStream_t st = H.stream();
+    const size_t vb = n * sizeof(double2);
+    // three vectors in turn
+    auto vec = [&](int i) { return H.krylov_vector((size_t)(i % 3), vb); };
+    double2* v0 = static_cast<double2*>(vec(0));
+    double2* v1 = static_cast<double2*>(vec(1));
+    QKG_CUDA(cudaMemcpyAsync(H.permuted() ? v1 : v0, v_ref, vb, cudaMemcpyHostToDevice, st));
+    if (H.permuted()) H.to_internal_f64(v1, v0, st);
+    const double norm2 = nrm2sq_f64(v0, n, H.reduction_scratch(1 << 16), st);
+    const double nr = std::sqrt(norm2);
+    if (nr < min_norm || n_steps <= 0) return norm2;
+    Recurrence64 R(H, n_steps, false);
+    R.run(nr != 0.0 ? 1.0 / nr : 1.0, [](int i) { return (size_t)(i % 3); }, vec, [&](int j) {
+        alphas.push_back(R.ah[j]);
+        if (R.bh[j] < 1e-15) return false;
+        betas.push_back(R.bh[j]);
+        return true;
+    });
+    return norm2;
 }
 
 }  // namespace qkg

@@ -475,6 +475,11 @@ void release_workspace_if_short(Hamiltonian& H, size_t bytes) {
 }
 
 LanczosOut lanczos_f64(Hamiltonian& H, const LanczosOpts& o) {
+    if (!o.selective) {
+        const size_t steps = (size_t)std::min<uint64_t>((uint64_t)std::max(o.maxiter, 0), H.dim());
+        release_workspace_if_short(H, (steps + 3) * H.dim() * sizeof(double2));
+        return lanczos_f64_device(H, o);
+    }
     LanczosOut out;
     const uint64_t n = H.dim();
     if (n == 0) return out;
@@ -527,15 +532,7 @@ LanczosOut lanczos_f64(Hamiltonian& H, const LanczosOpts& o) {
         ++out.n_spmv;
         alphas.push_back(alpha);
         double b2 = lanczos_update_f64(w.as<double2>(), v, vp, alpha, iter > 0 ? betas.back() : 0.0, n, ws, st);
-        if (!o.selective) {
-            // full reorthogonalisation against every stored vector (:148-151), one CGS pass
-            const int k = (int)V.size();
-            c.assign(k, 0.0);
-            mdot_f64(V.dev(), k, w.as<double2>(), n, c.data(), ws, st);
-            for (auto& x : c) x = -x;
-            mcombine_f64(V.dev(), k, c.data(), w.as<double2>(), n, ws, st);
-            b2 = nrm2sq_f64(w.as<double2>(), n, ws, st);
-        } else if (psi.size()) {
+        if (psi.size()) {
             c.assign(psi.size(), 0.0);
             mdot_f64(psi.dev(), (int)psi.size(), w.as<double2>(), n, c.data(), ws, st);
             for (auto& x : c) x = -x;
@@ -556,7 +553,7 @@ LanczosOut lanczos_f64(Hamiltonian& H, const LanczosOpts& o) {
             if (std::abs(e - e_old) < o.tol) { out.converged = true; break; }
             e_old = e;
         }
-        if (o.selective && k >= 4) {
+        if (k >= 4) {
             for (double theta : ritz_to_lock(alphas.data(), betas.data(), k, beta, so_tol, locked, o.ritz_guard)) {
                 std::vector<double> sv;
                 if (!tridiag_vector(alphas.data(), betas.data(), k, theta, sv)) continue;
@@ -726,33 +723,9 @@ LanczosOut lanczos_mixed(Hamiltonian& H, const LanczosOpts& o) {
 // ============================================================ continued fraction
 CFOut cf_f64(Hamiltonian& H, const cd* phi0_ref, int n_iter) {
     CFOut out;
-    const uint64_t n = H.dim();
-    if (n == 0) return out;
-    cudaStream_t st = H.stream();
-    Workspace ws(ws_cap(2));
-    DBuf a(n * sizeof(double2)), b(n * sizeof(double2)), w(n * sizeof(double2)), tmp;
-    double2 *v = a.as<double2>(), *vp = b.as<double2>();
-    upload_ref_f64(H, phi0_ref, v, tmp);
-    const double np = std::sqrt(nrm2sq_f64(v, n, ws, st));
-    if (np < 1e-15) return out;  // src/solvers/dynamics.cpp:26
-    scal_f64(1.0 / np, v, n, st);
-    out.norm = np;
-    for (int it = 0; it < n_iter; ++it) {
-        H.apply_f64(v, w.as<double2>(), st);
-        const double alpha = dot_f64(v, w.as<double2>(), n, ws, st).real();
-        out.alphas.push_back(alpha);
-        const double b2 = lanczos_update_f64(w.as<double2>(), v, it > 0 ? vp : nullptr, alpha,
-                                             it > 0 ? out.betas.back() : 0.0, n, ws, st);
-        const double beta = std::sqrt(b2);
-        if (beta < 1e-15) break;
-        out.betas.push_back(beta);
-        // rotate: vp <- v, v <- w / beta, w <- old vp buffer
-        std::swap(vp, v);
-        double2* wp = w.as<double2>();
-        QKG_CUDA(cudaMemcpyAsync(v, wp, n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-        scal_f64(1.0 / beta, v, n, st);
-    }
-    QKG_CUDA(cudaStreamSynchronize(st));
+    if (H.dim() == 0) return out;
+    const double np = std::sqrt(three_term_f64(H, phi0_ref, n_iter, 1e-15, out.alphas, out.betas));
+    if (np >= 1e-15) out.norm = np;  // src/solvers/dynamics.cpp:26
     return out;
 }
 
@@ -773,33 +746,13 @@ std::vector<FTLMTri> ftlm_tridiags_f64(Hamiltonian& H, int n_random, int n_steps
     std::vector<FTLMTri> out;
     const uint64_t n = H.dim();
     if (n == 0 || n_random <= 0) return out;
-    cudaStream_t st = H.stream();
-    Workspace ws(ws_cap(2));
-    DBuf a(n * sizeof(double2)), b(n * sizeof(double2)), w(n * sizeof(double2)), tmp;
     NormalStream stream(f32_stream);  // mt19937(42), src/solvers/ftlm.cpp:133-134
     std::vector<cd> h(n);
     for (int r = 0; r < n_random; ++r) {
         stream.fill(n, h.data());
-        double2 *v = a.as<double2>(), *vp = b.as<double2>();
-        upload_ref_f64(H, h.data(), v, tmp);
         FTLMTri t;
-        t.norm2 = nrm2sq_f64(v, n, ws, st);
-        const double nr = std::sqrt(t.norm2);
-        if (nr != 0.0) scal_f64(1.0 / nr, v, n, st);
         std::vector<double> al, be;
-        for (int i = 0; i < n_steps; ++i) {
-            H.apply_f64(v, w.as<double2>(), st);
-            const double alpha = dot_f64(v, w.as<double2>(), n, ws, st).real();
-            al.push_back(alpha);
-            const double b2 = lanczos_update_f64(w.as<double2>(), v, i > 0 ? vp : nullptr, alpha, i > 0 ? be.back() : 0.0,
-                                                 n, ws, st);
-            const double beta = std::sqrt(b2);
-            if (beta < 1e-15) break;
-            be.push_back(beta);
-            std::swap(vp, v);
-            QKG_CUDA(cudaMemcpyAsync(v, w.p, n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-            scal_f64(1.0 / beta, v, n, st);
-        }
+        t.norm2 = three_term_f64(H, h.data(), n_steps, 0.0, al, be);
         std::vector<double> z;
         tridiag_eig(al.data(), be.data(), (int)al.size(), t.evals, {0}, z);
         t.w0.resize(t.evals.size());

@@ -132,6 +132,11 @@ bool lanczos_device_supported(const Hamiltonian& H);
 // device memory a device-resident mixed run of maxiter steps holds
 size_t lanczos_device_bytes(const Hamiltonian& H, int maxiter);
 LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o);
+// lanczos_f64 without o.selective, the recurrence's scalars on the device
+LanczosOut lanczos_f64_device(Hamiltonian& H, const LanczosOpts& o);
+// Three-term recurrence in FP64 from a host vector; see lanczos_dev.cu.
+double three_term_f64(Hamiltonian& H, const cd* v_ref, int n_steps, double min_norm, std::vector<double>& alphas,
+                      std::vector<double>& betas);
 
 // ---- continued fraction (src/solvers/dynamics.cpp:13-89) --------------------------
 struct CFOut { std::vector<double> alphas, betas; double norm = 0.0; };

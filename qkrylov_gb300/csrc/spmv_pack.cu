@@ -369,57 +369,85 @@ __global__ void __launch_bounds__(kThreads, kCtas32)
     }
 }
 
-// FP64.  EQUAL: every amplitude has the same magnitude p.u (sums of aligned integers).
-template <int MODE, bool CPLX, bool EQUAL, int NQ>
+// FP64.  EQUAL: every amplitude has the same magnitude p.u (sums of aligned
+// integers).  LZ as above.
+template <int MODE, bool CPLX, bool EQUAL, bool LZ, int NQ>
 __global__ void __launch_bounds__(kThreads, kCtas64)
-    pack64_kernel(const Params<double> p, const double2* __restrict__ x, double2* __restrict__ y) {
+    pack64_kernel(const Params<double> p, const double2* __restrict__ x_in, double2* __restrict__ y_in) {
     __shared__ double s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
     if (MODE == AMP_CODED) load_amps(p, s_amp);
+    const double2* __restrict__ x = x_in;
+    double2* __restrict__ y = y_in;
+    double scale = 1.0, bprev = 0.0, dot = 0.0;
+    const double2* __restrict__ vprev = nullptr;
+    if (LZ) {
+        const LzOperands o = *p.lz;
+        x = static_cast<const double2*>(o.x);
+        y = static_cast<double2*>(o.y);
+        vprev = static_cast<const double2*>(o.vprev);
+        scale = o.scale;
+        bprev = o.bprev;
+    }
     const uint32_t wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     const uint32_t id = NQ == 4 ? wid : wid >> 2, q0 = NQ == 4 ? 0u : wid & 3u;
-    if (id >= p.n_items) return;
-    const uint4 i4 = __ldg(reinterpret_cast<const uint4*>(p.items) + id);
-    const Item it{i4.x, i4.y, i4.z, i4.w};
-    const uint32_t cnt = it.tc & 0xFFu;
-    double orr[NQ], oi[NQ];
-    bool redo = !EQUAL;
-    if constexpr (EQUAL) {
-        SumI64 acc[NQ];
-        walk<double, SumI64, MODE, false, NQ>(p, it, q0, x, s_amp, acc);
-        const double v = fabs(p.u) * 0x1p-56;
-        bool bad = false;
+    if (id < p.n_items) {
+        const uint4 i4 = __ldg(reinterpret_cast<const uint4*>(p.items) + id);
+        const Item it{i4.x, i4.y, i4.z, i4.w};
+        const uint32_t cnt = it.tc & 0xFFu;
+        double orr[NQ], oi[NQ];
+        bool redo = !EQUAL;
+        if constexpr (EQUAL) {
+            SumI64 acc[NQ];
+            walk<double, SumI64, MODE, false, NQ>(p, it, q0, x, s_amp, acc);
+            const double v = fabs(p.u) * 0x1p-56;
+            bool bad = false;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                bad = bad || (lane + 32u * (q0 + q) < cnt && acc[q].bad());
+                orr[q] = acc[q].r.value(v);
+                oi[q] = acc[q].i.value(v);
+            }
+            redo = __any_sync(0xffffffffu, bad);
+        }
+        if (redo) {
+            SumF64 acc[NQ];
+            walk<double, SumF64, MODE, CPLX, NQ>(p, it, q0, x, s_amp, acc);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                orr[q] = acc[q].r;
+                oi[q] = acc[q].i;
+            }
+        }
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            bad = bad || (lane + 32u * (q0 + q) < cnt && acc[q].bad());
-            orr[q] = acc[q].r.value(v);
-            oi[q] = acc[q].i.value(v);
+            if (lane + 32u * (q0 + q) >= cnt) continue;
+            const uint32_t row = it.row0 + lane + 32u * (q0 + q);
+            double dr, di;
+            diag_at(p, row, dr, di);
+            const double2 xv = __ldg(x + row);
+            double2 o;
+            o.x = fma(dr, xv.x, orr[q]);
+            o.y = fma(dr, xv.y, oi[q]);
+            if (p.cdiag) {
+                o.x = fma(-di, xv.y, o.x);
+                o.y = fma(di, xv.x, o.y);
+            }
+            if (LZ) {
+                o.x *= scale;
+                o.y *= scale;
+                if (vprev) {
+                    const double2 pv = __ldcs(vprev + row);
+                    o.x = fma(-bprev, pv.x, o.x);
+                    o.y = fma(-bprev, pv.y, o.y);
+                }
+                dot = fma(xv.y, o.y, fma(xv.x, o.x, dot));
+            }
+            __stcs(y + row, o);
         }
-        redo = __any_sync(0xffffffffu, bad);
     }
-    if (redo) {
-        SumF64 acc[NQ];
-        walk<double, SumF64, MODE, CPLX, NQ>(p, it, q0, x, s_amp, acc);
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            orr[q] = acc[q].r;
-            oi[q] = acc[q].i;
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        if (lane + 32u * (q0 + q) >= cnt) continue;
-        const uint32_t row = it.row0 + lane + 32u * (q0 + q);
-        double dr, di;
-        diag_at(p, row, dr, di);
-        const double2 xv = __ldg(x + row);
-        double2 o;
-        o.x = fma(dr, xv.x, orr[q]);
-        o.y = fma(dr, xv.y, oi[q]);
-        if (p.cdiag) {
-            o.x = fma(-di, xv.y, o.x);
-            o.y = fma(di, xv.x, o.y);
-        }
-        __stcs(y + row, o);
+    if (LZ) {
+        dot = block_sum_d(dot);
+        if (threadIdx.x == 0) p.apart[blockIdx.x] = make_double2(dot, 0.0);
     }
 }
 
@@ -473,11 +501,13 @@ void pack_apply_f64(const PackPlan& P, Params<double>& p, const double2* x, doub
         constexpr bool C = decltype(c)::value;
         if constexpr (M != AMP_CODED) {
             if (P.equal_magnitude()) {
-                pack64_kernel<M, C, true, N><<<g, t, 0, s>>>(p, x, y);
+                if (p.lz) pack64_kernel<M, C, true, true, N><<<g, t, 0, s>>>(p, x, y);
+                else pack64_kernel<M, C, true, false, N><<<g, t, 0, s>>>(p, x, y);
                 return;
             }
         }
-        pack64_kernel<M, C, false, N><<<g, t, 0, s>>>(p, x, y);
+        if (p.lz) pack64_kernel<M, C, false, true, N><<<g, t, 0, s>>>(p, x, y);
+        else pack64_kernel<M, C, false, false, N><<<g, t, 0, s>>>(p, x, y);
     });
     QKG_LAUNCHED();
 }
