@@ -624,7 +624,7 @@ public:
                 mode_ = plan_of[h]->mode();
                 n = (plan_of[h]->n_items() + run_ - 1) / run_;
             } else {
-                std::memset(&P[h], 0, sizeof(P[h]));
+                P[h] = packk::Params<T>{};
             }
             range.push_back(range.back() + n);
             rrange.push_back(rrange.back() + (uint32_t)((H.dim() + blockk::kRowChunk - 1) / blockk::kRowChunk));

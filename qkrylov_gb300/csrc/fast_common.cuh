@@ -165,6 +165,56 @@ __device__ __forceinline__ double block_sum_d(double v) {
     return v;
 }
 
+// Whether this CTA is the last of the grid to get here; its threads then see what
+// every CTA wrote to global memory before.  `arrived` is 0 again afterwards.
+__device__ __forceinline__ bool last_cta(unsigned int* arrived) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    if (threadIdx.x == 0) *arrived = 0u;
+    return true;
+}
+// Sum of n partials (real parts) by one CTA, valid in thread 0.
+__device__ __forceinline__ double sum_partials(const double2* part, int n) {
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s += __ldcg(&part[i].x);
+    return block_sum_d(s);
+}
+// Step k's scalars (one thread).
+__device__ __forceinline__ void lz_set_alpha(const LzDev& d, double xy) {
+    const int k = d.st->k;
+    const double a = d.sig[k] * xy;
+    d.alpha[k] = a;
+    d.alpha_host[k] = a;
+    d.st->a = a * d.sig[k];
+}
+// beta_k, sig_{k+1}, k + 1, and the next step's SpMV operands:
+// y = sig_{k+1} H V_{k+1} - beta_k sig_k V_k into V_{k+2}.
+__device__ __forceinline__ void lz_set_beta(const LzDev& d, int k, double norm2) {
+    const double b = sqrt(norm2);
+    const double sn = b > 0.0 ? 1.0 / b : 0.0;
+    d.beta[k] = b;
+    d.beta_host[k] = b;
+    d.sig[k + 1] = sn;
+    d.st->k = k + 1;
+    LzOperands o;
+    o.x = d.vtab[min(k + 1, d.nmax)];
+    o.y = d.vtab[min(k + 2, d.nmax)];  // no step runs past nmax - 1
+    o.vprev = d.vtab[k];
+    o.scale = sn;
+    o.bprev = b * d.sig[k];
+    o.scale32 = (float)o.scale;
+    o.bprev32 = (float)o.bprev;
+    *d.op = o;
+}
+
 __device__ __forceinline__ bool in_basis_fast(int ng, uint32_t g0, uint32_t g1, int p0, int p1, int no_double, int N,
                                               uint32_t s) {
     if (ng > 0 && __popc(s & g0) != p0) return false;

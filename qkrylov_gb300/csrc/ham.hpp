@@ -68,9 +68,28 @@ struct LzOperands {
     double scale = 1.0, bprev = 0.0;
     float scale32 = 1.f, bprev32 = 0.f;  // the same, rounded once for FP32 kernels
 };
+constexpr int kMaxLzRitz = 4;  // Ritz vectors a device-resident run may hold
+struct LzState {
+    int k;
+    int orth;               // this step's correction along the Ritz vectors is still to be applied
+    double a;               // update coefficient of the current step
+    double pre[kMaxLzRitz], pim[kMaxLzRitz];  // projections on the Ritz vectors (selective reorthogonalisation)
+};
+// The recurrence's scalars on the device: v_k = sig[k] V_k, alpha and beta (also
+// written to mapped host memory), the vectors' pointers V_0 .. V_nmax, the next
+// SpMV's operands, and a counter of CTAs that have finished.
+struct LzDev {
+    LzState* st = nullptr;
+    double *alpha = nullptr, *beta = nullptr, *sig = nullptr, *alpha_host = nullptr, *beta_host = nullptr;
+    void* const* vtab = nullptr;
+    int nmax = 0;
+    LzOperands* op = nullptr;
+    unsigned int* arrived = nullptr;
+};
 struct LanczosHooks {
     const LzOperands* op = nullptr;  // device
     double2* apart = nullptr;        // per-block partials of Re<x, y>
+    LzDev fin;                       // st set: the SpMV's last CTA adds the partials and sets alpha
 };
 
 namespace fastk {

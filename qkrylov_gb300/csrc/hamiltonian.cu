@@ -1848,6 +1848,7 @@ void Hamiltonian::apply_lanczos_f32(const LanczosHooks& lz, cudaStream_t s) cons
         pack_params(p, *pack_);
         p.lz = lz.op;
         p.apart = lz.apart;
+        p.fin = lz.fin;
         pack_apply_f32(*pack_, p, nullptr, nullptr, s);
         return;
     }
@@ -1876,6 +1877,7 @@ bool Hamiltonian::apply_lanczos_f64(const LanczosHooks& lz, cudaStream_t s) cons
     pack_params(p, *pack_);
     p.lz = lz.op;
     p.apart = lz.apart;
+    p.fin = lz.fin;
     pack_apply_f64(*pack_, p, nullptr, nullptr, s);
     return true;
 }

@@ -253,45 +253,57 @@ __global__ void lupd32_kernel(float2* __restrict__ w, const float2* __restrict__
 // columns of one row chunk run side by side on the same elements and w (or W)
 // comes from DRAM once and from L2 for the other columns.
 constexpr int KB = 8;
-template <class T2, bool F32>
-__global__ void mdot_kernel(const T2* const* __restrict__ V, int k, const T2* __restrict__ w, uint64_t n, double2* part,
-                            int stride) {
+// FP64 projections <V_j, w> for up to KB vectors per block column.  Bound by the FP64
+// pipe (four FMAs an element of V), so the CTA's sums are arranged to cost it little:
+// the threads' values go through shared memory and each thread adds sixteen of them, 17
+// double additions a warp where shuffles would take 160 (n = 184,756, 40 vectors: 97 us).
+__global__ void __launch_bounds__(kThreads) mdot64_kernel(const double2* const* __restrict__ V, int k,
+                                                          const double2* __restrict__ w, uint64_t n, double2* part,
+                                                          int stride) {
+    __shared__ double red[kThreads][2 * KB + 1];
     const int j0 = blockIdx.x * KB;
     const int kk = min(KB, k - j0);
     double re[KB], im[KB];
-    FF fre[KB], fim[KB];
+    const double2* vp[KB];
 #pragma unroll
-    for (int q = 0; q < KB; ++q) { re[q] = im[q] = 0.0; fre[q] = fim[q] = FF{0.f, 0.f}; }
-    const T2* vp[KB];
-#pragma unroll
-    for (int q = 0; q < KB; ++q) vp[q] = (q < kk) ? V[j0 + q] : nullptr;
+    for (int q = 0; q < KB; ++q) {
+        re[q] = im[q] = 0.0;
+        vp[q] = V[j0 + (q < kk ? q : 0)];
+    }
     for (uint64_t i = blockIdx.y * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.y * blockDim.x) {
-        const T2 b = w[i];
+        const double2 b = w[i];
 #pragma unroll
         for (int q = 0; q < KB; ++q) {
             if (q < kk) {
-                const T2 a = vp[q][i];
-                if (F32) {
-                    ff_add_prod(fre[q], (float)a.x, (float)b.x);
-                    ff_add_prod(fre[q], (float)a.y, (float)b.y);
-                    ff_add_prod(fim[q], (float)a.x, (float)b.y);
-                    ff_add_prod(fim[q], -(float)a.y, (float)b.x);
-                } else {
-                    re[q] = fma((double)a.x, (double)b.x, re[q]);
-                    re[q] = fma((double)a.y, (double)b.y, re[q]);
-                    im[q] = fma((double)a.x, (double)b.y, im[q]);
-                    im[q] = fma(-(double)a.y, (double)b.x, im[q]);
-                }
+                const double2 a = vp[q][i];
+                re[q] = fma(a.x, b.x, re[q]);
+                im[q] = fma(a.x, b.y, im[q]);
+                re[q] = fma(a.y, b.y, re[q]);
+                im[q] = fma(-a.y, b.x, im[q]);
             }
         }
     }
 #pragma unroll
     for (int q = 0; q < KB; ++q) {
-        if (q < kk) {
-            const double2 v = F32 ? make_double2(ff_value(fre[q]), ff_value(fim[q])) : make_double2(re[q], im[q]);
-            const double2 s = block_sum(v);
-            if (threadIdx.x == 0) part[(size_t)(j0 + q) * stride + blockIdx.y] = s;
-        }
+        red[threadIdx.x][2 * q] = re[q];
+        red[threadIdx.x][2 * q + 1] = im[q];
+    }
+    __syncthreads();
+    // thread t: value t % 16 of the threads 16 (t / 16) ..
+    static_assert(2 * KB == 16 && kThreads == 256, "sixteen values, sixteen groups of sixteen threads");
+    const int v = threadIdx.x & 15, g = threadIdx.x >> 4;
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s += red[16 * g + i][v];
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    __syncthreads();
+    if ((threadIdx.x & 16) == 0) red[threadIdx.x >> 5][v] = s;
+    __syncthreads();
+    if (threadIdx.x < 16 && (v >> 1) < kk) {
+        double t = 0.0;
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; ++i) t += red[i][v];
+        reinterpret_cast<double*>(part + (size_t)(j0 + (v >> 1)) * stride + blockIdx.y)[v & 1] = t;
     }
 }
 
@@ -733,8 +745,10 @@ static void mdot_impl(const T2* const* V, int k, const T2* w, uint64_t n, std::c
         mdot32_kernel<<<grid, kThreads, 0, s>>>(reinterpret_cast<const float2* const*>(V), k,
                                                 reinterpret_cast<const float2*>(w), n, ws.partial.as<double2>(), g);
     } else {
-        dim3 grid((k + KB - 1) / KB, g);
-        mdot_kernel<T2, F32><<<grid, kThreads, 0, s>>>(V, k, w, n, ws.partial.as<double2>(), g);
+        g = std::max(1, std::min(g, mdot_f64_chunks(k, n)));
+        mdot64_kernel<<<dim3((k + KB - 1) / KB, g), kThreads, 0, s>>>(reinterpret_cast<const double2* const*>(V), k,
+                                                                     reinterpret_cast<const double2*>(w), n,
+                                                                     ws.partial.as<double2>(), g);
     }
     QKG_LAUNCHED();
     const double2* r = finish(ws, g, g, k, s);
@@ -744,14 +758,13 @@ void mdot_f64(const double2* const* V, int k, const double2* w, uint64_t n, std:
               cudaStream_t s) {
     mdot_impl<double2, false>(V, k, w, n, out, ws, s);
 }
-// Row chunks of the FP64 projections: every CTA ends with two double sums a vector
-// over its threads, which cost more than an element's products on the FP64 pipe, so
-// the chunks are few (six CTAs a SM over all columns) and a thread has at least four
+// Row chunks of the FP64 projections: every CTA ends with sums over its threads, so
+// the chunks are few (four CTAs a SM over all columns) and a thread has at least four
 // elements where there are that many.
 int mdot_f64_chunks(int k, uint64_t n) {
     const int cols = std::max(1, (k + KB - 1) / KB);
     const uint64_t most = std::max<uint64_t>(1, n / (4 * kThreads));
-    return (int)std::max<uint64_t>(1, std::min<uint64_t>(most, std::max(8, 152 * 6 / cols)));
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(most, std::max(8, 152 * 4 / cols)));
 }
 size_t mdot_f64_most_partials(int k_max, uint64_t n) {
     size_t m = 0;
@@ -761,7 +774,7 @@ size_t mdot_f64_most_partials(int k_max, uint64_t n) {
 void mdot_f64_partials(const double2* const* V, int k, const double2* w, uint64_t n, double2* part, int g,
                        cudaStream_t s) {
     if (k <= 0) return;
-    mdot_kernel<double2, false><<<dim3((k + KB - 1) / KB, g), kThreads, 0, s>>>(V, k, w, n, part, g);
+    mdot64_kernel<<<dim3((k + KB - 1) / KB, g), kThreads, 0, s>>>(V, k, w, n, part, g);
     QKG_LAUNCHED();
 }
 void mdot_f32(const float2* const* V, int k, const float2* w, uint64_t n, std::complex<double>* out, Workspace& ws,

@@ -1,4 +1,4 @@
-// Device-resident mixed-precision Lanczos: one step = four kernels that read
+// Device-resident mixed-precision Lanczos: one step = two or three kernels that read
 // the step index, the vector pointers and the recurrence scalars from device
 // memory, so the step is captured once as a CUDA graph and replayed.
 //
@@ -12,13 +12,16 @@
 //      sig_k * sum = <v_k, H v_k - beta_{k-1} v_{k-1}> (the modified
 //      Gram-Schmidt order of Paige's Lanczos variant: equal to <v_k, H v_k> in
 //      exact arithmetic, one pass over a vector fewer per step).
-//   2. lz_alpha: alpha_k and the coefficient a = alpha_k sig_k.
-//   3. lz_update: V_{k+1} -= a V_k; compensated |V_{k+1}|^2 partials.
-//      (selective reorthogonalisation adds lz_proj, lz_proj_finish, lz_orth)
-//   4. lz_beta: beta_k, sig_{k+1}, k += 1.
+//      The last CTA adds the partials and sets alpha_k and a = alpha_k sig_k (a
+//      kernel of its own, lz_alpha, where the grid is large).
+//   2. lz_update: V_{k+1} -= a V_k; compensated |V_{k+1}|^2, and the projections on
+//      the Ritz vectors held; the last CTA sets beta_k, sig_{k+1} and k += 1.
+//   3. lz_orth, with Ritz vectors held: the correction along them where the
+//      projections ask for it, and beta_k from the corrected vector.
 // alpha/beta are also written to mapped pinned host memory; the host reads
 // them a few steps behind the GPU (convergence test, selective
 // reorthogonalisation trigger) without stalling the stream.
+#include "fast_common.cuh"
 #include "solvers.hpp"
 
 #include <algorithm>
@@ -29,6 +32,7 @@
 #include <type_traits>
 
 namespace qkg {
+using namespace fastk;
 
 namespace {
 constexpr int kT = 256;
@@ -38,13 +42,8 @@ constexpr int kInFlight = 6;    // steps the host lets the GPU run ahead of its 
 constexpr double kOrthTol = 3.4526698300124393e-4;  // sqrt(2^-23): FP32 semiorthogonality level
 
 constexpr int kMaxPsi = kMaxRitzLocked;  // converged Ritz vectors held for selective reorthogonalisation
+static_assert(kMaxPsi <= kMaxLzRitz, "the step's state holds a projection for every Ritz vector");
 
-struct LzState {
-    int k;
-    int orth;               // this step's correction along the Ritz vectors is applied
-    double a, b;            // update coefficients of the current step
-    double pre[kMaxPsi], pim[kMaxPsi];  // projections on the Ritz vectors (selective reorthogonalisation)
-};
 struct PsiTab {
     const float2* p[kMaxPsi];
 };
@@ -58,59 +57,32 @@ __device__ __forceinline__ void ff_acc(float& hi, float& lo, float a, float b) {
     hi = t;
 }
 
-__device__ __forceinline__ double2 bsum2(double x, double y) {
-    __shared__ double2 sh[32];
-    for (int o = 16; o > 0; o >>= 1) {
-        x += __shfl_down_sync(0xffffffffu, x, o);
-        y += __shfl_down_sync(0xffffffffu, y, o);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[wid] = make_double2(x, y);
-    __syncthreads();
-    double2 v = (threadIdx.x < (blockDim.x >> 5)) ? sh[lane] : make_double2(0.0, 0.0);
-    if (wid == 0)
-        for (int o = 16; o > 0; o >>= 1) {
-            v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-            v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-        }
-    return v;
-}
-
-// alpha from the SpMV's per-CTA partials: kAlphaBlocks blocks sum fixed
-// slices, the last block to finish (arrival counter) adds their sums in block
-// order and does the step's bookkeeping; the result does not depend on which
-// block finishes last.
-constexpr int kAlphaBlocks = 64;
-__global__ void lz_alpha_kernel(const double2* __restrict__ apart, int nparts, LzState* st, double* alpha,
-                                const double* beta, const double* sig, double* alpha_host, double* part2,
-                                unsigned int* arrived) {
+// alpha from the SpMV's per-CTA partials where its grid is too large for its last
+// CTA to add them: blocks sum fixed slices, the last one to finish adds their sums in
+// block order; the result does not depend on which block that is.
+constexpr int kAlphaBlocks = 64, kAlphaThreads = 1024;
+// SpMV grids up to this add their own partials: every CTA then passes a fence and an
+// atomic, 4 us on 380 CTAs (L = 18, FP64) where the kernel of its own takes 7, but 7 us on
+// 1,700 (L = 20) and 15 us on 5,400 (L = 24, FP32).
+constexpr int kFusedParts = 1024;
+// One block for up to eight partials a thread.
+inline int alpha_blocks(int nparts) { return nparts <= 8 * kAlphaThreads ? 1 : kAlphaBlocks; }
+__global__ void __launch_bounds__(kAlphaThreads) lz_alpha_kernel(const double2* __restrict__ apart, int nparts, const LzDev d, double2* part2) {
     double s = 0.0;
+#pragma unroll 8
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nparts; i += gridDim.x * blockDim.x) s += apart[i].x;
-    const double2 t = bsum2(s, 0.0);
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        part2[blockIdx.x] = t.x;
-        __threadfence();
-        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    s = block_sum_d(s);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) lz_set_alpha(d, s);
+        return;
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const double v = threadIdx.x < gridDim.x ? *(volatile double*)(part2 + threadIdx.x) : 0.0;
-    const double2 u = bsum2(v, 0.0);
-    if (threadIdx.x == 0) {
-        const int k = st->k;
-        const double a = sig[k] * u.x;
-        alpha[k] = a;
-        alpha_host[k] = a;
-        st->a = a * sig[k];
-        st->b = 0.0;  // the SpMV already subtracted beta_{k-1} v_{k-1}
-        *arrived = 0u;  // ready for the next step
-    }
+    if (threadIdx.x == 0) part2[blockIdx.x] = make_double2(s, 0.0);
+    if (!last_cta(d.arrived)) return;
+    const double t = sum_partials(part2, gridDim.x);
+    if (threadIdx.x == 0) lz_set_alpha(d, t);
 }
 
-// One element of the update w -= a v + b v_prev with its ||w||^2 (and, with
+// One element of the update w -= a v with its ||w||^2 (and, with
 // NP Ritz vectors psi_p, the <psi_p, w>) contributions.
 template <int NP>
 struct UpdAcc {
@@ -118,14 +90,9 @@ struct UpdAcc {
     float rh[NP > 0 ? NP : 1] = {}, rl[NP > 0 ? NP : 1] = {}, ih[NP > 0 ? NP : 1] = {}, il[NP > 0 ? NP : 1] = {};
 };
 template <int NP>
-__device__ __forceinline__ float2 upd_elem(float2 x, float2 c, float2 d, const float2 (&p)[NP > 0 ? NP : 1], float a,
-                                           float b, bool has_prev, UpdAcc<NP>& s) {
+__device__ __forceinline__ float2 upd_elem(float2 x, float2 c, const float2 (&p)[NP > 0 ? NP : 1], float a, UpdAcc<NP>& s) {
     x.x = fmaf(-a, c.x, x.x);
     x.y = fmaf(-a, c.y, x.y);
-    if (has_prev) {
-        x.x = fmaf(-b, d.x, x.x);
-        x.y = fmaf(-b, d.y, x.y);
-    }
     ff_acc(s.hi, s.lo, x.x, x.x);
     ff_acc(s.hi, s.lo, x.y, x.y);
 #pragma unroll
@@ -138,28 +105,24 @@ __device__ __forceinline__ float2 upd_elem(float2 x, float2 c, float2 d, const f
     return x;
 }
 
-// w -= a v + b v_prev in place (b = 0: the SpMV applied the previous-vector
-// term, and v_prev is not read), ||w||^2 partials (and the <psi_q, w> partials
-// of the NP Ritz vectors, for selective reorthogonalisation): two elements per
-// thread and iteration with 16-byte accesses (the Krylov vectors are 256-byte
-// aligned).  ppart[q * gridDim.x + block] holds Ritz vector q's partial.
+// w -= a v in place (the SpMV applied the previous-vector term), ||w||^2 (and the
+// <psi_q, w> of the NP Ritz vectors, for selective reorthogonalisation), and from them
+// beta: two elements per thread and iteration with 16-byte accesses (the Krylov vectors
+// are 256-byte aligned).  ppart[q * gridDim.x + block] holds Ritz vector q's partial.
 template <int NP>
-__global__ void lz_update_t(void* const* __restrict__ vtab, const LzState* __restrict__ st, uint64_t n,
-                            const PsiTab psi, double2* __restrict__ bpart, double2* __restrict__ ppart) {
-    const int k = st->k;
-    float2* __restrict__ w = static_cast<float2*>(vtab[k + 1]);
-    const float2* __restrict__ v = static_cast<const float2*>(vtab[k]);
-    const float a = (float)st->a, b = (float)st->b;
-    const bool has_prev = k > 0 && b != 0.f;
-    const float2* __restrict__ vp = has_prev ? static_cast<const float2*>(vtab[k - 1]) : v;
+__global__ void __launch_bounds__(kT) lz_update_t(const LzDev d, uint64_t n, const PsiTab psi, double orth_tol,
+                                                  double2* __restrict__ bpart, double2* __restrict__ ppart) {
+    const int k = d.st->k;
+    float2* __restrict__ w = static_cast<float2*>(d.vtab[k + 1]);
+    const float2* __restrict__ v = static_cast<const float2*>(d.vtab[k]);
+    const float a = (float)d.st->a;
     UpdAcc<NP> s;
     constexpr int NQ = NP > 0 ? NP : 1;
     const uint64_t n2 = n / 2, step = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll 2
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n2; i += step) {
         const float4 x4 = reinterpret_cast<const float4*>(w)[i];
         const float4 c4 = reinterpret_cast<const float4*>(v)[i];
-        float4 d4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (has_prev) d4 = reinterpret_cast<const float4*>(vp)[i];
         float2 p0[NQ], p1[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
@@ -168,67 +131,70 @@ __global__ void lz_update_t(void* const* __restrict__ vtab, const LzState* __res
             p0[q] = make_float2(p4.x, p4.y);
             p1[q] = make_float2(p4.z, p4.w);
         }
-        const float2 y0 = upd_elem<NP>(make_float2(x4.x, x4.y), make_float2(c4.x, c4.y), make_float2(d4.x, d4.y),
-                                       p0, a, b, has_prev, s);
-        const float2 y1 = upd_elem<NP>(make_float2(x4.z, x4.w), make_float2(c4.z, c4.w), make_float2(d4.z, d4.w),
-                                       p1, a, b, has_prev, s);
+        const float2 y0 = upd_elem<NP>(make_float2(x4.x, x4.y), make_float2(c4.x, c4.y), p0, a, s);
+        const float2 y1 = upd_elem<NP>(make_float2(x4.z, x4.w), make_float2(c4.z, c4.w), p1, a, s);
         reinterpret_cast<float4*>(w)[i] = make_float4(y0.x, y0.y, y1.x, y1.y);
     }
     if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
         float2 pl[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) pl[q] = q < NP ? psi.p[q][n - 1] : make_float2(0.f, 0.f);
-        w[n - 1] = upd_elem<NP>(w[n - 1], v[n - 1], vp[n - 1], pl, a, b, has_prev, s);
+        w[n - 1] = upd_elem<NP>(w[n - 1], v[n - 1], pl, a, s);
     }
-    const double2 t = bsum2((double)s.hi + (double)s.lo, 0.0);
+    // block sums in float-float FP32 arithmetic: a double sum in each of the CTAs
+    // cost as much as the pass on GB300's narrow FP64 pipe (L = 24, no Ritz vector 18.5
+    // us, one 29.5 us)
+    const float2 t = block_sum_ff(s.hi, s.lo);
+    if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2((double)t.x + (double)t.y, 0.0);
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        const double2 r = bsum2((double)s.rh[q] + (double)s.rl[q], (double)s.ih[q] + (double)s.il[q]);
-        if (threadIdx.x == 0) ppart[(size_t)q * gridDim.x + blockIdx.x] = r;
+        const float2 r = block_sum_ff(s.rh[q], s.rl[q]);
+        const float2 m = block_sum_ff(s.ih[q], s.il[q]);
+        if (threadIdx.x == 0)
+            ppart[(size_t)q * gridDim.x + blockIdx.x] = make_double2((double)r.x + (double)r.y, (double)m.x + (double)m.y);
     }
-    if (threadIdx.x == 0) bpart[blockIdx.x] = t;
-}
-
-// c_q = <psi_q, W> for the NP Ritz vectors; the correction is applied only
-// when some |c_q| exceeds orth_tol ||W|| (components below the square root of
-// the working precision are harmless, Parlett & Scott 1979), so most steps skip
-// the extra pass over W.
-template <int NP>
-__global__ void lz_proj_finish_kernel(const double2* __restrict__ ppart, const double2* __restrict__ bpart,
-                                      int nparts, LzState* st, double orth_tol) {
-    double w2 = 0.0;
-    for (int j = threadIdx.x; j < nparts; j += blockDim.x) w2 += bpart[j].x;
-    const double2 u = bsum2(w2, 0.0);
+    if (!last_cta(d.arrived)) return;
+    // the last CTA: ||w||^2, c_q = <psi_q, w>.  The correction is applied only when
+    // some |c_q| exceeds orth_tol ||w|| (components below the square root of the working
+    // precision are harmless, Parlett & Scott 1979), so most steps skip the extra pass.
+    const double w2 = sum_partials(bpart, gridDim.x);
     int orth = 0;
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        double r = 0.0, i = 0.0;
-        for (int j = threadIdx.x; j < nparts; j += blockDim.x) {
-            r += ppart[(size_t)q * nparts + j].x;
-            i += ppart[(size_t)q * nparts + j].y;
+        double r = 0.0, m = 0.0;
+        for (int j = threadIdx.x; j < gridDim.x; j += blockDim.x) {
+            const double2 e = __ldcg(ppart + (size_t)q * gridDim.x + j);
+            r += e.x;
+            m += e.y;
         }
-        const double2 t = bsum2(r, i);
+        r = block_sum_d(r);
+        m = block_sum_d(m);
         if (threadIdx.x == 0) {
-            st->pre[q] = t.x;
-            st->pim[q] = t.y;
-            orth |= (t.x * t.x + t.y * t.y) > orth_tol * orth_tol * u.x ? 1 : 0;
+            d.st->pre[q] = r;
+            d.st->pim[q] = m;
+            orth |= r * r + m * m > orth_tol * orth_tol * w2 ? 1 : 0;
         }
     }
-    if (threadIdx.x == 0) st->orth = orth;
+    if (threadIdx.x == 0) {
+        d.st->orth = orth;
+        if (!orth) lz_set_beta(d, k, w2);  // else after the correction
+    }
 }
-// W -= sum_q c_q psi_q with c_q = <psi_q, W>; |W|^2 partials.
+
+// W -= sum_q c_q psi_q with c_q = <psi_q, W>, then beta from the corrected W.
 template <int NP>
-__global__ void lz_orth_kernel(void* const* __restrict__ vtab, const LzState* __restrict__ st, const PsiTab psi,
-                               uint64_t n, double2* __restrict__ bpart) {
-    if (!st->orth) return;  // bpart keeps the partials of the unchanged W
-    float2* __restrict__ w = static_cast<float2*>(vtab[st->k + 1]);
+__global__ void __launch_bounds__(kT) lz_orth_kernel(const LzDev d, const PsiTab psi, uint64_t n, double2* __restrict__ bpart) {
+    if (!d.st->orth) return;
+    const int k = d.st->k;
+    float2* __restrict__ w = static_cast<float2*>(d.vtab[k + 1]);
     float cr[NP], ci[NP];
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        cr[q] = (float)st->pre[q];
-        ci[q] = (float)st->pim[q];
+        cr[q] = (float)d.st->pre[q];
+        ci[q] = (float)d.st->pim[q];
     }
     float hi = 0.f, lo = 0.f;
+#pragma unroll 2
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         float2 x = w[i];
 #pragma unroll
@@ -241,45 +207,33 @@ __global__ void lz_orth_kernel(void* const* __restrict__ vtab, const LzState* __
         ff_acc(hi, lo, x.x, x.x);
         ff_acc(hi, lo, x.y, x.y);
     }
-    const double2 s = bsum2((double)hi + (double)lo, 0.0);
-    if (threadIdx.x == 0) bpart[blockIdx.x] = s;
-}
-
-// beta_k, sig_{k+1}, k += 1, and the next step's SpMV operands:
-// y = sig_{k+1} H V_{k+1} - beta_k sig_k V_k into V_{k+2}.
-__global__ void lz_beta_kernel(const double2* __restrict__ bpart, int nparts, LzState* st, double* beta, double* sig,
-                               double* beta_host, void* const* __restrict__ vtab, int nmax, LzOperands* op) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += bpart[i].x;
-    const double2 t = bsum2(s, 0.0);
+    const float2 s = block_sum_ff(hi, lo);
+    if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2((double)s.x + (double)s.y, 0.0);
+    if (!last_cta(d.arrived)) return;
+    const double w2 = sum_partials(bpart, gridDim.x);
     if (threadIdx.x == 0) {
-        const int k = st->k;
-        const double b = sqrt(t.x);
-        const double sn = b > 0.0 ? 1.0 / b : 0.0;
-        beta[k] = b;
-        beta_host[k] = b;
-        sig[k + 1] = sn;
-        st->k = k + 1;
-        LzOperands o;
-        o.x = vtab[min(k + 1, nmax)];
-        o.y = vtab[min(k + 2, nmax)];  // no step runs past nmax - 1
-        o.vprev = vtab[k];
-        o.scale = sn;
-        o.bprev = b * sig[k];
-        o.scale32 = (float)o.scale;
-        o.bprev32 = (float)o.bprev;
-        *op = o;
+        d.st->orth = 0;
+        lz_set_beta(d, k, w2);
     }
 }
 
 // ---- FP64 ---------------------------------------------------------------------
-// w -= a v in place, ||w||^2 partials.
-__global__ void lz64_update(void* const* __restrict__ vtab, const LzState* __restrict__ st, uint64_t n,
-                            double2* __restrict__ bpart) {
-    const int k = st->k;
-    double2* __restrict__ w = static_cast<double2*>(vtab[k + 1]);
-    const double2* __restrict__ v = static_cast<const double2*>(vtab[k]);
-    const double a = -st->a;
+// Per-CTA partials of ||w||^2; the last CTA adds them and sets beta_k.
+__device__ __forceinline__ void finish_beta(const LzDev& d, int k, double acc, double2* bpart) {
+    const double t = block_sum_d(acc);
+    if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2(t, 0.0);
+    if (!last_cta(d.arrived)) return;
+    const double w2 = sum_partials(bpart, gridDim.x);
+    if (threadIdx.x == 0) lz_set_beta(d, k, w2);
+}
+// w -= a v in place, and beta.
+// FULL: a reorthogonalisation follows, which sets beta.
+template <bool FULL>
+__global__ void __launch_bounds__(kT) lz64_update(const LzDev d, uint64_t n, double2* __restrict__ bpart) {
+    const int k = d.st->k;
+    double2* __restrict__ w = static_cast<double2*>(d.vtab[k + 1]);
+    const double2* __restrict__ v = static_cast<const double2*>(d.vtab[k]);
+    const double a = -d.st->a;
     double acc = 0.0;
 #pragma unroll 4
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -288,10 +242,9 @@ __global__ void lz64_update(void* const* __restrict__ vtab, const LzState* __res
         x.x = fma(a, c.x, x.x);
         x.y = fma(a, c.y, x.y);
         w[i] = x;
-        acc = fma(x.y, x.y, fma(x.x, x.x, acc));
+        if (!FULL) acc = fma(x.y, x.y, fma(x.x, x.x, acc));
     }
-    const double2 t = bsum2(acc, 0.0);
-    if (threadIdx.x == 0) bpart[blockIdx.x] = t;
+    if (!FULL) finish_beta(d, k, acc, bpart);
 }
 // y = scale y - bprev vprev and Re<x, y> partials, for an SpMV that does not do it.
 __global__ void lz64_post(const LzOperands* __restrict__ op, uint64_t n, double2* __restrict__ apart) {
@@ -313,8 +266,8 @@ __global__ void lz64_post(const LzOperands* __restrict__ op, uint64_t n, double2
         y[i] = w;
         acc = fma(c.y, w.y, fma(c.x, w.x, acc));
     }
-    const double2 t = bsum2(acc, 0.0);
-    if (threadIdx.x == 0) apart[blockIdx.x] = t;
+    acc = block_sum_d(acc);
+    if (threadIdx.x == 0) apart[blockIdx.x] = make_double2(acc, 0.0);
 }
 // coef_j = -sig_j^2 <V_j, w> from the projections' partials (column j at part[j * nparts]).
 __global__ void lz64_coef(const double2* __restrict__ part, int nparts, const double* __restrict__ sig,
@@ -326,15 +279,17 @@ __global__ void lz64_coef(const double2* __restrict__ part, int nparts, const do
         re += v.x;
         im += v.y;
     }
-    const double2 s = bsum2(re, im);
+    re = block_sum_d(re);
+    im = block_sum_d(im);
     if (threadIdx.x == 0) {
         const double f = -sig[j] * sig[j];
-        coef[j] = make_double2(f * s.x, f * s.y);
+        coef[j] = make_double2(f * re, f * im);
     }
 }
-// w += sum_j coef_j V_j (j < k), ||w||^2 partials; w = V_k.
-__global__ void __launch_bounds__(kT) lz64_subtract(void* const* __restrict__ vtab, int k, const double2* __restrict__ coef,
-                                                    uint64_t n, double2* __restrict__ bpart) {
+// w += sum_j coef_j V_j (j < k; w = V_k), and beta_{k-1}.
+__global__ void __launch_bounds__(kT) lz64_subtract(const LzDev d, int k, const double2* __restrict__ coef, uint64_t n,
+                                                    double2* __restrict__ bpart) {
+    void* const* vtab = d.vtab;
     extern __shared__ double2 s_c[];
     const double2** s_v = reinterpret_cast<const double2**>(s_c + k);
     for (int j = threadIdx.x; j < k; j += blockDim.x) {
@@ -366,8 +321,7 @@ __global__ void __launch_bounds__(kT) lz64_subtract(void* const* __restrict__ vt
         w[i] = x;
         acc = fma(x.y, x.y, fma(x.x, x.x, acc));
     }
-    const double2 t = bsum2(acc, 0.0);
-    if (threadIdx.x == 0) bpart[blockIdx.x] = t;
+    finish_beta(d, k - 1, acc, bpart);
 }
 
 using clk = std::chrono::steady_clock;
@@ -434,7 +388,7 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
     DBuf apart(std::max<size_t>(1, H.lanczos_parts()) * sizeof(double2)), bpart(kUpdGrid * sizeof(double2)),
         ppart((size_t)kMaxPsi * kUpdGrid * sizeof(double2)), psitab(kMaxPsi * sizeof(float2*));
     Mapped ah(nmax + 2), bh(nmax + 2);
-    DBuf part2(kAlphaBlocks * sizeof(double)), arrived(sizeof(unsigned int));
+    DBuf part2(kAlphaBlocks * sizeof(double2)), arrived(sizeof(unsigned int));
     QKG_CUDA(cudaMemsetAsync(arrived.p, 0, sizeof(unsigned int), st));
     Workspace ws(std::max<size_t>(1 << 16, (size_t)1216 * (size_t)(nmax + 2)));
     DBuf tmp;
@@ -475,10 +429,25 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
         QKG_CUDA(cudaStreamSynchronize(st));
     }
 
+    LzDev dev;
+    dev.st = state.as<LzState>();
+    dev.alpha = alpha.as<double>();
+    dev.beta = beta.as<double>();
+    dev.sig = sig.as<double>();
+    dev.alpha_host = ah.d;
+    dev.beta_host = bh.d;
+    dev.vtab = static_cast<void* const*>(vtab.p);
+    dev.nmax = nmax;
+    dev.op = lzop.as<LzOperands>();
+    dev.arrived = arrived.as<unsigned int>();
     LanczosHooks hooks;
     hooks.op = lzop.as<LzOperands>();
     hooks.apart = apart.as<double2>();
     const int nparts = (int)H.lanczos_parts();
+    const bool own_alpha = H.packed() && nparts <= kFusedParts;
+    if (own_alpha) hooks.fin = dev;
+    // CTAs of the update: four 16-byte elements a thread at least, up to a resident wave
+    const int ug = (int)std::max<uint64_t>(1, std::min<uint64_t>(n / (8 * kT), kUpdGrid));
     PsiTab psi{};   // converged Ritz vectors (selective reorthogonalisation)
     int npsi = 0;   // how many are held
     std::vector<double> locked;  // their Ritz values
@@ -486,21 +455,16 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
         if (timer) timer->start();
         H.apply_lanczos_f32(hooks, st);
         if (timer) timer->stop();
-        lz_alpha_kernel<<<kAlphaBlocks, kT, 0, st>>>(apart.as<double2>(), nparts, state.as<LzState>(),
-                                                     alpha.as<double>(), beta.as<double>(), sig.as<double>(), ah.d,
-                                                     part2.as<double>(), arrived.as<unsigned int>());
-        QKG_LAUNCHED();
-        void* const* vt = static_cast<void* const*>(vtab.p);
+        if (!own_alpha) {
+            lz_alpha_kernel<<<alpha_blocks(nparts), kAlphaThreads, 0, st>>>(apart.as<double2>(), nparts, dev, part2.as<double2>());
+            QKG_LAUNCHED();
+        }
         auto sel = [&](auto npc) {
             constexpr int NP = decltype(npc)::value;
-            lz_update_t<NP><<<kUpdGrid, kT, 0, st>>>(vt, state.as<LzState>(), n, psi, bpart.as<double2>(),
-                                                     ppart.as<double2>());
+            lz_update_t<NP><<<ug, kT, 0, st>>>(dev, n, psi, kOrthTol, bpart.as<double2>(), ppart.as<double2>());
             QKG_LAUNCHED();
             if constexpr (NP > 0) {
-                lz_proj_finish_kernel<NP><<<1, kT, 0, st>>>(ppart.as<double2>(), bpart.as<double2>(), kUpdGrid,
-                                                            state.as<LzState>(), kOrthTol);
-                QKG_LAUNCHED();
-                lz_orth_kernel<NP><<<kUpdGrid, kT, 0, st>>>(vt, state.as<LzState>(), psi, n, bpart.as<double2>());
+                lz_orth_kernel<NP><<<ug, kT, 0, st>>>(dev, psi, n, bpart.as<double2>());
                 QKG_LAUNCHED();
             }
         };
@@ -511,10 +475,6 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
             case 3: sel(std::integral_constant<int, 3>{}); break;
             default: sel(std::integral_constant<int, 4>{}); break;
         }
-        lz_beta_kernel<<<1, kT, 0, st>>>(bpart.as<double2>(), kUpdGrid, state.as<LzState>(), beta.as<double>(),
-                                         sig.as<double>(), bh.d, static_cast<void* const*>(vtab.p), nmax,
-                                         lzop.as<LzOperands>());
-        QKG_LAUNCHED();
     };
     int kernels[kMaxPsi + 1] = {};  // kernels per step graph (by Ritz vectors held), counted at capture
     auto capture = [&](int np) {
@@ -715,7 +675,7 @@ struct Recurrence64 {
         auto take = [&](size_t b) { const size_t o = off; off += al(b); return o; };
         const size_t o_st = take(sizeof(LzState)), o_op = take(sizeof(LzOperands)), o_tab = take(N * sizeof(void*)),
                      o_al = take(N * 8), o_be = take(N * 8), o_sg = take(N * 8), o_co = take((size_t)N * 16),
-                     o_ap = take((size_t)nparts * 16), o_bp = take((size_t)kUpdGrid * 16), o_p2 = take(kAlphaBlocks * 8),
+                     o_ap = take((size_t)nparts * 16), o_bp = take((size_t)kUpdGrid * 16), o_p2 = take(kAlphaBlocks * 16),
                      o_ar = take(sizeof(unsigned int));
         Workspace& ws = H.reduction_scratch(std::max<size_t>(1 << 16, off / sizeof(double2) + 1 + (full ? mdot_f64_most_partials(N, n) : 0)));
         char* base = ws.partial.as<char>();
@@ -726,7 +686,7 @@ struct Recurrence64 {
              *sig = reinterpret_cast<double*>(base + o_sg);
         auto* coef = reinterpret_cast<double2*>(base + o_co);
         auto *apart = reinterpret_cast<double2*>(base + o_ap), *bpart = reinterpret_cast<double2*>(base + o_bp);
-        auto* part2 = reinterpret_cast<double*>(base + o_p2);
+        auto* part2 = reinterpret_cast<double2*>(base + o_p2);
         auto* arrived = reinterpret_cast<unsigned int*>(base + o_ar);
         double2* ppart = reinterpret_cast<double2*>(base + off);
         const auto m = H.mapped_scalars(2 * (size_t)N);
@@ -750,9 +710,22 @@ struct Recurrence64 {
         std::memcpy(image.data() + o_tab, ptr.data(), (size_t)known * sizeof(void*));
         std::memcpy(image.data() + o_sg, &sig0, sizeof(double));
         QKG_CUDA(cudaMemcpyAsync(base, image.data(), image.size(), cudaMemcpyHostToDevice, st));
+        LzDev d;
+        d.st = state;
+        d.alpha = alpha;
+        d.beta = beta;
+        d.sig = sig;
+        d.alpha_host = m.dev;
+        d.beta_host = m.dev + N;
+        d.vtab = tab;
+        d.nmax = nmax;
+        d.op = op;
+        d.arrived = arrived;
         LanczosHooks hooks;
         hooks.op = op;
         hooks.apart = apart;
+        const bool own_alpha = H.packed() && nparts <= kFusedParts;
+        if (own_alpha) hooks.fin = d;
         struct Events {
             std::vector<cudaEvent_t> e;
             ~Events() { for (auto x : e) if (x) cudaEventDestroy(x); }
@@ -779,9 +752,12 @@ struct Recurrence64 {
                 lz64_post<<<kUpdGrid, kT, 0, st>>>(op, n, apart);
                 QKG_LAUNCHED();
             }
-            lz_alpha_kernel<<<kAlphaBlocks, kT, 0, st>>>(apart, nparts, state, alpha, beta, sig, m.dev, part2, arrived);
-            QKG_LAUNCHED();
-            lz64_update<<<g, kT, 0, st>>>(tab, state, n, bpart);
+            if (!own_alpha) {
+                lz_alpha_kernel<<<alpha_blocks(nparts), kAlphaThreads, 0, st>>>(apart, nparts, d, part2);
+                QKG_LAUNCHED();
+            }
+            if (full) lz64_update<true><<<g, kT, 0, st>>>(d, n, bpart);
+            else lz64_update<false><<<g, kT, 0, st>>>(d, n, bpart);
             QKG_LAUNCHED();
             if (full) {
                 const int gm = mdot_f64_chunks(k + 1, n);
@@ -789,11 +765,9 @@ struct Recurrence64 {
                                   n, ppart, gm, st);
                 lz64_coef<<<k + 1, kT, 0, st>>>(ppart, gm, sig, coef);
                 QKG_LAUNCHED();
-                lz64_subtract<<<g, kT, (size_t)(k + 1) * (sizeof(double2) + sizeof(void*)), st>>>(tab, k + 1, coef, n, bpart);
+                lz64_subtract<<<g, kT, (size_t)(k + 1) * (sizeof(double2) + sizeof(void*)), st>>>(d, k + 1, coef, n, bpart);
                 QKG_LAUNCHED();
             }
-            lz_beta_kernel<<<1, kT, 0, st>>>(bpart, g, state, beta, sig, m.dev + N, tab, nmax, op);
-            QKG_LAUNCHED();
         };
         try {
             while (launched < nmax && go) {

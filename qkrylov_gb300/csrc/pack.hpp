@@ -76,6 +76,7 @@ struct Params {
     const A* dtab;
     const LzOperands* lz;   // Lanczos mode, as FastParams::lz
     double2* apart;
+    LzDev fin;              // st set: the last CTA adds the partials and sets alpha
 };
 
 }  // namespace packk

@@ -553,7 +553,7 @@ int packed_apply_host(const Basis& B, SiteKind site, const std::vector<Term>& te
 
 template <class A>
 void PackPlan::params(Params<A>& p) const {
-    std::memset(&p, 0, sizeof(p));
+    p = Params<A>{};
     const bool d = sizeof(A) == 8;
     p.items = at<Item>(items_);
     p.n_items = n_items_;

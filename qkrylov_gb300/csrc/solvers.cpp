@@ -794,28 +794,6 @@ void ftlm_observables(const std::vector<FTLMTri>& tri, const double* betas, int 
 namespace {
 // Vector operations of one storage precision.
 template <class T2> struct DavOps;
-template <> struct DavOps<double2> {
-    static void apply(Hamiltonian& H, const double2* x, double2* y, cudaStream_t s) { H.apply_f64(x, y, s); }
-    static void mdot(const double2* const* V, int k, const double2* w, uint64_t n, cd* o, Workspace& ws, cudaStream_t s) {
-        mdot_f64(V, k, w, n, o, ws, s);
-    }
-    static void mcomb(const double2* const* V, int k, const cd* c, double2* w, uint64_t n, Workspace& ws, cudaStream_t s) {
-        mcombine_f64(V, k, c, w, n, ws, s);
-    }
-    static void mmulti(const double2* const* V, int k, const cd* c, double2* const* W, int no, uint64_t n, bool acc,
-                       Workspace& ws, cudaStream_t s) {
-        mcombine_multi_f64(V, k, c, W, no, n, acc, ws, s);
-    }
-    static double nrm2sq(const double2* x, uint64_t n, Workspace& ws, cudaStream_t s) { return nrm2sq_f64(x, n, ws, s); }
-    static void scal(double a, double2* x, uint64_t n, cudaStream_t s) { scal_f64(a, x, n, s); }
-    static void precond(const double2* r, const double2* d, double l, double2* t, uint64_t n, cudaStream_t s) {
-        davidson_precond_f64(r, d, l, t, n, s);
-    }
-    static void from64(const double2* x, double2* y, uint64_t n, cudaStream_t s) {
-        QKG_CUDA(cudaMemcpyAsync(y, x, n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
-    }
-    static void to64(const double2* x, double2* y, uint64_t n, cudaStream_t s) { from64(x, y, n, s); }
-};
 template <> struct DavOps<float2> {
     static void apply(Hamiltonian& H, const float2* x, float2* y, cudaStream_t s) { H.apply_f32(x, y, s); }
     static void mdot(const float2* const* V, int k, const float2* w, uint64_t n, cd* o, Workspace& ws, cudaStream_t s) {
@@ -845,10 +823,6 @@ inline void mdot_block(const float2* const* V, int k, float2* const* W, int nw, 
                        cudaStream_t s) {
     mdot_multi_f32(V, k, W, nw, n, o, ws, s);
 }
-inline void mdot_block(const double2* const*, int, double2* const*, int, uint64_t, cd*, Workspace&, cudaStream_t) {
-    QKG_REQUIRE(false, "block projection is used by the mixed form only");
-}
-
 // src/solvers/davidson.cpp:86-227 with the Krylov vectors stored in T2.
 // Projections <V_i, HV_j> of vectors that did not change are kept from the
 // previous iteration (the reference recomputes them; the values are the same
@@ -1101,10 +1075,6 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
 }
 }  // namespace
 
-DavidsonOut davidson_f64(Hamiltonian& H, int n_eig, int max_sub, double tol, bool want_vecs, bool f32_stream,
-                         int max_iter) {
-    return davidson_impl<double2>(H, n_eig, max_sub, tol, want_vecs, f32_stream, max_iter);
-}
 DavidsonOut davidson_mixed(Hamiltonian& H, int n_eig, int max_sub, double tol, bool want_vecs, int max_iter) {
     return davidson_impl<float2>(H, n_eig, max_sub, tol, want_vecs, false, max_iter);
 }

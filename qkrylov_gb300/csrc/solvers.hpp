@@ -119,6 +119,8 @@ private:
     cudaStream_t s_;
     cudaEvent_t a_ = nullptr, b_ = nullptr;
 };
+// Frees a Krylov workspace kept on H where `bytes` more would not fit beside it.
+void release_workspace_if_short(Hamiltonian& H, size_t bytes);
 // Plain FP64 path with the reference's semantics (full reorthogonalisation,
 // convergence when |E_k - E_{k-1}| < tol; src/solvers/lanczos.cpp:101-202).
 LanczosOut lanczos_f64(Hamiltonian& H, const LanczosOpts& o);

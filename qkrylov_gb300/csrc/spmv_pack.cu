@@ -310,6 +310,14 @@ __device__ __forceinline__ void diag_at(const Params<T>& p, uint32_t row, T& dr,
     di = __ldg(p.dtab + 2 * c + 1);
 }
 
+// Lanczos mode: the last CTA adds the grid's partials and sets alpha.
+template <class T>
+__device__ __forceinline__ void finish_alpha(const Params<T>& p) {
+    if (!p.fin.st || !last_cta(p.fin.arrived)) return;
+    const double t = sum_partials(p.apart, gridDim.x);
+    if (threadIdx.x == 0) lz_set_alpha(p.fin, t);
+}
+
 // FP32.  LZ: the Lanczos step's form (operands from *p.lz, y = scale H x -
 // bprev vprev, per-CTA partials of Re<x, y>).
 template <int MODE, bool CPLX, bool LZ, int NQ>
@@ -366,6 +374,7 @@ __global__ void __launch_bounds__(kThreads, kCtas32)
     if (LZ) {
         const float2 t = block_sum_ff(dot_hi, dot_lo);
         if (threadIdx.x == 0) p.apart[blockIdx.x] = make_double2((double)t.x + (double)t.y, 0.0);
+        finish_alpha(p);
     }
 }
 
@@ -448,6 +457,7 @@ __global__ void __launch_bounds__(kThreads, kCtas64)
     if (LZ) {
         dot = block_sum_d(dot);
         if (threadIdx.x == 0) p.apart[blockIdx.x] = make_double2(dot, 0.0);
+        finish_alpha(p);
     }
 }
 
