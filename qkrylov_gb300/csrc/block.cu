@@ -609,6 +609,9 @@ public:
         const uint32_t groups = blockk::kBT / std::max(1, Rp / (Rp % 4 == 0 ? 4 : Rp % 2 == 0 ? 2 : 1));
         run_ = (int)std::max<uint64_t>(1, std::min<uint64_t>({(uint64_t)kPasses * groups / blockk::kTile,
                                                               total / (152 * 4) / blockk::kTile, blockk::kMaxRun}));
+        // rows of an update CTA: a small batch is spread over the SMs (12-site sectors, 16
+        // vectors: 15.8 us an update with 512 rows a CTA)
+        chunk_ = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, total / (152 * 4) / 32 * 32));
         std::vector<packk::Params<T>> P(hs.size());
         std::vector<blockk::Ham> hams(hs.size());
         std::vector<uint32_t> range(1, 0), rrange(1, 0);
@@ -627,7 +630,7 @@ public:
                 P[h] = packk::Params<T>{};
             }
             range.push_back(range.back() + n);
-            rrange.push_back(rrange.back() + (uint32_t)((H.dim() + blockk::kRowChunk - 1) / blockk::kRowChunk));
+            rrange.push_back(rrange.back() + (uint32_t)((H.dim() + chunk_ - 1) / chunk_));
             rows_ += H.dim();
         }
         n_ctas_ = range.back();
@@ -677,9 +680,9 @@ public:
         if (!n_row_ctas_) return;
         constexpr int W = sizeof(T) == 4 ? 2 : 1;
         if (Rp_ % W == 0)
-            blockk::block_pack_update<T, W><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), Rp_, y, u, up, ca, cb, part);
+            blockk::block_pack_update<T, W><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), chunk_, Rp_, y, u, up, ca, cb, part);
         else
-            blockk::block_pack_update<T, 1><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), Rp_, y, u, up, ca, cb, part);
+            blockk::block_pack_update<T, 1><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), chunk_, Rp_, y, u, up, ca, cb, part);
         QKG_LAUNCHED();
     }
     void finish(const double* part, int mode, const BState& st) {
@@ -691,7 +694,7 @@ public:
         if (!n_row_ctas_) return;
         int streams = 1;  // streams a Hamiltonian: the vectors padded to a power of two
         while (streams < Ruser_) streams *= 2;
-        blockk::block_pack_philox<T2, sizeof(T) == 8><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), Rp_, Ruser_,
+        blockk::block_pack_philox<T2, sizeof(T) == 8><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), chunk_, Rp_, Ruser_,
                                                                                           streams, seed, u);
         QKG_LAUNCHED();
     }
@@ -752,6 +755,7 @@ private:
 
     std::vector<Hamiltonian*> hs_;
     int Rp_, Ruser_, run_ = 1;
+    uint32_t chunk_ = 512;
     std::unique_lock<std::mutex> ws_lock_;  // the first Hamiltonian's workspace, held for the engine's life
     cudaStream_t s_ = nullptr;
     packk::AmpMode mode_ = packk::AMP_UNIFORM;

@@ -23,13 +23,12 @@ constexpr int kMaxList = 96;   // outer (and straddling) entries of its blocks s
 
 // One Hamiltonian of the batch: its rows [base, base + dim) of the block vector,
 // its CTAs' range in the SpMV grid (runs of `run` tiles) and in the row grid
-// (chunks of kRowChunk rows).
+// (chunks of `chunk` rows).
 struct Ham {
     uint64_t base, dim;
     uint32_t cta0, row_cta0;
     const uint32_t* perm;  // reference index of each internal row (null: the same)
 };
-constexpr uint32_t kRowChunk = 512;
 // the Hamiltonian whose range holds CTA c
 template <class F>
 __device__ __forceinline__ int find_ham(const Ham* __restrict__ hams, int n, uint32_t c, F first) {
@@ -465,17 +464,17 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
 
 // w = y - ca u - cb up in place on y, and per CTA the partial ||w_v||^2 (u ==
 // nullptr: only the norms of y; Up == nullptr: no previous vector).  A CTA takes
-// kRowChunk rows of one Hamiltonian, a lane one 16-byte unit (VPL values) of a row.
+// `chunk` rows of one Hamiltonian, a lane one 16-byte unit (VPL values) of a row.
 template <class T, int VPL>
 __global__ void __launch_bounds__(kBT)
-    block_pack_update(const Ham* __restrict__ hams, int n_hams, int Rp, typename V2<T>::t* __restrict__ Y,
+    block_pack_update(const Ham* __restrict__ hams, int n_hams, uint32_t chunk, int Rp, typename V2<T>::t* __restrict__ Y,
                       const typename V2<T>::t* __restrict__ U, const typename V2<T>::t* __restrict__ Up,
                       const double* __restrict__ ca, const double* __restrict__ cb, double* __restrict__ part) {
     using R = Row<T, VPL>;
     __shared__ double red[kBT * VPL];
     const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.row_cta0; });
-    const uint32_t row0 = (blockIdx.x - hams[ham].row_cta0) * kRowChunk;
-    const uint32_t count = (uint32_t)min((unsigned long long)kRowChunk, (unsigned long long)(hams[ham].dim - row0));
+    const uint32_t row0 = (blockIdx.x - hams[ham].row_cta0) * chunk;
+    const uint32_t count = (uint32_t)min((unsigned long long)chunk, (unsigned long long)(hams[ham].dim - row0));
     const int G = Rp / VPL, NG = kBT / G;
     const int l = threadIdx.x % G, grp = threadIdx.x / G;
     Dots<T, VPL> dots;
@@ -516,13 +515,13 @@ __global__ void __launch_bounds__(kBT)
 // the Philox block (counter i, stream h * streams + v); padding vectors are zero.
 template <class T2, bool F64>
 __global__ void __launch_bounds__(kBT)
-    block_pack_philox(const Ham* __restrict__ hams, int n_hams, int Rp, int Ruser, int streams, uint64_t seed,
+    block_pack_philox(const Ham* __restrict__ hams, int n_hams, uint32_t chunk, int Rp, int Ruser, int streams, uint64_t seed,
                       T2* __restrict__ U) {
     const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.row_cta0; });
     const uint64_t base = hams[ham].base;
     const uint32_t* __restrict__ perm = hams[ham].perm;
-    const uint32_t i0 = (blockIdx.x - hams[ham].row_cta0) * kRowChunk;
-    const uint32_t count = (uint32_t)min((unsigned long long)kRowChunk, (unsigned long long)(hams[ham].dim - i0));
+    const uint32_t i0 = (blockIdx.x - hams[ham].row_cta0) * chunk;
+    const uint32_t count = (uint32_t)min((unsigned long long)chunk, (unsigned long long)(hams[ham].dim - i0));
     for (uint32_t e = threadIdx.x; e < count * (uint32_t)Rp; e += kBT) {
         const uint32_t i = i0 + e / Rp, v = e % Rp;
         T2 o;
