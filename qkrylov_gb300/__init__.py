@@ -172,6 +172,21 @@ class QKrylovError(RuntimeError):
         self.code = code
 
 
+_torch_module = None
+
+
+def _torch():
+    """torch, imported on first use (host arrays do without it)."""
+    global _torch_module, _raw_stream
+    if _torch_module is None:
+        import torch
+        # the stream handle alone, without a Stream object where torch has the call
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        _raw_stream = raw if raw is not None else (lambda d: torch.cuda.current_stream(d).cuda_stream)
+        _torch_module = torch
+    return _torch_module
+
+
 def _check(rc):
     if rc != SUCCESS:
         raise QKrylovError(rc, (lib().qkrylov_last_error() or b"").decode())
@@ -398,6 +413,7 @@ class MatrixFreeHamiltonian(_Handle):
         self._h = lib().qkrylov_hamiltonian_create(basis._h, site._h, ops._h)
         if not self._h:
             raise ValueError((lib().qkrylov_last_error() or b"").decode() or "hamiltonian creation failed")
+        self._dim = int(lib().qkrylov_hamiltonian_dimension(self._h))
 
     def to(self, device=None, dtype=None):
         """A new Hamiltonian of the same basis, site and terms on ``device`` with ``dtype``."""
@@ -406,7 +422,7 @@ class MatrixFreeHamiltonian(_Handle):
 
     @property
     def dimension(self):
-        return int(lib().qkrylov_hamiltonian_dimension(self._h))
+        return self._dim
 
     def apply(self, x):
         """y = H x.  Host arrays (NumPy, complex128) go through host memory;
@@ -421,16 +437,23 @@ class MatrixFreeHamiltonian(_Handle):
         return y.astype(_np.complex64) if self.dtype == _np.float32 else y
 
     def _apply_cuda(self, x):
-        import torch
+        # a small apply takes the GPU 6 us: nothing here is looked up or wrapped twice
+        # (14-site ring, calls in a row: 15 us a call before, 10.7 now)
+        torch = _torch()
         if not isinstance(x, torch.Tensor):
             raise TypeError("device arrays other than torch tensors: use apply_device with raw pointers")
-        if x.dtype not in (torch.complex128, torch.complex64):
+        if x.dtype is torch.complex128:
+            fn = _lib.qkrylov_hamiltonian_apply_device_f64
+        elif x.dtype is torch.complex64:
+            fn = _lib.qkrylov_hamiltonian_apply_device_f32
+        else:
             raise TypeError("device vectors must be complex128 or complex64")
-        if x.dim() != 1 or x.numel() != self.dimension or not x.is_contiguous():
-            raise ValueError(f"expected a contiguous vector of length {self.dimension}")
+        if x.dim() != 1 or x.numel() != self._dim or not x.is_contiguous():
+            raise ValueError(f"expected a contiguous vector of length {self._dim}")
         y = torch.empty_like(x)
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        self.apply_device(x.data_ptr(), y.data_ptr(), stream=stream, fp32=x.dtype == torch.complex64)
+        rc = fn(self._h, x.data_ptr(), y.data_ptr(), _raw_stream(x.get_device()))
+        if rc:
+            _check(rc)
         return y
 
     __matmul__ = apply

@@ -396,56 +396,78 @@ double tridiag_ground_ql(const double* a, const double* b, int n, std::vector<do
     return d[mi];
 }
 
+// Cyclic complex Jacobi.  Columns are stored contiguously, real and imaginary
+// parts apart, so a rotation is two passes of real multiply-adds over two columns of A
+// and of V; the rows of A follow from its Hermitian symmetry.
 void hermitian_eig(const std::vector<cd>& H, int m, std::vector<double>& evals, std::vector<std::vector<cd>>& vecs) {
-    std::vector<cd> A = H, V((size_t)m * m, 0.0);
-    for (int i = 0; i < m; ++i) V[(size_t)i * m + i] = 1.0;
-    auto at = [&](std::vector<cd>& M, int i, int j) -> cd& { return M[(size_t)i * m + j]; };
+    const size_t mm = (size_t)m * m;
+    std::vector<double> buf(4 * mm, 0.0);
+    double *Ar = buf.data(), *Ai = Ar + mm, *Vr = Ai + mm, *Vi = Vr + mm;  // column p at [p * m ..]
+    for (int i = 0; i < m; ++i) {
+        for (int j = 0; j < m; ++j) {
+            Ar[(size_t)j * m + i] = H[(size_t)i * m + j].real();
+            Ai[(size_t)j * m + i] = H[(size_t)i * m + j].imag();
+        }
+        Vr[(size_t)i * m + i] = 1.0;
+    }
+    // columns p, q <- (p c + q u_qp, p s + q u_qq) with u_qp = -s e, u_qq = c e
+    auto rotate = [m](double* __restrict__ xr, double* __restrict__ xi, double* __restrict__ yr, double* __restrict__ yi, double c, double s, double er, double ei) {
+#pragma omp simd
+        for (int k = 0; k < m; ++k) {
+            const double pr = xr[k], pi = xi[k];
+            const double qr = yr[k] * er - yi[k] * ei, qi = yr[k] * ei + yi[k] * er;
+            xr[k] = c * pr - s * qr;
+            xi[k] = c * pi - s * qi;
+            yr[k] = s * pr + c * qr;
+            yi[k] = s * pi + c * qi;
+        }
+    };
     for (int sweep = 0; sweep < 100; ++sweep) {
         double off = 0.0, diag = 0.0;
         for (int i = 0; i < m; ++i) {
-            diag += std::norm(at(A, i, i));
-            for (int j = i + 1; j < m; ++j) off += std::norm(at(A, i, j));
+            diag += Ar[(size_t)i * m + i] * Ar[(size_t)i * m + i];
+            for (int j = i + 1; j < m; ++j) {
+                const size_t ij = (size_t)j * m + i;
+                off += Ar[ij] * Ar[ij] + Ai[ij] * Ai[ij];
+            }
         }
         if (off <= 1e-32 * std::max(diag, 1e-300)) break;
         for (int p = 0; p < m; ++p)
             for (int q = p + 1; q < m; ++q) {
-                const cd apq = at(A, p, q);
-                const double mag = std::abs(apq);
+                double *pr = Ar + (size_t)p * m, *pi = Ai + (size_t)p * m, *qr = Ar + (size_t)q * m, *qi = Ai + (size_t)q * m;
+                const double xr = qr[p], xi = qi[p];  // A_pq
+                const double mag = std::sqrt(xr * xr + xi * xi);
                 if (mag < 1e-300) continue;
-                const cd ph = apq / mag;  // e^{i phi}
-                const double app = at(A, p, p).real(), aqq = at(A, q, q).real();
+                const double app = pr[p], aqq = qr[q];
                 const double tau = (aqq - app) / (2.0 * mag);
                 const double t = (tau >= 0 ? 1.0 : -1.0) / (std::abs(tau) + std::sqrt(1.0 + tau * tau));
                 const double c = 1.0 / std::sqrt(1.0 + t * t), s = t * c;
-                // U on (p,q): U_pp = c, U_pq = s, U_qp = -s e^{-i phi}, U_qq = c e^{-i phi}
-                const cd upp = c, upq = s, uqp = -s * std::conj(ph), uqq = c * std::conj(ph);
-                for (int k = 0; k < m; ++k) {  // A <- A U, V <- V U
-                    const cd akp = at(A, k, p), akq = at(A, k, q);
-                    at(A, k, p) = akp * upp + akq * uqp;
-                    at(A, k, q) = akp * upq + akq * uqq;
-                    const cd vkp = at(V, k, p), vkq = at(V, k, q);
-                    at(V, k, p) = vkp * upp + vkq * uqp;
-                    at(V, k, q) = vkp * upq + vkq * uqq;
+                // U on (p, q): U_pp = c, U_pq = s, U_qp = -s e^{-i phi}, U_qq = c e^{-i phi}, A_pq = mag e^{i phi}
+                const double er = xr / mag, ei = -xi / mag;
+                rotate(pr, pi, qr, qi, c, s, er, ei);                                                    // A <- A U
+                rotate(Vr + (size_t)p * m, Vi + (size_t)p * m, Vr + (size_t)q * m, Vi + (size_t)q * m, c, s, er, ei);
+                for (int k = 0; k < m; ++k) {  // A <- U^H A: rows p, q of the other columns are the columns' conjugates
+                    if (k == p || k == q) continue;
+                    Ar[(size_t)k * m + p] = pr[k];
+                    Ai[(size_t)k * m + p] = -pi[k];
+                    Ar[(size_t)k * m + q] = qr[k];
+                    Ai[(size_t)k * m + q] = -qi[k];
                 }
-                for (int k = 0; k < m; ++k) {  // A <- U^H A
-                    const cd apk = at(A, p, k), aqk = at(A, q, k);
-                    at(A, p, k) = std::conj(upp) * apk + std::conj(uqp) * aqk;
-                    at(A, q, k) = std::conj(upq) * apk + std::conj(uqq) * aqk;
-                }
-                at(A, p, q) = at(A, q, p) = 0.0;
-                at(A, p, p) = at(A, p, p).real();
-                at(A, q, q) = at(A, q, q).real();
+                pr[p] = app - t * mag;
+                qr[q] = aqq + t * mag;
+                pi[p] = qi[q] = 0.0;
+                pr[q] = pi[q] = qr[p] = qi[p] = 0.0;
             }
     }
     std::vector<int> idx(m);
     std::iota(idx.begin(), idx.end(), 0);
-    std::stable_sort(idx.begin(), idx.end(), [&](int i, int j) { return at(A, i, i).real() < at(A, j, j).real(); });
+    std::stable_sort(idx.begin(), idx.end(), [&](int i, int j) { return Ar[(size_t)i * m + i] < Ar[(size_t)j * m + j]; });
     evals.clear();
     vecs.clear();
     for (int i : idx) {
-        evals.push_back(at(A, i, i).real());
+        evals.push_back(Ar[(size_t)i * m + i]);
         std::vector<cd> v(m);
-        for (int k = 0; k < m; ++k) v[k] = at(V, k, i);
+        for (int k = 0; k < m; ++k) v[k] = cd(Vr[(size_t)i * m + k], Vi[(size_t)i * m + k]);
         vecs.push_back(std::move(v));
     }
 }
@@ -729,16 +751,27 @@ CFOut cf_f64(Hamiltonian& H, const cd* phi0_ref, int n_iter) {
     return out;
 }
 
-// Backward continued fraction at z = omega + E0 + i eta (dynamics.cpp:61-89).
+// Backward continued fraction at z = omega + E0 + i eta (dynamics.cpp:61-89):
+// f <- 1 / (z - alpha_i - beta_i^2 f), in real arithmetic with one division a level.
 double spectral(const double* alphas, const double* betas, size_t n, double norm, double omega, double E0, double eta) {
     if (n == 0) return 0.0;
-    const cd z(omega + E0, eta);
-    cd f = 0.0;
+    const double zr = omega + E0, zi = eta;
+    double fr = 0.0, fi = 0.0;
     for (int i = (int)n - 1; i >= 0; --i) {
-        if (i == (int)n - 1) f = 1.0 / (z - alphas[i]);
-        else f = 1.0 / (z - alphas[i] - betas[i] * betas[i] * f);
+        const double b2 = i == (int)n - 1 ? 0.0 : betas[i] * betas[i];
+        const double dr = zr - alphas[i] - b2 * fr, di = zi - b2 * fi;
+        const double m = dr * dr + di * di;
+        if (m > 1e-200 && m < 1e200) {
+            const double inv = 1.0 / m;
+            fr = dr * inv;
+            fi = -di * inv;
+        } else {  // a square outside the range: the library's scaled division
+            const cd f = 1.0 / cd(dr, di);
+            fr = f.real();
+            fi = f.imag();
+        }
     }
-    return -1.0 / M_PI * std::imag(norm * norm * f);
+    return -1.0 / M_PI * (norm * norm * fi);
 }
 
 // ============================================================ FTLM
