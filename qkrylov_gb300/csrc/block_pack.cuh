@@ -9,12 +9,13 @@
 #pragma once
 
 #include "pack.hpp"
+#include "pair.cuh"
 
 namespace qkg {
 namespace blockk {
 using namespace fastk;
 using namespace packk;
-using u64 = unsigned long long;
+using namespace pairk;
 
 constexpr int kBT = 256;       // threads of a CTA
 constexpr int kBatch = 4;      // outer entries loaded together
@@ -39,44 +40,6 @@ __device__ __forceinline__ int find_ham(const Ham* __restrict__ hams, int n, uin
         else hi = mid - 1;
     }
     return lo;
-}
-
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ u64 pk(float x, float y) {
-    u64 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-    return d;
-}
-__device__ __forceinline__ float2 unpk(u64 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-constexpr u64 kMinusOne2 = 0xBF800000BF800000ull;  // (-1, -1)
-__device__ __forceinline__ u64 sub2(u64 a, u64 b) { return fma2(b, kMinusOne2, a); }  // a - b, rounded once
-// (hi, lo) += a * b elementwise, compensated (TwoProduct, TwoSum), both halves at once
-__device__ __forceinline__ void acc2(u64& hi, u64& lo, u64 a, u64 b) {
-    const u64 p = mul2(a, b);
-    const u64 e = fma2(a, b, mul2(p, kMinusOne2));
-    const u64 t = add2(hi, p);
-    const u64 z = sub2(t, hi);
-    const u64 err = add2(sub2(hi, sub2(t, z)), sub2(p, z));
-    lo = add2(lo, add2(err, e));
-    hi = t;
 }
 
 // p + a * b bytes (one 32 x 32 + 64 bit multiply-add)
@@ -105,6 +68,17 @@ template <int VPL> struct Row<float, VPL> {
                 v[2 * j] = q.x;
                 v[2 * j + 1] = q.y;
             }
+        }
+    }
+    __device__ __forceinline__ void load_if(const float2* p, int G, bool on) {
+        if constexpr (VPL == 1) {
+            v[0] = 0ull;
+            if (on) v[0] = *reinterpret_cast<const u64*>(p);
+        } else {
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+                asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.b64 %0, 0;\n\tmov.b64 %1, 0;\n\t@p ld.global.v2.b64 {%0, %1}, [%2];\n\t}"
+                    : "=l"(v[2 * j]), "=l"(v[2 * j + 1]) : "l"(p + 2 * j * G), "r"((uint32_t)on));
         }
     }
     __device__ __forceinline__ void store(float2* p, int G) const {
@@ -150,6 +124,13 @@ template <int VPL> struct Row<double, VPL> {
     __device__ __forceinline__ void load(const double2* p, int G) {
 #pragma unroll
         for (int j = 0; j < VPL; ++j) v[j] = p[j * G];
+    }
+    __device__ __forceinline__ void load_if(const double2* p, int G, bool on) {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            v[j] = make_double2(0.0, 0.0);
+            if (on) v[j] = p[j * G];
+        }
     }
     __device__ __forceinline__ void store(double2* p, int G) const {
 #pragma unroll
@@ -419,18 +400,16 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                         nxt = __ldg(tab + at);
                         if (MODE == AMP_CODED) cn = __ldg(codes + at);
                     }
-                    // a row's entries fill its first slots
                     const uint32_t w[4] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16};
+                    // the four rows' loads go out together; an empty slot reads zero
+                    R v[4];
 #pragma unroll
-                    for (int h = 0; h < 4; h += 2) {
-                        const int r0 = rank_of(w[h]), r1 = rank_of(w[h + 1]);
-                        if (r0 == kNone) break;
-                        R v0, v1;
-                        v0.load(offset(xl, r0, rb), G);
-                        if (r1 != kNone) v1.load(offset(xl, r1, rb), G);
-                        amp_add(w[h], c >> (8 * h), u, v0);
-                        if (r1 != kNone) amp_add(w[h + 1], c >> (8 * h + 8), u, v1);
+                    for (int h = 0; h < 4; ++h) {
+                        const int to = rank_of(w[h]);
+                        v[h].load_if(offset(xl, to, rb), G, to != kNone);
                     }
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) amp_add(w[h], c >> (8 * h), u, v[h]);
                 }
                 for (uint32_t j = 0; j < ns; ++j) {
                     const Str<T> s = strl[j];

@@ -13,39 +13,23 @@
 // FP64: the integer pipe (60% busy) for equal magnitudes, 1.65 ms; the FP64 pipe (88%
 // busy) otherwise and before, 2.80 ms.
 #include "pack.hpp"
+#include "pair.cuh"
 
 #include <type_traits>
 
 namespace qkg {
 using namespace fastk;
 using namespace packk;
+using namespace pairk;
 namespace {
-
-using u64 = unsigned long long;
 
 // CTAs of four warps.  Resident CTAs the register allocation is held to: the
 // kernels wait for gathers, so FP32 takes 48 warps a SM at 40 registers (L = 28
-// ring: 32 warps 0.47 ms, 40 0.46, 48 0.42, 56 0.44), FP64 24 warps at 80 (16
-// warps 2.05 ms, 24 1.65, 32 1.65).
+// ring: 32 warps 0.47 ms, 40 0.46, 48 0.42, 56 0.44) and 40 warps at 48 where signs,
+// codes or the Lanczos step's terms need more (L = 28 Lanczos step 0.55 to 0.54 ms, L = 14
+// Hubbard ring 0.153 to 0.148), FP64 24 warps at 80 (16 warps 2.05 ms, 24 1.65, 32 1.65).
 constexpr int kThreads = 128;
-constexpr int kCtas32 = 12, kCtas64 = 6;
-
-// Two FP32 FMAs in one instruction: d = a * b + c on (re, im) pairs.
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ u64 pair(float x, float y) {
-    u64 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-    return d;
-}
-__device__ __forceinline__ float2 unpair(u64 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
+constexpr int kCtas32 = 12, kCtas32more = 10, kCtas64 = 6;
 
 // ---- sums of one row -------------------------------------------------------
 // FP32, real amplitudes.
@@ -53,11 +37,11 @@ struct SumF32 {
     using V = u64;  // one complex element
     u64 s;
     __device__ __forceinline__ void init() { s = 0ull; }
-    __device__ __forceinline__ void add(float a, V x) { s = fma2(pair(a, a), x, s); }
+    __device__ __forceinline__ void add(float a, V x) { s = fma2(pk(a, a), x, s); }
     __device__ __forceinline__ void add(float ar, float ai, V x) {
-        const float2 v = unpair(x);
-        s = fma2(pair(ar, ar), x, s);
-        s = fma2(pair(-ai, ai), pair(v.y, v.x), s);
+        const float2 v = unpk(x);
+        s = fma2(pk(ar, ar), x, s);
+        s = fma2(pk(-ai, ai), pk(v.y, v.x), s);
     }
 };
 // FP64 on the FP64 pipe.
@@ -321,7 +305,7 @@ __device__ __forceinline__ void finish_alpha(const Params<T>& p) {
 // FP32.  LZ: the Lanczos step's form (operands from *p.lz, y = scale H x -
 // bprev vprev, per-CTA partials of Re<x, y>).
 template <int MODE, bool CPLX, bool LZ, int NQ>
-__global__ void __launch_bounds__(kThreads, kCtas32)
+__global__ void __launch_bounds__(kThreads, LZ || MODE != AMP_UNIFORM ? kCtas32more : kCtas32)
     pack32_kernel(const Params<float> p, const float2* __restrict__ x_in, float2* __restrict__ y_in) {
     __shared__ float s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
     if (MODE == AMP_CODED) load_amps(p, s_amp);
@@ -339,40 +323,48 @@ __global__ void __launch_bounds__(kThreads, kCtas32)
     }
     const uint32_t wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     const uint32_t id = NQ == 4 ? wid : wid >> 2, q0 = NQ == 4 ? 0u : wid & 3u;
-    float dot_hi = 0.f, dot_lo = 0.f;
+    u64 dot_hi = 0ull, dot_lo = 0ull;  // real and imaginary products apart
     if (id < p.n_items) {
         const uint4 i4 = __ldg(reinterpret_cast<const uint4*>(p.items) + id);
         const Item it{i4.x, i4.y, i4.z, i4.w};
         SumF32 acc[NQ];
         walk<float, SumF32, MODE, CPLX, NQ>(p, it, q0, x, s_amp, acc);
-        const uint32_t cnt = it.tc & 0xFFu;
+        const uint32_t cnt = it.tc & 0xFFu, row0 = it.row0 + lane + 32u * q0;
+        uint32_t dc[NQ];
+        u64 xv[NQ], pv[NQ];
+        auto own = [&](int q) {  // row q's own values
+            const uint32_t row = lane + 32u * (q0 + q) < cnt ? row0 + 32u * q : it.row0;
+            dc[q] = p.diag_mode == DIAG_U8 ? (uint32_t)__ldg(static_cast<const uint8_t*>(p.dcode) + row)
+                                           : (uint32_t)__ldg(static_cast<const uint16_t*>(p.dcode) + row);
+            xv[q] = Elem<float>::load(x + row);
+            pv[q] = 0ull;
+            // read once a step: evict-first, so x keeps more of L2
+            if (LZ && vprev) pv[q] = __ldcs(reinterpret_cast<const u64*>(vprev + row));
+        };
+        if (LZ)  // all in flight together (L = 28: 0.59 to 0.54 ms; without v_{k-1} it costs registers: 0.42 to 0.43)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) own(q);
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
             if (lane + 32u * (q0 + q) >= cnt) continue;
-            const uint32_t row = it.row0 + lane + 32u * (q0 + q);
-            float dr, di;
-            diag_at(p, row, dr, di);
-            const u64 xv = Elem<float>::load(x + row);
-            if (p.cdiag) acc[q].add(dr, di, xv);
-            else acc[q].add(dr, xv);
-            float2 o = unpair(acc[q].s);
+            if (!LZ) own(q);
+            const float dr = __ldg(p.dtab + 2 * dc[q]);
+            if (p.cdiag) acc[q].add(dr, __ldg(p.dtab + 2 * dc[q] + 1), xv[q]);
+            else acc[q].add(dr, xv[q]);
+            u64 o = acc[q].s;
             if (LZ) {
-                o.x *= scale;
-                o.y *= scale;
-                if (vprev) {  // read once a step: evict-first, so x keeps more of L2
-                    const float2 pv = __ldcs(vprev + row);
-                    o.x = fmaf(-bprev, pv.x, o.x);
-                    o.y = fmaf(-bprev, pv.y, o.y);
-                }
-                const float2 xf = unpair(xv);
-                ffma_acc(dot_hi, dot_lo, xf.x, o.x);
-                ffma_acc(dot_hi, dot_lo, xf.y, o.y);
+                o = mul2(o, pk(scale, scale));
+                if (vprev) o = fma2(pk(-bprev, -bprev), pv[q], o);
+                acc2(dot_hi, dot_lo, xv[q], o);
             }
-            __stcs(y + row, o);
+            __stcs(reinterpret_cast<u64*>(y + row0 + 32u * q), o);
         }
     }
     if (LZ) {
-        const float2 t = block_sum_ff(dot_hi, dot_lo);
+        const float2 h = unpk(dot_hi), l = unpk(dot_lo);
+        float hi = h.x, lo = l.x;
+        ff_add(hi, lo, h.y, l.y);
+        const float2 t = block_sum_ff(hi, lo);
         if (threadIdx.x == 0) p.apart[blockIdx.x] = make_double2((double)t.x + (double)t.y, 0.0);
         finish_alpha(p);
     }
