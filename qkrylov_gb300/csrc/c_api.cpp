@@ -640,7 +640,7 @@ VectorScratch& vector_scratch() {  // caller holds vector_scratch_lock()
     QKG_CUDA(cudaGetDevice(&dev));
     VectorScratch& sc = scratch[dev];
     if (!sc.ws) {
-        sc.tab.alloc((size_t)kMdotMaxVectors * sizeof(void*));
+        sc.tab.alloc(((size_t)kMdotMaxVectors + 8) * sizeof(void*) + 1024 * sizeof(double2));  // pointers, coefficients
         sc.ws = std::make_unique<qkg::Workspace>(1 << 16);
     }
     return sc;
@@ -664,13 +664,21 @@ int qkrylov_vector_mdot_device_f32(const void* const* v_dev, int k, const void* 
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         auto lk = vector_scratch_lock();
         VectorScratch& sc = vector_scratch();
-        QKG_CUDA(cudaMemcpyAsync(sc.tab.p, v_dev, (size_t)k * sizeof(void*), cudaMemcpyHostToDevice, s));
+        // both pointer tables in one copy
+        std::vector<const void*> tab(v_dev, v_dev + k);
+        tab.insert(tab.end(), w_dev, w_dev + nw);
+        QKG_CUDA(cudaMemcpyAsync(sc.tab.p, tab.data(), tab.size() * sizeof(void*), cudaMemcpyHostToDevice, s));
         std::vector<float2*> w(nw);
         for (int o = 0; o < nw; ++o) w[o] = const_cast<float2*>(static_cast<const float2*>(w_dev[o]));
         std::vector<cd> r((size_t)k * nw);
         const auto* V = static_cast<const float2* const*>(sc.tab.p);
         if (method == 1) qkg::mdot_multi_f32_tc(V, k, w.data(), nw, n, r.data(), *sc.ws, s);
-        else if (method == 2) qkg::mdot_multi_f32_fast(V, k, w.data(), nw, n, r.data(), *sc.ws, s);
+        else if (method == 2) {
+            bool al = true;
+            for (int j = 0; j < k; ++j) al = al && on_grid(v_dev[j], 16);
+            for (int o = 0; o < nw; ++o) al = al && on_grid(w_dev[o], 16);
+            qkg::mdot_multi_f32_fast(V, k, w.data(), nw, n, r.data(), *sc.ws, s, al, V + k);
+        }
         else qkg::mdot_multi_f32_cuda(V, k, w.data(), nw, n, r.data(), *sc.ws, s);
         for (size_t i = 0; i < r.size(); ++i) {
             out[2 * i] = r[i].real();
@@ -691,14 +699,20 @@ int qkrylov_vector_mcombine_device_f32(const void* const* v_dev, int k, const do
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         auto lk = vector_scratch_lock();
         VectorScratch& sc = vector_scratch();
-        if (k > 0)
-            QKG_CUDA(cudaMemcpyAsync(sc.tab.p, v_dev, (size_t)k * sizeof(void*), cudaMemcpyHostToDevice, s));
-        std::vector<float2*> w(nw);
-        for (int o = 0; o < nw; ++o) w[o] = static_cast<float2*>(w_dev[o]);
-        std::vector<cd> c((size_t)k * nw);
-        for (size_t i = 0; i < c.size(); ++i) c[i] = {coeffs[2 * i], coeffs[2 * i + 1]};
-        qkg::mcombine_multi_f32(static_cast<const float2* const*>(sc.tab.p), k, c.data(), w.data(), nw, n,
-                                accumulate != 0, *sc.ws, s);
+        // coefficients, then the pointer tables, in one copy
+        std::vector<char> image((size_t)k * nw * sizeof(double2) + ((size_t)k + nw) * sizeof(void*));
+        char* p = image.data();
+        if (k > 0) {
+            std::memcpy(p, coeffs, (size_t)k * nw * sizeof(double2));
+            std::memcpy(p + (size_t)k * nw * sizeof(double2), v_dev, (size_t)k * sizeof(void*));
+        }
+        const size_t at_v = (size_t)k * nw * sizeof(double2), at_w = at_v + (size_t)k * sizeof(void*);
+        std::memcpy(p + at_w, w_dev, (size_t)nw * sizeof(void*));
+        QKG_CUDA(cudaMemcpyAsync(sc.tab.p, p, image.size(), cudaMemcpyHostToDevice, s));
+        const char* d = sc.tab.as<char>();
+        qkg::mcombine_multi_f32_dev(reinterpret_cast<const float2* const*>(d + at_v), k, reinterpret_cast<const double2*>(d),
+                                    reinterpret_cast<float2* const*>(d + at_w), nw, n, accumulate != 0, s);
+        QKG_CUDA(cudaStreamSynchronize(s));  // the scratch is free for the next call, on any stream
     });
 }
 

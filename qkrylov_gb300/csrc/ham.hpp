@@ -337,6 +337,7 @@ struct Workspace {
     DBuf partial;     // per-block partial sums
     DBuf result;      // device-side result slots
     double* host = nullptr;  // pinned host result slots
+    double* host_dev = nullptr;  // their device address
     size_t cap_partials = 0;
     explicit Workspace(size_t max_blocks_times_k = 1 << 16);
     ~Workspace();
@@ -376,8 +377,11 @@ void mdot_multi_f32(const float2* const* V_dev, int k, float2* const* W, int nw,
 void mdot_multi_f32_cuda(const float2* const* V_dev, int k, float2* const* W, int nw, uint64_t n,
                          std::complex<double>* out, Workspace& ws, cudaStream_t s);
 // the same with FP32 sums over runs of 32 elements (projection mode 2)
+// (aligned16: every vector starts on a 16-byte boundary; w_dev: the device copy of W where the
+// caller has one)
 void mdot_multi_f32_fast(const float2* const* V_dev, int k, float2* const* W, int nw, uint64_t n,
-                         std::complex<double>* out, Workspace& ws, cudaStream_t s);
+                         std::complex<double>* out, Workspace& ws, cudaStream_t s, bool aligned16,
+                         const float2* const* w_dev = nullptr);
 // The same on the tensor cores (tcgen05, 3xTF32 products, FP32 accumulation
 // read out into FP64 every thousand or so terms; mdot_tc.cu): k <= 128, nw <= 4.
 bool mdot_tc_supported(int k, int nw);
@@ -400,6 +404,9 @@ void mcombine_multi_f64(const double2* const* V_dev, int k, const std::complex<d
                         uint64_t n, bool accumulate, Workspace& ws, cudaStream_t s);
 void mcombine_multi_f32(const float2* const* V_dev, int k, const std::complex<double>* c, float2* const* W, int nout,
                         uint64_t n, bool accumulate, Workspace& ws, cudaStream_t s);
+// The same with coefficients and output pointers on the device; queued, not waited for.
+void mcombine_multi_f32_dev(const float2* const* V_dev, int k, const double2* c_dev, float2* const* W_dev, int nout,
+                            uint64_t n, bool accumulate, cudaStream_t s);
 // Davidson preconditioner t_i = r_i / (d_i - lambda) with the reference's clamp.
 void davidson_precond_f64(const double2* r, const double2* d, double lambda, double2* t, uint64_t n, cudaStream_t s);
 void davidson_precond_f32(const float2* r, const double2* d, double lambda, float2* t, uint64_t n, cudaStream_t s);

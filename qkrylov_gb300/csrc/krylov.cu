@@ -16,11 +16,13 @@
 // precision.  Partials are then combined in FP64.  This keeps the reductions
 // off GB300's low-rate FP64 pipe.
 #include "fast_common.cuh"
+#include "pair.cuh"
 
 #include <algorithm>
 #include <atomic>
 
 namespace qkg {
+using namespace pairk;
 
 namespace {
 constexpr int kThreads = 256;
@@ -545,6 +547,139 @@ __global__ void __launch_bounds__(kThreads, KC == 4 ? 2 : 3) mdot32_multi_fast_k
             if (q < kk) block_sum_cff(re[q][o], im[q][o], part + ((size_t)(j0 + q) * NW + o) * stride + blockIdx.y);
 }
 
+// The run-summed projections for large aligned vectors, streamed through shared
+// memory: a CTA (16 warps, one per SM) takes a column of up to 16 vectors V_j (the k are
+// dealt out evenly) and the NW vectors
+// W_o in tiles of 256 elements, copied asynchronously three tiles ahead, so every V_j
+// comes from DRAM once, every W_o once a column, and the loads in flight (120 KB a SM) do
+// not depend on the registers.  Warps 2g, 2g + 1 hold vectors 2g and 2g + 1 of the
+// column; products, runs of 32 elements and their float-float folds run on (re, im) pairs.
+// bound by DRAM: k = 32, nw = 4, n = 11.8 M 0.60 ms, 5.7 TB/s
+// of V and W (register-held 0.92 ms).
+constexpr int kStreamVecs = 16, kStreamTile = 256, kStreamStages = 4, kStreamThreads = 512;
+template <int NW>
+constexpr size_t stream_smem() { return (size_t)kStreamStages * (kStreamVecs + NW) * kStreamTile * sizeof(float2); }
+// a += t elementwise in float-float (TwoSum)
+__device__ __forceinline__ void ff2_add(u64& hi, u64& lo, u64 t) {
+    const u64 s = add2(hi, t), z = sub2(s, hi);
+    lo = add2(lo, add2(sub2(hi, sub2(s, z)), sub2(t, z)));
+    hi = s;
+}
+template <int NW>
+__global__ void __launch_bounds__(kStreamThreads, 1) mdot32_stream_kernel(const float2* const* __restrict__ V, int k,
+                                                                          const float2* const* __restrict__ W, uint64_t n,
+                                                                          int per, double2* part, int stride) {
+    extern __shared__ __align__(16) unsigned char ring[];
+    __shared__ const float2* s_ptr[kStreamVecs + NW];
+    __shared__ double2 s_sum[kStreamThreads / 32][2 * NW];
+    constexpr int kVec = kStreamTile * (int)sizeof(float2);  // bytes of a vector's tile
+    constexpr int kStage = (kStreamVecs + NW) * kVec;
+    const int j0 = blockIdx.x * per, kk = min(per, k - j0);
+    if (threadIdx.x < kStreamVecs + NW)
+        s_ptr[threadIdx.x] = threadIdx.x < kStreamVecs ? V[j0 + max(0, min((int)threadIdx.x, kk - 1))] : W[threadIdx.x - kStreamVecs];
+    __syncthreads();
+    const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring);
+    const uint64_t tiles = (n + kStreamTile - 1) / kStreamTile;
+    // tile t into stage s: 16-byte pieces (two elements), zero past the end
+    auto copy = [&](uint64_t t, int s) {
+        if (t < tiles) {
+#pragma unroll
+            for (int i = 0; i < (kStreamVecs + NW + 3) / 4; ++i) {
+                const int v = (int)(threadIdx.x >> 7) + 4 * i;
+                if (v >= kStreamVecs + NW || (v < kStreamVecs && v >= kk)) continue;
+                const uint64_t e = t * kStreamTile + 2 * (threadIdx.x & 127);
+                const int bytes = e + 1 < n ? 16 : e < n ? 8 : 0;
+                const float2* src = s_ptr[v] + (bytes ? e : 0);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring_at + s * kStage + v * kVec + 16 * (threadIdx.x & 127)),
+                             "l"(src), "r"(bytes)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int q0 = 2 * (int)(threadIdx.x >> 6);  // this warp's vectors q0, q0 + 1 of the column
+    const bool on0 = q0 < kk, on1 = q0 + 1 < kk;
+    u64 run[2][NW], hi[2][NW], lo[2][NW];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int o = 0; o < NW; ++o) run[q][o] = hi[q][o] = lo[q][o] = 0ull;
+    auto fold = [&] {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int o = 0; o < NW; ++o) {
+                ff2_add(hi[q][o], lo[q][o], run[q][o]);
+                run[q][o] = 0ull;
+            }
+    };
+#pragma unroll
+    for (int s = 0; s < kStreamStages - 1; ++s) copy(blockIdx.y + (uint64_t)s * gridDim.y, s);
+    int stage = 0, in_run = 0;
+    for (uint64_t t = blockIdx.y; t < tiles; t += gridDim.y) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStreamStages - 2) : "memory");
+        __syncthreads();  // every thread's pieces of this tile are there; the stage refilled next has been read
+        copy(t + (uint64_t)(kStreamStages - 1) * gridDim.y, (stage + kStreamStages - 1) % kStreamStages);
+        if (on0) {
+            const unsigned char* base = ring + stage * kStage;
+#pragma unroll
+            for (int i = 0; i < kStreamTile / 128; ++i) {
+                const int at = 16 * ((threadIdx.x & 63) + 64 * i);
+                const float4 a0 = *reinterpret_cast<const float4*>(base + q0 * kVec + at);
+                const float4 a1 = *reinterpret_cast<const float4*>(base + (on1 ? q0 + 1 : q0) * kVec + at);
+#pragma unroll
+                for (int o = 0; o < NW; ++o) {
+                    const float4 b = *reinterpret_cast<const float4*>(base + (kStreamVecs + o) * kVec + at);
+                    // conj(a) b = (ax bx + ay by, ax by - ay bx), two elements
+                    const u64 b0 = pk(b.x, b.y), b1 = pk(b.z, b.w), c0 = pk(b.y, -b.x), c1 = pk(b.w, -b.z);
+                    u64 r = run[0][o];
+                    r = fma2(pk(a0.x, a0.x), b0, r);
+                    r = fma2(pk(a0.y, a0.y), c0, r);
+                    r = fma2(pk(a0.z, a0.z), b1, r);
+                    run[0][o] = fma2(pk(a0.w, a0.w), c1, r);
+                    r = run[1][o];
+                    r = fma2(pk(a1.x, a1.x), b0, r);
+                    r = fma2(pk(a1.y, a1.y), c0, r);
+                    r = fma2(pk(a1.z, a1.z), b1, r);
+                    run[1][o] = fma2(pk(a1.w, a1.w), c1, r);
+                }
+            }
+            if (++in_run == 32 / (2 * (kStreamTile / 128))) {  // 32 elements a thread
+                fold();
+                in_run = 0;
+            }
+        }
+        stage = (stage + 1) % kStreamStages;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    fold();
+    // sums over the warp, then over the group's two warps
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int o = 0; o < NW; ++o) {
+            u64 h = hi[q][o], l = lo[q][o];
+#pragma unroll
+            for (int m = 16; m > 0; m >>= 1) {
+                const u64 h2 = __shfl_down_sync(0xffffffffu, h, m), l2 = __shfl_down_sync(0xffffffffu, l, m);
+                ff2_add(h, l, h2);
+                l = add2(l, l2);
+            }
+            if ((threadIdx.x & 31) == 0) {
+                const float2 x = unpk(h), y = unpk(l);
+                s_sum[threadIdx.x >> 5][q * NW + o] = make_double2((double)x.x + (double)y.x, (double)x.y + (double)y.y);
+            }
+        }
+    __syncthreads();
+    if (threadIdx.x < kStreamVecs * NW) {
+        const int v = threadIdx.x / NW, o = threadIdx.x % NW;
+        if (v < kk) {
+            const double2 a = s_sum[(v >> 1) * 2][(v & 1) * NW + o], b = s_sum[(v >> 1) * 2 + 1][(v & 1) * NW + o];
+            part[((size_t)(j0 + v) * NW + o) * stride + blockIdx.y] = make_double2(a.x + b.x, a.y + b.y);
+        }
+    }
+}
+
 // w += sum_j c_j V_j ; coefficients (complex double) in global memory.
 template <class T2, class A>
 __global__ void mcomb_kernel(const T2* const* __restrict__ V, int k, const double2* __restrict__ c, T2* __restrict__ w,
@@ -649,9 +784,9 @@ __global__ void philox_normal_kernel(uint64_t seed, uint64_t stream, T2* out, ui
 }
 
 double2* finish(Workspace& ws, int nparts, int stride, int k, cudaStream_t s) {
-    finish_kernel<<<k, kThreads, 0, s>>>(ws.partial.as<double2>(), nparts, stride, ws.result.as<double2>());
+    // straight into the pinned slots: no copy between the sums and the host
+    finish_kernel<<<k, kThreads, 0, s>>>(ws.partial.as<double2>(), nparts, stride, reinterpret_cast<double2*>(ws.host_dev));
     QKG_LAUNCHED();
-    QKG_CUDA(cudaMemcpyAsync(ws.host, ws.result.p, (size_t)k * sizeof(double2), cudaMemcpyDeviceToHost, s));
     QKG_CUDA(cudaStreamSynchronize(s));
     return reinterpret_cast<double2*>(ws.host);
 }
@@ -661,7 +796,12 @@ double2* finish(Workspace& ws, int nparts, int stride, int k, cudaStream_t s) {
 Workspace::Workspace(size_t cap) : cap_partials(cap) {
     partial.alloc(cap * sizeof(double2));
     result.alloc(4096 * sizeof(double2));
-    QKG_CUDA(cudaMallocHost(&host, 4096 * sizeof(double2)));
+    QKG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host), 4096 * sizeof(double2), cudaHostAllocMapped));
+    const cudaError_t e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&host_dev), host, 0);
+    if (e != cudaSuccess) {
+        cudaFreeHost(host);
+        QKG_CUDA(e);
+    }
 }
 Workspace::~Workspace() {
     if (host) cudaFreeHost(host);
@@ -798,7 +938,7 @@ void mdot_multi_f32(const float2* const* V, int k, float2* const* W, int nw, uin
         return;
     }
     if (mode == 2) {
-        mdot_multi_f32_fast(V, k, W, nw, n, out, ws, s);
+        mdot_multi_f32_fast(V, k, W, nw, n, out, ws, s, true);  // the solvers' vectors are whole allocations
         return;
     }
     mdot_multi_f32_cuda(V, k, W, nw, n, out, ws, s);
@@ -818,12 +958,41 @@ static int balanced_chunks(int ncol, int slots, int g_max) {
     return g_max;
 }
 
+namespace {
+// The streaming kernel is taken for three and four right-hand vectors (calls of n = 11.8 M,
+// register-held against streamed: k = 8, nw = 4 283 against 235 us, k = 16 497 / 341, k = 32
+// 940 / 640) from 2^18 elements (k = 32, nw = 4 63 / 59 us; below, the two are level); with
+// one or two the kernel above already reads at 6.2 TB/s (k = 32, nw = 1 478 / 533 us, k = 17,
+// nw = 2 348 / 410).
+constexpr uint64_t kStreamMin = 1u << 18;
+// Lets the streaming kernel take its dynamic shared memory, once per width and device.
+template <int NW>
+void allow_stream_smem() {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    QKG_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+    if (bit && (done.load() & bit)) return;
+    QKG_CUDA(cudaFuncSetAttribute(mdot32_stream_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem<NW>()));
+    done.fetch_or(bit);
+}
+template <int NW>
+void launch_stream(dim3 grid, const float2* const* V, int k, const float2* const* W, uint64_t n, double2* part, cudaStream_t s) {
+    allow_stream_smem<NW>();
+    mdot32_stream_kernel<NW><<<grid, kStreamThreads, stream_smem<NW>(), s>>>(V, k, W, n, (k + (int)grid.x - 1) / (int)grid.x, part, (int)grid.y);
+}
+}  // namespace
+
 void mdot_multi_f32_fast(const float2* const* V, int k, float2* const* W, int nw, uint64_t n, std::complex<double>* out,
-                         Workspace& ws, cudaStream_t s) {
+                         Workspace& ws, cudaStream_t s, bool aligned16, const float2* const* w_dev) {
     if (k <= 0 || nw <= 0) return;
     QKG_REQUIRE(nw <= 4 && (size_t)k * nw <= 4088, "mdot_multi: at most 4 right-hand vectors and 4088 products");
-    float2** dw = reinterpret_cast<float2**>(ws.result.as<double2>() + 4096 - 8);
-    QKG_CUDA(cudaMemcpyAsync(dw, W, (size_t)nw * sizeof(float2*), cudaMemcpyHostToDevice, s));
+    const float2* const* dw = w_dev;
+    if (!dw) {
+        void* t = ws.result.as<double2>() + 4096 - 8;
+        QKG_CUDA(cudaMemcpyAsync(t, W, (size_t)nw * sizeof(float2*), cudaMemcpyHostToDevice, s));
+        dw = static_cast<const float2* const*>(t);
+    }
     int g = stream_grid(n);
     g = (int)std::min<size_t>((size_t)g, ws.cap_partials / ((size_t)k * nw));
     g = std::max(1, g);
@@ -834,6 +1003,18 @@ void mdot_multi_f32_fast(const float2* const* V, int k, float2* const* W, int nw
     // of whole chunks would double the time): at k = 32, nw = 4, n = 11.8 M
     // 0.93 ms, against 1.02 ms for 512 chunks and 1.71 ms for one wave rounded up.
     double2* part = ws.partial.as<double2>();
+    if (aligned16 && nw >= 3 && n >= kStreamMin) {
+        const int ncol = (k + kStreamVecs - 1) / kStreamVecs;
+        g = std::max(1, std::min(g, 152 / ncol));  // one CTA a SM
+        const dim3 grid(ncol, g);
+        if (nw == 3) launch_stream<3>(grid, V, k, dw, n, part, s);
+        else launch_stream<4>(grid, V, k, dw, n, part, s);
+        QKG_LAUNCHED();
+        const double2* r = finish(ws, g, g, k * nw, s);
+        for (int j = 0; j < k; ++j)
+            for (int o = 0; o < nw; ++o) out[(size_t)o * k + j] = {r[(size_t)j * nw + o].x, r[(size_t)j * nw + o].y};
+        return;
+    }
     auto launch = [&](auto kern, int kc) {
         const int ncol = (k + kc - 1) / kc;
         int per_sm = 1;
@@ -907,16 +1088,8 @@ void philox_normal_f32(uint64_t seed, uint64_t stream, float2* out, uint64_t n, 
     QKG_LAUNCHED();
 }
 template <class T2, class A>
-static void mcomb_multi_impl(const T2* const* V, int k, const std::complex<double>* c, T2* const* W, int nout,
-                             uint64_t n, bool accumulate, Workspace& ws, cudaStream_t s) {
-    QKG_REQUIRE(nout >= 1 && nout <= 8, "mcombine_multi: 1..8 outputs");
-    QKG_REQUIRE(k >= 0 && nout * k <= 1024, "mcombine_multi: at most 1024 coefficients");
-    if (!n) return;
-    // coefficients and the output pointer table go through the workspace result slots
-    double2* dc = ws.result.as<double2>();
-    QKG_CUDA(cudaMemcpyAsync(dc, c, (size_t)nout * k * sizeof(double2), cudaMemcpyHostToDevice, s));
-    T2** dw = reinterpret_cast<T2**>(dc + 1024);
-    QKG_CUDA(cudaMemcpyAsync(dw, W, (size_t)nout * sizeof(T2*), cudaMemcpyHostToDevice, s));
+static void mcomb_multi_launch(const T2* const* V, int k, const double2* dc, T2* const* dw, int nout, uint64_t n,
+                               bool accumulate, cudaStream_t s) {
     const size_t sm = (size_t)nout * k * sizeof(double2);
     const int g = stream_grid(n);
     const int acc = accumulate ? 1 : 0;
@@ -931,8 +1104,26 @@ static void mcomb_multi_impl(const T2* const* V, int k, const std::complex<doubl
         default: mcomb_multi_kernel<T2, A, 8><<<g, kThreads, sm, s>>>(V, k, dc, dw, n, acc); break;
     }
     QKG_LAUNCHED();
+}
+template <class T2, class A>
+static void mcomb_multi_impl(const T2* const* V, int k, const std::complex<double>* c, T2* const* W, int nout,
+                             uint64_t n, bool accumulate, Workspace& ws, cudaStream_t s) {
+    QKG_REQUIRE(nout >= 1 && nout <= 8, "mcombine_multi: 1..8 outputs");
+    QKG_REQUIRE(k >= 0 && nout * k <= 1024, "mcombine_multi: at most 1024 coefficients");
+    if (!n) return;
+    // coefficients and the output pointer table go through the workspace result slots
+    double2* dc = ws.result.as<double2>();
+    QKG_CUDA(cudaMemcpyAsync(dc, c, (size_t)nout * k * sizeof(double2), cudaMemcpyHostToDevice, s));
+    T2** dw = reinterpret_cast<T2**>(dc + 1024);
+    QKG_CUDA(cudaMemcpyAsync(dw, W, (size_t)nout * sizeof(T2*), cudaMemcpyHostToDevice, s));
+    mcomb_multi_launch<T2, A>(V, k, dc, dw, nout, n, accumulate, s);
     // the host arrays may be reused once the copies have been consumed
     QKG_CUDA(cudaStreamSynchronize(s));
+}
+void mcombine_multi_f32_dev(const float2* const* V, int k, const double2* c, float2* const* W, int nout, uint64_t n,
+                            bool accumulate, cudaStream_t s) {
+    QKG_REQUIRE(nout >= 1 && nout <= 8 && k >= 0 && nout * k <= 1024, "mcombine_multi: at most 8 outputs, 1024 coefficients");
+    if (n) mcomb_multi_launch<float2, float>(V, k, c, W, nout, n, accumulate, s);
 }
 void mcombine_multi_f64(const double2* const* V, int k, const std::complex<double>* c, double2* const* W, int nout,
                         uint64_t n, bool accumulate, Workspace& ws, cudaStream_t s) {
