@@ -2,10 +2,18 @@
 // interleaved vectors of several Hamiltonians in one launch.
 //
 // A CTA takes a run of the plan's 128-row tiles.  G lanes share a row; lane l
-// holds the row's 16-byte units l, l + G, ... (a unit: two FP32 or one FP64
-// vector), so that the G lanes of a row read consecutive units: whole sectors and
-// whole 128-byte lines a load instruction.  A row's index work (its quads, its
-// ranks) is shared by its Rp values.
+// holds the row's units l, l + G, ... (16 bytes: two FP32 vectors or one FP64; at
+// four FP32 vectors a lane one unit of 32 bytes, loaded by one instruction), so
+// that the G lanes of a row read consecutive units: whole sectors and whole
+// 128-byte lines a load instruction.  A row's index work (its quads, its ranks) is
+// shared by its Rp values.
+//
+// What bounds it (FP32, 32 vectors): the L1 data pipe and issue (246 us a launch on
+// the 2^20 rows of a Heisenberg ring of 20 sites, every sector; 119 us at 12
+// vectors).  Taken one after the other at 32 / 12 vectors: 310 / 154 us before, the
+// sums in shared memory and not in spilled registers 262 / 140, rests of the outer
+// list as shorter batches and the row's own values last 253 / 139, 32-byte accesses
+// 246 / 119.
 #pragma once
 
 #include "pack.hpp"
@@ -18,7 +26,9 @@ using namespace packk;
 using namespace pairk;
 
 constexpr int kBT = 256;       // threads of a CTA
-constexpr int kBatch = 4;      // outer entries loaded together
+constexpr int kBatch = 3;      // outer entries loaded together
+constexpr int kStrBatch = 2;   // straddling entries loaded together
+template <int N> struct Int { static constexpr int value = N; };
 constexpr int kMaxRun = 8;     // tiles of a CTA
 constexpr int kMaxList = 96;   // outer (and straddling) entries of its blocks staged in shared memory
 
@@ -56,11 +66,13 @@ __device__ __forceinline__ E* offset(E* p, int a, int b) {
 // FP32: pairs (re, im) packed in 64 bits.
 template <class T, int VPL> struct Row;
 template <int VPL> struct Row<float, VPL> {
-    static constexpr int U = VPL >= 2 ? VPL / 2 : 1;  // units (VPL = 1: half a unit)
+    static constexpr int U = VPL >= 2 ? VPL / 2 : 1;  // 16-byte units (VPL = 1: half a unit)
     u64 v[VPL];
     __device__ __forceinline__ void load(const float2* p, int G) {  // p: the lane's first unit
         if constexpr (VPL == 1) {
             v[0] = *reinterpret_cast<const u64*>(p);
+        } else if constexpr (VPL == 4) {
+            asm("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
         } else {
 #pragma unroll
             for (int j = 0; j < U; ++j) {
@@ -74,6 +86,10 @@ template <int VPL> struct Row<float, VPL> {
         if constexpr (VPL == 1) {
             v[0] = 0ull;
             if (on) v[0] = *reinterpret_cast<const u64*>(p);
+        } else if constexpr (VPL == 4) {
+            asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.b64 %0, 0;\n\tmov.b64 %1, 0;\n\tmov.b64 %2, 0;\n\tmov.b64 %3, 0;\n\t"
+                "@p ld.global.v4.b64 {%0, %1, %2, %3}, [%4];\n\t}"
+                : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p), "r"((uint32_t)on));
         } else {
 #pragma unroll
             for (int j = 0; j < U; ++j)
@@ -84,6 +100,8 @@ template <int VPL> struct Row<float, VPL> {
     __device__ __forceinline__ void store(float2* p, int G) const {
         if constexpr (VPL == 1) {
             __stcs(reinterpret_cast<u64*>(p), v[0]);
+        } else if constexpr (VPL == 4) {
+            asm volatile("st.global.cs.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v[0]), "l"(v[1]), "l"(v[2]), "l"(v[3]) : "memory");
         } else {
 #pragma unroll
             for (int j = 0; j < U; ++j)
@@ -169,6 +187,7 @@ template <int VPL> struct Row<double, VPL> {
 // Vector of a lane's j-th value.
 template <class T, int VPL>
 __device__ __forceinline__ int vec_of(int l, int j, int G) {
+    if (sizeof(T) == 4 && VPL == 4) return 4 * l + j;
     if (sizeof(T) == 4 && VPL >= 2) return 2 * (l + (j / 2) * G) + (j & 1);
     return l + j * G;
 }
@@ -223,6 +242,50 @@ template <int VPL> struct Dots<double, VPL> {
     }
     __device__ __forceinline__ double2 get(int j) const { return make_double2(s[j], 0.0); }
 };
+// The SpMV's sums and scales.  FP32: in shared memory, touched once a row (16-byte
+// accesses, one per value); in registers beside the rows in flight they spilled, and
+// every row wrote the spills through to L2 (Heisenberg L = 20, every sector, 32
+// vectors: 310 -> 262 us a launch).
+template <class T, int VPL> struct RowSums : Dots<T, VPL> {
+    static constexpr int kBytes = 0;
+    __device__ __forceinline__ explicit RowSums(char*) {}
+};
+template <int VPL> struct RowSums<float, VPL> {
+    static constexpr int kBytes = kBT * VPL * 20;
+    ulonglong2* s;  // (hi, lo) of the thread's j-th value at j * kBT
+    float* sc;
+    __device__ __forceinline__ explicit RowSums(char* mem)
+        : s(reinterpret_cast<ulonglong2*>(mem) + threadIdx.x), sc(reinterpret_cast<float*>(mem + kBT * VPL * 16) + threadIdx.x * VPL) {}
+    __device__ __forceinline__ void init(int j, double scale) {
+        s[j * kBT] = make_ulonglong2(0ull, 0ull);
+        sc[j] = (float)scale;
+    }
+    __device__ __forceinline__ void finish(Row<float, VPL>& y, const Row<float, VPL>& x, bool dot) {
+        float f[VPL];
+        if constexpr (VPL == 4) {
+            const float4 f4 = *reinterpret_cast<const float4*>(sc);
+            f[0] = f4.x, f[1] = f4.y, f[2] = f4.z, f[3] = f4.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < VPL; ++j) f[j] = sc[j];
+        }
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) {
+            y.v[j] = mul2(y.v[j], pk(f[j], f[j]));
+            if (dot) {
+                ulonglong2 a = s[j * kBT];
+                acc2(a.x, a.y, x.v[j], y.v[j]);
+                s[j * kBT] = a;
+            }
+        }
+    }
+    __device__ __forceinline__ double2 get(int j) const {
+        Dots<float, VPL> d;
+        d.hi[j] = s[j * kBT].x;
+        d.lo[j] = s[j * kBT].y;
+        return d.get(j);
+    }
+};
 // Partial sums as the CTA adds them: FP32 as float pairs (a double-precision
 // reduction in every CTA would cost more than its rows on the narrow FP64 pipe).
 template <class T> struct Part;
@@ -271,7 +334,8 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                       const double* __restrict__ scale, double* __restrict__ apart, int* kstep) {
     using T2 = typename V2<T>::t;
     using R = Row<T, VPL>;
-    __shared__ double red[kBT * VPL];
+    __shared__ alignas(16) char sums_mem[RowSums<T, VPL>::kBytes > kBT * VPL * 8 ? RowSums<T, VPL>::kBytes : kBT * VPL * 8];
+    double* const red = reinterpret_cast<double*>(sums_mem);  // once the rows are done
     __shared__ T s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
     if (kstep && blockIdx.x == 0 && threadIdx.x == 0) ++*kstep;  // the step whose kernels follow
     const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.cta0; });
@@ -285,8 +349,8 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
     }
     const int G = Rp / VPL, NG = kBT / G;
     const int l = threadIdx.x % G, grp = threadIdx.x / G;
-    constexpr int W0 = (sizeof(T) == 4 && VPL >= 2) ? 2 : 1;  // complex values of a unit
-    Dots<T, VPL> dots;
+    constexpr int W0 = (sizeof(T) == 4 && VPL >= 2) ? VPL : 1;  // complex values of a unit
+    RowSums<T, VPL> dots(sums_mem);
 #pragma unroll
     for (int j = 0; j < VPL; ++j)
         dots.init(j, scale ? scale[(size_t)ham * Rp + vec_of<T, VPL>(l, j, G)] : 1.0);
@@ -353,26 +417,9 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                                                            : (uint32_t)__ldg(static_cast<const uint16_t*>(p.dcode) + row);
                 const T2* xo = offset(Xh, (int)row, rb);
                 const T2* xl = offset(Xh, (int)(it.row0 - tin * (uint32_t)kTile), rb);  // the block's rows
-                R acc;
-                acc.zero();
-                // outer entries, kBatch rows in flight
-                uint32_t k = 0;
-                for (; k + kBatch <= no; k += kBatch) {
-                    R v[kBatch];
-#pragma unroll
-                    for (int i = 0; i < kBatch; ++i) v[i].load(offset(xo, outl[k + i].delta, rb), G);
-#pragma unroll
-                    for (int i = 0; i < kBatch; ++i) {
-                        if (CPLX) acc.add(outl[k + i].ar, outl[k + i].ai, v[i]);
-                        else acc.add(outl[k + i].ar, v[i]);
-                    }
-                }
-                for (; k < no; ++k) {
-                    R v;
-                    v.load(offset(xo, outl[k].delta, rb), G);
-                    if (CPLX) acc.add(outl[k].ar, outl[k].ai, v);
-                    else acc.add(outl[k].ar, v);
-                }
+                auto rank_of = [](uint32_t w16) { return (int)(MODE == AMP_SIGNED ? w16 & 0x7FFFu : w16); };
+                constexpr int kNone = MODE == AMP_SIGNED ? (int)kNone15 : (int)kNone16;
+                // the row's index words before its values: the first quad, the straddling entries
                 uint32_t first = rec.x;
                 if (q > 0) first += ((rec.y & 0xFFu) + 3u) >> 2;
                 if (q > 1) first += (((rec.y >> 8) & 0xFFu) + 3u) >> 2;
@@ -381,6 +428,39 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                 uint32_t at = first * 32u + lane;
                 uint2 nxt = __ldg(tab + at);
                 uint32_t cn = MODE == AMP_CODED ? __ldg(codes + at) : 0u;
+                uint32_t sw[kStrBatch], sc[kStrBatch];
+                auto straddles = [&](uint32_t j) {
+#pragma unroll
+                    for (int i = 0; i < kStrBatch; ++i) {
+                        sw[i] = (uint32_t)kNone;
+                        sc[i] = 0u;
+                        if (j + i < ns) {
+                            const uint32_t as = strl[j + i].tab + tin * 32u + lane;
+                            sw[i] = __ldg(reinterpret_cast<const uint16_t*>(tab + as) + q);
+                            if (MODE == AMP_CODED) sc[i] = __ldg(reinterpret_cast<const uint8_t*>(codes + as) + q);
+                        }
+                    }
+                };
+                straddles(0);
+                R acc;
+                acc.zero();
+                // outer entries, the rows of up to kBatch of them in flight; their number is the
+                // warp's, so that a short rest is a shorter batch and not a chain of loads
+                auto outer = [&](uint32_t k, auto batch) {
+                    constexpr int N = decltype(batch)::value;
+                    R v[N];
+#pragma unroll
+                    for (int i = 0; i < N; ++i) v[i].load(offset(xo, outl[k + i].delta, rb), G);
+#pragma unroll
+                    for (int i = 0; i < N; ++i) {
+                        if (CPLX) acc.add(outl[k + i].ar, outl[k + i].ai, v[i]);
+                        else acc.add(outl[k + i].ar, v[i]);
+                    }
+                };
+                uint32_t k = 0;
+                for (; k + kBatch <= no; k += kBatch) outer(k, Int<kBatch>{});
+                if (no - k == 2) outer(k, Int<2>{});
+                else if (no - k == 1) outer(k, Int<1>{});
                 auto amp_add = [&](uint32_t w16, uint32_t code, T a, const R& v) {
                     if (MODE == AMP_CODED) {
                         const uint32_t c = code & 0xFFu;
@@ -390,8 +470,6 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                         acc.add(MODE == AMP_SIGNED && (w16 & 0x8000u) ? -a : a, v);
                     }
                 };
-                auto rank_of = [](uint32_t w16) { return (int)(MODE == AMP_SIGNED ? w16 & 0x7FFFu : w16); };
-                constexpr int kNone = MODE == AMP_SIGNED ? (int)kNone15 : (int)kNone16;
                 for (int n = slots; n > 0; n -= 4) {
                     const uint2 e = nxt;
                     const uint32_t c = cn;
@@ -401,6 +479,7 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                         if (MODE == AMP_CODED) cn = __ldg(codes + at);
                     }
                     const uint32_t w[4] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16};
+                    if (rank_of(w[0]) == kNone) break;  // a row's entries come first
                     // the four rows' loads go out together; an empty slot reads zero
                     R v[4];
 #pragma unroll
@@ -411,17 +490,17 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
 #pragma unroll
                     for (int h = 0; h < 4; ++h) amp_add(w[h], c >> (8 * h), u, v[h]);
                 }
-                for (uint32_t j = 0; j < ns; ++j) {
-                    const Str<T> s = strl[j];
-                    const uint32_t as = s.tab + tin * 32u + lane;
-                    const uint2 e = __ldg(tab + as);
-                    const uint32_t w = (q & 2u) ? e.y : e.x, w16 = (q & 1u) ? w >> 16 : w & 0xFFFFu;
-                    const uint32_t c = MODE == AMP_CODED ? __ldg(codes + as) >> (8 * q) : 0u;
-                    const int to = rank_of(w16);
-                    if (to == kNone) continue;
-                    R v;
-                    v.load(offset(Xh, (int)s.off + to, rb), G);
-                    amp_add(w16, c, s.ar, v);
+                for (uint32_t j = 0; j < ns; j += kStrBatch) {
+                    if (j) straddles(j);
+                    R v[kStrBatch];
+#pragma unroll
+                    for (int i = 0; i < kStrBatch; ++i) {
+                        const int to = rank_of(sw[i]);
+                        v[i].load_if(offset(Xh, j + i < ns ? (int)strl[j + i].off + to : 0, rb), G, to != kNone);
+                    }
+#pragma unroll
+                    for (int i = 0; i < kStrBatch; ++i)
+                        if (j + i < ns) amp_add(sw[i], sc[i], strl[j + i].ar, v[i]);
                 }
                 R x;
                 x.load(xo, G);
@@ -433,9 +512,13 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
             }
     }
     if (apart) {
+        double own[VPL];
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) own[j] = dots.get(j).x;
+        __syncthreads();  // red lies over the sums
         if (grp < NG)
 #pragma unroll
-            for (int j = 0; j < VPL; ++j) red[grp * Rp + vec_of<T, VPL>(l, j, G)] = dots.get(j).x;
+            for (int j = 0; j < VPL; ++j) red[grp * Rp + vec_of<T, VPL>(l, j, G)] = own[j];
         __syncthreads();
         reduce_vectors<T>(red, NG, Rp, apart + (size_t)blockIdx.x * Rp);
     }
