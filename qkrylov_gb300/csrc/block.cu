@@ -333,63 +333,22 @@ __global__ void __launch_bounds__(kBlock) block_update_kernel(const BItem* __res
     }
 }
 
-struct BState {
-    double *c_cur, *c_prev, *beta_prev, *ca, *cb, *norm2;
-    double *alpha, *beta;  // [k * V + vid]
-    int *active, *n_alpha, *n_beta, *kstep;
-    int V, Rp, Ruser;
-};
-
-enum { FIN_INIT = 0, FIN_ALPHA = 1, FIN_BETA = 2 };
+using blockk::BState;
+using blockk::FIN_ALPHA;
+using blockk::FIN_BETA;
+using blockk::FIN_INIT;
 
 // Per vector (one CTA each): the sum of its CTA partials over its
-// Hamiltonian's CTA range (fixed order), then the scalar bookkeeping.
+// Hamiltonian's CTA range (fixed order), then the scalar bookkeeping of step k (k < 0: the step on the device).
 __global__ void __launch_bounds__(kBlock) block_finish_kernel(const double* __restrict__ part,
                                                               const uint32_t* __restrict__ cta_range, int mode,
-                                                              BState st) {
+                                                              BState st, int k) {
     const int vid = blockIdx.x, h = vid / st.Rp, v = vid % st.Rp;
     double acc = 0.0;
     for (uint32_t c = cta_range[h] + threadIdx.x; c < cta_range[h + 1]; c += blockDim.x) acc += part[(size_t)c * st.Rp + v];
     acc = block_sum_d(acc);
     if (threadIdx.x) return;
-    if (mode == FIN_INIT) {
-        st.norm2[vid] = acc;
-        const double nr = sqrt(acc);
-        const bool on = v < st.Ruser && nr >= 1e-15;  // dynamics.cpp:27
-        st.active[vid] = on;
-        st.c_cur[vid] = on ? 1.0 / nr : 0.0;
-        st.c_prev[vid] = 0.0;
-        st.beta_prev[vid] = 0.0;
-        st.n_alpha[vid] = 0;
-        st.n_beta[vid] = 0;
-        return;
-    }
-    const int k = *st.kstep;
-    if (mode == FIN_ALPHA) {
-        if (st.active[vid]) {
-            const double a = st.c_cur[vid] * acc;
-            st.alpha[(size_t)k * st.V + vid] = a;
-            st.n_alpha[vid] = k + 1;
-            st.ca[vid] = a * st.c_cur[vid];
-            st.cb[vid] = st.beta_prev[vid] * st.c_prev[vid];
-        } else {
-            st.ca[vid] = 0.0;
-            st.cb[vid] = 0.0;
-        }
-        return;
-    }
-    if (!st.active[vid]) return;
-    const double b = sqrt(acc);
-    st.c_prev[vid] = st.c_cur[vid];
-    if (b < 1e-15) {  // ftlm.cpp:45, dynamics.cpp:52
-        st.active[vid] = 0;
-        st.c_cur[vid] = 0.0;
-        return;
-    }
-    st.beta[(size_t)k * st.V + vid] = b;
-    st.n_beta[vid] = k + 1;
-    st.c_cur[vid] = 1.0 / b;
-    st.beta_prev[vid] = b;
+    blockk::finish_vector(st, vid, acc, mode, k >= 0 ? k : *st.kstep);
 }
 
 __global__ void block_advance_kernel(int* k) { ++*k; }
@@ -537,7 +496,7 @@ public:
         QKG_LAUNCHED();
     }
     void finish(const double* part, int mode, const BState& st) {
-        block_finish_kernel<<<(unsigned)(hs_.size() * Rp_), kBlock, 0, s_>>>(part, range_.as<uint32_t>(), mode, st);
+        block_finish_kernel<<<(unsigned)(hs_.size() * Rp_), kBlock, 0, s_>>>(part, range_.as<uint32_t>(), mode, st, mode == FIN_INIT ? 0 : -1);
         QKG_LAUNCHED();
     }
     void philox(uint64_t seed, T2* u) {
@@ -614,7 +573,7 @@ public:
         chunk_ = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, total / (152 * 4) / 32 * 32));
         std::vector<packk::Params<T>> P(hs.size());
         std::vector<blockk::Ham> hams(hs.size());
-        std::vector<uint32_t> range(1, 0), rrange(1, 0);
+        std::vector<uint32_t> range(1, 0), rrange(1, 0);  // CTAs by Hamiltonian
         for (size_t h = 0; h < hs.size(); ++h) {
             Hamiltonian& H = *hs[h];
             QKG_REQUIRE(H.device() == hs[0]->device(), "batched Lanczos needs every Hamiltonian on one device");
@@ -636,6 +595,7 @@ public:
         n_ctas_ = range.back();
         n_row_ctas_ = rrange.back();
         range.insert(range.end(), rrange.begin(), rrange.end());
+        range.insert(range.end(), hams.size(), 0u);  // the arrival counters
         // the workspace: three vectors, then everything else, 256-byte aligned
         auto al = [](size_t b) { return (b + 255) / 256 * 256; };
         const size_t vbytes = al(std::max<uint64_t>(1, rows_) * Rp * sizeof(T2));
@@ -645,13 +605,14 @@ public:
         for (int i = 0; i < 3; ++i) buf_[i] = ws + (size_t)i * vbytes;
         char* q = ws + 3 * vbytes;
         std::vector<char> image(pb + hb + rb);
+        std::memcpy(image.data() + pb + hb, range.data(), range.size() * 4);
         std::memcpy(image.data(), P.data(), P.size() * sizeof(P[0]));
         std::memcpy(image.data() + pb, hams.data(), hams.size() * sizeof(hams[0]));
-        std::memcpy(image.data() + pb + hb, range.data(), range.size() * 4);
         QKG_CUDA(cudaMemcpyAsync(q, image.data(), image.size(), cudaMemcpyHostToDevice, s_));  // pageable: copied on return
         params_ = reinterpret_cast<packk::Params<T>*>(q);
         hams_ = reinterpret_cast<blockk::Ham*>(q + pb);
         range_ = reinterpret_cast<uint32_t*>(q + pb + hb);
+        arrived_ = range_ + 2 * (hams.size() + 1);
         apart_ = reinterpret_cast<double*>(q + pb + hb + rb);
         bpart_ = reinterpret_cast<double*>(q + pb + hb + rb + ab);
         extra_ = q + pb + hb + rb + ab + bb;
@@ -670,25 +631,25 @@ public:
         return Rp_ % 4 == 0 ? 4 : Rp_ % 2 == 0 ? 2 : 1;
     }
 
-    void spmv(int vpl, const T2* x, T2* y, const double* scale, double* apart, int* kstep) {
+    void spmv(int vpl, const T2* x, T2* y, const double* scale, double* apart, const BState& st, int k) {
         if (!n_ctas_) return;
-        if (vpl == 4) spmv_v<4>(x, y, scale, apart, kstep);
-        else if (vpl == 2) spmv_v<2>(x, y, scale, apart, kstep);
-        else spmv_v<1>(x, y, scale, apart, kstep);
+        const bool fused = n_ctas_ <= kFusedCtas;
+        const blockk::Finish fin{st, arrived_, FIN_ALPHA, k};
+        if (vpl == 4) spmv_v<4>(x, y, scale, apart, fin, fused);
+        else if (vpl == 2) spmv_v<2>(x, y, scale, apart, fin, fused);
+        else spmv_v<1>(x, y, scale, apart, fin, fused);
+        if (!fused) finish(apart, range_, FIN_ALPHA, st, k);
     }
-    void update(const T2* u, const T2* up, T2* y, const double* ca, const double* cb, double* part) {
+    void update(const T2* u, const T2* up, T2* y, const double* ca, const double* cb, double* part, int mode, const BState& st, int k) {
         if (!n_row_ctas_) return;
+        const bool fused = n_row_ctas_ <= kFusedCtas;
+        const blockk::Finish fin{st, arrived_, mode, k};
         constexpr int W = sizeof(T) == 4 ? 2 : 1;
-        if (Rp_ % W == 0)
-            blockk::block_pack_update<T, W><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), chunk_, Rp_, y, u, up, ca, cb, part);
-        else
-            blockk::block_pack_update<T, 1><<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), chunk_, Rp_, y, u, up, ca, cb, part);
+        auto* kernel = Rp_ % W == 0 ? (fused ? blockk::block_pack_update<T, W, true> : blockk::block_pack_update<T, W, false>)
+                                    : (fused ? blockk::block_pack_update<T, 1, true> : blockk::block_pack_update<T, 1, false>);
+        kernel<<<n_row_ctas_, blockk::kBT, 0, s_>>>(hams_, (int)hs_.size(), chunk_, Rp_, y, u, up, ca, cb, part, fin);
         QKG_LAUNCHED();
-    }
-    void finish(const double* part, int mode, const BState& st) {
-        const uint32_t* r = range_ + (mode == FIN_ALPHA ? 0 : hs_.size() + 1);
-        block_finish_kernel<<<(unsigned)(hs_.size() * Rp_), kBlock, 0, s_>>>(part, r, mode, st);
-        QKG_LAUNCHED();
+        if (!fused) finish(part, range_ + hs_.size() + 1, mode, st, k);
     }
     void philox(uint64_t seed, T2* u) {
         if (!n_row_ctas_) return;
@@ -717,6 +678,17 @@ public:
 
 private:
     static constexpr uint32_t kPasses = 8;
+    // Up to one wave of CTAs the last CTA of a Hamiltonian sums up and does the scalars
+    // itself (40 steps of every sector: L = 10, 4 vectors 1.11 -> 0.87 ms, L = 14, 24 vectors
+    // 1.42 -> 1.24); beyond, each CTA's fence, behind all its stores, would keep the next one
+    // from its place (L = 20, 32 vectors 16.9 -> 17.4 ms; L = 22, 12 vectors, Sz = 0, 120 steps
+    // 18.9 -> 22.8).
+    static constexpr unsigned kFusedCtas = 4 * 152;
+
+    void finish(const double* part, const uint32_t* range, int mode, const BState& st, int k) {
+        block_finish_kernel<<<(unsigned)(hs_.size() * Rp_), kBlock, 0, s_>>>(part, range, mode, st, k);
+        QKG_LAUNCHED();
+    }
 
     static bool plans(const std::vector<Hamiltonian*>& hs, std::vector<const PackPlan*>& out) {
         int form = packk::AMP_UNIFORM;
@@ -738,12 +710,12 @@ private:
     }
 
     template <int VPL>
-    void spmv_v(const T2* x, T2* y, const double* scale, double* apart, int* kstep) {
+    void spmv_v(const T2* x, T2* y, const double* scale, double* apart, const blockk::Finish& fin, bool fused) {
         auto go = [&](auto mode, auto cplx) {
             constexpr int M = decltype(mode)::value;
             constexpr bool C = decltype(cplx)::value;
-            blockk::block_pack_kernel<T, M, C, VPL><<<n_ctas_, blockk::kBT, 0, s_>>>(params_, hams_, (int)hs_.size(), run_, Rp_,
-                                                                                    x, y, scale, apart, kstep);
+            auto* kernel = fused ? blockk::block_pack_kernel<T, M, C, VPL, true> : blockk::block_pack_kernel<T, M, C, VPL, false>;
+            kernel<<<n_ctas_, blockk::kBT, 0, s_>>>(params_, hams_, (int)hs_.size(), run_, Rp_, x, y, scale, apart, fin);
         };
         using std::integral_constant;
         if (mode_ == packk::AMP_UNIFORM) go(integral_constant<int, packk::AMP_UNIFORM>{}, std::false_type{});
@@ -766,6 +738,7 @@ private:
     packk::Params<T>* params_ = nullptr;
     blockk::Ham* hams_ = nullptr;
     uint32_t* range_ = nullptr;
+    unsigned int* arrived_ = nullptr;
     double *apart_ = nullptr, *bpart_ = nullptr;
     void* extra_ = nullptr;
     void* buf_[3] = {nullptr, nullptr, nullptr};
@@ -957,14 +930,13 @@ BlockTridiag run_packed(const std::vector<Hamiltonian*>& hs, const BlockOpts& o,
     const int V = out.n_ham * Rp;
     const int M = std::max(0, o.steps);
     // device state: six scalars a vector, alpha and beta of every step, then integers
-    const size_t nd = 6 * (size_t)V + 2 * (size_t)M * V, ni = 3 * (size_t)V + 1;
+    const size_t nd = 6 * (size_t)V + 2 * (size_t)M * V, ni = 3 * (size_t)V;
     Engine E(hs, Rp, o.R, nd * sizeof(double) + ni * sizeof(int));
     cudaStream_t s = E.stream();
     out.rows = E.rows();
     double* d = static_cast<double*>(E.extra());
     int* ip = reinterpret_cast<int*>(d + nd);
     QKG_CUDA(cudaMemsetAsync(d, 0, nd * sizeof(double) + ni * sizeof(int), s));
-    QKG_CUDA(cudaMemsetAsync(ip + 3 * (size_t)V, 0xFF, sizeof(int), s));  // the first SpMV makes it step 0
     BState st;
     st.c_cur = d;
     st.c_prev = d + V;
@@ -977,7 +949,7 @@ BlockTridiag run_packed(const std::vector<Hamiltonian*>& hs, const BlockOpts& o,
     st.active = ip;
     st.n_alpha = ip + V;
     st.n_beta = ip + 2 * V;
-    st.kstep = ip + 3 * V;
+    st.kstep = nullptr;  // the host counts
     st.V = V;
     st.Rp = Rp;
     st.Ruser = o.R;
@@ -1013,19 +985,16 @@ BlockTridiag run_packed(const std::vector<Hamiltonian*>& hs, const BlockOpts& o,
     std::vector<std::unique_ptr<LaunchTimer>> tsp;
     for (int k = 0; k < std::min(M, kTimed); ++k) tsp.push_back(std::make_unique<LaunchTimer>(s));
     total.start();
-    E.update(nullptr, nullptr, U0, nullptr, nullptr, E.bpart());  // ||u_0||^2 partials
-    E.finish(E.bpart(), FIN_INIT, st);
+    E.update(nullptr, nullptr, U0, nullptr, nullptr, E.bpart(), FIN_INIT, st, 0);  // ||u_0||^2
     // step k: u_k = buf[k % 3], u_{k-1} = buf[(k + 2) % 3], y = buf[(k + 1) % 3]
     for (int k = 0; k < M; ++k) {
         T2* u = E.buf(k % 3);
         T2* up = k ? E.buf((k + 2) % 3) : nullptr;
         T2* y = E.buf((k + 1) % 3);
         if (k < kTimed) tsp[k]->start();
-        E.spmv(vpl, u, y, st.c_cur, E.apart(), st.kstep);
+        E.spmv(vpl, u, y, st.c_cur, E.apart(), st, k);
         if (k < kTimed) tsp[k]->stop();
-        E.finish(E.apart(), FIN_ALPHA, st);
-        E.update(u, up, y, st.ca, st.cb, E.bpart());
-        E.finish(E.bpart(), FIN_BETA, st);
+        E.update(u, up, y, st.ca, st.cb, E.bpart(), FIN_BETA, st, k);
     }
     total.stop();
     std::vector<double> hd(nd);

@@ -40,6 +40,65 @@ struct Ham {
     uint32_t cta0, row_cta0;
     const uint32_t* perm;  // reference index of each internal row (null: the same)
 };
+// The vectors' scalars on the device.
+struct BState {
+    double *c_cur, *c_prev, *beta_prev, *ca, *cb, *norm2;
+    double *alpha, *beta;  // [k * V + vid]
+    int *active, *n_alpha, *n_beta, *kstep;
+    int V, Rp, Ruser;
+};
+enum { FIN_INIT = 0, FIN_ALPHA = 1, FIN_BETA = 2 };
+
+// The bookkeeping of vector vid from its sum: the norm of the start vector, step k's
+// alpha or its beta.
+__device__ __forceinline__ void finish_vector(const BState& st, int vid, double acc, int mode, int k) {
+    if (mode == FIN_INIT) {
+        st.norm2[vid] = acc;
+        const double nr = sqrt(acc);
+        const bool on = vid % st.Rp < st.Ruser && nr >= 1e-15;  // dynamics.cpp:27
+        st.active[vid] = on;
+        st.c_cur[vid] = on ? 1.0 / nr : 0.0;
+        st.c_prev[vid] = 0.0;
+        st.beta_prev[vid] = 0.0;
+        st.n_alpha[vid] = 0;
+        st.n_beta[vid] = 0;
+        return;
+    }
+    if (mode == FIN_ALPHA) {
+        if (st.active[vid]) {
+            const double a = st.c_cur[vid] * acc;
+            st.alpha[(size_t)k * st.V + vid] = a;
+            st.n_alpha[vid] = k + 1;
+            st.ca[vid] = a * st.c_cur[vid];
+            st.cb[vid] = st.beta_prev[vid] * st.c_prev[vid];
+        } else {
+            st.ca[vid] = 0.0;
+            st.cb[vid] = 0.0;
+        }
+        return;
+    }
+    if (!st.active[vid]) return;
+    const double b = sqrt(acc);
+    st.c_prev[vid] = st.c_cur[vid];
+    if (b < 1e-15) {  // ftlm.cpp:45, dynamics.cpp:52
+        st.active[vid] = 0;
+        st.c_cur[vid] = 0.0;
+        return;
+    }
+    st.beta[(size_t)k * st.V + vid] = b;
+    st.n_beta[vid] = k + 1;
+    st.c_cur[vid] = 1.0 / b;
+    st.beta_prev[vid] = b;
+}
+
+// What the last CTA of a Hamiltonian does with its CTAs' partial sums (in the
+// kernels' FUSED form; else they are left to a kernel of their own).
+struct Finish {
+    BState st;
+    unsigned int* arrived;  // per Hamiltonian, 0 between launches
+    int mode, k;
+};
+
 // the Hamiltonian whose range holds CTA c
 template <class F>
 __device__ __forceinline__ int find_ham(const Ham* __restrict__ hams, int n, uint32_t c, F first) {
@@ -327,17 +386,52 @@ __device__ __forceinline__ void reduce_vectors(double* red, int n_groups, int Rp
     if ((int)threadIdx.x < Rp) part[threadIdx.x] = a.value();  // s = 0
 }
 
-template <class T, int MODE, bool CPLX, int VPL>
+// The last of a Hamiltonian's n_ctas CTAs (partials part[c * Rp + v], this CTA's
+// written by its first Rp threads) adds them up, in CTA order by rows of kBT / Rp, and
+// does the vectors' bookkeeping.
+__device__ __forceinline__ void finish_ham(const Finish& f, int ham, uint32_t n_ctas, int Rp, const double* part, double* red) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(f.arrived + ham, 1u) == n_ctas - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x == 0) f.arrived[ham] = 0u;
+    const int v = threadIdx.x % Rp, s = threadIdx.x / Rp, ns = kBT / Rp;
+    double a = 0.0;
+    if (s < ns) {
+#pragma unroll 8
+        for (uint32_t c = s; c < n_ctas; c += ns) a += __ldcg(part + (size_t)c * Rp + v);
+        red[s * Rp + v] = a;
+    }
+    __syncthreads();
+    for (int n = ns; n > 1;) {  // halves onto each other
+        const int h = (n + 1) / 2;
+        if (s < n - h) {
+            a += red[(s + h) * Rp + v];
+            red[s * Rp + v] = a;
+        }
+        n = h;
+        __syncthreads();
+    }
+    if ((int)threadIdx.x < Rp) finish_vector(f.st, ham * Rp + v, a, f.mode, f.k);
+}
+
+// FUSED: the bookkeeping in the Hamiltonian's last CTA (an instantiation of its own: the
+// code alone cost the large batches 2 %).
+template <class T, int MODE, bool CPLX, int VPL, bool FUSED>
 __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
     block_pack_kernel(const Params<T>* __restrict__ P, const Ham* __restrict__ hams, int n_hams, int run, int Rp,
                       const typename V2<T>::t* __restrict__ X, typename V2<T>::t* __restrict__ Y,
-                      const double* __restrict__ scale, double* __restrict__ apart, int* kstep) {
+                      const double* __restrict__ scale, double* __restrict__ apart, const Finish fin) {
     using T2 = typename V2<T>::t;
     using R = Row<T, VPL>;
     __shared__ alignas(16) char sums_mem[RowSums<T, VPL>::kBytes > kBT * VPL * 8 ? RowSums<T, VPL>::kBytes : kBT * VPL * 8];
     double* const red = reinterpret_cast<double*>(sums_mem);  // once the rows are done
     __shared__ T s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
-    if (kstep && blockIdx.x == 0 && threadIdx.x == 0) ++*kstep;  // the step whose kernels follow
     const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.cta0; });
     const Params<T>& p = P[ham];
     const uint32_t tile0 = (blockIdx.x - hams[ham].cta0) * (uint32_t)run;
@@ -521,17 +615,18 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
             for (int j = 0; j < VPL; ++j) red[grp * Rp + vec_of<T, VPL>(l, j, G)] = own[j];
         __syncthreads();
         reduce_vectors<T>(red, NG, Rp, apart + (size_t)blockIdx.x * Rp);
+        if constexpr (FUSED) finish_ham(fin, ham, (p.n_items + run - 1) / run, Rp, apart + (size_t)hams[ham].cta0 * Rp, red);
     }
 }
 
 // w = y - ca u - cb up in place on y, and per CTA the partial ||w_v||^2 (u ==
 // nullptr: only the norms of y; Up == nullptr: no previous vector).  A CTA takes
 // `chunk` rows of one Hamiltonian, a lane one 16-byte unit (VPL values) of a row.
-template <class T, int VPL>
+template <class T, int VPL, bool FUSED>
 __global__ void __launch_bounds__(kBT)
     block_pack_update(const Ham* __restrict__ hams, int n_hams, uint32_t chunk, int Rp, typename V2<T>::t* __restrict__ Y,
                       const typename V2<T>::t* __restrict__ U, const typename V2<T>::t* __restrict__ Up,
-                      const double* __restrict__ ca, const double* __restrict__ cb, double* __restrict__ part) {
+                      const double* __restrict__ ca, const double* __restrict__ cb, double* __restrict__ part, const Finish fin) {
     using R = Row<T, VPL>;
     __shared__ double red[kBT * VPL];
     const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.row_cta0; });
@@ -570,6 +665,7 @@ __global__ void __launch_bounds__(kBT)
     }
     __syncthreads();
     reduce_vectors<T>(red, NG, Rp, part + (size_t)blockIdx.x * Rp);
+    if constexpr (FUSED) finish_ham(fin, ham, (uint32_t)((hams[ham].dim + chunk - 1) / chunk), Rp, part + (size_t)hams[ham].row_cta0 * Rp, red);
 }
 
 // Seeded Philox Gaussian start vectors in reference order: vector v of
