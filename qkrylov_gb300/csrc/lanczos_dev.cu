@@ -22,6 +22,7 @@
 // them a few steps behind the GPU (convergence test, selective
 // reorthogonalisation trigger) without stalling the stream.
 #include "fast_common.cuh"
+#include "pair.cuh"
 #include "solvers.hpp"
 
 #include <algorithm>
@@ -33,10 +34,15 @@
 
 namespace qkg {
 using namespace fastk;
+using namespace pairk;
 
 namespace {
 constexpr int kT = 256;
 constexpr int kUpdGrid = 152 * 8;
+// CTAs of the FP32 update and correction: each ends in block sums, a fence and an atomic, so
+// fewer of them with more bytes in flight each (100 steps at L = 24: 8 CTAs an SM and 16-byte
+// accesses 8.91 ms, 32-byte accesses 8.98, with 4 CTAs an SM 8.63, with 2 8.73).
+constexpr int kUpdGrid32 = 152 * 4;
 constexpr int kTimedSteps = 8;  // steps launched one by one with an SpMV timer before the graph takes over
 constexpr int kInFlight = 6;    // steps the host lets the GPU run ahead of its checks
 constexpr double kOrthTol = 3.4526698300124393e-4;  // sqrt(2^-23): FP32 semiorthogonality level
@@ -82,74 +88,90 @@ __global__ void __launch_bounds__(kAlphaThreads) lz_alpha_kernel(const double2* 
     if (threadIdx.x == 0) lz_set_alpha(d, t);
 }
 
-// One element of the update w -= a v with its ||w||^2 (and, with
-// NP Ritz vectors psi_p, the <psi_p, w>) contributions.
+// Four elements of the update w -= a v with its ||w||^2 (and, with NP Ritz vectors psi_p,
+// the <psi_p, w>) contributions: compensated sums of (re, im) pairs.
 template <int NP>
 struct UpdAcc {
-    float hi = 0.f, lo = 0.f;
-    float rh[NP > 0 ? NP : 1] = {}, rl[NP > 0 ? NP : 1] = {}, ih[NP > 0 ? NP : 1] = {}, il[NP > 0 ? NP : 1] = {};
+    static constexpr int NQ = NP > 0 ? NP : 1;
+    u64 hi = 0, lo = 0;                                   // Re^2, Im^2 of w
+    u64 rh[NQ] = {}, rl[NQ] = {}, ih[NQ] = {}, il[NQ] = {};  // the two products of Re and of Im <psi, w>
 };
+constexpr u64 kConj2 = 0x8000000000000000ull;  // the sign of the imaginary part
 template <int NP>
-__device__ __forceinline__ float2 upd_elem(float2 x, float2 c, const float2 (&p)[NP > 0 ? NP : 1], float a, UpdAcc<NP>& s) {
-    x.x = fmaf(-a, c.x, x.x);
-    x.y = fmaf(-a, c.y, x.y);
-    ff_acc(s.hi, s.lo, x.x, x.x);
-    ff_acc(s.hi, s.lo, x.y, x.y);
-#pragma unroll
-    for (int q = 0; q < NP; ++q) {
-        ff_acc(s.rh[q], s.rl[q], p[q].x, x.x);
-        ff_acc(s.rh[q], s.rl[q], p[q].y, x.y);
-        ff_acc(s.ih[q], s.il[q], p[q].x, x.y);
-        ff_acc(s.ih[q], s.il[q], -p[q].y, x.x);
-    }
-    return x;
+__device__ __forceinline__ void upd_elem(u64& x, u64 c, u64 a2, UpdAcc<NP>& s) {
+    x = fma2(a2, c, x);
+    acc2(s.hi, s.lo, x, x);
 }
+template <int NP>
+__device__ __forceinline__ void upd_psi(u64 x, u64 p, int q, UpdAcc<NP>& s) {
+    const float2 f = unpk(x);
+    acc2(s.rh[q], s.rl[q], p, x);
+    acc2(s.ih[q], s.il[q], p ^ kConj2, pk(f.y, f.x));
+}
+// the two halves of a compensated pair sum added
+__device__ __forceinline__ float2 halves(u64 hi, u64 lo) {
+    const float2 h = unpk(hi), l = unpk(lo);
+    float a = h.x, b = l.x;
+    ff_add(a, b, h.y, l.y);
+    return make_float2(a, b);
+}
+struct Four {
+    u64 v[4];
+    __device__ __forceinline__ explicit Four(const float2* p) {
+        asm("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
+    }
+    __device__ __forceinline__ void store(float2* p) const {
+        asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v[0]), "l"(v[1]), "l"(v[2]), "l"(v[3]) : "memory");
+    }
+};
 
 // w -= a v in place (the SpMV applied the previous-vector term), ||w||^2 (and the
 // <psi_q, w> of the NP Ritz vectors, for selective reorthogonalisation), and from them
-// beta: two elements per thread and iteration with 16-byte accesses (the Krylov vectors
-// are 256-byte aligned).  ppart[q * gridDim.x + block] holds Ritz vector q's partial.
+// beta: four elements per thread and iteration with 32-byte accesses (the Krylov vectors
+// and the Ritz vectors are 256-byte aligned).  ppart[q * gridDim.x + block] holds Ritz
+// vector q's partial.
 template <int NP>
 __global__ void __launch_bounds__(kT) lz_update_t(const LzDev d, uint64_t n, const PsiTab psi, double orth_tol,
                                                   double2* __restrict__ bpart, double2* __restrict__ ppart) {
     const int k = d.st->k;
-    float2* __restrict__ w = static_cast<float2*>(d.vtab[k + 1]);
-    const float2* __restrict__ v = static_cast<const float2*>(d.vtab[k]);
-    const float a = (float)d.st->a;
+    float2* w = static_cast<float2*>(d.vtab[k + 1]);
+    const float2* v = static_cast<const float2*>(d.vtab[k]);
+    const float a = -(float)d.st->a;
+    const u64 a2 = pk(a, a);
     UpdAcc<NP> s;
-    constexpr int NQ = NP > 0 ? NP : 1;
-    const uint64_t n2 = n / 2, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t n4 = n / 4, step = (uint64_t)gridDim.x * blockDim.x;
 #pragma unroll 2
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n2; i += step) {
-        const float4 x4 = reinterpret_cast<const float4*>(w)[i];
-        const float4 c4 = reinterpret_cast<const float4*>(v)[i];
-        float2 p0[NQ], p1[NQ];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n4; i += step) {
+        Four x(w + 4 * i);
+        const Four c(v + 4 * i);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            float4 p4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (q < NP) p4 = reinterpret_cast<const float4*>(psi.p[q])[i];
-            p0[q] = make_float2(p4.x, p4.y);
-            p1[q] = make_float2(p4.z, p4.w);
+        for (int e = 0; e < 4; ++e) upd_elem<NP>(x.v[e], c.v[e], a2, s);
+        x.store(w + 4 * i);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const Four p(psi.p[q] + 4 * i);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) upd_psi<NP>(x.v[e], p.v[e], q, s);
         }
-        const float2 y0 = upd_elem<NP>(make_float2(x4.x, x4.y), make_float2(c4.x, c4.y), p0, a, s);
-        const float2 y1 = upd_elem<NP>(make_float2(x4.z, x4.w), make_float2(c4.z, c4.w), p1, a, s);
-        reinterpret_cast<float4*>(w)[i] = make_float4(y0.x, y0.y, y1.x, y1.y);
     }
-    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
-        float2 pl[NQ];
+    if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
+        const uint64_t i = 4 * n4 + threadIdx.x;
+        u64 x = reinterpret_cast<const u64*>(w)[i];
+        upd_elem<NP>(x, reinterpret_cast<const u64*>(v)[i], a2, s);
+        reinterpret_cast<u64*>(w)[i] = x;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) pl[q] = q < NP ? psi.p[q][n - 1] : make_float2(0.f, 0.f);
-        w[n - 1] = upd_elem<NP>(w[n - 1], v[n - 1], pl, a, s);
+        for (int q = 0; q < NP; ++q) upd_psi<NP>(x, reinterpret_cast<const u64*>(psi.p[q])[i], q, s);
     }
     // block sums in float-float FP32 arithmetic: a double sum in each of the CTAs
-    // cost as much as the pass on GB300's narrow FP64 pipe (L = 24, no Ritz vector 18.5
-    // us, one 29.5 us)
-    const float2 t = block_sum_ff(s.hi, s.lo);
+    // cost as much as the pass on GB300's narrow FP64 pipe
+    float2 t = halves(s.hi, s.lo);
+    t = block_sum_ff(t.x, t.y);
     if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2((double)t.x + (double)t.y, 0.0);
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        const float2 r = block_sum_ff(s.rh[q], s.rl[q]);
-        const float2 m = block_sum_ff(s.ih[q], s.il[q]);
+        float2 r = halves(s.rh[q], s.rl[q]), m = halves(s.ih[q], s.il[q]);
+        r = block_sum_ff(r.x, r.y);
+        m = block_sum_ff(m.x, m.y);
         if (threadIdx.x == 0)
             ppart[(size_t)q * gridDim.x + blockIdx.x] = make_double2((double)r.x + (double)r.y, (double)m.x + (double)m.y);
     }
@@ -186,28 +208,43 @@ template <int NP>
 __global__ void __launch_bounds__(kT) lz_orth_kernel(const LzDev d, const PsiTab psi, uint64_t n, double2* __restrict__ bpart) {
     if (!d.st->orth) return;
     const int k = d.st->k;
-    float2* __restrict__ w = static_cast<float2*>(d.vtab[k + 1]);
-    float cr[NP], ci[NP];
+    float2* w = static_cast<float2*>(d.vtab[k + 1]);
+    u64 cr[NP], ci[NP];  // -(c, c) and (im c, -im c)
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        cr[q] = (float)d.st->pre[q];
-        ci[q] = (float)d.st->pim[q];
+        const float r = (float)d.st->pre[q], m = (float)d.st->pim[q];
+        cr[q] = pk(-r, -r);
+        ci[q] = pk(m, -m);
     }
-    float hi = 0.f, lo = 0.f;
+    auto take = [&](u64 x, u64 p, int q) {
+        const float2 f = unpk(p);
+        return fma2(ci[q], pk(f.y, f.x), fma2(cr[q], p, x));
+    };
+    u64 h2 = 0, l2 = 0;
+    const uint64_t n4 = n / 4;
 #pragma unroll 2
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        float2 x = w[i];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n4; i += (uint64_t)gridDim.x * blockDim.x) {
+        Four x(w + 4 * i);
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
-            const float2 p = psi.p[q][i];
-            x.x -= cr[q] * p.x - ci[q] * p.y;
-            x.y -= cr[q] * p.y + ci[q] * p.x;
+            const Four p(psi.p[q] + 4 * i);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x.v[e] = take(x.v[e], p.v[e], q);
         }
-        w[i] = x;
-        ff_acc(hi, lo, x.x, x.x);
-        ff_acc(hi, lo, x.y, x.y);
+        x.store(w + 4 * i);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc2(h2, l2, x.v[e], x.v[e]);
     }
-    const float2 s = block_sum_ff(hi, lo);
+    if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
+        const uint64_t i = 4 * n4 + threadIdx.x;
+        u64 x = reinterpret_cast<const u64*>(w)[i];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) x = take(x, reinterpret_cast<const u64*>(psi.p[q])[i], q);
+        reinterpret_cast<u64*>(w)[i] = x;
+        acc2(h2, l2, x, x);
+    }
+    float2 s = halves(h2, l2);
+    s = block_sum_ff(s.x, s.y);
     if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2((double)s.x + (double)s.y, 0.0);
     if (!last_cta(d.arrived)) return;
     const double w2 = sum_partials(bpart, gridDim.x);
@@ -447,7 +484,7 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
     const bool own_alpha = H.packed() && nparts <= kFusedParts;
     if (own_alpha) hooks.fin = dev;
     // CTAs of the update: four 16-byte elements a thread at least, up to a resident wave
-    const int ug = (int)std::max<uint64_t>(1, std::min<uint64_t>(n / (8 * kT), kUpdGrid));
+    const int ug = (int)std::max<uint64_t>(1, std::min<uint64_t>(n / (8 * kT), kUpdGrid32));
     PsiTab psi{};   // converged Ritz vectors (selective reorthogonalisation)
     int npsi = 0;   // how many are held
     std::vector<double> locked;  // their Ritz values
