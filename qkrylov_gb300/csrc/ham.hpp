@@ -408,7 +408,6 @@ void mcombine_multi_f32(const float2* const* V_dev, int k, const std::complex<do
 void mcombine_multi_f32_dev(const float2* const* V_dev, int k, const double2* c_dev, float2* const* W_dev, int nout,
                             uint64_t n, bool accumulate, cudaStream_t s);
 // Davidson preconditioner t_i = r_i / (d_i - lambda) with the reference's clamp.
-void davidson_precond_f64(const double2* r, const double2* d, double lambda, double2* t, uint64_t n, cudaStream_t s);
 void davidson_precond_f32(const float2* r, const double2* d, double lambda, float2* t, uint64_t n, cudaStream_t s);
 
 }  // namespace qkg

@@ -258,7 +258,7 @@ constexpr int KB = 8;
 // FP64 projections <V_j, w> for up to KB vectors per block column.  Bound by the FP64
 // pipe (four FMAs an element of V), so the CTA's sums are arranged to cost it little:
 // the threads' values go through shared memory and each thread adds sixteen of them, 17
-// double additions a warp where shuffles would take 160 (n = 184,756, 40 vectors: 97 us).
+// double additions a warp where shuffles would take 160 (n = 184,756, 40 vectors: 73 us; shuffles 97).
 __global__ void __launch_bounds__(kThreads) mdot64_kernel(const double2* const* __restrict__ V, int k,
                                                           const double2* __restrict__ w, uint64_t n, double2* part,
                                                           int stride) {
@@ -751,7 +751,8 @@ __global__ void mcomb_multi_kernel(const T2* const* __restrict__ V, int k, const
     }
 }
 
-// The Davidson preconditioner for FP32 vectors (difference taken in FP64).
+// The Davidson preconditioner for FP32 vectors (difference taken in FP64):
+// src/solvers/davidson.cpp:171-175, diff = d_i - lambda, clamped to +-1e-10.
 __global__ void precond32_kernel(const float2* __restrict__ r, const double2* __restrict__ d, double lambda,
                                  float2* __restrict__ t, uint64_t n) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -760,18 +761,6 @@ __global__ void precond32_kernel(const float2* __restrict__ r, const double2* __
         const float2 a = r[i];
         const float den = fr * fr + fi * fi;
         t[i] = make_float2((a.x * fr + a.y * fi) / den, (a.y * fr - a.x * fi) / den);
-    }
-}
-
-__global__ void precond_kernel(const double2* __restrict__ r, const double2* __restrict__ d, double lambda,
-                               double2* __restrict__ t, uint64_t n) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        // src/solvers/davidson.cpp:171-175: diff = d_i - lambda, clamped to +-1e-10.
-        double dr = d[i].x - lambda, di = d[i].y;
-        if (sqrt(dr * dr + di * di) < 1e-10) { dr = (dr >= 0) ? 1e-10 : -1e-10; di = 0.0; }
-        const double2 a = r[i];
-        const double den = dr * dr + di * di;
-        t[i] = make_double2((a.x * dr + a.y * di) / den, (a.y * dr - a.x * di) / den);
     }
 }
 
@@ -1135,10 +1124,6 @@ void mcombine_multi_f32(const float2* const* V, int k, const std::complex<double
 }
 void davidson_precond_f32(const float2* r, const double2* d, double lambda, float2* t, uint64_t n, cudaStream_t s) {
     precond32_kernel<<<stream_grid(n), kThreads, 0, s>>>(r, d, lambda, t, n);
-    QKG_LAUNCHED();
-}
-void davidson_precond_f64(const double2* r, const double2* d, double lambda, double2* t, uint64_t n, cudaStream_t s) {
-    precond_kernel<<<stream_grid(n), kThreads, 0, s>>>(r, d, lambda, t, n);
     QKG_LAUNCHED();
 }
 

@@ -54,15 +54,6 @@ struct PsiTab {
     const float2* p[kMaxPsi];
 };
 
-__device__ __forceinline__ void ff_acc(float& hi, float& lo, float a, float b) {
-    const float p = a * b;
-    const float e = fmaf(a, b, -p);
-    const float t = hi + p;
-    const float z = t - hi;
-    lo += ((hi - (t - z)) + (p - z)) + e;
-    hi = t;
-}
-
 // alpha from the SpMV's per-CTA partials where its grid is too large for its last
 // CTA to add them: blocks sum fixed slices, the last one to finish adds their sums in
 // block order; the result does not depend on which block that is.

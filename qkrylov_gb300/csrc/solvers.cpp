@@ -826,8 +826,7 @@ void ftlm_observables(const std::vector<FTLMTri>& tri, const double* betas, int 
 // ============================================================ Davidson
 namespace {
 // Vector operations of one storage precision.
-template <class T2> struct DavOps;
-template <> struct DavOps<float2> {
+struct DavOps {
     static void apply(Hamiltonian& H, const float2* x, float2* y, cudaStream_t s) { H.apply_f32(x, y, s); }
     static void mdot(const float2* const* V, int k, const float2* w, uint64_t n, cd* o, Workspace& ws, cudaStream_t s) {
         mdot_f32(V, k, w, n, o, ws, s);
@@ -844,10 +843,6 @@ template <> struct DavOps<float2> {
     static void precond(const float2* r, const double2* d, double l, float2* t, uint64_t n, cudaStream_t s) {
         davidson_precond_f32(r, d, l, t, n, s);
     }
-    static void mdot_multi(const float2* const* V, int k, float2* const* W, int nw, uint64_t n, cd* o, Workspace& ws,
-                           cudaStream_t s) {
-        mdot_multi_f32(V, k, W, nw, n, o, ws, s);
-    }
     static void from64(const double2* x, float2* y, uint64_t n, cudaStream_t s) { f64_to_f32(x, y, n, s); }
     static void to64(const float2* x, double2* y, uint64_t n, cudaStream_t s) { f32_to_f64(x, y, n, s); }
 };
@@ -856,18 +851,16 @@ inline void mdot_block(const float2* const* V, int k, float2* const* W, int nw, 
                        cudaStream_t s) {
     mdot_multi_f32(V, k, W, nw, n, o, ws, s);
 }
-// src/solvers/davidson.cpp:86-227 with the Krylov vectors stored in T2.
+// src/solvers/davidson.cpp:86-227 with the Krylov vectors stored in FP32.
 // Projections <V_i, HV_j> of vectors that did not change are kept from the
 // previous iteration (the reference recomputes them; the values are the same
 // dot products), the k residuals and the restart's Ritz vectors are formed in
-// one pass over V and HV each.  MIXED (FP32 storage): SpMV in FP32, projections
+// one pass over V and HV each.  FP32 storage: SpMV in FP32, projections
 // and norms by compensated reductions in FP64, corrections orthogonalised twice,
 // and the final Ritz pairs refined in FP64 (Rayleigh quotient, residual).
-template <class T2>
-DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bool want_vecs, bool f32_stream,
-                          int max_iter) {
-    using Op = DavOps<T2>;
-    constexpr bool MIXED = std::is_same<T2, float2>::value;
+DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bool want_vecs, int max_iter) {
+    using T2 = float2;
+    using Op = DavOps;
     DavidsonOut out;
     const uint64_t n = H.dim();
     if (n == 0) return out;
@@ -889,8 +882,6 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
     // std::sort leaves them (davidson.cpp:111-121); the diagonal is taken in the
     // reference's order so ties resolve as they do there.
     std::vector<cd> dref = H.diagonal_host_ref();
-    if (f32_stream)  // the FP32 engine sorts its float diagonal
-        for (auto& d : dref) d = cd((double)(float)d.real(), 0.0);
     std::vector<uint64_t> di(n);
     std::iota(di.begin(), di.end(), 0);
     if (n <= (1ull << 23)) {
@@ -903,11 +894,10 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
     std::vector<cd>().swap(dref);
     std::mt19937 rng(1234);
     std::uniform_real_distribution<double> dist(-1.0, 1.0);
-    std::uniform_real_distribution<float> dist32(-1.0f, 1.0f);
     VecPool pool(n * sizeof(T2));  // declared before the lists, so it outlives them
     VecList<T2> V(n, &pool), HV(n, &pool);
     std::vector<cd> hv(n), c;
-    const int passes = MIXED ? 2 : 1;
+    const int passes = 2;
     // t -= V[from..] (V[from..]^H t), passes times, and ||t||
     auto orthonormalize = [&](T2* t, size_t from) -> double {
         const int kv = (int)(V.size() - std::min(from, V.size()));
@@ -927,8 +917,7 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
         Op::from64(d64.as<double2>(), seed.as<T2>(), n, st);
         double nrm = orthonormalize(seed.as<T2>(), 0);
         if (nrm < 1e-10) {
-            if (f32_stream) fill_stream(rng, dist32, n, hv.data());
-            else fill_stream(rng, dist, n, hv.data());
+            fill_stream(rng, dist, n, hv.data());
             upload_ref_f64(H, hv.data(), d64.as<double2>(), tmp);
             Op::from64(d64.as<double2>(), seed.as<T2>(), n, st);
             nrm = orthonormalize(seed.as<T2>(), 0);
@@ -947,7 +936,7 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
     for (auto& r : rbuf) rptr.push_back(r.as<T2>());
     for (int iter = 0; iter < max_iter; ++iter) {
         const int m = (int)V.size();
-        if (MIXED && m - (int)rows.size() > 1) {
+        if (m - (int)rows.size() > 1) {
             // the new rows together: one pass over HV_0..HV_{m-1} for up to four new V_i
             for (int i0 = (int)rows.size(); i0 < m; i0 += 4) {
                 const int nw = std::min(4, m - i0);
@@ -1015,38 +1004,30 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
                 Op::mmulti(V.dev(), m, cs.data() + (size_t)k0 * m, rptr.data() + k0, std::min(kc, n_eig - k0), n, false,
                            ws, st);
             DBuf e64, h64;
-            if (MIXED) {
-                // FP64 refinement: Rayleigh quotient and residual of each normalised Ritz vector
-                V.clear();
-                HV.clear();
-                pool.free.clear();  // give the basis memory back before the FP64 vectors
-                e64.alloc(n * sizeof(double2));
-                h64.alloc(n * sizeof(double2));
-                bool conv64 = true;
-                for (int k = 0; k < n_eig; ++k) {
-                    Op::to64(rptr[k], e64.as<double2>(), n, st);
-                    const double nr = std::sqrt(nrm2sq_f64(e64.as<double2>(), n, ws, st));
-                    if (nr > 0.0) scal_f64(1.0 / nr, e64.as<double2>(), n, st);
-                    H.apply_f64(e64.as<double2>(), h64.as<double2>(), st);
-                    const double lam = dot_f64(e64.as<double2>(), h64.as<double2>(), n, ws, st).real();
-                    axpy_f64(cd(-lam, 0.0), e64.as<double2>(), h64.as<double2>(), n, st);
-                    out.residuals[k] = std::sqrt(nrm2sq_f64(h64.as<double2>(), n, ws, st));
-                    out.evals[k] = lam;
-                    if (out.residuals[k] > tol) conv64 = false;
-                    if (want_vecs) {
-                        std::vector<cd> h(n);
-                        download_ref_f64(H, e64.as<double2>(), h.data(), tmp);
-                        out.evecs.push_back(std::move(h));
-                    }
-                }
-                out.converged = conv64;
-            } else if (want_vecs) {
-                for (int k = 0; k < n_eig; ++k) {
+            // FP64 refinement: Rayleigh quotient and residual of each normalised Ritz vector
+            V.clear();
+            HV.clear();
+            pool.free.clear();  // give the basis memory back before the FP64 vectors
+            e64.alloc(n * sizeof(double2));
+            h64.alloc(n * sizeof(double2));
+            bool conv64 = true;
+            for (int k = 0; k < n_eig; ++k) {
+                Op::to64(rptr[k], e64.as<double2>(), n, st);
+                const double nr = std::sqrt(nrm2sq_f64(e64.as<double2>(), n, ws, st));
+                if (nr > 0.0) scal_f64(1.0 / nr, e64.as<double2>(), n, st);
+                H.apply_f64(e64.as<double2>(), h64.as<double2>(), st);
+                const double lam = dot_f64(e64.as<double2>(), h64.as<double2>(), n, ws, st).real();
+                axpy_f64(cd(-lam, 0.0), e64.as<double2>(), h64.as<double2>(), n, st);
+                out.residuals[k] = std::sqrt(nrm2sq_f64(h64.as<double2>(), n, ws, st));
+                out.evals[k] = lam;
+                if (out.residuals[k] > tol) conv64 = false;
+                if (want_vecs) {
                     std::vector<cd> h(n);
-                    download_ref_f64(H, reinterpret_cast<const double2*>(rptr[k]), h.data(), tmp);
+                    download_ref_f64(H, e64.as<double2>(), h.data(), tmp);
                     out.evecs.push_back(std::move(h));
                 }
             }
+            out.converged = conv64;
             QKG_CUDA(cudaStreamSynchronize(st));
             out.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
             return out;
@@ -1072,13 +1053,13 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
             HV.take(nh);
             rows.clear();
         }
-        // Orthogonalise each correction and extend (:213-223).  Mixed form: all
+        // Orthogonalise each correction and extend (:213-223): all
         // corrections are first projected off the current basis together (one
         // pass over V per Gram-Schmidt pass for all of them), then each off the
         // corrections accepted before it; in exact arithmetic the same as the
         // sequential projection off the growing basis.
         size_t from = 0;
-        if (MIXED && corr.size() > 1 && V.size()) {
+        if (corr.size() > 1 && V.size()) {
             const int kv = (int)V.size(), nc = (int)corr.size();
             std::vector<T2*> tp;
             for (auto& t : corr) tp.push_back(t.as<T2>());
@@ -1109,7 +1090,7 @@ DavidsonOut davidson_impl(Hamiltonian& H, int n_eig, int max_sub, double tol, bo
 }  // namespace
 
 DavidsonOut davidson_mixed(Hamiltonian& H, int n_eig, int max_sub, double tol, bool want_vecs, int max_iter) {
-    return davidson_impl<float2>(H, n_eig, max_sub, tol, want_vecs, false, max_iter);
+    return davidson_impl(H, n_eig, max_sub, tol, want_vecs, max_iter);
 }
 
 }  // namespace qkg
