@@ -27,7 +27,8 @@ using namespace pairk;
 
 constexpr int kBT = 256;       // threads of a CTA
 constexpr int kBatch = 3;      // outer entries loaded together
-constexpr int kStrBatch = 2;   // straddling entries loaded together
+constexpr int kStrBatch = 2;   // straddling entries loaded together (the FP64 form takes its two by name)
+static_assert(kStrBatch == 2);
 template <int N> struct Int { static constexpr int value = N; };
 constexpr int kMaxRun = 8;     // tiles of a CTA
 constexpr int kMaxList = 96;   // outer (and straddling) entries of its blocks staged in shared memory
@@ -572,6 +573,30 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                         nxt = __ldg(tab + at);
                         if (MODE == AMP_CODED) cn = __ldg(codes + at);
                     }
+                    if constexpr (sizeof(T) == 8) {
+                        // one at a time, an empty slot ends the row: bound by the FP64 pipe, on
+                        // which the empty slots' products would count like the others (2^20 rows,
+                        // 32 vectors: 1.98 -> 1.78 ms)
+                        unsigned long long e64 = (unsigned long long)e.y << 32 | e.x;
+                        uint32_t c1 = c;
+                        bool more = true;
+#pragma unroll 1
+                        for (int h = 0; h < 4; ++h) {
+                            const uint32_t w16 = (uint32_t)e64 & 0xFFFFu;
+                            const int to = rank_of(w16);
+                            if (to == kNone) {
+                                more = false;
+                                break;
+                            }
+                            R v;
+                            v.load(offset(xl, to, rb), G);
+                            amp_add(w16, c1, u, v);
+                            e64 >>= 16;
+                            c1 >>= 8;
+                        }
+                        if (!more) break;
+                        continue;
+                    }
                     const uint32_t w[4] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16};
                     if (rank_of(w[0]) == kNone) break;  // a row's entries come first
                     // the four rows' loads go out together; an empty slot reads zero
@@ -586,6 +611,18 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                 }
                 for (uint32_t j = 0; j < ns; j += kStrBatch) {
                     if (j) straddles(j);
+                    if constexpr (sizeof(T) == 8) {
+#pragma unroll 1
+                        for (uint32_t i = 0; i < (uint32_t)kStrBatch && j + i < ns; ++i) {
+                            const uint32_t w16 = i ? sw[1] : sw[0];
+                            const int to = rank_of(w16);
+                            if (to == kNone) continue;
+                            R v;
+                            v.load(offset(Xh, (int)strl[j + i].off + to, rb), G);
+                            amp_add(w16, i ? sc[1] : sc[0], strl[j + i].ar, v);
+                        }
+                        continue;
+                    }
                     R v[kStrBatch];
 #pragma unroll
                     for (int i = 0; i < kStrBatch; ++i) {

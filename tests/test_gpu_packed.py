@@ -79,6 +79,18 @@ def test_block_widths_against_single_vectors(qk, name, R):
             np.testing.assert_allclose(got[r].betas[:5], one.betas[:5], rtol=0, atol=64 * eps * bound)
 
 
+@pytest.mark.parametrize("L", [20, 21])
+def test_block_fp64_large_batches(qk, L):
+    """32 FP64 vectors on both sides of 2^25 block elements: either engine's first steps are the single vector's."""
+    hams = [ham(qk, M.heisenberg(L, True, s)) for s in range(L % 2, L + 1, 2)] * 2
+    got = qk.block_lanczos_tridiag(hams, 32, 4, mixed=False, start="philox", seed=5)
+    few = qk.block_lanczos_tridiag(hams[:1], 32, 4, mixed=False, start="philox", seed=5)
+    for v in (0, 31):
+        # four steps of 2^-53 rounding on numbers up to ||H|| <= 0.75 L
+        np.testing.assert_allclose(got.alphas[v], few.alphas[v], rtol=0, atol=64 * 2.0 ** -53 * 0.75 * L)
+        np.testing.assert_allclose(got.betas[v][:3], few.betas[v][:3], rtol=0, atol=64 * 2.0 ** -53 * 0.75 * L)
+
+
 # dimensions 4845, 2002, 6435, 3432: every remainder of four, Ritz vectors locked on the way
 @pytest.mark.parametrize("L,sz2", [(20, 12), (14, 4), (15, 1), (14, 0)])
 def test_lanczos_fp32_remainders(qk, L, sz2):
