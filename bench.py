@@ -344,11 +344,11 @@ def main():
     alg_bytes = (3 * (LANCZOS_STEPS - 1) + 2) * DIM * BYTES_PER_ELEM_F32 / LANCZOS_STEPS
     achieved = alg_bytes / spmv_s / 1e9
     variant, _ = H.tuning(fp32=True)
-    tr = profile_traffic() if variant == "rows4" else None  # the summary covers the four-rows kernel
+    tr = profile_traffic() if variant == "packed" else None  # the summary covers the packed kernel
     kname = {"rows4": "spmv_rows_kernel<float>", "rows4_staged": "spmv_rows_kernel<float, staged>",
              "rows4_wide": "spmv_rows_kernel<float, 4 CTAs/SM>",
              "row": "spmv_fast_kernel<float>",
-             "staged": "spmv_fast_kernel<float, staged>"}.get(variant, "spmv_kernel<float>")
+             "staged": "spmv_fast_kernel<float, staged>", "packed": "pack32_kernel"}.get(variant, "spmv_kernel<float>")
     out["roofline"] = {"kernel": kname + " (FP32 SpMV fused with the three-term recurrence)", "bound": "hbm",
                        "achieved": achieved,
                        "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / hbm_peak,
@@ -441,7 +441,7 @@ def ftlm_batch(qk, seed, hbm_peak, peak_kind, cpu=True):
             "e2e_vectors_per_s": nvec / w32, "loop_s": st["seconds"],
             "fp64_vectors_per_s": nvec / r64.stats["seconds"], "fp64_loop_s": r64.stats["seconds"],
             "tile": {"vectors_per_lane": st["vectors_per_lane"], "tune_ms": st["tune_ms"]},
-            "roofline": {"kernel": "spmv_block_kernel<float> (FP32 block SpMV, 32 vectors)", "bound": "hbm",
+            "roofline": {"kernel": "block_pack_kernel<float> (FP32 block SpMV, 32 vectors)", "bound": "hbm",
                          "achieved": achieved, "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / hbm_peak, "algorithmic_bytes_per_launch": alg,
                          "launch_ms": st["spmv_ms"]},
@@ -545,7 +545,7 @@ def cf_batch(qk, hbm_peak, peak_kind, cpu=True):
             "rhs_steps_per_s": nrhs * CF_STEPS / st32["seconds"], "loop_s": st32["seconds"],
             "e2e_s": w32, "fp64_rhs_steps_per_s": nrhs * CF_STEPS / st64["seconds"], "fp64_loop_s": st64["seconds"],
             "tile": {"vectors_per_lane": st32["vectors_per_lane"], "padded_vectors": st32["padded_vectors"]},
-            "roofline": {"kernel": "spmv_block_kernel<float> (FP32 block SpMV, 16 vectors)", "bound": "hbm",
+            "roofline": {"kernel": "block_pack_kernel<float> (FP32 block SpMV, 16 vectors)", "bound": "hbm",
                          "achieved": achieved, "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / hbm_peak, "algorithmic_bytes_per_launch": alg,
                          "launch_ms": st32["spmv_ms"]},

@@ -363,9 +363,10 @@ int qkrylov_ftlm_multi_beta_f64(qkrylov_hamiltonian_h h, const double* betas, in
 int qkrylov_hamiltonian_info(qkrylov_hamiltonian_h h, int* n_outer, int* n_inner, int* n_mixed, int* n_diag,
                              int* diag_mode);
 
-/* SpMV kernel choice: generic = 0 lets the library use its table-driven fast
- * kernel when the Hamiltonian qualifies (32-bit states, coded diagonal), in
- * the variant its autotuner measured fastest at creation; generic = 1 forces
+/* SpMV kernel choice: generic = 0 lets the library use its packed kernel when
+ * the Hamiltonian has a packed plan, else its table-driven fast kernel when it
+ * qualifies (32-bit states, coded diagonal), in the variant its autotuner
+ * measured fastest; generic = 1 forces
  * the generic kernel; 2 the fast kernel with one row per thread; 3 the fast
  * kernel with shared-memory staging of each outer block's slice of x (when a
  * block fits); 4 the fast kernel with four rows per thread; 5 four rows per
@@ -387,7 +388,8 @@ int qkrylov_hamiltonian_select_kernel(qkrylov_hamiltonian_h h, int generic, int*
 int qkrylov_hamiltonian_tuning(qkrylov_hamiltonian_h h, int fp32, int* variant, double* ms_per_variant);
 
 /* The same with every variant: *variant 0..4 as above, 5, 6, 7 the tiled
- * kernel over 1, 2, 4 outer blocks per CTA, 8 the class-persistent kernel; ms_per_variant receives n_ms
+ * kernel over 1, 2, 4 outer blocks per CTA, 8 the class-persistent kernel, 9 the packed
+ * kernel (chosen by rule, not timed); ms_per_variant receives n_ms
  * entries (variants beyond those the library has read 0). */
 int qkrylov_hamiltonian_tuning_ex(qkrylov_hamiltonian_h h, int fp32, int* variant, double* ms_per_variant, int n_ms);
 
@@ -396,7 +398,8 @@ int qkrylov_hamiltonian_tuning_ex(qkrylov_hamiltonian_h h, int fp32, int* varian
 int qkrylov_basis_states(qkrylov_basis_h basis, uint64_t first, uint64_t count, uint64_t* out);
 
 /* Device memory the Hamiltonian keeps between solver calls (the FP32 Krylov
- * space of the mixed Lanczos: maxiter + 7 vectors): *bytes receives its size;
+ * space of the mixed Lanczos: maxiter + 7 vectors; the FP64 solvers' and the
+ * batched forms' vectors): *bytes receives its size;
  * release != 0 frees it now (it is also freed with the Hamiltonian). */
 int qkrylov_hamiltonian_workspace(qkrylov_hamiltonian_h h, int release, uint64_t* bytes);
 
@@ -430,8 +433,8 @@ int qkrylov_hamiltonian_entries(qkrylov_hamiltonian_h h, uint64_t* nnz_out, uint
 typedef struct {
     double seconds;         /* device time of the Lanczos loop (CUDA events; start vectors excluded) */
     double spmv_ms;         /* mean CUDA-event time of one block SpMV launch (first steps) */
-    int vectors_per_lane;   /* block-SpMV tile shape picked by the autotuner (1, 2 or 4) */
-    int padded_vectors;     /* vectors per row in the block (n_vec rounded up to a power of two) */
+    int vectors_per_lane;   /* block-SpMV tile shape (1, 2 or 4) */
+    int padded_vectors;     /* vectors per row in the block (n_vec rounded up to a multiple of four or a power of two) */
     uint64_t rows;          /* sum of the Hamiltonians' dimensions */
     double tune_ms[3];      /* autotuner timings for 1, 2, 4 vectors per lane (0: not measured) */
 } qkrylov_block_stats_t;
