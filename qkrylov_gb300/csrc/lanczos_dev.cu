@@ -314,18 +314,23 @@ __global__ void lz64_coef(const double2* __restrict__ part, int nparts, const do
         coef[j] = make_double2(f * re, f * im);
     }
 }
-// w += sum_j coef_j V_j (j < k; w = V_k), and beta_{k-1}.
-__global__ void __launch_bounds__(kT) lz64_subtract(const LzDev d, int k, const double2* __restrict__ coef, uint64_t n,
-                                                    double2* __restrict__ bpart) {
+// w += sum_j coef_j V_j for the k vectors from j0 (w = V_kw); the launch that reaches
+// V_{kw-1} also sets beta_{kw-1}.  Coefficients and pointers take 24 bytes of shared
+// memory a vector: kSubtractMost of them a launch keep to 24 KB.
+constexpr int kSubtractMost = 1024;
+// vectors a run reorthogonalises against
+constexpr int kMaxBasis = 4096;
+__global__ void __launch_bounds__(kT) lz64_subtract(const LzDev d, int kw, int j0, int k, const double2* __restrict__ coef,
+                                                    uint64_t n, double2* __restrict__ bpart) {
     void* const* vtab = d.vtab;
     extern __shared__ double2 s_c[];
     const double2** s_v = reinterpret_cast<const double2**>(s_c + k);
     for (int j = threadIdx.x; j < k; j += blockDim.x) {
-        s_c[j] = coef[j];
-        s_v[j] = static_cast<const double2*>(vtab[j]);
+        s_c[j] = coef[j0 + j];
+        s_v[j] = static_cast<const double2*>(vtab[j0 + j]);
     }
     __syncthreads();
-    double2* __restrict__ w = static_cast<double2*>(vtab[k]);
+    double2* __restrict__ w = static_cast<double2*>(vtab[kw]);
     double acc = 0.0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         double2 x = w[i];
@@ -349,7 +354,7 @@ __global__ void __launch_bounds__(kT) lz64_subtract(const LzDev d, int k, const 
         w[i] = x;
         acc = fma(x.y, x.y, fma(x.x, x.x, acc));
     }
-    finish_beta(d, k - 1, acc, bpart);
+    if (j0 + k == kw) finish_beta(d, kw - 1, acc, bpart);
 }
 
 using clk = std::chrono::steady_clock;
@@ -705,7 +710,7 @@ struct Recurrence64 {
                      o_al = take(N * 8), o_be = take(N * 8), o_sg = take(N * 8), o_co = take((size_t)N * 16),
                      o_ap = take((size_t)nparts * 16), o_bp = take((size_t)kUpdGrid * 16), o_p2 = take(kAlphaBlocks * 16),
                      o_ar = take(sizeof(unsigned int));
-        Workspace& ws = H.reduction_scratch(std::max<size_t>(1 << 16, off / sizeof(double2) + 1 + (full ? mdot_f64_most_partials(N, n) : 0)));
+        Workspace& ws = H.reduction_scratch(std::max<size_t>(1 << 16, off / sizeof(double2) + 1 + (full ? mdot_f64_most_partials(std::min(N, kMaxBasis), n) : 0)));
         char* base = ws.partial.as<char>();
         auto* state = reinterpret_cast<LzState*>(base + o_st);
         auto* op = reinterpret_cast<LzOperands*>(base + o_op);
@@ -788,13 +793,17 @@ struct Recurrence64 {
             else lz64_update<false><<<g, kT, 0, st>>>(d, n, bpart);
             QKG_LAUNCHED();
             if (full) {
+                QKG_REQUIRE(k < kMaxBasis, "Lanczos with full reorthogonalisation: at most 4096 vectors");
                 const int gm = mdot_f64_chunks(k + 1, n);
                 mdot_f64_partials(reinterpret_cast<const double2* const*>(tab), k + 1, static_cast<const double2*>(ptr[k + 1]),
                                   n, ppart, gm, st);
                 lz64_coef<<<k + 1, kT, 0, st>>>(ppart, gm, sig, coef);
                 QKG_LAUNCHED();
-                lz64_subtract<<<g, kT, (size_t)(k + 1) * (sizeof(double2) + sizeof(void*)), st>>>(d, k + 1, coef, n, bpart);
-                QKG_LAUNCHED();
+                for (int j0 = 0; j0 <= k; j0 += kSubtractMost) {
+                    const int kk = std::min(kSubtractMost, k + 1 - j0);
+                    lz64_subtract<<<g, kT, (size_t)kk * (sizeof(double2) + sizeof(void*)), st>>>(d, k + 1, j0, kk, coef, n, bpart);
+                    QKG_LAUNCHED();
+                }
             }
         };
         try {
