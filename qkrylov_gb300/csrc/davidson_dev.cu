@@ -98,7 +98,9 @@ __global__ void __launch_bounds__(kT) dav_scale(const double2* __restrict__ norm
 
 // For K Ritz pairs: r = sum_j s_j (HV_j - lambda V_j), t = r / (d - lambda) with the
 // reference's clamp (davidson.cpp:171-175), and ||r||^2 in norm[k].x.
-// cs[k * m + j] = s_j of pair k.
+// cs[k * m + j] = s_j of pair k.  The coefficients are in shared memory: at most
+// kResidualCoefs of them a pass (32 KB), so a wide basis takes its pairs in more passes.
+constexpr int kResidualCoefs = 2048;
 template <int K>
 __global__ void __launch_bounds__(kT) dav_residual(const double2* const* __restrict__ V, const double2* const* __restrict__ HV,
                                                    int m, const double2* __restrict__ cs, const double* __restrict__ lambda,
@@ -338,8 +340,8 @@ DavidsonOut davidson_f64(Hamiltonian& H, int n_eig, int max_sub, double tol, boo
             for (int i = 0; i < m; ++i) cs[(size_t)k * m + i] = evec[k][i];
         QKG_CUDA(cudaMemcpyAsync(coef, cs.data(), cs.size() * sizeof(cd), cudaMemcpyHostToDevice, st));
         QKG_CUDA(cudaMemcpyAsync(dlam, ev.data(), n_eig * sizeof(double), cudaMemcpyHostToDevice, st));
-        for (int k0 = 0; k0 < n_eig; k0 += KB) {
-            const int nk = std::min(KB, n_eig - k0);
+        for (int k0 = 0, nk; k0 < n_eig; k0 += nk) {
+            nk = std::min({KB, n_eig - k0, std::max(1, kResidualCoefs / m)});
             auto go = [&](auto kc) {
                 constexpr int K = decltype(kc)::value;
                 dav_residual<K><<<g, kT, (size_t)K * m * sizeof(double2), st>>>(

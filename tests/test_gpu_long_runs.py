@@ -40,3 +40,30 @@ def test_lanczos_fp64_past_one_launch_of_coefficients(qk, steps):
     # FP64 Ritz values of the converged ends: thousands of roundings of 2^-53 on numbers up to ||H|| < 16
     np.testing.assert_allclose(values[:40], want[:40], rtol=0, atol=steps * 2.0 ** -53 * 16)
     np.testing.assert_allclose(values[-40:], want[-40:], rtol=0, atol=steps * 2.0 ** -53 * 16)
+
+
+def test_davidson_fp64_wide_basis(qk):
+    """256 states in a basis that grows to 768: residual passes narrower than four pairs.
+
+    Three bonds with hops between strongly staggered sites, eleven sites in weak fields: a seed and its
+    corrections stay in a block of eight states that no other seed reaches, so the 768-wide projected
+    matrix is three-by-three blocks and its diagonalisation cheap."""
+    L, J = 17, (1.0, 0.8, 1.2)
+    rng = np.random.default_rng(7)
+    h = np.concatenate([np.tile([10.0, -10.0], 3), rng.uniform(-0.5, 0.5, 11)])
+    terms = [(h[i], [("Sz", i)]) for i in range(L)]
+    for b in range(3):
+        terms += [(0.5 * J[b], [("Sp", 2 * b), ("Sm", 2 * b + 1)]), (0.5 * J[b], [("Sm", 2 * b), ("Sp", 2 * b + 1)])]
+    H = qk.MatrixFreeHamiltonian(*make_model(qk, M.SPIN, L, M.sector(sz2=-1), terms))
+    r = qk.davidson_lowest_ex(H, n_eig=256, max_subspace=768, tol=1e-12, max_iter=3, return_vectors=True)
+    assert r.iterations == 3
+    # ground states of the three bonds (fields +-10) and the 256 lowest arrangements of the other sites
+    from itertools import combinations
+    rest = np.sort([h[6:][list(c)].sum() - 0.5 * h[6:].sum() for c in combinations(range(11), 5)])[:256]
+    want = rest - sum(0.5 * np.sqrt(20.0 ** 2 + j ** 2) for j in J)
+    scale = 64 * 2.0 ** -53 * 34  # roundings of numbers up to ||H||
+    assert np.all(np.abs(r.eigenvalues - want) <= r.residuals + scale)
+    for k in range(0, 256, 5):  # the residuals are those of the vectors handed back
+        v = r.eigenvectors[k]
+        assert abs(np.linalg.norm(H.apply(v) - r.eigenvalues[k] * v) - r.residuals[k]) <= scale
+    assert r.residuals.min() > 1e-9  # not converged yet: the pass had something to compute
