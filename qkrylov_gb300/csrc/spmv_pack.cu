@@ -29,7 +29,9 @@ namespace {
 // codes or the Lanczos step's terms need more (L = 28 Lanczos step 0.55 to 0.54 ms, L = 14
 // Hubbard ring 0.153 to 0.148), FP64 24 warps at 80 (16 warps 2.05 ms, 24 1.65, 32 1.65).
 constexpr int kThreads = 128;
-constexpr int kCtas32 = 12, kCtas32more = 10, kCtas64 = 6;
+// Integer sums of four rows a lane with signs or the Lanczos step's terms: 20 warps at 96 registers
+// (100 recurrence steps at L = 24: 19.1 ms with 24 warps and their spills, 18.4; 13-site Hubbard ring 151 and 150 us).
+constexpr int kCtas32 = 12, kCtas32more = 10, kCtas64 = 6, kCtas64more = 5;
 
 // ---- sums of one row -------------------------------------------------------
 // FP32, real amplitudes.
@@ -66,10 +68,19 @@ struct SumF64 {
 // integers at 64.  The significand keeps 4 bits below its last place and 6
 // above its first (up to 64 addends), so an addend loses less than 2^-56 of the
 // largest one where a chain of FP64 additions rounds each partial sum to 2^-53.
-// Infinities, NaN and rows below 2^-959 are left to the FP64 pipe (bad()).
+// Infinities, NaN and rows below 2^-959 are left to the FP64 pipe (bad()), but for sums of
+// nothing but zeros: every imaginary part of a real vector and most rows of a sparse one are
+// that, and a warp that walks twice takes longer than the FP64 pipe alone (real vector, L = 24
+// ring: 264 us walked twice, 237 on the FP64 pipe in the older kernels, 122 now).  What tells
+// zeros from the smallest numbers is one FP32 addition an addend, on a pipe that is idle (on
+// the integer pipe, two addends an OR: L = 28 1.97 against 1.94 ms); aligning the sum once
+// for two addends pays for it (complex vectors without either and with both: L = 28 1.92 and
+// 1.88 ms, L = 24 122 and 121 us, 13-site Hubbard ring 149 and 149, 23-site transverse-field
+// ring 407 and 414).
 struct IntSum {
     long long s;
     int e;
+    float any;  // sum of the magnitudes of the addends' high words read as floats: 0 where those are all +-0
     // PTX shifts clamp: a distance of 64 or more leaves nothing
     static __device__ __forceinline__ u64 shift(u64 v, int d) {
         u64 r;
@@ -84,22 +95,33 @@ struct IntSum {
     __device__ __forceinline__ void init() {
         s = 0;
         e = 0;
+        any = 0.f;
     }
-    // x with its sign bit flipped by the top bit of `flip`
-    __device__ __forceinline__ void add(uint32_t flip, double x) {
-        const uint32_t hi = (uint32_t)__double2hiint(x);
-        const uint32_t lo = (uint32_t)__double2loint(x);
-        const int ex = (int)((hi >> 20) & 0x7FFu);
-        const int em = max(e, ex);
+    // the x, each with its sign bit flipped by the top bit of its flip
+    template <int N>
+    __device__ __forceinline__ void add(const uint32_t (&flip)[N], const double (&x)[N]) {
+        int em = e, ex[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            ex[k] = (int)(((uint32_t)__double2hiint(x[k]) >> 20) & 0x7FFu);
+            em = max(em, ex[k]);
+        }
         s = shift(s, em - e);
         e = em;
-        u64 m = ((u64)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
-        m = shift(m << 4, em - ex);
-        const long long sg = (long long)((int)(hi ^ flip) >> 31);  // 0 or -1
-        s += ((long long)m ^ sg) - sg;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const uint32_t hi = (uint32_t)__double2hiint(x[k]), lo = (uint32_t)__double2loint(x[k]);
+            any += fabsf(__uint_as_float(hi));
+            u64 m = ((u64)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+            m = shift(m << 4, em - ex[k]);
+            const long long sg = (long long)((int)(hi ^ flip[k]) >> 31);  // 0 or -1
+            s += ((long long)m ^ sg) - sg;
+        }
     }
-    __device__ __forceinline__ bool bad() const { return e == 0x7FF || e < 64; }
-    // u times the sum (s counts units of 2^(e - 1079)); v = u * 2^-56
+    // Whether the sum is one of zeros: with every high word +-0 the addends are below 2^32 units
+    // of 2^-1074, and their sum is what s holds below the weight 2^56 of the (absent) leading ones.
+    __device__ __forceinline__ bool zeros() const { return any == 0.f && (s << 8) == 0; }
+    __device__ __forceinline__ bool bad() const { return e == 0x7FF || (e < 64 && !zeros()); }
     __device__ __forceinline__ double value(double v) const { return v * __hiloint2double(e << 20, 0) * (double)s; }
 };
 struct SumI64 {
@@ -109,10 +131,22 @@ struct SumI64 {
         r.init();
         i.init();
     }
-    __device__ __forceinline__ void add(double a, V x) {  // a = +-u
-        const uint32_t flip = (uint32_t)__double2hiint(a);
-        r.add(flip, x.x);
-        i.add(flip, x.y);
+    template <int N>
+    __device__ __forceinline__ void add_n(const double (&a)[N], const V* x) {  // a = +-u
+        uint32_t flip[N];
+        double re[N], im[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            flip[k] = (uint32_t)__double2hiint(a[k]);
+            re[k] = x[k].x;
+            im[k] = x[k].y;
+        }
+        r.add(flip, re);
+        i.add(flip, im);
+    }
+    __device__ __forceinline__ void add(double a, V x) {
+        const double a1[1] = {a};
+        add_n(a1, &x);
     }
     __device__ __forceinline__ void add(double, double, V) {}  // never called: coded amplitudes go to SumF64
     __device__ __forceinline__ bool bad() const { return r.bad() || i.bad(); }
@@ -166,8 +200,21 @@ __device__ __forceinline__ void walk(const Params<T>& p, const Item& it, uint32_
     // outer entries: one offset and amplitude for the whole block
     const auto* xr = x + it.row0 + lane + 32u * q0;
     if (cnt >= 32u * (q0 + NQ)) {
+        uint32_t k = b4.x;
+        if constexpr (std::is_same<Sum, SumI64>::value) {
+            for (; k + 2 <= b4.y; k += 2) {
+                const Out<T> o0 = p.out[k], o1 = p.out[k + 1];
+                const auto *x0 = xr + o0.delta, *x1 = xr + o1.delta;
+                const T a[2] = {o0.ar, o1.ar};
+                V v[NQ][2];
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) v[q][0] = E::load(x0 + 32 * q), v[q][1] = E::load(x1 + 32 * q);
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) acc[q].add_n(a, v[q]);
+            }
+        }
 #pragma unroll(NQ == 4 ? 2 : 4)
-        for (uint32_t k = b4.x; k < b4.y; ++k) {
+        for (; k < b4.y; ++k) {
             const Out<T> o = p.out[k];
             const auto* xo = xr + o.delta;
             V v[NQ];
@@ -242,6 +289,16 @@ __device__ __forceinline__ void walk(const Params<T>& p, const Item& it, uint32_
                     bool on;
                     const uint32_t r = rank_of(e, k, on);
                     v[k] = E::load_if(xb + r, on);
+                }
+                if constexpr (std::is_same<Sum, SumI64>::value) {
+                    auto pair = [&](uint32_t w, const V* v2) {
+                        const T a[2] = {MODE == AMP_SIGNED ? with_sign(p.u, w << 16) : p.u,
+                                        MODE == AMP_SIGNED ? with_sign(p.u, w) : p.u};
+                        acc[q].add_n(a, v2);
+                    };
+                    pair(e.x, v);
+                    if (n > 2) pair(e.y, v + 2);
+                    continue;
                 }
                 add_entry(e, 0, c, acc[q], v[0], p.u);
                 add_entry(e, 1, c, acc[q], v[1], p.u);
@@ -373,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, LZ || MODE != AMP_UNIFORM ? kCtas32m
 // FP64.  EQUAL: every amplitude has the same magnitude p.u (sums of aligned
 // integers).  LZ as above.
 template <int MODE, bool CPLX, bool EQUAL, bool LZ, int NQ>
-__global__ void __launch_bounds__(kThreads, kCtas64)
+__global__ void __launch_bounds__(kThreads, EQUAL && NQ == 4 && (LZ || MODE == AMP_SIGNED) ? kCtas64more : kCtas64)
     pack64_kernel(const Params<double> p, const double2* __restrict__ x_in, double2* __restrict__ y_in) {
     __shared__ double s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
     if (MODE == AMP_CODED) load_amps(p, s_amp);

@@ -123,3 +123,70 @@ def test_streamed_projections(qk, n, k, nw, shift):
             want = complex(torch.vdot(v, w).cpu())
             # runs of at most 64 products added in FP32, the runs in float pairs
             assert abs(P[o, j] - want) <= 64 * 2.0 ** -24 * float((v.abs() * w.abs()).sum().cpu())
+
+
+def sparse_values(kind, n, rng):
+    x = np.zeros(n, dtype=np.complex128)
+    some = rng.integers(0, n, n // 50 + 1)
+    if kind == "real":
+        x.real = rng.standard_normal(n)
+    elif kind == "imaginary":
+        x.imag = rng.standard_normal(n)
+    elif kind == "unit":
+        x[n // 2] = 1.0
+    elif kind == "sparse":
+        x[some] = rng.standard_normal(len(some)) + 1j * rng.standard_normal(len(some))
+    elif kind == "negative zeros":
+        x = np.full(n, complex(-0.0, -0.0))
+        x[some] = 1.0
+    elif kind == "subnormal ones":  # whole rows of one power: 2^-1023, 2^-1043 and 2^-1074 (top bits of the words)
+        x.real = rng.standard_normal(n)
+        x.imag = np.array([2.0 ** -1023, 2.0 ** -1043, 2.0 ** -1074])[rng.integers(0, 3)] * rng.integers(-1, 2, n)
+    elif kind == "subnormal twos":  # two sizes of 2^-1043 and 2^-1023 in one row
+        x.real = np.where(rng.integers(0, 2, n) == 1, 2.0 ** -1043, 2.0 ** -1023)
+        x.imag = 2.0 ** -1023
+    elif kind == "large":
+        x = (rng.standard_normal(n) + 1j * rng.standard_normal(n)) * 2.0 ** 1012
+    return x
+
+
+@pytest.mark.parametrize("kind", ["real", "imaginary", "unit", "sparse", "negative zeros", "subnormal ones", "subnormal twos",
+                                  "large"])
+@pytest.mark.parametrize("model", [M.heisenberg(13, True, 1), M.heisenberg(24, True), M.hubbard(8, True, 4, 4)],
+                         ids=["ring13", "ring24_whole_tiles", "hubbard8_signs"])
+def test_integer_sums_of_zeros(qk, model, kind):
+    H = ham(qk, model)
+    x = sparse_values(kind, H.dimension, np.random.default_rng(5))
+    y = H.apply(x)
+    H.select_kernel(mode=1)
+    want = H.apply(x)
+    # every row: up to 64 products of numbers up to the largest, each rounded at 2^-53 (or to 2^-1074), in either kernel
+    top = 64.0 * max(np.abs(x.real).max(), np.abs(x.imag).max())
+    assert np.all(np.abs(y - want) <= 64 * 2.0 ** -53 * top + 128 * 2.0 ** -1074)
+    for part, got in ((x.real, y.real), (x.imag, y.imag)):
+        if not np.any(part):
+            assert not np.any(got)
+
+
+@pytest.mark.parametrize("kind", ["real", "unit"])
+def test_integer_sums_of_zeros_walk_once(qk, kind):
+    """A real vector costs an apply what a complex one does (a second walk doubled it)."""
+    torch = pytest.importorskip("torch")
+    H = ham(qk, M.heisenberg(24, True))
+    full = torch.randn(H.dimension, dtype=torch.complex128, device="cuda")
+    x = torch.from_numpy(sparse_values(kind, H.dimension, np.random.default_rng(5))).cuda()
+
+    def us(v):
+        best = float("inf")
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                H.apply(v)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    us(full)
+    assert us(x) <= 1.5 * us(full)
