@@ -24,6 +24,7 @@ constexpr uint32_t kClassTarget = 5000;  // rows of the largest inner class aime
 constexpr int kTile = 128;        // rows of a table tile: one warp, four rows a lane
 constexpr uint32_t kNone16 = 0xFFFFu, kNone15 = 0x7FFFu;
 constexpr int kMaxAmps = 256;     // distinct amplitudes of the coded form
+constexpr double kMinEqual = 0x1p-900;
 constexpr int kMaxRowEntries = 63;  // entries a row of the integer-aligned FP64 sum may have
 
 // How the amplitudes of table entries are given.
@@ -71,6 +72,7 @@ struct Params {
     const A* amps;          // CODED: (re, im) pairs
     int n_amps;
     A u;                    // UNIFORM / SIGNED: the inner amplitude
+    int e_min;              // integer sums: exponents below are left to the FP64 pipe
     int diag_mode, cdiag;   // cdiag: the diagonal has imaginary parts
     const void* dcode;
     const A* dtab;
@@ -86,7 +88,7 @@ struct PackTables {
     packk::AmpMode mode = packk::AMP_UNIFORM;
     bool real = true;
     // every entry has the same |amplitude| and rows are short enough: the FP64
-    // kernel sums aligned integers
+    // kernel sums aligned integers (not for magnitudes below kMinEqual, 0 apart)
     bool equal = false;
     double u = 0.0;
     uint64_t dim = 0;

@@ -428,7 +428,7 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
     } else {
         equal = false;
     }
-    if (longest + outer_most + mixed_most > (size_t)kMaxRowEntries) equal = false;
+    if (longest + outer_most + mixed_most > (size_t)kMaxRowEntries || (u != 0.0 && std::abs(u) < kMinEqual)) equal = false;
     // --- items: the tiles of every block; blocks that a straddling flip of the
     // highest outer bit joins run side by side, so that the rows they gather from
     // one another are still in L2
@@ -566,6 +566,8 @@ void PackPlan::params(Params<A>& p) const {
     p.amps = mode_ == AMP_CODED ? at<A>(d ? amps64_ : amps32_) : nullptr;
     p.n_amps = n_amps_;
     p.u = (A)u_;
+    // u 2^-56 2^(e - 1023) is a normal number for the exponents that the integer sums keep
+    p.e_min = std::max(64, u_ != 0.0 ? 57 - std::ilogb(u_) : 0);
 }
 template void PackPlan::params<float>(Params<float>&) const;
 template void PackPlan::params<double>(Params<double>&) const;

@@ -68,9 +68,10 @@ struct SumF64 {
 // integers at 64.  The significand keeps 4 bits below its last place and 6
 // above its first (up to 64 addends), so an addend loses less than 2^-56 of the
 // largest one where a chain of FP64 additions rounds each partial sum to 2^-53.
-// Infinities, NaN and rows below 2^-959 are left to the FP64 pipe (bad()), but for sums of
-// nothing but zeros: every imaginary part of a real vector and most rows of a sparse one are
-// that, and a warp that walks twice takes longer than the FP64 pipe alone (real vector, L = 24
+// Infinities, NaN and rows whose sum, or its product with the magnitude, comes near the
+// subnormal numbers (below 2^-959 for magnitudes from 2^-7 up) are left to the FP64 pipe
+// (bad()), but for sums of nothing but zeros: every imaginary part of a real vector and most
+// rows of a sparse one are that, and a warp that walks twice takes longer than the FP64 pipe alone (real vector, L = 24
 // ring: 264 us walked twice, 237 on the FP64 pipe in the older kernels, 122 now).  What tells
 // zeros from the smallest numbers is one FP32 addition an addend, on a pipe that is idle (on
 // the integer pipe, two addends an OR: L = 28 1.97 against 1.94 ms); aligning the sum once
@@ -121,7 +122,7 @@ struct IntSum {
     // Whether the sum is one of zeros: with every high word +-0 the addends are below 2^32 units
     // of 2^-1074, and their sum is what s holds below the weight 2^56 of the (absent) leading ones.
     __device__ __forceinline__ bool zeros() const { return any == 0.f && (s << 8) == 0; }
-    __device__ __forceinline__ bool bad() const { return e == 0x7FF || (e < 64 && !zeros()); }
+    __device__ __forceinline__ bool bad(int e_min) const { return e == 0x7FF || (e < e_min && !zeros()); }
     __device__ __forceinline__ double value(double v) const { return v * __hiloint2double(e << 20, 0) * (double)s; }
 };
 struct SumI64 {
@@ -149,7 +150,7 @@ struct SumI64 {
         add_n(a1, &x);
     }
     __device__ __forceinline__ void add(double, double, V) {}  // never called: coded amplitudes go to SumF64
-    __device__ __forceinline__ bool bad() const { return r.bad() || i.bad(); }
+    __device__ __forceinline__ bool bad(int e_min) const { return r.bad(e_min) || i.bad(e_min); }
 };
 
 // a with the sign of the top bit of w applied
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(kThreads, EQUAL && NQ == 4 && (LZ || MODE == A
             bool bad = false;
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
-                bad = bad || (lane + 32u * (q0 + q) < cnt && acc[q].bad());
+                bad = bad || (lane + 32u * (q0 + q) < cnt && acc[q].bad(p.e_min));
                 orr[q] = acc[q].r.value(v);
                 oi[q] = acc[q].i.value(v);
             }

@@ -190,3 +190,21 @@ def test_integer_sums_of_zeros_walk_once(qk, kind):
 
     us(full)
     assert us(x) <= 1.5 * us(full)
+
+
+@pytest.mark.parametrize("model", [M.heisenberg(13, True, 1, 1.1 * 2.0 ** -500), M.heisenberg(24, True, 0, 1.1 * 2.0 ** -500),
+                                   M.hubbard(8, True, 4, 4, 1.1 * 2.0 ** -500, 2.0 ** -499),
+                                   M.heisenberg(13, True, 1, 1.1 * 2.0 ** -950)],
+                         ids=["ring13", "ring24_whole_tiles", "hubbard8_signs", "ring13_smaller"])
+def test_integer_sums_of_small_couplings(qk, model):
+    """Products near the smallest normal number although coupling and vector are far from it."""
+    H = ham(qk, model)
+    rng = np.random.default_rng(5)
+    J = abs(model[3][0][0])
+    x = (rng.standard_normal(H.dimension) + 1j * rng.standard_normal(H.dimension)) * (2.0 ** -1000 / J)
+    y = H.apply(x)
+    H.select_kernel(mode=1)
+    want = H.apply(x)
+    top = 64.0 * J * max(np.abs(x.real).max(), np.abs(x.imag).max())
+    assert top > 0.0
+    assert np.all(np.abs(y - want) <= 64 * 2.0 ** -53 * top + 128 * 2.0 ** -1074)
