@@ -1038,14 +1038,10 @@ BlockTridiag block_lanczos(const std::vector<Hamiltonian*>& hs, const BlockOpts&
     QKG_CUDA(cudaGetDevice(&dev));
     QKG_REQUIRE(dev == hs[0]->device(), "current device differs from the Hamiltonians' device");
     if (o.mixed) return PackedBlockEngine<float>::usable(hs) ? run_packed<float>(hs, o, Rq) : run_block<float, float>(hs, o, Rp);
-    // FP64, both bound by the FP64 pipe: without padding to save, large batches stay on the other
-    // engine (SpMV, packed against other: 2^20 rows, 32 vectors 1.78 / 1.67 ms; 2^22 rows, 14 of 16
-    // vectors 3.86 / 3.67; 2^20 rows, 12 vectors 0.75 / 1.00, 4 vectors 0.27 / 0.57; 24 steps of 2^18
-    // rows, 16 vectors 8.5 / 9.3 ms)
-    uint64_t rows = 0;
-    for (const auto* h : hs) rows += h->dim();
-    const bool unpadded = Rq == Rp && Rp >= 16 && rows * Rp >= (1ull << 25);
-    return !unpadded && PackedBlockEngine<double>::usable(hs) ? run_packed<double>(hs, o, Rq) : run_block<double, double>(hs, o, Rp);
+    // FP64: both engines are bound by the FP64 pipe, and unpadded the other one's SpMV is up to 6 %
+    // faster on large batches (2^20 rows, 32 vectors 1.78 / 1.67 ms), but the tables it would build
+    // first cost what it saves in some 400 steps (21 sectors of the 20-site ring: 44 ms)
+    return PackedBlockEngine<double>::usable(hs) ? run_packed<double>(hs, o, Rq) : run_block<double, double>(hs, o, Rp);
 }
 
 void ftlm_observables_block(const BlockTridiag& t, const double* betas, int nb, double* Zo, double* Eo, double* Co,

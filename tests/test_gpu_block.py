@@ -233,3 +233,15 @@ def test_ftlm_sectors_host_reduction_matches(qk):
     np.testing.assert_allclose(Z * np.exp(ls), r.partition_function * np.exp(r.log_shift), rtol=1e-9)
     np.testing.assert_allclose(E, r.internal_energy, rtol=1e-9, atol=1e-9)
     np.testing.assert_allclose(C, r.specific_heat, rtol=1e-8, atol=1e-8)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_batch_builds_nothing_it_would_have_to_keep(qk, mixed):
+    """A large unpadded batch runs on the tables its Hamiltonians came with: what it leaves on the
+    device beside the workspace is what was there before."""
+    hams = [qk.MatrixFreeHamiltonian(*make_model(qk, *M.heisenberg(20, True, s))) for s in range(-20, 21, 2)]
+    before = qk.lib().qkrylov_debug_live_allocations()
+    qk.block_lanczos_tridiag(hams, 32, 2, mixed=mixed, start="philox", seed=3)
+    for H in hams:
+        H.workspace_bytes(release=True)
+    assert qk.lib().qkrylov_debug_live_allocations() == before
