@@ -237,7 +237,7 @@ public:
         return basis_->permuted ? static_cast<const uint32_t*>(db_->ref_of_int) : nullptr;
     }
     bool uniform_inner() const { return unif_; }
-    const WorkItem* items_device() const { return items_.as<WorkItem>(); }
+    const WorkItem* items_device() const { return fast_items().as<WorkItem>(); }
     // host copy of the fast kernel's work items
     std::vector<WorkItem> items_host() const;
     size_t lanczos_parts() const;  // partial sums written by apply_lanczos_f32
@@ -285,6 +285,12 @@ private:
     int mode_ = 0;
     FastVariant pref_[2] = {FV_ROWS4, FV_ROWS4};
     double tune_ms_[2][kFastVariants] = {};
+    std::mutex lazy_tables_mu_;  // ensure_fast
+    // the fast kernels' work items: items_ with their own fields and order, beside it where they
+    // are built after construction (the generic kernel may be running on items_ then)
+    DBuf items_fast_;
+    DBuf& fast_items() { return pack_ ? items_fast_ : items_; }
+    const DBuf& fast_items() const { return pack_ ? items_fast_ : items_; }
     DBuf items_blk_;            // one work item per outer block (staged kernel)
     size_t n_items_blk_ = 0, max_block_ = 0;
     DBuf class_blocks_, class_info_;  // class-persistent kernel: sorted blocks, per-class table ranges

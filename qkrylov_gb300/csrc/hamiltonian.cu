@@ -957,9 +957,13 @@ Hamiltonian::Hamiltonian(std::shared_ptr<Basis> basis, SiteKind site, const std:
 }
 
 // The tables of the other fast kernels, for a Hamiltonian on the packed one:
-// built when a kernel mode or the batched engine first asks for them.
+// built when a kernel mode, or a batch with a Hamiltonian that has no packed plan,
+// first asks for them.  Batches on several threads may share a Hamiltonian.
 void Hamiltonian::ensure_fast() {
-    if (pack_ && !fast_tried_) build_fast();
+    std::lock_guard<std::mutex> lk(lazy_tables_mu_);
+    if (!pack_ || fast_tried_) return;
+    build_fast();
+    fast_tried_ = true;  // not after an exception: the next call builds them again
 }
 void Hamiltonian::set_kernel_mode(int m) {
     if (m >= 2) ensure_fast();
@@ -983,7 +987,6 @@ static void allow_stage_smem(size_t bytes);
 void Hamiltonian::build_fast() {
     const Basis& B = *basis_;
     fast_ = false;
-    fast_tried_ = true;
     if (B.rank_kind != RANK_TABLE || wide_ || dim() == 0 || dim() >= (1ull << 31) || diag_mode_ == DIAG_FULL) return;
     const uint64_t inm = db_->in_mask;
     std::vector<const HostTerm*> outer, inner, mixed;
@@ -1080,7 +1083,7 @@ void Hamiltonian::build_fast() {
         auto items = B.work_items(kChunk);
         set_groups(items);
         pair_order(items);
-        upload_vec(items_, items);
+        upload_vec(fast_items(), items);
     }
     u_ar_ = amp0.real();
     u_ai_ = amp0.imag();
@@ -1231,8 +1234,8 @@ void Hamiltonian::build_fast() {
     }
     if (stage_bytes(8) <= kStageLimit) allow_stage_smem<float, float>(stage_bytes(8));
     if (stage_bytes(16) <= kStageLimit) allow_stage_smem<double, double>(stage_bytes(16));
-    fast_ = true;
-    {
+    fast_ = true;  // can_tile asks for it
+    try {
         size_t t32 = 0, t64 = 0;
         for (int G : {1, 2, 4}) {
             if (can_tile(G, 8)) t32 = std::max(t32, tile_smem_bytes(G, 8));
@@ -1240,6 +1243,9 @@ void Hamiltonian::build_fast() {
         }
         if (t32) tilek::tile_allow_smem<float, float>(t32);
         if (t64) tilek::tile_allow_smem<double, double>(t64);
+    } catch (...) {
+        fast_ = false;
+        throw;
     }
 }
 
@@ -1413,7 +1419,7 @@ void Hamiltonian::fast_params(FastParams<A>& p) const {
     p.outer_off = static_cast<const uint32_t*>(b.outer_off);
     p.inner_rank = b.inner_all ? nullptr : b.inner_rank;
     p.inner_state = b.inner_all ? nullptr : b.inner_state;
-    p.items = items_.as<WorkItem>();
+    p.items = fast_items().as<WorkItem>();
     p.iptr = iptr_.as<uint32_t>();
     p.ient = ient_.as<uint32_t>();
     p.rbits = rbits_;
@@ -1503,7 +1509,7 @@ DBuf& Hamiltonian::krylov_workspace(size_t bytes) const {
 
 std::vector<WorkItem> Hamiltonian::items_host() const {
     std::vector<WorkItem> v(n_items_);
-    if (n_items_) QKG_CUDA(cudaMemcpy(v.data(), items_.p, n_items_ * sizeof(WorkItem), cudaMemcpyDeviceToHost));
+    if (n_items_) QKG_CUDA(cudaMemcpy(v.data(), fast_items().p, n_items_ * sizeof(WorkItem), cudaMemcpyDeviceToHost));
     return v;
 }
 template void Hamiltonian::fast_params<double>(FastParams<double>&) const;
@@ -1898,7 +1904,7 @@ const WorkItem* Hamiltonian::items_of(FastVariant v, size_t* n) const {
         return items_blk_.as<WorkItem>();
     }
     *n = n_items_;
-    return items_.as<WorkItem>();
+    return fast_items().as<WorkItem>();
 }
 
 void Hamiltonian::apply_f32(const float2* x, float2* y, cudaStream_t s) const {

@@ -245,3 +245,37 @@ def test_batch_builds_nothing_it_would_have_to_keep(qk, mixed):
     for H in hams:
         H.workspace_bytes(release=True)
     assert qk.lib().qkrylov_debug_live_allocations() == before
+
+
+def test_batches_on_two_threads_share_a_hamiltonian(qk):
+    """A batch with a sector that has no packed plan (more amplitudes than codes) builds the other
+    engine's tables of the rest on first use; two threads that share a sector give what one does."""
+    import threading
+
+    L = 24
+    many = (M.SPIN, L, M.sector(sz2=18), [(1.0 + 0.001 * (i * L + j), [(a, i), (b, j)]) for i in range(L) for j in range(i)
+                                          for a, b in (("Sp", "Sm"), ("Sm", "Sp"))]
+            + [(0.1 + 0.0003 * (i * L + j), [(a, i), (b, j), ("Sz", (i + 1) % L)]) for i in range(L) for j in range(i - 1)
+               if (i + 1) % L != j for a, b in (("Sp", "Sm"), ("Sm", "Sp"))])
+    ham = lambda model: qk.MatrixFreeHamiltonian(*make_model(qk, *model))
+    assert ham(many).tuning()[0] not in ("packed", "generic")
+    run = lambda hams: qk.block_lanczos_tridiag(hams, 4, 6, mixed=False, start="philox", seed=9)
+    want = [run([ham(many), ham(M.heisenberg(L, True, s))]) for s in (12, 14)]
+    for _ in range(3):
+        shared, got = [ham(M.heisenberg(L, True, s)) for s in (12, 14)], [None, None]
+        firsts = [ham(many), ham(many)]
+
+        def work(t):
+            # both threads need the tables of both shared sectors, in opposite orders
+            a, b = shared if t == 0 else shared[::-1]
+            r = run([firsts[t], a, b])
+            got[t] = r
+
+        th = [threading.Thread(target=work, args=(t,)) for t in (0, 1)]
+        [x.start() for x in th]
+        [x.join() for x in th]
+        for t in (0, 1):
+            assert got[t] is not None
+            for v in range(8):  # the first two Hamiltonians' vectors: the same streams as in the runs of one thread
+                np.testing.assert_array_equal(got[t].alphas[v], want[t].alphas[v])
+                np.testing.assert_array_equal(got[t].betas[v], want[t].betas[v])
