@@ -193,13 +193,7 @@ DavidsonOut davidson_f64(Hamiltonian& H, int n_eig, int max_sub, double tol, boo
     const size_t vb = n * sizeof(double2);
     release_workspace_if_short(H, (size_t)(2 * (max_sub + 2 * n_eig) + 4) * vb);
     const auto lock = H.workspace_lock();
-    struct Trim {  // a large basis is not kept
-        Hamiltonian& H;
-        ~Trim() {
-            cudaStreamSynchronize(H.stream());
-            H.trim_vectors(2ull << 30);
-        }
-    } trim{H};
+    const TrimVectors trim{H};
 
     // vectors by slot of the kept Krylov memory
     std::vector<int> spare;

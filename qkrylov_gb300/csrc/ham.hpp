@@ -254,11 +254,15 @@ public:
     void release_workspace() const;
     size_t workspace_bytes() const;
     // Also kept between calls and covered by the lock and the two above: vectors of
-    // `bytes` each for the FP64 Lanczos (slabs of up to 256 MB, allocated as the run
-    // grows), the reductions' scratch, and mapped host memory for scalars.
+    // `bytes` each for the FP64 solvers (slabs of up to 256 MB, allocated as the run
+    // grows; at most kKeptBytes over all Hamiltonians of a device once the runs are over),
+    // the reductions' scratch, and mapped host memory for scalars.
     void* krylov_vector(size_t i, size_t bytes) const;
     bool has_krylov_vector(size_t i) const;  // of the size last asked for
-    void trim_vectors(size_t keep_bytes) const;  // frees slabs from the last while they hold more
+    // frees slabs, the last first, while they and those of the device's other idle Hamiltonians
+    // hold more than kKeptBytes (at the end of a run)
+    void trim_vectors() const;
+    static constexpr size_t kKeptBytes = 2ull << 30;
     Workspace& reduction_scratch(size_t partials) const;
     struct MappedScalars {
         double *host = nullptr, *dev = nullptr;
@@ -329,10 +333,21 @@ private:
     mutable std::vector<DBuf> slabs_;
     mutable size_t slab_vec_bytes_ = 0;
     static constexpr size_t kSlabBytes = 256ull << 20;
+    size_t slab_vectors(size_t slab) const;  // vectors of a slab
+    mutable size_t kept_ = 0;                // bytes that count as kept
     mutable std::unique_ptr<Workspace> red_;
     mutable MappedScalars mapped_;
     mutable size_t mapped_n_ = 0;
     mutable std::mutex kws_mu_;
+};
+
+// Trims the vectors when a run is over, however it ends.
+struct TrimVectors {
+    const Hamiltonian& H;
+    ~TrimVectors() {
+        cudaStreamSynchronize(H.stream());
+        H.trim_vectors();
+    }
 };
 
 // ------------------------------------------------------------ Krylov algebra

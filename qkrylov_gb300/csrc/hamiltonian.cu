@@ -1620,6 +1620,7 @@ static void allow_stage_smem(size_t bytes) {
 void Hamiltonian::release_workspace() const {
     kws_.reset();
     slabs_.clear();
+    trim_vectors();
     red_.reset();
 }
 size_t Hamiltonian::workspace_bytes() const {
@@ -1627,32 +1628,62 @@ size_t Hamiltonian::workspace_bytes() const {
     for (const auto& s : slabs_) b += s.bytes;
     return b;
 }
+// Slab 0 holds the few vectors of a three-term recurrence, the others up to 64 each.
+size_t Hamiltonian::slab_vectors(size_t slab) const {
+    const size_t per = std::max<size_t>(1, std::min<size_t>(64, kSlabBytes / slab_vec_bytes_));
+    return slab ? per : std::min<size_t>(4, per);
+}
 void* Hamiltonian::krylov_vector(size_t i, size_t bytes) const {
     bytes = (bytes + 255) / 256 * 256;
     if (slab_vec_bytes_ != bytes) {
         slabs_.clear();
         slab_vec_bytes_ = bytes;
     }
-    const size_t per = std::max<size_t>(1, std::min<size_t>(64, kSlabBytes / bytes));
-    while (slabs_.size() <= i / per) {
-        size_t fr = 0, tot = 0;
-        QKG_CUDA(cudaMemGetInfo(&fr, &tot));
-        if (fr < per * bytes + (64ull << 20))
-            throw Error(CUDA_ERR, "out of device memory for the Krylov basis (" + std::to_string(slabs_.size() * per) + " vectors held)");
-        slabs_.emplace_back(per * bytes);
+    const size_t first = slab_vectors(0), per = slab_vectors(1);
+    const size_t slab = i < first ? 0 : 1 + (i - first) / per, at = i < first ? i : (i - first) % per;
+    while (slabs_.size() <= slab) {
+        const size_t need = slab_vectors(slabs_.size()) * bytes;
+        auto fits = [&] {
+            size_t fr = 0, tot = 0;
+            QKG_CUDA(cudaMemGetInfo(&fr, &tot));
+            return fr >= need + (64ull << 20);
+        };
+        if (!fits()) {
+            kws_.reset();  // the contiguous workspace is not in use beside the vectors
+            if (!fits())
+                throw Error(CUDA_ERR, "out of device memory for the Krylov basis (" +
+                                          std::to_string(slabs_.empty() ? 0 : first + (slabs_.size() - 1) * per) + " vectors held)");
+        }
+        slabs_.emplace_back(need);
     }
-    return slabs_[i / per].as<char>() + (i % per) * bytes;
+    return slabs_[slab].as<char>() + at * bytes;
 }
 bool Hamiltonian::has_krylov_vector(size_t i) const {
-    return slab_vec_bytes_ && i < slabs_.size() * std::max<size_t>(1, std::min<size_t>(64, kSlabBytes / slab_vec_bytes_));
+    return !slabs_.empty() && i < slab_vectors(0) + (slabs_.size() - 1) * slab_vectors(1);
 }
-void Hamiltonian::trim_vectors(size_t keep_bytes) const {
+namespace {
+// bytes of vectors kept by idle Hamiltonians, by device
+struct KeptVectors {
+    std::mutex mu;
+    std::map<int, size_t> bytes;
+};
+KeptVectors& kept_vectors() {
+    static KeptVectors* k = new KeptVectors;  // outlives every Hamiltonian
+    return *k;
+}
+}  // namespace
+void Hamiltonian::trim_vectors() const {
+    std::lock_guard<std::mutex> lk(kept_vectors().mu);
+    size_t& all = kept_vectors().bytes[dev_];
+    all -= kept_;
     size_t b = 0;
     for (const auto& s : slabs_) b += s.bytes;
-    while (!slabs_.empty() && b > keep_bytes) {
+    while (!slabs_.empty() && all + b > kKeptBytes) {
         b -= slabs_.back().bytes;
         slabs_.pop_back();
     }
+    kept_ = b;
+    all += b;
 }
 Workspace& Hamiltonian::reduction_scratch(size_t partials) const {
     if (!red_ || red_->cap_partials < partials) {
@@ -1674,6 +1705,8 @@ Hamiltonian::MappedScalars Hamiltonian::mapped_scalars(size_t n) const {
 }
 
 Hamiltonian::~Hamiltonian() {
+    slabs_.clear();
+    trim_vectors();
     if (mapped_.host) {
         if (stream_) cudaStreamSynchronize(stream_);
         cudaFreeHost(mapped_.host);

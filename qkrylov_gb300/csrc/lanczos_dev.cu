@@ -845,10 +845,7 @@ LanczosOut lanczos_f64_device(Hamiltonian& H, const LanczosOpts& o) {
     const int nmax = (int)std::min<uint64_t>((uint64_t)std::max(o.maxiter, 0), n);
     const size_t vb = n * sizeof(double2);
     auto vec = [&](int i) { return H.krylov_vector((size_t)i, vb); };
-    struct Trim {  // a long run's vectors are not kept
-        Hamiltonian& H;
-        ~Trim() { H.trim_vectors(2ull << 30); }
-    } trim{H};
+    const TrimVectors trim{H};
     double2* v0 = static_cast<double2*>(vec(0));
     double2* v1 = static_cast<double2*>(vec(1));
     if (o.device_start) {
@@ -949,6 +946,7 @@ double three_term_f64(Hamiltonian& H, const cd* v_ref, int n_steps, double min_n
     const auto lock = H.workspace_lock();
     cudaStream_t st = H.stream();
     const size_t vb = n * sizeof(double2);
+    const TrimVectors trim{H};
     // three vectors in turn
     auto vec = [&](int i) { return H.krylov_vector((size_t)(i % 3), vb); };
     double2* v0 = static_cast<double2*>(vec(0));
