@@ -253,6 +253,7 @@ public:
     DBuf& krylov_workspace(size_t bytes) const;
     void release_workspace() const;
     size_t workspace_bytes() const;
+    size_t krylov_workspace_bytes() const { return kws_.bytes; }  // of the contiguous one alone
     // Also kept between calls and covered by the lock and the two above: vectors of
     // `bytes` each for the FP64 solvers (slabs of up to 256 MB, allocated as the run
     // grows; at most kKeptBytes over all Hamiltonians of a device once the runs are over),

@@ -1501,7 +1501,10 @@ static void launch_tile_variant(const Hamiltonian& H, const FastParams<A>& p, Fa
 
 DBuf& Hamiltonian::krylov_workspace(size_t bytes) const {
     if (kws_.bytes < bytes) {
-        kws_.reset();  // free first: the old and new spaces need not fit together
+        // free first: the old and new spaces, and the FP64 vectors beside them, need not fit together
+        kws_.reset();
+        slabs_.clear();
+        trim_vectors();
         kws_.alloc(bytes);
     }
     return kws_;

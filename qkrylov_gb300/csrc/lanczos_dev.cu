@@ -399,8 +399,8 @@ LanczosOut lanczos_mixed_device(Hamiltonian& H, const LanczosOpts& o) {
     // cover whole 128-byte lines)
     const uint64_t stride = (n + 31) / 32 * 32;
     const size_t need = lanczos_device_bytes(H, o.maxiter);
-    if (H.workspace_bytes() < need) {
-        H.release_workspace();
+    if (H.krylov_workspace_bytes() < need) {
+        H.release_workspace();  // with the FP64 vectors, which the new space need not fit beside
         size_t fr = 0, tot = 0;
         QKG_CUDA(cudaMemGetInfo(&fr, &tot));
         if (need + (512ull << 20) > fr)

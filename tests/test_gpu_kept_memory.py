@@ -45,3 +45,18 @@ def test_three_term_recurrence_keeps_its_few_vectors(qk):
     v0 = np.random.default_rng(1).standard_normal(H.dimension).astype(complex)
     qk.continued_fraction_coeffs(H, v0, n_iter=20)
     assert 0 < H.workspace_bytes() <= 4 * (16 * H.dimension + 256)
+
+
+def test_contiguous_workspace_takes_the_place_of_fp64_vectors(qk):
+    """The mixed Lanczos and a batch allocate one block; the FP64 vectors kept before it, although larger, go first."""
+    H = ham(qk, M.heisenberg(16, True))
+    vector = 8 * H.dimension + 256
+    qk.lanczos_fixed_steps(H, 80, mixed=False)
+    assert H.workspace_bytes() > 80 * 2 * vector
+    qk.lanczos_fixed_steps(H, 20, mixed=True)
+    assert 20 * (vector - 256) < H.workspace_bytes() <= (20 + 16) * vector
+    H.workspace_bytes(release=True)
+    qk.lanczos_fixed_steps(H, 80, mixed=False)
+    qk.block_lanczos_tridiag([H], 4, 5, mixed=True, start="philox", seed=1)
+    # three block vectors of four, and under 2 MB of tables and partial sums
+    assert 12 * (vector - 256) < H.workspace_bytes() <= 12 * vector + (2 << 20)
