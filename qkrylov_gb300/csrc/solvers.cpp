@@ -747,7 +747,7 @@ CFOut cf_f64(Hamiltonian& H, const cd* phi0_ref, int n_iter) {
     CFOut out;
     if (H.dim() == 0) return out;
     const double np = std::sqrt(three_term_f64(H, phi0_ref, n_iter, 1e-15, out.alphas, out.betas));
-    if (np >= 1e-15) out.norm = np;  // src/solvers/dynamics.cpp:26
+    if (!(np < 1e-15)) out.norm = np;  // src/solvers/dynamics.cpp:26; NaN passes, as there
     return out;
 }
 

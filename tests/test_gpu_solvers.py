@@ -271,3 +271,15 @@ def test_selective_reorth_holds_several_ritz_vectors(qk):
     np.testing.assert_allclose(full, exact, rtol=0, atol=1e-9)
     np.testing.assert_allclose(sel, exact, rtol=0, atol=1e-9)
     np.testing.assert_allclose(mix, exact, rtol=0, atol=5e-5)  # FP32 vectors
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_continued_fraction_of_a_vector_that_is_not_finite(qk, bad):
+    """The norm and the spectrum are not finite either: they are not those of an empty recurrence."""
+    H = qk.MatrixFreeHamiltonian(*make_model(qk, *M.heisenberg(10, True)))
+    phi = np.ones(H.dimension, dtype=complex)
+    phi[3] = bad
+    r = qk.continued_fraction_coeffs(H, phi, n_iter=8)
+    assert not np.isfinite(r.norm_phi0)
+    assert len(r.alphas) and not np.isfinite(r.alphas).any()
+    assert not np.isfinite(qk.evaluate_spectral_function(r, np.array([0.5]), 0.0, 0.1)).any()
