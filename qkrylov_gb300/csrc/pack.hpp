@@ -102,7 +102,8 @@ struct PackTables {
 
     // False where the plan does not apply: ranks by search, states over 32 bits,
     // classes of more than 65,534 rows, more than 256 distinct amplitudes (coded
-    // form), tables over 256 MB, more than 24 straddling terms with one flip.
+    // form), amplitudes that are not finite in FP32, tables over 256 MB, more than 24
+    // straddling terms with one flip.
     // at_least: the least general amplitude form to give.
     bool build(const Basis& B, SiteKind site, const std::vector<Term>& terms,
                packk::AmpMode at_least = packk::AMP_UNIFORM);

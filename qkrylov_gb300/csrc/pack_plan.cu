@@ -235,7 +235,7 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         return m;
     };
     std::vector<uint32_t> ctile(ncls, 0);  // first inner tile of a class
-        std::vector<uint16_t> er, ec;  // entries: [(slot * 32 + lane) * 4 + q]
+    std::vector<uint16_t> er, ec;  // entries: [(slot * 32 + lane) * 4 + q]
     size_t longest = 0;            // inner entries of a row
     auto tiles_of = [&](int c) { return (uint32_t)((members[c].size() + kTile - 1) / kTile); };
     // emit(row, target rank, amplitude index) for the rows of class c on which the
@@ -388,6 +388,12 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         mixed_most = std::max<size_t>(mixed_most, blk[a].m1 - blk[a].m0);
         if (olist.size() > 0x7FFFFFFFull || slist.size() > 0x7FFFFFFFull) return false;
     }
+    // an empty slot adds amplitude * 0: that is nothing only for finite amplitudes, in FP32 too
+    auto finite32 = [](cd a) { return std::isfinite((float)a.real()) && std::isfinite((float)a.imag()); };
+    for (const cd& a : amps)
+        if (!finite32(a)) return false;
+    for (const auto& o : olist)
+        if (!finite32(o.a)) return false;
     // --- amplitude mode: one magnitude per inner table and per straddling table?
     size_t widest = 0;
     for (int c = 0; c < ncls; ++c)

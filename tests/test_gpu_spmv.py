@@ -332,3 +332,17 @@ def test_full_size_hubbard_L16_properties(qk):
     assert abs(lhs - rhs) <= 1e-12 * abs(lhs)
     d = H.diagonal()
     assert d.min() == 0.0 and d.max() == 4.0 * 8  # U * number of doubly occupied sites
+
+
+def test_rows_without_an_overflowing_coupling_stay_finite(qk):
+    """A coupling beyond FP32: the FP32 rows it does not reach are those of the generic kernel."""
+    L = 9
+    terms = [(1e39 if i == L - 2 else 1.0, [(a, i), (b, i + 1)]) for i in range(L - 1) for a, b in (("Sp", "Sm"), ("Sm", "Sp"))]
+    torch = pytest.importorskip("torch")
+    H = qk.MatrixFreeHamiltonian(*make_model(qk, M.SPIN, L, M.sector(sz2=1), terms))
+    x = torch.ones(H.dimension, dtype=torch.complex64, device="cuda")
+    y = H.apply(x).cpu().numpy()
+    H.select_kernel(mode=1)
+    want = H.apply(x).cpu().numpy()
+    assert np.isfinite(want).any() and not np.isfinite(want).all()
+    np.testing.assert_array_equal(np.isfinite(y), np.isfinite(want))

@@ -103,3 +103,15 @@ def test_plan_declines(qk):
     assert packed_apply(qk, (M.SPIN, 40, M.sector(sz2=38), M.heisenberg_terms(40, True)), x)[1] == -1
     many = [(1.0 + 0.001 * (i * 18 + j), [("Sp", i), ("Sm", j)]) for i in range(18) for j in range(18) if i != j]
     assert packed_apply(qk, (M.SPIN, 18, M.sector(sz2=16), many), x[:18])[1] == -1
+
+
+@pytest.mark.parametrize("J", [np.inf, np.nan, 1e39])
+def test_plan_declines_amplitudes_that_are_not_finite(qk, J):
+    """Empty slots are products with zero, also where the amplitude overflows FP32 only."""
+    import math
+    for L, n in ((9, 4), (16, 8)):  # one block; outer and straddling entries too
+        terms = [(J if i == L - 2 else 1.0, [(a, i), (b, i + 1)]) for i in range(L - 1) for a, b in (("Sp", "Sm"), ("Sm", "Sp"))]
+        x = np.zeros(math.comb(L, n), dtype=np.complex128)
+        assert packed_apply(qk, (M.SPIN, L, M.sector(sz2=2 * n - L), terms), x)[1] == -1
+    terms = [(1e38, t) for _, t in M.heisenberg_terms(9, True) if t[0][0] != "Sz"]
+    assert packed_apply(qk, (M.SPIN, 9, M.sector(sz2=1), terms), np.zeros(126, dtype=np.complex128))[1] >= 0
