@@ -6,8 +6,11 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <map>
+#include <memory>
 #include <tuple>
+#include <type_traits>
 
 namespace qkg {
 using namespace packk;
@@ -47,6 +50,13 @@ bool simplify(const HostTerm& h, PTerm& t, bool& dead) {
     if (popc(pinned & t.V) & 1) t.amp = -t.amp;
     t.J &= ~pinned;
     return true;
+}
+
+// parity of 16 bits without a population count (which takes Arm a trip through its vector unit)
+inline uint32_t parity16(uint32_t x) {
+    x ^= x >> 8;
+    x ^= x >> 4;
+    return (0x6996u >> (x & 15u)) & 1u;
 }
 
 int top_bit(uint64_t x) { return x ? 63 - __builtin_clzll(x) : -1; }
@@ -123,11 +133,10 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         return k0 * w1 + k1;
     };
     std::vector<std::vector<uint32_t>> members(ncls);
-    std::vector<uint16_t> rank(1ull << n_in), cls(1ull << n_in);
+    std::vector<uint32_t> place(1ull << n_in);  // class << 16 | rank in it
     for (uint64_t b = 0; b <= inm; ++b) {
         const int c = class_of_inner(b);
-        cls[b] = (uint16_t)c;
-        rank[b] = (uint16_t)std::min<size_t>(members[c].size(), 0xFFFF);
+        place[b] = (uint32_t)c << 16 | (uint32_t)std::min<size_t>(members[c].size(), 0xFFFF);
         members[c].push_back((uint32_t)b);
     }
     const uint64_t n_a = 1ull << n_out;
@@ -180,146 +189,208 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
             }
         return any;
     };
-    // --- raw tables: (rank, amplitude) per slot and row, then packed by mode
-    struct Raw {
-        std::vector<uint16_t> r;  // [slot][row of the class, padded to tiles]
-        std::vector<uint16_t> c;  // amplitude index
-    };
-    std::map<std::pair<uint64_t, uint64_t>, uint32_t> amp_id;
-    bool too_many = false;
-    // codes met since `used` was last cleared, and the last ones looked up
-    std::vector<char> used;
-    cd seen[4];
-    uint16_t seen_id[4];
-    int n_seen = 0, next_seen = 0;
-    auto code_of = [&](cd a) -> uint16_t {
-        for (int i = 0; i < n_seen; ++i)
-            if (seen[i] == a) {
-                used[seen_id[i]] = 1;
-                return seen_id[i];
+    // --- tables: a 16-bit rank and an amplitude index per entry, packed by mode at the end.
+    // Each class's inner table and each straddling table is built by one thread with amplitude
+    // indexes of its own; they are joined in order, so the outcome is that of one thread.
+    struct Codes {
+        std::vector<cd> amps;
+        std::map<std::pair<uint64_t, uint64_t>, uint32_t> id;
+        cd seen[4];  // the last ones looked up
+        uint16_t seen_id[4];
+        int n_seen = 0, next_seen = 0;
+        bool too_many = false;
+        uint16_t operator()(cd a) {
+            for (int i = 0; i < n_seen; ++i)
+                if (seen[i] == a) return seen_id[i];
+            uint64_t k[2];
+            const double re = a.real() + 0.0, im = a.imag() + 0.0;  // no negative zeros
+            std::memcpy(k, &re, 8);
+            std::memcpy(k + 1, &im, 8);
+            auto it = id.find({k[0], k[1]});
+            if (it == id.end()) {
+                if (amps.size() >= 4096) { too_many = true; return 0; }
+                it = id.emplace(std::make_pair(k[0], k[1]), (uint32_t)amps.size()).first;
+                amps.push_back(cd(re, im));
             }
-        uint64_t k[2];
-        const double re = a.real() + 0.0, im = a.imag() + 0.0;  // no negative zeros
-        std::memcpy(k, &re, 8);
-        std::memcpy(k + 1, &im, 8);
-        auto it = amp_id.find({k[0], k[1]});
-        if (it == amp_id.end()) {
-            if (amps.size() >= 4096) { too_many = true; return 0; }
-            it = amp_id.emplace(std::make_pair(k[0], k[1]), (uint32_t)amps.size()).first;
-            amps.push_back(cd(re, im));
-            used.push_back(0);
+            seen[next_seen] = cd(re, im);
+            seen_id[next_seen] = (uint16_t)it->second;
+            n_seen = std::min(n_seen + 1, 4);
+            next_seen = (next_seen + 1) & 3;
+            return (uint16_t)it->second;
         }
-        seen[next_seen] = cd(re, im);
-        seen_id[next_seen] = (uint16_t)it->second;
-        n_seen = std::min(n_seen + 1, 4);
-        next_seen = (next_seen + 1) & 3;
-        used[it->second] = 1;
-        return (uint16_t)it->second;
     };
-    // the magnitude of the used codes (-1: none used), and which signs occur; one =
-    // false: several magnitudes
+    // the magnitude of a set of amplitudes (-1: none), and which signs occur; one = false:
+    // several magnitudes
     struct Mag {
         double mag = -1.0;
         bool plus = false, minus = false, one = true;
-    };
-    auto magnitude = [&]() {
-        Mag m;
-        for (size_t i = 0; i < amps.size(); ++i) {
-            if (!used[i]) continue;
-            const double v = amps[i].real();
-            if (m.mag < 0.0) m.mag = std::abs(v);
-            m.one = m.one && std::abs(v) == m.mag;
-            (std::signbit(v) ? m.minus : m.plus) = true;
+        void add(const std::vector<cd>& amps) {
+            for (const cd& a : amps) {
+                const double v = a.real();
+                if (mag < 0.0) mag = std::abs(v);
+                one = one && std::abs(v) == mag;
+                (std::signbit(v) ? minus : plus) = true;
+            }
         }
-        std::fill(used.begin(), used.end(), 0);
-        return m;
+    };
+    struct Built {
+        std::vector<uint16_t> er, ec;  // entries: [(slot * 32 + lane) * 4 + q]
+        std::vector<uint2> tile;
+        Codes code;
+        size_t longest = 0;  // inner entries of a row
+        bool any = false;
+    };
+    Codes code;                    // of all tables
+    std::vector<uint16_t> er, ec;  // entries of all tables
+    // appends b's entries
+    auto join = [&](Built& b) {
+        std::vector<uint16_t> to(b.code.amps.size());
+        bool same = true;
+        for (size_t i = 0; i < to.size(); ++i) {
+            to[i] = code(b.code.amps[i]);
+            same = same && to[i] == i;
+        }
+        if (!same)
+            for (size_t e = 0; e < b.er.size(); ++e)
+                if (b.er[e] != kNone16) b.ec[e] = to[b.ec[e]];
+        er.insert(er.end(), b.er.begin(), b.er.end());
+        ec.insert(ec.end(), b.ec.begin(), b.ec.end());
+        return er.size() / 4 <= kMaxTable && !code.too_many && !b.code.too_many;
+    };
+    // body(i) for i < n on several threads where there is work for them: a region costs some 20 us,
+    // 20,000 rows tested 70 us (16 cores: 12-site Hubbard ring 5.9 to 2.1 ms, with next-nearest hops
+    // 9.8 to 4.1, 20-site ring 0.86 to 0.46; one class, 14-site ring, 0.22)
+    auto threads = [](size_t n, size_t work, auto&& body) {
+        std::exception_ptr failed;
+#pragma omp parallel for schedule(dynamic) if (n > 1 && work > 20000)
+        for (long long i = 0; i < (long long)n; ++i) {
+            try {
+                body((size_t)i);
+            } catch (...) {
+#pragma omp critical(qkg_pack_plan)
+                failed = std::current_exception();
+            }
+        }
+        if (failed) std::rethrow_exception(failed);
     };
     std::vector<uint32_t> ctile(ncls, 0);  // first inner tile of a class
-    std::vector<uint16_t> er, ec;  // entries: [(slot * 32 + lane) * 4 + q]
-    size_t longest = 0;            // inner entries of a row
+    size_t longest = 0;                    // inner entries of a row
+    Mag inner_mag;
     auto tiles_of = [&](int c) { return (uint32_t)((members[c].size() + kTile - 1) / kTile); };
-    // emit(row, target rank, amplitude index) for the rows of class c on which the
-    // merged terms ts give an entry in class c2.  A few terms have a few sums: the
-    // amplitude index is looked up by which terms hold, and with which signs.
-    std::vector<int> sums;
-    auto each = [&](int c, int c2, const std::vector<PTerm>& ts, uint32_t flip, auto&& emit) {
-        const size_t T = ts.size();
+    // emit(row, target rank, amplitude index) for the rows of class c on which the merged
+    // terms ts give an entry in class c2.  A few terms have a few sums: the amplitude index is
+    // looked up by which terms hold, and with which signs.
+    auto each = [&](int c, int c2, const std::vector<PTerm>& ts, uint32_t flip, Codes& code_of, auto&& emit) {
+        const int T = (int)ts.size();
         const bool few = T <= 5;
-        if (few) sums.assign((size_t)1 << (2 * T), -1);
+        int sums[1 << 10];
+        if (few) std::fill(sums, sums + ((size_t)1 << (2 * T)), -1);
         uint32_t C[5], V[5], J[5];
-        for (size_t k = 0; few && k < T; ++k) C[k] = (uint32_t)ts[k].C, V[k] = (uint32_t)ts[k].V, J[k] = (uint32_t)ts[k].J;
-        const auto& mem = members[c];
-        for (uint32_t r = 0; r < mem.size(); ++r) {
-            const uint32_t bb = mem[r], b2 = bb ^ flip;
+        for (int k = 0; few && k < T; ++k) C[k] = (uint32_t)ts[k].C, V[k] = (uint32_t)ts[k].V, J[k] = (uint32_t)ts[k].J;
+        const uint32_t *mem = members[c].data(), *at = place.data();
+        const uint32_t n = (uint32_t)members[c].size();
+        for (uint32_t r = 0; r < n; ++r) {
+            const uint32_t bb = mem[r];
+            cd amp;
             if (few) {
                 uint32_t key = 0;
-                for (size_t k = 0; k < T; ++k)
-                    if ((bb & C[k]) == V[k]) key |= (J[k] && __builtin_parity(bb & J[k]) ? ((1u << T) | 1u) : 1u) << k;
-                if (!key || cls[b2] != c2) continue;
+                for (int k = 0; k < T; ++k)
+                    if ((bb & C[k]) == V[k]) key |= (J[k] && parity16(bb & J[k]) ? ((1u << T) | 1u) : 1u) << k;
+                if (!key) continue;
+                const uint32_t to = at[bb ^ flip];
+                if ((to >> 16) != (uint32_t)c2) continue;
                 int& id = sums[key];
-                if (id < 0) {  // code_of also marks the code as used
-                    cd amp;
+                if (id < 0) {
                     sum_at(ts, bb, amp);
                     id = code_of(amp);
                 }
-                emit(r, rank[b2], (uint16_t)id);
+                emit(r, (uint16_t)to, (uint16_t)id);
             } else {
-                cd amp;
-                if (!sum_at(ts, bb, amp) || cls[b2] != c2) continue;
-                emit(r, rank[b2], code_of(amp));
+                const uint32_t to = at[bb ^ flip];
+                if (!sum_at(ts, bb, amp) || (to >> 16) != (uint32_t)c2) continue;
+                emit(r, (uint16_t)to, code_of(amp));
             }
         }
     };
-    std::vector<uint16_t> rr, rc;  // a class' rows: entries in group order
-    std::vector<uint8_t> rn;       // how many
-    for (int c = 0; c < ncls; ++c) {
-        ctile[c] = (uint32_t)tile.size();
-        if (!present[c]) continue;
-        const size_t W = members[c].size(), most_slots = inner.size();
-        if (most_slots > 255) return false;
-        rn.assign(W, 0);
-        rr.resize(W * most_slots);
-        rc.resize(W * most_slots);
-        for (const auto& g : inner)
-            each(c, c, g.t, (uint32_t)g.X, [&](uint32_t r, uint16_t to, uint16_t code) {
-                const size_t at = r * most_slots + rn[r]++;
-                rr[at] = to;
-                rc[at] = code;
-            });
-        for (uint32_t t = 0; t < tiles_of(c); ++t) {
-            uint2 rec = make_uint2((uint32_t)(er.size() / kTile), 0u);
-            for (uint32_t q = 0; q < 4; ++q) {
-                const size_t r0 = (size_t)t * kTile + q * 32, r1 = std::min(W, r0 + 32);
-                size_t most = 0;
-                for (size_t r = r0; r < r1; ++r) most = std::max<size_t>(most, rn[r]);
-                rec.y |= (uint32_t)most << (8 * q);
-                longest = std::max(longest, most);
-                const size_t e0 = er.size(), nq = (most + 3) / 4;
-                er.resize(e0 + nq * kTile, (uint16_t)kNone16);
-                ec.resize(er.size(), 0);
-                for (size_t r = r0; r < r1; ++r)
-                    for (size_t j = 0; j < rn[r]; ++j) {
-                        const size_t at = e0 + ((j / 4) * 32 + (r - r0)) * 4 + (j & 3);
-                        er[at] = rr[r * most_slots + j];
-                        ec[at] = rc[r * most_slots + j];
-                    }
+    if (inner.size() > 255) return false;
+    {
+        std::vector<int> list;       // the classes that occur
+        std::vector<size_t> row_at;  // their first rows in the scratch below
+        size_t rows = 0;
+        for (int c = 0; c < ncls; ++c)
+            if (present[c]) {
+                list.push_back(c);
+                row_at.push_back(rows);
+                rows += members[c].size();
             }
-            tile.push_back(rec);
-            if (er.size() / 4 > kMaxTable || too_many) return false;
+        // rows: entries in group order (not initialised), and how many
+        const size_t stride = inner.size();
+        const std::unique_ptr<uint16_t[]> rows_r(new uint16_t[rows * stride]), rows_c(new uint16_t[rows * stride]);
+        std::vector<uint16_t> rows_n(rows, 0);
+        std::vector<Built> built(list.size());
+        threads(list.size(), rows * inner.size(), [&](size_t n) {
+            const int c = list[n];
+            Built& b = built[n];
+            const size_t W = members[c].size();
+            uint16_t *rr = rows_r.get() + row_at[n] * stride, *rc = rows_c.get() + row_at[n] * stride, *rn = rows_n.data() + row_at[n];
+            for (const auto& g : inner)
+                each(c, c, g.t, (uint32_t)g.X, b.code, [stride, R = rr, A = rc, N = rn](uint32_t r, uint16_t to, uint16_t code) {
+                    const size_t at = r * stride + N[r]++;
+                    R[at] = to;
+                    A[at] = code;
+                });
+            b.er.reserve((size_t)tiles_of(c) * kTile * ((stride + 7) / 8 * 4));
+            b.ec.reserve((size_t)tiles_of(c) * kTile * ((stride + 7) / 8 * 4));
+            for (uint32_t t = 0; t < tiles_of(c); ++t) {
+                uint2 rec = make_uint2((uint32_t)(b.er.size() / kTile), 0u);
+                for (uint32_t q = 0; q < 4; ++q) {
+                    const size_t r0 = (size_t)t * kTile + q * 32, r1 = std::min(W, r0 + 32);
+                    size_t most = 0;
+                    for (size_t r = r0; r < r1; ++r) most = std::max<size_t>(most, rn[r]);
+                    rec.y |= (uint32_t)most << (8 * q);
+                    b.longest = std::max(b.longest, most);
+                    const size_t e0 = b.er.size(), nq = (most + 3) / 4;
+                    b.er.resize(e0 + nq * kTile, (uint16_t)kNone16);
+                    b.ec.resize(b.er.size(), 0);
+                    for (size_t r = r0; r < r1; ++r)
+                        for (size_t j = 0; j < rn[r]; j += 4) {  // a quad, or the rest of the row
+                            const size_t at = e0 + ((j / 4) * 32 + (r - r0)) * 4, k = std::min<size_t>(4, rn[r] - j) * 2;
+                            std::memcpy(&b.er[at], &rr[r * stride + j], k);
+                            std::memcpy(&b.ec[at], &rc[r * stride + j], k);
+                        }
+                }
+                b.tile.push_back(rec);
+            }
+        });
+        for (size_t n = 0; n < list.size(); ++n) {
+            Built& b = built[n];
+            ctile[list[n]] = (uint32_t)tile.size();
+            for (uint2 rec : b.tile) tile.push_back(make_uint2(rec.x + (uint32_t)(er.size() / kTile), rec.y));
+            longest = std::max(longest, b.longest);
+            inner_mag.add(b.code.amps);
+            if (!join(b)) return false;
+            b = Built();
         }
     }
     // the kernels read one quad ahead
     er.resize(er.size() + kTile, (uint16_t)kNone16);
     ec.resize(er.size(), 0);
-    const Mag inner_mag = magnitude();
     // --- per block: outer entries and straddling tables
     blk.assign(n_a, Blk{});
     struct O { int32_t d; cd a; };
-    struct M { uint32_t tab, off; };
+    struct M { uint32_t tab, off; };  // tab: index in `tables` first, its entries in the end
     std::vector<O> olist;
     std::vector<M> slist;
-    std::map<std::tuple<int, uint32_t, uint32_t, uint32_t, int>, uint32_t> tables;  // -> first entry / 4 (uint2 index)
-    std::vector<std::pair<uint32_t, Mag>> table_mag;  // of each straddling table
+    struct Table {
+        int c, c2;
+        uint32_t group, valid, neg;
+        uint32_t id;  // first entry / 4 (uint2 index), kNoTable: no row of the class has an entry
+    };
+    constexpr uint32_t kNoTable = 0xFFFFFFFFu;
+    std::vector<Table> tables;
+    // by class and group, a few each: (valid, neg, c2) -> index in tables
+    std::vector<std::map<std::tuple<uint32_t, uint32_t, int>, uint32_t>> known((size_t)ncls * mixed.size());
+    std::vector<std::pair<uint32_t, Mag>> table_mag;                        // of each straddling table
     size_t outer_most = 0, mixed_most = 0;
     for (uint64_t a = 0; a < n_a; ++a) {
         blk[a].o0 = (uint32_t)olist.size();
@@ -340,54 +411,77 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
                 for (size_t k = 0; k < g.t.size(); ++k)
                     if ((sa & g.t[k].C & ~inm) == (g.t[k].V & ~inm)) {
                         valid |= 1u << k;
-                        if (popc(sa & g.t[k].J & ~inm) & 1) neg |= 1u << k;
+                        const uint64_t J = g.t[k].J & ~inm;
+                        if (J && (popc(sa & J) & 1)) neg |= 1u << k;
                     }
                 if (!valid) continue;
-                const auto key = std::make_tuple(bcls[a], (uint32_t)gi, valid, neg, bcls[a2]);
-                auto it = tables.find(key);
-                if (it == tables.end()) {
-                    std::vector<PTerm> ts;
-                    for (size_t k = 0; k < g.t.size(); ++k)
-                        if (valid >> k & 1) {
-                            PTerm t = g.t[k];
-                            t.C &= inm;
-                            t.V &= inm;
-                            t.J &= inm;
-                            if (neg >> k & 1) t.amp = -t.amp;
-                            ts.push_back(t);
-                        }
-                    const int c = bcls[a], c2 = bcls[a2];
-                    const size_t e0 = er.size();
-                    er.resize(e0 + (size_t)tiles_of(c) * kTile, (uint16_t)kNone16);
-                    ec.resize(er.size(), 0);
-                    bool any = false;
-                    each(c, c2, ts, (uint32_t)(g.X & inm), [&](uint32_t r, uint16_t to, uint16_t code) {
-                        const size_t t = r / kTile, i = r % kTile;
-                        const size_t at = e0 + (t * 32 + (i & 31)) * 4 + (i >> 5);
-                        er[at] = to;
-                        ec[at] = code;
-                        any = true;
-                    });
-                    if (er.size() / 4 > kMaxTable || too_many) return false;
-                    uint32_t id = 0xFFFFFFFFu;  // no row of the class has an entry
-                    if (any) {
-                        id = (uint32_t)(e0 / 4);
-                        table_mag.push_back({id, magnitude()});
-                    } else {
-                        er.resize(e0);
-                        ec.resize(e0);
-                    }
-                    it = tables.emplace(key, id).first;
-                }
-                if (it->second != 0xFFFFFFFFu) slist.push_back({it->second, off[a2]});
+                const auto [it, fresh] = known[bcls[a] * mixed.size() + gi].try_emplace({valid, neg, bcls[a2]}, (uint32_t)tables.size());
+                if (fresh) tables.push_back({bcls[a], bcls[a2], (uint32_t)gi, valid, neg, kNoTable});
+                slist.push_back({it->second, off[a2]});
             }
         }
         blk[a].o1 = (uint32_t)olist.size();
         blk[a].m1 = (uint32_t)slist.size();
         outer_most = std::max<size_t>(outer_most, blk[a].o1 - blk[a].o0);
-        mixed_most = std::max<size_t>(mixed_most, blk[a].m1 - blk[a].m0);
         if (olist.size() > 0x7FFFFFFFull || slist.size() > 0x7FFFFFFFull) return false;
     }
+    // the tables, some at a time (what is built before it is joined stays below 8 M entries)
+    for (size_t t0 = 0, t1; t0 < tables.size(); t0 = t1) {
+        size_t rows = 0, work = 0;
+        for (t1 = t0; t1 < tables.size() && rows < (8u << 20); ++t1) {
+            rows += (size_t)tiles_of(tables[t1].c) * kTile;
+            work += members[tables[t1].c].size() * mixed[tables[t1].group].t.size();
+        }
+        std::vector<Built> built(t1 - t0);
+        threads(t1 - t0, work, [&](size_t n) {
+            const Table& tb = tables[t0 + n];
+            const Group& g = mixed[tb.group];
+            Built& b = built[n];
+            std::vector<PTerm> ts;
+            for (size_t k = 0; k < g.t.size(); ++k)
+                if (tb.valid >> k & 1) {
+                    PTerm t = g.t[k];
+                    t.C &= inm;
+                    t.V &= inm;
+                    t.J &= inm;
+                    if (tb.neg >> k & 1) t.amp = -t.amp;
+                    ts.push_back(t);
+                }
+            b.er.resize((size_t)tiles_of(tb.c) * kTile, (uint16_t)kNone16);
+            b.ec.resize(b.er.size(), 0);
+            bool any = false;
+            each(tb.c, tb.c2, ts, (uint32_t)(g.X & inm), b.code, [&any, R = b.er.data(), A = b.ec.data()](uint32_t r, uint16_t to, uint16_t code) {
+                const uint32_t t = r / kTile, i = r % kTile;
+                const size_t at = (t * 32 + (i & 31)) * 4 + (i >> 5);
+                R[at] = to;
+                A[at] = code;
+                any = true;
+            });
+            b.any = any;
+        });
+        for (size_t n = 0; n < built.size(); ++n) {
+            if (!built[n].any) continue;
+            tables[t0 + n].id = (uint32_t)(er.size() / 4);
+            Mag m;
+            m.add(built[n].code.amps);
+            table_mag.push_back({tables[t0 + n].id, m});
+            if (!join(built[n])) return false;
+        }
+    }
+    // the blocks' entries of tables that are there
+    {
+        uint32_t n = 0;
+        for (uint64_t a = 0; a < n_a; ++a) {
+            const uint32_t m0 = n;
+            for (uint32_t k = blk[a].m0; k < blk[a].m1; ++k)
+                if (tables[slist[k].tab].id != kNoTable) slist[n++] = {tables[slist[k].tab].id, slist[k].off};
+            blk[a].m0 = m0;
+            blk[a].m1 = n;
+            mixed_most = std::max<size_t>(mixed_most, n - m0);
+        }
+        slist.resize(n);
+    }
+    amps = code.amps;
     // an empty slot adds amplitude * 0: that is nothing only for finite amplitudes, in FP32 too
     auto finite32 = [](cd a) { return std::isfinite((float)a.real()) && std::isfinite((float)a.imag()); };
     for (const cd& a : amps)
@@ -416,8 +510,11 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
             // rank | sign << 15; amplitudes are magnitudes
             std::vector<uint16_t> bit(amps.size());
             for (size_t i = 0; i < amps.size(); ++i) bit[i] = std::signbit(amps[i].real()) ? 0x8000u : 0u;
-            for (size_t e = 0; e < er.size(); ++e)
-                er[e] = er[e] == kNone16 ? (uint16_t)kNone15 : (uint16_t)(er[e] | bit[ec[e]]);
+            constexpr size_t kChunk = 1 << 14;
+            threads((er.size() + kChunk - 1) / kChunk, er.size(), [&](size_t n) {
+                for (size_t e = n * kChunk; e < std::min(er.size(), (n + 1) * kChunk); ++e)
+                    er[e] = er[e] == kNone16 ? (uint16_t)kNone15 : (uint16_t)(er[e] | bit[ec[e]]);
+            });
             u = std::max(umag, 0.0);
         }
         for (const auto& t : table_mag)
@@ -441,13 +538,15 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
     int pair_bit = -1;
     for (const auto& g : mixed) pair_bit = std::max(pair_bit, top_bit(g.X >> n_in));
     std::vector<uint32_t> order;
-    for (uint64_t a = 0; a < n_a; ++a)
+    const uint32_t pair = pair_bit >= 0 ? 1u << pair_bit : 0u;
+    for (uint64_t a = 0; a < n_a; ++a) {
+        if (a & pair) continue;  // comes with its partner
         if (bcls[a] >= 0) order.push_back((uint32_t)a);
-    if (pair_bit >= 0) {
-        const uint32_t m = 1u << pair_bit;
-        auto key = [&](uint32_t a) { return ((uint64_t)(a & ~m) << 1) | ((a & m) ? 1u : 0u); };
-        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return key(x) < key(y); });
+        if (pair && bcls[a | pair] >= 0) order.push_back((uint32_t)a | pair);
     }
+    size_t n_tiles = 0;
+    for (uint32_t a : order) n_tiles += tiles_of(bcls[a]);
+    items.reserve(n_tiles);
     for (uint32_t a : order) {
         const size_t W = members[bcls[a]].size();
         for (size_t t = 0; t * kTile < W; ++t)
@@ -462,6 +561,8 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         for (size_t e = 0; e < codes.size(); ++e)
             codes[e] = (uint32_t)ec[4 * e] | (uint32_t)ec[4 * e + 1] << 8 | (uint32_t)ec[4 * e + 2] << 16 | (uint32_t)ec[4 * e + 3] << 24;
     }
+    out.reserve(olist.size());
+    str.reserve(slist.size());
     for (const auto& o : olist) out.push_back({o.d, 0u, o.a.real(), o.a.imag()});
     for (const auto& m : slist) {
         const double v = mode == AMP_CODED ? 0.0 : smag[m.tab];
