@@ -100,11 +100,36 @@ __device__ __forceinline__ void upd_psi(u64 x, u64 p, int q, UpdAcc<NP>& s) {
     acc2(s.ih[q], s.il[q], p ^ kConj2, pk(f.y, f.x));
 }
 // the two halves of a compensated pair sum added
-__device__ __forceinline__ float2 halves(u64 hi, u64 lo) {
+__device__ __forceinline__ double halves(u64 hi, u64 lo) {
     const float2 h = unpk(hi), l = unpk(lo);
     float a = h.x, b = l.x;
     ff_add(a, b, h.y, l.y);
-    return make_float2(a, b);
+    return (double)a + (double)b;
+}
+// CTA sums of M values a thread, in double and in a fixed order, valid in thread 0: the values
+// go through shared memory and a warp takes one of them, eight additions a lane and a tree, so
+// that GB300's narrow FP64 pipe sees 13 additions a value and CTA where shuffles in every warp
+// would take 45.  As fast as float pairs throughout (100 steps at L = 24 7.82 and 7.82 ms, 60 at
+// L = 28 54.9 and 54.9, 100 at L = 18 3.30 and 3.30) without their 48 bits; a thread's own sums
+// are brought to one pair in FP32 first (two conversions a value and not four: 8.03 ms).
+template <int M>
+__device__ __forceinline__ void block_sums_d(double (&v)[M]) {
+    __shared__ double red[M][kT], sum[M];
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int m = 0; m < M; ++m) red[m][threadIdx.x] = v[m];
+    __syncthreads();
+    for (int m = threadIdx.x >> 5; m < M; m += kT / 32) {
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < kT / 32; ++i) s += red[m][lane + 32 * i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) sum[m] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = sum[m];
 }
 struct Four {
     u64 v[4];
@@ -153,18 +178,18 @@ __global__ void __launch_bounds__(kT) lz_update_t(const LzDev d, uint64_t n, con
 #pragma unroll
         for (int q = 0; q < NP; ++q) upd_psi<NP>(x, reinterpret_cast<const u64*>(psi.p[q])[i], q, s);
     }
-    // block sums in float-float FP32 arithmetic: a double sum in each of the CTAs
-    // cost as much as the pass on GB300's narrow FP64 pipe
-    float2 t = halves(s.hi, s.lo);
-    t = block_sum_ff(t.x, t.y);
-    if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2((double)t.x + (double)t.y, 0.0);
+    double t[1 + 2 * NP];
+    t[0] = halves(s.hi, s.lo);
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        float2 r = halves(s.rh[q], s.rl[q]), m = halves(s.ih[q], s.il[q]);
-        r = block_sum_ff(r.x, r.y);
-        m = block_sum_ff(m.x, m.y);
-        if (threadIdx.x == 0)
-            ppart[(size_t)q * gridDim.x + blockIdx.x] = make_double2((double)r.x + (double)r.y, (double)m.x + (double)m.y);
+        t[1 + 2 * q] = halves(s.rh[q], s.rl[q]);
+        t[2 + 2 * q] = halves(s.ih[q], s.il[q]);
+    }
+    block_sums_d(t);
+    if (threadIdx.x == 0) {
+        bpart[blockIdx.x] = make_double2(t[0], 0.0);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) ppart[(size_t)q * gridDim.x + blockIdx.x] = make_double2(t[1 + 2 * q], t[2 + 2 * q]);
     }
     if (!last_cta(d.arrived)) return;
     // the last CTA: ||w||^2, c_q = <psi_q, w>.  The correction is applied only when
@@ -234,9 +259,9 @@ __global__ void __launch_bounds__(kT) lz_orth_kernel(const LzDev d, const PsiTab
         reinterpret_cast<u64*>(w)[i] = x;
         acc2(h2, l2, x, x);
     }
-    float2 s = halves(h2, l2);
-    s = block_sum_ff(s.x, s.y);
-    if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2((double)s.x + (double)s.y, 0.0);
+    double s[1] = {halves(h2, l2)};
+    block_sums_d(s);
+    if (threadIdx.x == 0) bpart[blockIdx.x] = make_double2(s[0], 0.0);
     if (!last_cta(d.arrived)) return;
     const double w2 = sum_partials(bpart, gridDim.x);
     if (threadIdx.x == 0) {
