@@ -203,13 +203,6 @@ template <int VPL> struct Row<double, VPL> {
 #pragma unroll
         for (int j = 0; j < VPL; ++j) v[j] = p[j * G];
     }
-    __device__ __forceinline__ void load_if(const double2* p, int G, bool on) {
-#pragma unroll
-        for (int j = 0; j < VPL; ++j) {
-            v[j] = make_double2(0.0, 0.0);
-            if (on) v[j] = p[j * G];
-        }
-    }
     __device__ __forceinline__ void store(double2* p, int G) const {
 #pragma unroll
         for (int j = 0; j < VPL; ++j) __stcs(p + j * G, v[j]);
@@ -255,18 +248,8 @@ __device__ __forceinline__ int vec_of(int l, int j, int G) {
 // Per-vector sums Re sum conj(x) y.
 template <class T, int VPL> struct Dots;
 template <int VPL> struct Dots<float, VPL> {
-    u64 hi[VPL], lo[VPL], sc[VPL];
-    __device__ __forceinline__ void init(int j, double scale) {
-        hi[j] = lo[j] = 0ull;
-        sc[j] = pk((float)scale, (float)scale);
-    }
-    __device__ __forceinline__ void finish(Row<float, VPL>& y, const Row<float, VPL>& x, bool dot) {
-#pragma unroll
-        for (int j = 0; j < VPL; ++j) {
-            y.v[j] = mul2(y.v[j], sc[j]);
-            if (dot) acc2(hi[j], lo[j], x.v[j], y.v[j]);
-        }
-    }
+    u64 hi[VPL], lo[VPL];
+    __device__ __forceinline__ void init(int j, double) { hi[j] = lo[j] = 0ull; }
     __device__ __forceinline__ void square(const Row<float, VPL>& x) {
 #pragma unroll
         for (int j = 0; j < VPL; ++j) acc2(hi[j], lo[j], x.v[j], x.v[j]);
@@ -595,19 +578,19 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                             c1 >>= 8;
                         }
                         if (!more) break;
-                        continue;
-                    }
-                    const uint32_t w[4] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16};
-                    if (rank_of(w[0]) == kNone) break;  // a row's entries come first
-                    // the four rows' loads go out together; an empty slot reads zero
-                    R v[4];
+                    } else {
+                        const uint32_t w[4] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16};
+                        if (rank_of(w[0]) == kNone) break;  // a row's entries come first
+                        // the four rows' loads go out together; an empty slot reads zero
+                        R v[4];
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        const int to = rank_of(w[h]);
-                        v[h].load_if(offset(xl, to, rb), G, to != kNone);
-                    }
+                        for (int h = 0; h < 4; ++h) {
+                            const int to = rank_of(w[h]);
+                            v[h].load_if(offset(xl, to, rb), G, to != kNone);
+                        }
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) amp_add(w[h], c >> (8 * h), u, v[h]);
+                        for (int h = 0; h < 4; ++h) amp_add(w[h], c >> (8 * h), u, v[h]);
+                    }
                 }
                 for (uint32_t j = 0; j < ns; j += kStrBatch) {
                     if (j) straddles(j);
@@ -621,17 +604,17 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
                             v.load(offset(Xh, (int)strl[j + i].off + to, rb), G);
                             amp_add(w16, i ? sc[1] : sc[0], strl[j + i].ar, v);
                         }
-                        continue;
-                    }
-                    R v[kStrBatch];
+                    } else {
+                        R v[kStrBatch];
 #pragma unroll
-                    for (int i = 0; i < kStrBatch; ++i) {
-                        const int to = rank_of(sw[i]);
-                        v[i].load_if(offset(Xh, j + i < ns ? (int)strl[j + i].off + to : 0, rb), G, to != kNone);
-                    }
+                        for (int i = 0; i < kStrBatch; ++i) {
+                            const int to = rank_of(sw[i]);
+                            v[i].load_if(offset(Xh, j + i < ns ? (int)strl[j + i].off + to : 0, rb), G, to != kNone);
+                        }
 #pragma unroll
-                    for (int i = 0; i < kStrBatch; ++i)
-                        if (j + i < ns) amp_add(sw[i], sc[i], strl[j + i].ar, v[i]);
+                        for (int i = 0; i < kStrBatch; ++i)
+                            if (j + i < ns) amp_add(sw[i], sc[i], strl[j + i].ar, v[i]);
+                    }
                 }
                 R x;
                 x.load(xo, G);
