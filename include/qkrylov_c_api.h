@@ -398,8 +398,9 @@ int qkrylov_hamiltonian_tuning_ex(qkrylov_hamiltonian_h h, int fp32, int* varian
 int qkrylov_basis_states(qkrylov_basis_h basis, uint64_t first, uint64_t count, uint64_t* out);
 
 /* Device memory the Hamiltonian keeps between solver calls (the FP32 Krylov
- * space of the mixed Lanczos: maxiter + 7 vectors; the FP64 solvers' and the
- * batched forms' vectors): *bytes receives its size;
+ * space of the mixed Lanczos: maxiter + 7 vectors; the batched forms' vectors;
+ * the FP64 solvers' vectors, at most 2 GB over all Hamiltonians of a device):
+ * *bytes receives its size;
  * release != 0 frees it now (it is also freed with the Hamiltonian). */
 int qkrylov_hamiltonian_workspace(qkrylov_hamiltonian_h h, int release, uint64_t* bytes);
 

@@ -10,8 +10,8 @@
 // far flips, listed first, read one run.  L = 28 ring (40.1 M rows): 0.42 ms = 1.52
 // TB/s of x and y; the kernel on the domain-wall order 0.66 ms, and 0.19 ms for each of
 // the two permutation passes of an apply that this order does without.
-// FP64: the integer pipe (60% busy) for equal magnitudes, 1.65 ms; the FP64 pipe (88%
-// busy) otherwise and before, 2.80 ms.
+// FP64: the integer pipe for equal magnitudes (L = 28 1.87 ms, L = 24 121 us); the FP64 pipe
+// (88% busy) otherwise and in the older kernels (L = 24 197 us, and 40 of permutations).
 #include "pack.hpp"
 #include "pair.cuh"
 
@@ -27,7 +27,7 @@ namespace {
 // kernels wait for gathers, so FP32 takes 48 warps a SM at 40 registers (L = 28
 // ring: 32 warps 0.47 ms, 40 0.46, 48 0.42, 56 0.44) and 40 warps at 48 where signs,
 // codes or the Lanczos step's terms need more (L = 28 Lanczos step 0.55 to 0.54 ms, L = 14
-// Hubbard ring 0.153 to 0.148), FP64 24 warps at 80 (16 warps 2.05 ms, 24 1.65, 32 1.65).
+// Hubbard ring 0.153 to 0.148), FP64 24 warps at 80 (L = 28 ring: 16 warps 2.01 ms, 24 1.87, 32 1.93).
 constexpr int kThreads = 128;
 // Integer sums of four rows a lane with signs or the Lanczos step's terms: 20 warps at 96 registers
 // (100 recurrence steps at L = 24: 19.1 ms with 24 warps and their spills, 18.4; 13-site Hubbard ring 151 and 150 us).
@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(kThreads, EQUAL && NQ == 4 && (LZ || MODE == A
 // Four warps a tile (NQ = 1) below 24 tiles a SM: one warp a tile leaves the
 // SMs short of loads in flight there, and pays for itself above, where the four
 // rows share the block's entries.  FP32 / FP64, one against four warps: L = 14
-// 6.3 / 12.3 against 4.3 / 6.2 us, L = 20 (1,700 tiles) 8.5 / 18.5 against 6.3 /
-// 12.6 us, L = 24 (21,500 tiles) 28.9 / 112.9 against 43.2 / 126.0 us.
+// 6.3 / 10.3 against 4.2 / 6.2 us, L = 20 (1,700 tiles) 10.3 / 16.5 against 7.1 /
+// 13.5 us, L = 24 (21,500 tiles) 28.8 / 120.5 against 43.1 / 130.8 us.
 bool split_tiles(uint32_t n_items) { return n_items < 152u * 24u; }
 
 }  // namespace
