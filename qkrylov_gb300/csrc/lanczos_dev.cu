@@ -109,9 +109,10 @@ __device__ __forceinline__ double halves(u64 hi, u64 lo) {
 // CTA sums of M values a thread, in double and in a fixed order, valid in thread 0: the values
 // go through shared memory and a warp takes one of them, eight additions a lane and a tree, so
 // that GB300's narrow FP64 pipe sees 13 additions a value and CTA where shuffles in every warp
-// would take 45.  As fast as float pairs throughout (100 steps at L = 24 7.82 and 7.82 ms, 60 at
-// L = 28 54.9 and 54.9, 100 at L = 18 3.30 and 3.30) without their 48 bits; a thread's own sums
-// are brought to one pair in FP32 first (two conversions a value and not four: 8.03 ms).
+// would take 45.  About as fast as float pairs throughout (100 steps at L = 24, median of ten
+// processes 8.33 and 8.31 ms, 60 at L = 28 54.9 and 54.9, 100 at L = 18 3.30 and 3.30) without
+// their 48 bits; a thread's own sums are brought to one pair in FP32 first (two conversions a
+// value and not four: 0.2 ms at L = 24).
 template <int M>
 __device__ __forceinline__ void block_sums_d(double (&v)[M]) {
     __shared__ double red[M][kT], sum[M];
