@@ -1024,6 +1024,29 @@ BlockTridiag run_packed(const std::vector<Hamiltonian*>& hs, const BlockOpts& o,
 
 }  // namespace
 
+// Whether an FP64 batch of planned Hamiltonians runs on the other engine.  Both are bound by the
+// FP64 pipe; unpadded and without amplitude codes the other one's steps take 6-12 % less from 2^25
+// block elements on (ms a step, packed and other: L = 22, every sector, 32 vectors 9.4 / 8.8, L = 24
+// 39.0 / 35.5, L = 26, Sz = 0, 16 vectors 13.4 / 12.1, Hubbard 14 sites 17.7 / 15.9; level below: Hubbard
+// 12 sites, 32 vectors 2.41 / 2.41; with codes J1-J2 24 sites 5.3 / 5.6, complex field 22 sites 17 / 37).
+// Its tables cost about 0.7 ms a Hamiltonian on first use: the run has to be long enough to save
+// that itself (5 ps an element and step).
+static bool long_fp64_run(const std::vector<Hamiltonian*>& hs, const BlockOpts& o, int Rp, int Rq) {
+    uint64_t rows = 0;
+    for (const auto* h : hs) rows += h->dim();
+    const double elements = (double)rows * Rp;
+    if (Rq != Rp || Rp < 16 || elements < (double)(1ull << 25) ||
+        elements * o.steps < (double)(1ull << 27) * (double)hs.size())
+        return false;
+    for (auto* h : hs)
+        if (!h->dim() || h->plan_of_form(packk::AMP_UNIFORM)->mode() == packk::AMP_CODED) return false;
+    for (auto* h : hs) {
+        h->ensure_fast();
+        if (!h->has_fast_tables()) return false;
+    }
+    return true;
+}
+
 BlockTridiag block_lanczos(const std::vector<Hamiltonian*>& hs, const BlockOpts& o) {
     QKG_REQUIRE(!hs.empty(), "no Hamiltonians");
     QKG_REQUIRE(o.R >= 1 && o.R <= 32, "vectors per Hamiltonian must be 1..32");
@@ -1038,10 +1061,13 @@ BlockTridiag block_lanczos(const std::vector<Hamiltonian*>& hs, const BlockOpts&
     QKG_CUDA(cudaGetDevice(&dev));
     QKG_REQUIRE(dev == hs[0]->device(), "current device differs from the Hamiltonians' device");
     if (o.mixed) return PackedBlockEngine<float>::usable(hs) ? run_packed<float>(hs, o, Rq) : run_block<float, float>(hs, o, Rp);
-    // FP64: both engines are bound by the FP64 pipe, and unpadded the other one's SpMV is up to 6 %
-    // faster on large batches (2^20 rows, 32 vectors 1.78 / 1.67 ms), but the tables it would build
-    // first cost what it saves in some 400 steps (21 sectors of the 20-site ring: 44 ms)
-    return PackedBlockEngine<double>::usable(hs) ? run_packed<double>(hs, o, Rq) : run_block<double, double>(hs, o, Rp);
+    if (!PackedBlockEngine<double>::usable(hs)) return run_block<double, double>(hs, o, Rp);
+    if (long_fp64_run(hs, o, Rp, Rq)) {
+        BlockOpts w = o;
+        if (w.vpl <= 0) w.vpl = 4;  // the fastest of 1, 2, 4 on every model below, so none are timed
+        return run_block<double, double>(hs, w, Rp);
+    }
+    return run_packed<double>(hs, o, Rq);
 }
 
 void ftlm_observables_block(const BlockTridiag& t, const double* betas, int nb, double* Zo, double* Eo, double* Co,

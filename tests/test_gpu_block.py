@@ -237,8 +237,8 @@ def test_ftlm_sectors_host_reduction_matches(qk):
 
 @pytest.mark.parametrize("mixed", [False, True])
 def test_batch_builds_nothing_it_would_have_to_keep(qk, mixed):
-    """A large unpadded batch runs on the tables its Hamiltonians came with: what it leaves on the
-    device beside the workspace is what was there before."""
+    """A large unpadded batch of few steps runs on the tables its Hamiltonians came with: what it leaves
+    on the device beside the workspace is what was there before."""
     hams = [qk.MatrixFreeHamiltonian(*make_model(qk, *M.heisenberg(20, True, s))) for s in range(-20, 21, 2)]
     before = qk.lib().qkrylov_debug_live_allocations()
     qk.block_lanczos_tridiag(hams, 32, 2, mixed=mixed, start="philox", seed=3)
@@ -279,3 +279,22 @@ def test_batches_on_two_threads_share_a_hamiltonian(qk):
             for v in range(8):  # the first two Hamiltonians' vectors: the same streams as in the runs of one thread
                 np.testing.assert_array_equal(got[t].alphas[v], want[t].alphas[v])
                 np.testing.assert_array_equal(got[t].betas[v], want[t].betas[v])
+
+
+@pytest.mark.parametrize("case", ["long", "long_with_an_empty_sector", "codes"])
+def test_long_fp64_batches_against_few_steps(qk, case):
+    """FP64 batches long and large enough for the other engine, and those that stay on the packed one."""
+    L = 20
+    extra = [(0.2, [(a, i), (b, (i + 2) % L)]) for i in range(L) for a, b in (("Sp", "Sm"), ("Sm", "Sp"))] if case == "codes" else []
+    ham = lambda s: qk.MatrixFreeHamiltonian(*make_model(qk, M.SPIN, L, M.sector(sz2=s), M.heisenberg_terms(L, True) + extra))
+    hams = [ham(s) for s in (0, 2, -2, 4, -4, 6, -6)] * 2  # 2^21 rows
+    if case == "long_with_an_empty_sector":
+        hams.append(ham(1))
+        assert hams[-1].dimension == 0
+    got = qk.block_lanczos_tridiag(hams, 32, 40, mixed=False, start="philox", seed=5)
+    few = qk.block_lanczos_tridiag(hams[:1], 32, 4, mixed=False, start="philox", seed=5)
+    norm = 0.75 * L + (4.0 if case == "codes" else 0.0)
+    for v in (0, 31):
+        # four steps of 2^-53 rounding on numbers up to ||H||
+        np.testing.assert_allclose(got.alphas[v][:4], few.alphas[v], rtol=0, atol=64 * 2.0 ** -53 * norm)
+        np.testing.assert_allclose(got.betas[v][:3], few.betas[v][:3], rtol=0, atol=64 * 2.0 ** -53 * norm)
