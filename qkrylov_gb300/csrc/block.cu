@@ -568,9 +568,20 @@ public:
         const uint32_t groups = blockk::kBT / std::max(1, Rp / (Rp % 4 == 0 ? 4 : Rp % 2 == 0 ? 2 : 1));
         run_ = (int)std::max<uint64_t>(1, std::min<uint64_t>({(uint64_t)kPasses * groups / blockk::kTile,
                                                               total / (152 * 4) / blockk::kTile, blockk::kMaxRun}));
+        // small batches: a tile's rows over up to four CTAs, as far as that gives each row a group
+        // of its own and the last CTA no more than kSplitCtas partials to add (40 steps, FP64, tile by
+        // CTA and split: 12-site ring, 32 vectors 2.05 / 1.35 ms, 16 vectors 1.47 / 1.24; 8-site Hubbard
+        // ring, 32 vectors 2.84 / 2.2; 404 CTAs, 16-site ring 3.20 / 3.41)
+        uint64_t tiles = 0;
+        for (size_t h = 0; h < hs.size(); ++h)
+            if (hs[h]->dim()) tiles += plan_of[h]->n_items();
+        while (parts_ < 4 && (uint32_t)parts_ * groups < (uint32_t)blockk::kTile && tiles * parts_ * 2 <= kSplitCtas) parts_ *= 2;
         // rows of an update CTA: a small batch is spread over the SMs (12-site sectors, 16
-        // vectors: 15.8 us an update with 512 rows a CTA)
-        chunk_ = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, total / (152 * 4) / 32 * 32));
+        // vectors: 15.8 us an update with 512 rows a CTA), but where the last CTA adds the partials
+        // over one CTA an SM or so (40 steps, 32 FP32 / FP64 vectors, 32 rows and total / 152: 16-site
+        // ring 1.89 / 3.16 and 1.67 / 3.03 ms; 17 sites, 760 CTAs, 1.78 / 4.42 and 1.88 / 4.73)
+        const uint64_t ctas = total <= 32ull * kFusedCtas ? 152 : 152 * 4;
+        chunk_ = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(512, total / ctas / 32 * 32));
         std::vector<packk::Params<T>> P(hs.size());
         std::vector<blockk::Ham> hams(hs.size());
         std::vector<uint32_t> range(1, 0), rrange(1, 0);  // CTAs by Hamiltonian
@@ -584,7 +595,7 @@ public:
                 H.pack_params(P[h], *plan_of[h]);
                 real_ = real_ && plan_of[h]->real();
                 mode_ = plan_of[h]->mode();
-                n = (plan_of[h]->n_items() + run_ - 1) / run_;
+                n = (plan_of[h]->n_items() + run_ - 1) / run_ * parts_;
             } else {
                 P[h] = packk::Params<T>{};
             }
@@ -684,6 +695,8 @@ private:
     // from its place (L = 20, 32 vectors 16.9 -> 17.4 ms; L = 22, 12 vectors, Sz = 0, 120 steps
     // 18.9 -> 22.8).
     static constexpr unsigned kFusedCtas = 4 * 152;
+    static constexpr uint64_t kSplitCtas = 208;
+    static_assert(kSplitCtas <= kFusedCtas, "split tiles are one tile a run, in fused launches");
 
     void finish(const double* part, const uint32_t* range, int mode, const BState& st, int k) {
         block_finish_kernel<<<(unsigned)(hs_.size() * Rp_), kBlock, 0, s_>>>(part, range, mode, st, k);
@@ -715,7 +728,7 @@ private:
             constexpr int M = decltype(mode)::value;
             constexpr bool C = decltype(cplx)::value;
             auto* kernel = fused ? blockk::block_pack_kernel<T, M, C, VPL, true> : blockk::block_pack_kernel<T, M, C, VPL, false>;
-            kernel<<<n_ctas_, blockk::kBT, 0, s_>>>(params_, hams_, (int)hs_.size(), run_, Rp_, x, y, scale, apart, fin);
+            kernel<<<n_ctas_, blockk::kBT, 0, s_>>>(params_, hams_, (int)hs_.size(), run_, parts_, Rp_, x, y, scale, apart, fin);
         };
         using std::integral_constant;
         if (mode_ == packk::AMP_UNIFORM) go(integral_constant<int, packk::AMP_UNIFORM>{}, std::false_type{});
@@ -726,7 +739,7 @@ private:
     }
 
     std::vector<Hamiltonian*> hs_;
-    int Rp_, Ruser_, run_ = 1;
+    int Rp_, Ruser_, run_ = 1, parts_ = 1;
     uint32_t chunk_ = 512;
     std::unique_lock<std::mutex> ws_lock_;  // the first Hamiltonian's workspace, held for the engine's life
     cudaStream_t s_ = nullptr;

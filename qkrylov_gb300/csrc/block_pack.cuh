@@ -404,11 +404,11 @@ __device__ __forceinline__ void finish_ham(const Finish& f, int ham, uint32_t n_
     if ((int)threadIdx.x < Rp) finish_vector(f.st, ham * Rp + v, a, f.mode, f.k);
 }
 
-// FUSED: the bookkeeping in the Hamiltonian's last CTA (an instantiation of its own: the
-// code alone cost the large batches 2 %).
+// FUSED: the bookkeeping in the Hamiltonian's last CTA, and a tile dealt out to `parts` CTAs
+// (an instantiation of its own: the code alone cost the large batches 2 %).
 template <class T, int MODE, bool CPLX, int VPL, bool FUSED>
 __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
-    block_pack_kernel(const Params<T>* __restrict__ P, const Ham* __restrict__ hams, int n_hams, int run, int Rp,
+    block_pack_kernel(const Params<T>* __restrict__ P, const Ham* __restrict__ hams, int n_hams, int run, int parts, int Rp,
                       const typename V2<T>::t* __restrict__ X, typename V2<T>::t* __restrict__ Y,
                       const double* __restrict__ scale, double* __restrict__ apart, const Finish fin) {
     using T2 = typename V2<T>::t;
@@ -418,7 +418,8 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
     __shared__ T s_amp[MODE == AMP_CODED ? 2 * kMaxAmps : 1];
     const int ham = find_ham(hams, n_hams, blockIdx.x, [](const Ham& h) { return h.cta0; });
     const Params<T>& p = P[ham];
-    const uint32_t tile0 = (blockIdx.x - hams[ham].cta0) * (uint32_t)run;
+    const uint32_t tile0 = FUSED ? (blockIdx.x - hams[ham].cta0) / (uint32_t)parts * (uint32_t)run
+                                 : (blockIdx.x - hams[ham].cta0) * (uint32_t)run;
     const uint32_t count = min((uint32_t)run, p.n_items - tile0);
     const uint64_t base = hams[ham].base;
     if (MODE == AMP_CODED) {
@@ -474,8 +475,16 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
     T2* __restrict__ Yh = Y + base * (uint64_t)Rp + l * W0;
     {
         uint32_t ti = 0, oo = 0, so = 0;  // the row's tile and where its lists start
+        // the run's rows, or one of `parts` parts of its only tile's
+        int row_lo = grp, row_hi = (int)count * kTile;
+        if constexpr (FUSED)
+            if (parts > 1) {
+                const int lo = (int)((blockIdx.x - hams[ham].cta0) % (uint32_t)parts) * (kTile / parts);
+                row_lo += lo;
+                row_hi = lo + kTile / parts;
+            }
         if (grp < NG)
-            for (int rr = grp; rr < (int)count * kTile; rr += NG) {
+            for (int rr = row_lo; rr < row_hi; rr += NG) {
                 while (ti < (uint32_t)rr >> 7) {
                     oo += s_blk[ti].y - s_blk[ti].x;
                     so += s_blk[ti].w - s_blk[ti].z;
@@ -635,7 +644,7 @@ __global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 4 : 2)
             for (int j = 0; j < VPL; ++j) red[grp * Rp + vec_of<T, VPL>(l, j, G)] = own[j];
         __syncthreads();
         reduce_vectors<T>(red, NG, Rp, apart + (size_t)blockIdx.x * Rp);
-        if constexpr (FUSED) finish_ham(fin, ham, (p.n_items + run - 1) / run, Rp, apart + (size_t)hams[ham].cta0 * Rp, red);
+        if constexpr (FUSED) finish_ham(fin, ham, (p.n_items + run - 1) / run * parts, Rp, apart + (size_t)hams[ham].cta0 * Rp, red);
     }
 }
 

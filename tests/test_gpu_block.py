@@ -298,3 +298,26 @@ def test_long_fp64_batches_against_few_steps(qk, case):
         # four steps of 2^-53 rounding on numbers up to ||H||
         np.testing.assert_allclose(got.alphas[v][:4], few.alphas[v], rtol=0, atol=64 * 2.0 ** -53 * norm)
         np.testing.assert_allclose(got.betas[v][:3], few.betas[v][:3], rtol=0, atol=64 * 2.0 ** -53 * norm)
+
+
+@pytest.mark.parametrize("R", [3, 7, 12, 16, 20, 28, 32])
+@pytest.mark.parametrize("sz2", [10, 4, 0])
+def test_small_batches_split_tiles(qk, sz2, R):
+    """Tiles dealt out to two or four CTAs, rows of a tile in one, two and four parts, partial tiles
+    (11, 495 and 3,432 rows; with a second Hamiltonian beside it): every vector against its own run."""
+    L = {10: 12, 4: 12, 0: 14}[sz2]
+    H = qk.MatrixFreeHamiltonian(*make_model(qk, *M.heisenberg(L, True, sz2)))
+    other = qk.MatrixFreeHamiltonian(*make_model(qk, *M.heisenberg(10, True)))
+    rng = np.random.default_rng(R)
+    vec = lambda n: rng.standard_normal((R, n)) + 1j * rng.standard_normal((R, n))
+    P, Q = vec(H.dimension), vec(other.dimension)
+    steps = min(6, H.dimension)
+    for mixed, eps in ((False, 2.0 ** -53), (True, 2.0 ** -24)):
+        got = qk.block_lanczos_tridiag([other, H], R, steps, mixed=mixed, start="given", start_vectors=[Q, P])
+        for h, X, base in ((other, Q, 0), (H, P, R)):
+            bound = np.abs(h.diagonal()).max() + 2.0 * L
+            for r in sorted({0, R // 2, R - 1}):
+                one = qk.continued_fraction_coeffs(h, X[r], n_iter=steps)
+                # six steps of rounding, each step's error carried on by the next ones
+                np.testing.assert_allclose(got.alphas[base + r][:5], one.alphas[:5], rtol=0, atol=64 * eps * bound)
+                np.testing.assert_allclose(got.betas[base + r][:4], one.betas[:4], rtol=0, atol=64 * eps * bound)
