@@ -72,6 +72,16 @@ size_t append(std::vector<char>& image, const std::vector<T>& v) {
 
 constexpr size_t kMaxTable = 32ull << 20;  // uint2 entries of all tables (256 MB)
 
+// A vector whose resize leaves new elements as they are: the threads that write them touch
+// their pages first.
+template <class T>
+struct NoInit : std::allocator<T> {
+    template <class U> struct rebind { using other = NoInit<U>; };
+    template <class U> void construct(U* p) { ::new (static_cast<void*>(p)) U; }
+    template <class U, class A> void construct(U* p, A&& a) { ::new (static_cast<void*>(p)) U(std::forward<A>(a)); }
+};
+using Entries = std::vector<uint16_t, NoInit<uint16_t>>;
+
 }  // namespace
 
 bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& terms, AmpMode at_least) {
@@ -234,29 +244,15 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         }
     };
     struct Built {
-        std::vector<uint16_t> er, ec;  // entries: [(slot * 32 + lane) * 4 + q]
+        Entries er, ec;  // entries: [(slot * 32 + lane) * 4 + q]
         std::vector<uint2> tile;
         Codes code;
         size_t longest = 0;  // inner entries of a row
-        bool any = false;
+        size_t at = 0;       // its first entry among all tables'
+        bool any = false;    // whether it has entries at all
     };
-    Codes code;                    // of all tables
-    std::vector<uint16_t> er, ec;  // entries of all tables
-    // appends b's entries
-    auto join = [&](Built& b) {
-        std::vector<uint16_t> to(b.code.amps.size());
-        bool same = true;
-        for (size_t i = 0; i < to.size(); ++i) {
-            to[i] = code(b.code.amps[i]);
-            same = same && to[i] == i;
-        }
-        if (!same)
-            for (size_t e = 0; e < b.er.size(); ++e)
-                if (b.er[e] != kNone16) b.ec[e] = to[b.ec[e]];
-        er.insert(er.end(), b.er.begin(), b.er.end());
-        ec.insert(ec.end(), b.ec.begin(), b.ec.end());
-        return er.size() / 4 <= kMaxTable && !code.too_many && !b.code.too_many;
-    };
+    Codes code;      // of all tables
+    Entries er, ec;  // entries of all tables
     // body(i) for i < n on several threads where there is work for them: a region costs some 20 us,
     // 20,000 rows tested 70 us (16 cores: 12-site Hubbard ring 5.9 to 2.1 ms, with next-nearest hops
     // 9.8 to 4.1, 20-site ring 0.86 to 0.46; one class, 14-site ring, 0.22)
@@ -272,6 +268,38 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
             }
         }
         if (failed) std::rethrow_exception(failed);
+    };
+    // appends the entries of the tables that have any, in order
+    auto join = [&](std::vector<Built>& built) {
+        std::vector<std::vector<uint16_t>> to(built.size());  // codes, empty: the same
+        size_t n = er.size();
+        for (size_t t = 0; t < built.size(); ++t) {
+            Built& b = built[t];
+            if (!b.any) continue;
+            bool same = true;
+            for (size_t i = 0; i < b.code.amps.size(); ++i) {
+                to[t].push_back(code(b.code.amps[i]));
+                same = same && to[t][i] == i;
+            }
+            if (same) to[t].clear();
+            b.at = n;
+            n += b.er.size();
+            if (n / 4 > kMaxTable || code.too_many || b.code.too_many) return false;
+        }
+        const size_t added = n - er.size();
+        er.resize(n);
+        ec.resize(n);
+        threads(built.size(), added, [&](size_t t) {
+            const Built& b = built[t];
+            if (!b.any) return;
+            std::copy(b.er.begin(), b.er.end(), er.begin() + b.at);
+            if (to[t].empty()) {
+                std::copy(b.ec.begin(), b.ec.end(), ec.begin() + b.at);
+            } else {
+                for (size_t e = 0; e < b.ec.size(); ++e) ec[b.at + e] = b.er[e] == kNone16 ? (uint16_t)0 : to[t][b.ec[e]];
+            }
+        });
+        return true;
     };
     std::vector<uint32_t> ctile(ncls, 0);  // first inner tile of a class
     size_t longest = 0;                    // inner entries of a row
@@ -361,15 +389,15 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
                 }
                 b.tile.push_back(rec);
             }
+            b.any = true;
         });
+        if (!join(built)) return false;
         for (size_t n = 0; n < list.size(); ++n) {
-            Built& b = built[n];
+            const Built& b = built[n];
             ctile[list[n]] = (uint32_t)tile.size();
-            for (uint2 rec : b.tile) tile.push_back(make_uint2(rec.x + (uint32_t)(er.size() / kTile), rec.y));
+            for (uint2 rec : b.tile) tile.push_back(make_uint2(rec.x + (uint32_t)(b.at / kTile), rec.y));
             longest = std::max(longest, b.longest);
             inner_mag.add(b.code.amps);
-            if (!join(b)) return false;
-            b = Built();
         }
     }
     // the kernels read one quad ahead
@@ -425,6 +453,12 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
         outer_most = std::max<size_t>(outer_most, blk[a].o1 - blk[a].o0);
         if (olist.size() > 0x7FFFFFFFull || slist.size() > 0x7FFFFFFFull) return false;
     }
+    {
+        size_t all = er.size();
+        for (const Table& t : tables) all += (size_t)tiles_of(t.c) * kTile;
+        er.reserve(std::min(all, 4 * kMaxTable));
+        ec.reserve(std::min(all, 4 * kMaxTable));
+    }
     // the tables, some at a time (what is built before it is joined stays below 8 M entries)
     for (size_t t0 = 0, t1; t0 < tables.size(); t0 = t1) {
         size_t rows = 0, work = 0;
@@ -459,13 +493,13 @@ bool PackTables::build(const Basis& B, SiteKind site, const std::vector<Term>& t
             });
             b.any = any;
         });
+        if (!join(built)) return false;
         for (size_t n = 0; n < built.size(); ++n) {
             if (!built[n].any) continue;
-            tables[t0 + n].id = (uint32_t)(er.size() / 4);
+            tables[t0 + n].id = (uint32_t)(built[n].at / 4);
             Mag m;
             m.add(built[n].code.amps);
             table_mag.push_back({tables[t0 + n].id, m});
-            if (!join(built[n])) return false;
         }
     }
     // the blocks' entries of tables that are there
